@@ -10,7 +10,7 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kStageThreads = 512;
 constexpr int kPlanThreads = 256;
 constexpr int kReduceThreads = 512;
-constexpr int kZeroBytes = 2048;  // zero source of the padding rows
+constexpr int kZeroBytes = 2048;  // smallest zero source of the padding rows
 constexpr int kTagStage = 1, kTagPlan = 2, kTagPull = 3, kTagPush = 4, kTagReduce = 5, kTagBarrier = 6;
 
 __device__ __forceinline__ char* window(const CommonParams& c, int r) { return static_cast<char*>(c.peers[r]); }
@@ -577,49 +577,56 @@ __device__ void pull_body(const PullParams& p) {
     for (int i = 0; i < min(S - 1, n_my); ++i) issue(i);
 
     // Gaps between an expert's last real row and the next expert's first slot: zero rows are bulk
-    // stores from a small zero buffer behind the rings (few instructions, no LSU store traffic).
+    // stores from a zero buffer behind the rings (few instructions, no LSU store traffic).
     char* zero_buf = s_ring + (align_up(rb, 128) + 8) * int64_t(wpb) * S;
     zero_buf = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(zero_buf) + 127) & ~uintptr_t(127));
     if (p.expand && p.zero_padding) {
-        for (int i = threadIdx.x; i < kZeroBytes / 16; i += blockDim.x) reinterpret_cast<int4*>(zero_buf)[i] = make_int4(0, 0, 0, 0);
+        for (int i = threadIdx.x; i < p.zero_bytes / 16; i += blockDim.x) reinterpret_cast<int4*>(zero_buf)[i] = make_int4(0, 0, 0, 0);
         fence_proxy_async_smem();
         __syncthreads();
     }
-    if (p.expand) {
-        // Gap geometry is read 32 experts at a time (one coalesced load per lane) and handed round by
-        // shuffles: a scalar walk over the experts would cost one global-load latency per expert and warp.
-        int base = 0;
-        for (int l0 = 0; l0 < Le; l0 += 32) {
-          const int my_l = l0 + lane;
-          const int my_gs = my_l < Le ? int(p.expert_offsets[my_l] + p.expert_counts[my_l]) : 0;
-          const int my_len = my_l < Le ? int(p.expert_offsets[my_l + 1]) - my_gs : 0;
-          const int in_wave = min(32, Le - l0);
-          for (int li = 0; li < in_wave; ++li) {
-            const int gs = __shfl_sync(kFull, my_gs, li);
-            const int len = __shfl_sync(kFull, my_len, li);
-            int first = (gw - base) % GW;
-            if (first < 0) first += GW;
-            for (int j = first; j < len; j += GW) {
-                const int64_t row = gs + j;
-                if (p.zero_padding) {
-                    if (lane == 0) {
-                        char* dst = reinterpret_cast<char*>(p.x_out + row * H);
-                        for (int at = 0; at < H * 2; at += kZeroBytes) bulk_store(dst + at, zero_buf, uint32_t(min(kZeroBytes, H * 2 - at)));
-                        bulk_commit();
-                        if (p.w_out != nullptr) p.w_out[row] = 0.f;
-                    }
-                    if (p.tile_ready != nullptr) bulk_wait<0>();
-                }
-                if (lane == 0 && p.slot_map != nullptr) p.slot_map[row] = -1;
-                if (p.tile_ready != nullptr) {
-                    fence_proxy_async();
-                    __threadfence();
-                    __syncwarp();
-                    if (lane == 0) red_release_gpu_add(p.tile_ready + int(row / 128), 1);
-                }
+    if (p.expand && (p.zero_padding || p.slot_map != nullptr)) {
+        // Gap rows are dealt out over the warps without a walk over the experts: a lane reads the geometry of
+        // kGapWaves experts at once, a warp scan of the gap lengths numbers the gap rows of 32 experts, and a ballot
+        // finds the expert that owns a number.  (A scalar walk over 256 experts took 45 us of every warp's time, which
+        // was all of a one-token dispatch and ran ahead of the rows in a large one.)
+        constexpr int kGapWaves = 8;
+        int base = 0;  // gap rows of the experts before this wave, modulo the number of warps
+        for (int l0 = 0; l0 < Le; l0 += 32 * kGapWaves) {
+            int start[kGapWaves], len[kGapWaves];
+#pragma unroll
+            for (int u = 0; u < kGapWaves; ++u) {
+                const int l = l0 + 32 * u + lane;
+                start[u] = l < Le ? int(p.expert_offsets[l] + p.expert_counts[l]) : 0;
+                len[u] = l < Le ? int(p.expert_offsets[l + 1]) - start[u] : 0;
             }
-            base = (base + len) % GW;
-          }
+#pragma unroll
+            for (int u = 0; u < kGapWaves; ++u) {
+                if (!__any_sync(kFull, len[u] > 0)) continue;
+                const int incl = warp_inclusive_sum(len[u]);
+                const int total = __shfl_sync(kFull, incl, 31);
+                for (int j = gw >= base ? gw - base : gw - base + GW; j < total; j += GW) {
+                    const int owner = __ffs(__ballot_sync(kFull, incl > j)) - 1;
+                    const int64_t row = __shfl_sync(kFull, start[u] + len[u] - incl, owner) + j;
+                    if (p.zero_padding) {
+                        if (lane == 0) {
+                            char* dst = reinterpret_cast<char*>(p.x_out + row * H);
+                            for (int at = 0; at < H * 2; at += p.zero_bytes) bulk_store(dst + at, zero_buf, uint32_t(min(p.zero_bytes, H * 2 - at)));
+                            bulk_commit();
+                            if (p.w_out != nullptr) p.w_out[row] = 0.f;
+                        }
+                        if (p.tile_ready != nullptr) bulk_wait<0>();
+                    }
+                    if (lane == 0 && p.slot_map != nullptr) p.slot_map[row] = -1;
+                    if (p.tile_ready != nullptr) {
+                        fence_proxy_async();
+                        __threadfence();
+                        __syncwarp();
+                        if (lane == 0) red_release_gpu_add(p.tile_ready + int(row / 128), 1);
+                    }
+                }
+                base = (base + total) % GW;
+            }
         }
     }
 
@@ -1641,7 +1648,11 @@ RingPlan plan_ring(int64_t row_bytes, int max_smem_bytes) {
     }
     if (warps < 1) warps = 0;
     r.warps = warps > 8 ? 8 : warps;
-    r.smem_bytes = size_t(r.warps) * r.stages * (pitch + 8) + kZeroBytes + 256;
+    // What the rings leave goes to the zero source of the padding rows, up to a whole row: stores of 2 KB reach
+    // 4.8 TB/s, of 3.5 KB and more 5.9 TB/s (rows in random order).
+    const int64_t used = int64_t(r.warps) * r.stages * (pitch + 8);
+    r.zero_bytes = int(std::max<int64_t>(kZeroBytes, std::min(pitch, (int64_t(max_smem_bytes) - 512 - used) / 128 * 128)));
+    r.smem_bytes = size_t(used) + r.zero_bytes + 256;
     return r;
 }
 

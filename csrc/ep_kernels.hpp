@@ -70,6 +70,7 @@ struct PullParams {
     int zero_padding;
     int write_meta;
     int stages;
+    int zero_bytes;  // zero source in shared memory behind the rings (see RingPlan)
     __nv_bfloat16* x_out;
     int64_t* topk_out;   // compact [N,K]
     float* w_out;        // compact [N,K] / expanded [C], or null
@@ -194,6 +195,7 @@ cudaError_t launch_local_combine(const LocalCombineParams* params, LaunchShape s
 // Shared-memory plan of the pull/push rings: `warps` independent rings of `stages` row buffers.
 struct RingPlan {
     int warps, stages;
+    int zero_bytes;  // pull only: size of the zero source behind the rings
     size_t smem_bytes;
 };
 RingPlan plan_ring(int64_t row_bytes, int max_smem_bytes);

@@ -447,6 +447,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             p.zero_padding = zero_padding;
             p.write_meta = fresh;
             p.stages = ring.stages;
+            p.zero_bytes = ring.zero_bytes;
             p.x_out = reinterpret_cast<__nv_bfloat16*>(o[0].data_ptr());
             p.topk_out = expand ? nullptr : o[1].data_ptr<int64_t>();
             p.w_out = weighted ? o[2].data_ptr<float>() : nullptr;
