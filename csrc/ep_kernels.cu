@@ -1,6 +1,11 @@
 // Dispatch / combine kernels for sm_100a: stage, plan, pull, push, reduce, barrier.
 // See ep_kernels.hpp for the protocol.  All waits are bounded (prim.cuh); nothing traps.
 #include "ep_kernels.hpp"
+
+#include <map>
+#include <mutex>
+#include <utility>
+
 #include "prim.cuh"
 
 namespace nep {
@@ -9,7 +14,7 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kStageThreads = 512;
 constexpr int kPlanThreads = 256;
-constexpr int kReduceThreads = 512;
+constexpr int kRowSumThreads = 256, kRowSumBlocks = 2, kRowCopyBlocks = 5;  // blocks: resident per SM
 constexpr int kZeroBytes = 2048;  // smallest zero source of the padding rows
 constexpr int kTagStage = 1, kTagPlan = 2, kTagPull = 3, kTagPush = 4, kTagReduce = 5, kTagBarrier = 6;
 
@@ -1415,111 +1420,186 @@ __device__ void combine_body(const CombineParams& p) {
 }
 
 // ------------------------------------------------------------------------------------------
-// reduce alone: source-side sum of rows that another kernel pushed and a peer barrier made visible.
+// Sums of whole rows that are already in local memory: the reduction of a combine whose rows another kernel pushed
+// (`reduce`), and the combine of a single-rank group (`local_combine`).  Bound by reading up to K rows per token once.
+// // One work item is kItemVecs 16-byte columns of one token, so that a lane has all of its loads (eight rows x two
+// columns) in flight at once and a few tokens still occupy many warps; with a warp per token, one token took 14
+// dependent rounds of loads and 3001 tokens left a third of the warps without work.
+// Hidden 7168, top-8, local_combine with a cold L2, before and now: 1 token 32 -> 3.6 us, 128 tokens 38 -> 6.9 us; warm: 3001
+// tokens 84 -> 59 us, 4096 tokens (529 MB) 91 -> 80 us = 6.6 TB/s; reduce at 64 tokens 35 -> 4.7 us.  Two blocks of 256
+// threads per SM keep all loads of a lane in registers (126); three blocks (80 registers) took 217 us, a grid without the
+// loop 120 us.  Compact, 8192 x 4096: 40 -> 17 us.
 // ------------------------------------------------------------------------------------------
-__device__ void reduce_body(const ReduceParams& p) {
-    const WindowLayout& L = p.c.layout;
-    const int K = L.topk, Le = L.local_experts, E = int(L.num_experts);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const int gw = blockIdx.x * wpb + warp, GW = gridDim.x * wpb;
-    const float* ret_w = reinterpret_cast<const float*>(window(p.c, p.c.rank) + L.ret_w_offset);
-    for (int t = gw; t < p.tokens; t += GW) {
-        bool valid;
-        int dest;
-        const unsigned parts = expected_parts(p.topk, t, K, E, Le, p.sum_all_choices != 0, valid, dest);
-        reduce_columns(p.c, t, parts, L.rank_indexed ? dest : lane, p.bias, p.out, 0, 32, l2_evict_first_policy());
-        if (p.w_out != nullptr && lane < K) p.w_out[int64_t(t) * K + lane] = valid ? __ldcg(ret_w + int64_t(t) * K + lane) : 0.f;
+constexpr int kItemVecs = 64, kCopyItemVecs = 128;
+
+// FP32 sum of the rows named by the lanes in `mask`, in ascending lane order: lane k holds the row's index in `base`.
+// `a0`/`a1` take the columns col and col + 32 (16-byte units) where `one`/`two` say that they exist.
+__device__ __forceinline__ void sum_rows(const char* base, int64_t row_bytes, unsigned mask, int my_row, int col, bool one, bool two, float* a0,
+                                         float* a1, uint64_t once) {
+    while (mask) {
+        int row[8];
+        int4 d0[8], d1[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = mask ? __ffs(mask) - 1 : -1;
+            if (mask) mask &= mask - 1;
+            row[j] = __shfl_sync(kFull, my_row, k < 0 ? 0 : k);
+            if (k < 0) row[j] = -1;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (row[j] >= 0) {
+                const int4* src = reinterpret_cast<const int4*>(base + row[j] * row_bytes);
+                if (one) d0[j] = ld_cg_v4_hint(src + col, once);
+                if (two) d1[j] = ld_cg_v4_hint(src + col + 32, once);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (row[j] >= 0) {
+                if (one) accumulate8(a0, d0[j]);
+                if (two) accumulate8(a1, d1[j]);
+            }
+        }
     }
 }
 
-// ------------------------------------------------------------------------------------------
-// local combine (single-rank group): sum a row's expert outputs into its source token.
-// ------------------------------------------------------------------------------------------
+// Bias once, one bf16 round, store.
+__device__ __forceinline__ void finish_columns(float* a0, float* a1, int col, bool one, bool two, const __nv_bfloat16* bias_row,
+                                               __nv_bfloat16* out_row, uint64_t once) {
+    if (bias_row != nullptr) {
+        const int4* b = reinterpret_cast<const int4*>(bias_row);
+        if (one) accumulate8(a0, ld_nc_v4(b + col));
+        if (two) accumulate8(a1, ld_nc_v4(b + col + 32));
+    }
+    int4* o = reinterpret_cast<int4*>(out_row);
+    if (one) st_v4_hint(o + col, pack8(a0), once);
+    if (two) st_v4_hint(o + col + 32, pack8(a1), once);
+}
+
+__device__ void reduce_body(const ReduceParams& p) {
+    const WindowLayout& L = p.c.layout;
+    const int K = L.topk, Le = L.local_experts, E = int(L.num_experts), H = L.hidden;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const int gw = blockIdx.x * wpb + warp, GW = gridDim.x * wpb;
+    const int vecs = H / 8, per_token = (vecs + kItemVecs - 1) / kItemVecs;
+    const char* ret = window(p.c, p.c.rank) + L.ret_offset;
+    const float* ret_w = reinterpret_cast<const float*>(window(p.c, p.c.rank) + L.ret_w_offset);
+    const uint64_t once = l2_evict_first_policy();
+    const int64_t items = int64_t(p.tokens) * per_token;
+    for (int64_t item = gw; item < items; item += GW) {
+        const int t = int(item / per_token), c = int(item - int64_t(t) * per_token);
+        bool valid;
+        int dest;
+        const unsigned parts = expected_parts(p.topk, t, K, E, Le, p.sum_all_choices != 0, valid, dest);
+        const int part = L.rank_indexed ? dest : lane;
+        const int col = c * kItemVecs + lane;
+        const bool one = col < vecs, two = col + 32 < vecs;
+        float a0[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        float a1[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        sum_rows(ret, int64_t(H) * 2, parts, part * int(L.max_tokens) + t, col, one, two, a0, a1, once);
+        finish_columns(a0, a1, col, one, two, p.bias != nullptr ? p.bias + int64_t(t) * H : nullptr, p.out + int64_t(t) * H, once);
+        if (c == 0 && p.w_out != nullptr && lane < K) p.w_out[int64_t(t) * K + lane] = valid ? __ldcg(ret_w + int64_t(t) * K + lane) : 0.f;
+    }
+}
+
+// Tokens without any valid choice have no receive row: result = bias (or zero), weights = 0.
+__device__ void finish_rowless_tokens(const LocalCombineParams& p, int first, int step) {
+    if (p.rows == p.tokens) return;
+    const WindowLayout& L = p.c.layout;
+    const int lane = threadIdx.x & 31, K = L.topk, H = L.hidden;
+    for (int t = first; t < p.tokens; t += step) {
+        const int64_t e = lane < K ? p.topk[int64_t(t) * K + lane] : -1;
+        if (__ballot_sync(kFull, e >= 0 && e < L.num_experts) != 0) continue;
+        int4* out = reinterpret_cast<int4*>(p.out + int64_t(t) * H);
+        const int4* bias = p.bias != nullptr ? reinterpret_cast<const int4*>(p.bias + int64_t(t) * H) : nullptr;
+        for (int c = lane; c < H / 8; c += 32) out[c] = bias != nullptr ? ld_nc_v4(bias + c) : make_int4(0, 0, 0, 0);
+        if (p.w_out != nullptr && lane < K) p.w_out[int64_t(t) * K + lane] = 0.f;
+    }
+}
+
+// Token and choices of receive row r on all lanes: lane k holds choice k.  False: nothing to add up (or bad metadata).
+__device__ __forceinline__ bool local_row(const LocalCombineParams& p, int r, int& tok, int& v, unsigned& vm) {
+    const int lane = threadIdx.x & 31, K = p.c.layout.topk;
+    const int* m = p.meta + int64_t(r) * (K + 2);
+    const int src = m[0];
+    tok = m[1];
+    v = lane < K ? m[2 + lane] : -1;
+    if (src != p.c.rank || tok < 0 || tok >= p.tokens) {
+        if (lane == 0) report(status_of(p.c), kBadMetadata, uint32_t(r), kTagReduce);
+        return false;
+    }
+    vm = __ballot_sync(kFull, v >= 0 && (!p.expand || v < p.capacity));
+    return vm != 0;
+}
+
 __device__ void local_combine_body(const LocalCombineParams& p) {
     const WindowLayout& L = p.c.layout;
     const int K = L.topk, H = L.hidden;
-    const int E = int(L.num_experts);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     const int gw = blockIdx.x * wpb + warp, GW = gridDim.x * wpb;
-    const int MW = K + 2, vecs = H / 8;
-    const StatusRef status = status_of(p.c);
-    for (int r = gw; r < p.rows; r += GW) {
-        const int* m = p.meta + int64_t(r) * MW;
-        const int tok = m[1];
-        if (m[0] != p.c.rank || tok < 0 || tok >= p.tokens) {
-            if (lane == 0) report(status, kBadMetadata, uint32_t(r), kTagReduce);
-            continue;
+    const int vecs = H / 8, per_row = (vecs + kItemVecs - 1) / kItemVecs;
+    const uint64_t once = l2_evict_first_policy();
+    const int64_t items = int64_t(p.rows) * per_row;
+    for (int64_t item = gw; item < items; item += GW) {
+        const int r = int(item / per_row), c = int(item - int64_t(r) * per_row);
+        int tok, v;
+        unsigned vm;
+        if (!local_row(p, r, tok, v, vm)) continue;
+        const int col = c * kItemVecs + lane;
+        const bool one = col < vecs, two = col + 32 < vecs;
+        float a0[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        float a1[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        sum_rows(reinterpret_cast<const char*>(p.y), int64_t(H) * 2, vm, v, col, one, two, a0, a1, once);
+        if (p.round_partial) {
+            const int4 r0 = pack8(a0), r1 = pack8(a1);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a0[j] = a1[j] = 0.f;
+            accumulate8(a0, r0);
+            accumulate8(a1, r1);
         }
-        const int v = lane < K ? m[2 + lane] : -1;
-        const unsigned vm = __ballot_sync(kFull, p.expand ? (v >= 0 && v < p.capacity) : v >= 0);
-        if (vm == 0) continue;
+        finish_columns(a0, a1, col, one, two, p.bias != nullptr ? p.bias + int64_t(tok) * H : nullptr, p.out + int64_t(tok) * H, once);
+        if (c == 0 && p.w_out != nullptr && lane < K) p.w_out[int64_t(tok) * K + lane] = ((vm >> lane) & 1u) ? p.w[v] : 0.f;
+    }
+    finish_rowless_tokens(p, gw, GW);
+}
+
+// The compact layout: a row is its token's sum already.  A streaming copy (plus bias); few registers, so that many warps
+// are resident, each with kCopyItemVecs / 32 loads per lane in flight.
+__device__ void local_combine_compact_body(const LocalCombineParams& p) {
+    const WindowLayout& L = p.c.layout;
+    const int K = L.topk, H = L.hidden;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const int gw = blockIdx.x * wpb + warp, GW = gridDim.x * wpb;
+    constexpr int kCols = kCopyItemVecs / 32;
+    const int vecs = H / 8, per_row = (vecs + kCopyItemVecs - 1) / kCopyItemVecs;
+    const uint64_t once = l2_evict_first_policy();
+    const int64_t items = int64_t(p.rows) * per_row;
+    for (int64_t item = gw; item < items; item += GW) {
+        const int r = int(item / per_row), c = int(item - int64_t(r) * per_row);
+        const int col = c * kCopyItemVecs + lane;
+        const int4* from = reinterpret_cast<const int4*>(p.y + int64_t(r) * H);
+        int4 d[kCols];
+#pragma unroll
+        for (int j = 0; j < kCols; ++j)
+            if (col + 32 * j < vecs) d[j] = ld_cg_v4_hint(from + col + 32 * j, once);
+        int tok, v;
+        unsigned vm;
+        if (!local_row(p, r, tok, v, vm)) continue;
+        int4* to = reinterpret_cast<int4*>(p.out + int64_t(tok) * H);
         const int4* bias = p.bias != nullptr ? reinterpret_cast<const int4*>(p.bias + int64_t(tok) * H) : nullptr;
-        int4* out = reinterpret_cast<int4*>(p.out + int64_t(tok) * H);
-        for (int c = lane; c < vecs; c += 64) {
-            const bool two = c + 32 < vecs;
-            float a0[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            float a1[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (p.expand) {
-                unsigned left = vm;
-                while (left) {
-                    int k[4];
-                    int4 d0[4], d1[4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        k[j] = left ? __ffs(left) - 1 : -1;
-                        if (left) left &= left - 1;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int slot = __shfl_sync(kFull, v, k[j] < 0 ? 0 : k[j]);
-                        if (k[j] >= 0) {
-                            const int4* src = reinterpret_cast<const int4*>(p.y + int64_t(slot) * H);
-                            d0[j] = ld_nc_v4(src + c);
-                            if (two) d1[j] = ld_nc_v4(src + c + 32);
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        if (k[j] >= 0) {
-                            accumulate8(a0, d0[j]);
-                            if (two) accumulate8(a1, d1[j]);
-                        }
-                    }
-                }
-                if (p.round_partial) {
-                    const int4 r0 = pack8(a0), r1 = pack8(a1);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) a0[j] = a1[j] = 0.f;
-                    accumulate8(a0, r0);
-                    accumulate8(a1, r1);
-                }
-            } else {
-                const int4* src = reinterpret_cast<const int4*>(p.y + int64_t(r) * H);
-                accumulate8(a0, ld_nc_v4(src + c));
-                if (two) accumulate8(a1, ld_nc_v4(src + c + 32));
+        for (int j = 0; j < kCols; ++j) {
+            if (col + 32 * j < vecs) {
+                float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                accumulate8(a, d[j]);
+                if (bias != nullptr) accumulate8(a, ld_nc_v4(bias + col + 32 * j));
+                st_v4_hint(to + col + 32 * j, pack8(a), once);
             }
-            if (bias != nullptr) {
-                accumulate8(a0, ld_nc_v4(bias + c));
-                if (two) accumulate8(a1, ld_nc_v4(bias + c + 32));
-            }
-            out[c] = pack8(a0);
-            if (two) out[c + 32] = pack8(a1);
         }
-        if (p.w_out != nullptr && lane < K) {
-            float wv = 0.f;
-            if ((vm >> lane) & 1u) wv = p.expand ? p.w[v] : p.w[int64_t(r) * K + lane];
-            p.w_out[int64_t(tok) * K + lane] = wv;
-        }
+        if (c == 0 && p.w_out != nullptr && lane < K) p.w_out[int64_t(tok) * K + lane] = ((vm >> lane) & 1u) ? p.w[int64_t(r) * K + lane] : 0.f;
     }
-    // tokens without any valid choice have no receive row: result = bias (or zero), weights = 0
-    for (int t = gw; t < p.tokens; t += GW) {
-        const int64_t e = lane < K ? p.topk[int64_t(t) * K + lane] : -1;
-        if (__ballot_sync(kFull, e >= 0 && e < E) != 0) continue;
-        int4* out = reinterpret_cast<int4*>(p.out + int64_t(t) * H);
-        const int4* bias = p.bias != nullptr ? reinterpret_cast<const int4*>(p.bias + int64_t(t) * H) : nullptr;
-        for (int c = lane; c < vecs; c += 32) out[c] = bias != nullptr ? ld_nc_v4(bias + c) : make_int4(0, 0, 0, 0);
-        if (p.w_out != nullptr && lane < K) p.w_out[int64_t(t) * K + lane] = 0.f;
-    }
+    finish_rowless_tokens(p, gw, GW);
 }
 
 __device__ void barrier_body(const BarrierParams& p) {
@@ -1547,9 +1627,9 @@ __global__ void gate_kernel(volatile int* gate, uint64_t timeout_ns) {
 }
 
 // ---------------------------------------------------------------- wrappers
-#define NEP_KERNEL_PAIR(name, Params, threads)                                                                  \
-    __global__ void __launch_bounds__(threads) name##_kernel(const __grid_constant__ Params p) { name##_body(p); } \
-    __global__ void __launch_bounds__(threads) name##_multi_kernel(const Params* all) { name##_body(all[blockIdx.y]); }
+#define NEP_KERNEL_PAIR(name, Params, ...)                                                                          \
+    __global__ void __launch_bounds__(__VA_ARGS__) name##_kernel(const __grid_constant__ Params p) { name##_body(p); } \
+    __global__ void __launch_bounds__(__VA_ARGS__) name##_multi_kernel(const Params* all) { name##_body(all[blockIdx.y]); }
 
 __global__ void __launch_bounds__(kStageThreads) stage_kernel(const __grid_constant__ StageParams p) { stage_body(p); }
 __global__ void __launch_bounds__(kStageThreads) stage_multi_kernel(const StageParams* all) { stage_body(all[blockIdx.y]); }
@@ -1557,9 +1637,10 @@ NEP_KERNEL_PAIR(plan, PlanParams, kPlanThreads)
 NEP_KERNEL_PAIR(pull, PullParams, 256)
 __global__ void __launch_bounds__(kCombineThreads, 1) combine_kernel(const __grid_constant__ CombineParams p) { combine_body(p); }
 __global__ void __launch_bounds__(kCombineThreads, 1) combine_multi_kernel(const CombineParams* all) { combine_body(all[blockIdx.y]); }
-NEP_KERNEL_PAIR(reduce, ReduceParams, kReduceThreads)
+NEP_KERNEL_PAIR(reduce, ReduceParams, kRowSumThreads, kRowSumBlocks)
 NEP_KERNEL_PAIR(barrier, BarrierParams, 32)
-NEP_KERNEL_PAIR(local_combine, LocalCombineParams, kReduceThreads)
+NEP_KERNEL_PAIR(local_combine, LocalCombineParams, kRowSumThreads, kRowSumBlocks)
+NEP_KERNEL_PAIR(local_combine_compact, LocalCombineParams, kRowSumThreads, kRowCopyBlocks)
 
 // Fresh dispatch of a small call in ONE cooperative launch: stage (count exchange, peer barrier, prefixes, mailbox),
 // plan, pull.  Outputs are sized by the caller at an upper bound and trimmed on the host once N and C are known, so
@@ -1601,21 +1682,28 @@ __global__ void __launch_bounds__(256) fused_cached_dispatch_multi_kernel(const 
     pull_body(pp[blockIdx.y]);
 }
 
+// Raises a kernel's dynamic shared-memory limit when a launch needs more than it was granted so far.  The limit belongs
+// to the kernel on its device, not to a thread: the record is shared, and a smaller request never lowers it.
+cudaError_t allow_shared_memory(const void* fn, size_t smem) {
+    static std::mutex mutex;
+    static std::map<std::pair<const void*, int>, size_t> granted;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    const std::lock_guard<std::mutex> lock(mutex);
+    size_t& have = granted[{fn, device}];
+    if (smem <= have) return cudaSuccess;
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e == cudaSuccess) have = smem;
+    return e;
+}
+
 template <typename Params>
 cudaError_t launch_pair(void (*single)(const Params), void (*multi)(const Params*), const Params* params, LaunchShape shape, int threads,
                         size_t smem, cudaStream_t stream) {
     if (smem > 48 * 1024) {
-        // Raise the kernel's dynamic shared-memory limit once per (kernel, device) and only when it grows.
-        static thread_local size_t granted[2][64] = {};
-        int device = 0;
-        cudaGetDevice(&device);
-        size_t& have = granted[shape.ranks_y > 1 ? 1 : 0][device & 63];
-        if (smem > have) {
-            cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(shape.ranks_y > 1 ? (const void*)multi : (const void*)single),
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (e != cudaSuccess) return e;
-            have = smem;
-        }
+        const cudaError_t e = allow_shared_memory(shape.ranks_y > 1 ? (const void*)multi : (const void*)single, smem);
+        if (e != cudaSuccess) return e;
     }
     const dim3 grid(shape.grid_x, shape.ranks_y > 1 ? shape.ranks_y : 1);
     if (shape.ranks_y > 1)
@@ -1627,6 +1715,13 @@ cudaError_t launch_pair(void (*single)(const Params), void (*multi)(const Params
 
 }  // namespace
 
+int row_sum_grid(int64_t tokens, int hidden, bool sums, int sms) {
+    // one work item per warp until every SM is full; from there on the blocks loop (a larger grid measured slower)
+    const int64_t item_vecs = sums ? kItemVecs : kCopyItemVecs;
+    const int64_t items = tokens * ((hidden / 8 + item_vecs - 1) / item_vecs);
+    const int64_t blocks = (items + kRowSumThreads / 32 - 1) / (kRowSumThreads / 32);
+    return int(std::max<int64_t>(1, std::min<int64_t>(blocks, int64_t(sums ? kRowSumBlocks : kRowCopyBlocks) * sms)));
+}
 int stage_smem_bytes(const WindowLayout& l) { return int((l.ranks + l.num_experts) * 4); }
 int plan_smem_bytes(const WindowLayout& l) { return (kPlanThreads / 32) * 32 * l.topk * 4; }
 
@@ -1706,7 +1801,7 @@ cudaError_t launch_pull(const PullParams* params, LaunchShape shape, int warps, 
     return launch_pair<PullParams>(pull_kernel, pull_multi_kernel, params, shape, warps * 32, smem, stream);
 }
 cudaError_t launch_reduce(const ReduceParams* params, LaunchShape shape, cudaStream_t stream) {
-    return launch_pair<ReduceParams>(reduce_kernel, reduce_multi_kernel, params, shape, kReduceThreads, 0, stream);
+    return launch_pair<ReduceParams>(reduce_kernel, reduce_multi_kernel, params, shape, kRowSumThreads, 0, stream);
 }
 cudaError_t launch_barrier(const BarrierParams* params, LaunchShape shape, cudaStream_t stream) {
     return launch_pair<BarrierParams>(barrier_kernel, barrier_multi_kernel, params, shape, 32, 0, stream);
@@ -1715,19 +1810,12 @@ cudaError_t launch_barrier(const BarrierParams* params, LaunchShape shape, cudaS
 namespace {
 // Cooperative launch of a two-parameter-block kernel: fails instead of deadlocking if the grid cannot be resident at once.
 cudaError_t launch_cooperative(const void* single, const void* multi_fn, const void* first, const void* second, LaunchShape shape, int warps,
-                               size_t smem, cudaStream_t stream, size_t (*granted)[64]) {
+                               size_t smem, cudaStream_t stream) {
     const bool multi = shape.ranks_y > 1;
     const void* fn = multi ? multi_fn : single;
     if (smem > 48 * 1024) {
-        // as in launch_pair: raise the limit once per (kernel, device), and only when it grows
-        int device = 0;
-        cudaGetDevice(&device);
-        size_t& have = granted[multi ? 1 : 0][device & 63];
-        if (smem > have) {
-            cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (e != cudaSuccess) return e;
-            have = smem;
-        }
+        const cudaError_t e = allow_shared_memory(fn, smem);
+        if (e != cudaSuccess) return e;
     }
     const dim3 grid(shape.grid_x, multi ? shape.ranks_y : 1);
     // multi: the kernel takes the two device arrays; single: the two blocks by value
@@ -1739,25 +1827,17 @@ cudaError_t launch_cooperative(const void* single, const void* multi_fn, const v
 
 cudaError_t launch_fused_cached_dispatch(const StageParams* stage, const PullParams* pull, LaunchShape shape, int warps, size_t smem,
                                          cudaStream_t stream) {
-    static thread_local size_t granted[2][64] = {};
     return launch_cooperative((const void*)fused_cached_dispatch_kernel, (const void*)fused_cached_dispatch_multi_kernel, stage, pull, shape,
-                              warps, smem, stream, granted);
+                              warps, smem, stream);
 }
 
 cudaError_t launch_fused_fresh_dispatch(const StageParams* stage, const PlanParams* plan, const PullParams* pull, LaunchShape shape, int warps,
                                         size_t smem, cudaStream_t stream) {
     const bool multi = shape.ranks_y > 1;
     const void* fn = multi ? (const void*)fused_fresh_dispatch_multi_kernel : (const void*)fused_fresh_dispatch_kernel;
-    static thread_local size_t granted[2][64] = {};
     if (smem > 48 * 1024) {
-        int device = 0;
-        cudaGetDevice(&device);
-        size_t& have = granted[multi ? 1 : 0][device & 63];
-        if (smem > have) {
-            cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (e != cudaSuccess) return e;
-            have = smem;
-        }
+        const cudaError_t e = allow_shared_memory(fn, smem);
+        if (e != cudaSuccess) return e;
     }
     const dim3 grid(shape.grid_x, multi ? shape.ranks_y : 1);
     void* args_multi[3] = {(void*)&stage, (void*)&plan, (void*)&pull};
@@ -1769,16 +1849,9 @@ cudaError_t launch_combine(const CombineParams* params, LaunchShape shape, size_
     if (!cooperative) return launch_pair<CombineParams>(combine_kernel, combine_multi_kernel, params, shape, kCombineThreads, smem, stream);
     const bool multi = shape.ranks_y > 1;
     const void* fn = multi ? (const void*)combine_multi_kernel : (const void*)combine_kernel;
-    static thread_local size_t granted[2][64] = {};
     if (smem > 48 * 1024) {
-        int device = 0;
-        cudaGetDevice(&device);
-        size_t& have = granted[multi ? 1 : 0][device & 63];
-        if (smem > have) {
-            cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (e != cudaSuccess) return e;
-            have = smem;
-        }
+        const cudaError_t e = allow_shared_memory(fn, smem);
+        if (e != cudaSuccess) return e;
     }
     const dim3 grid(shape.grid_x, multi ? shape.ranks_y : 1);
     void* args[1] = {multi ? (void*)&params : (void*)params};
@@ -1790,8 +1863,10 @@ cudaError_t launch_gate(int* gate, uint64_t timeout_ns, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_local_combine(const LocalCombineParams* params, LaunchShape shape, cudaStream_t stream) {
-    return launch_pair<LocalCombineParams>(local_combine_kernel, local_combine_multi_kernel, params, shape, kReduceThreads, 0, stream);
+cudaError_t launch_local_combine(const LocalCombineParams* params, LaunchShape shape, bool compact, cudaStream_t stream) {
+    if (compact)
+        return launch_pair<LocalCombineParams>(local_combine_compact_kernel, local_combine_compact_multi_kernel, params, shape, kRowSumThreads, 0, stream);
+    return launch_pair<LocalCombineParams>(local_combine_kernel, local_combine_multi_kernel, params, shape, kRowSumThreads, 0, stream);
 }
 
 int kernel_table(KernelInfo* out, int capacity) {
@@ -1804,6 +1879,7 @@ int kernel_table(KernelInfo* out, int capacity) {
         {"combine", (const void*)combine_kernel}, {"reduce", (const void*)reduce_kernel}, {"barrier", (const void*)barrier_kernel},
         {"local_combine", (const void*)local_combine_kernel}, {"fused_cached_dispatch", (const void*)fused_cached_dispatch_kernel},
         {"fused_fresh_dispatch", (const void*)fused_fresh_dispatch_kernel},
+        {"local_combine_compact", (const void*)local_combine_compact_kernel},
     };
     int n = 0;
     for (const Entry& e : entries) {

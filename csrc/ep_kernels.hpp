@@ -190,7 +190,7 @@ cudaError_t launch_fused_cached_dispatch(const StageParams* stage, const PullPar
                                          cudaStream_t stream);
 // Test utility: one thread that waits (bounded) until gate[0] != 0; gate is pinned host memory that the host writes.
 cudaError_t launch_gate(int* gate, uint64_t timeout_ns, cudaStream_t stream);
-cudaError_t launch_local_combine(const LocalCombineParams* params, LaunchShape shape, cudaStream_t stream);
+cudaError_t launch_local_combine(const LocalCombineParams* params, LaunchShape shape, bool compact, cudaStream_t stream);
 
 // Shared-memory plan of the pull/push rings: `warps` independent rings of `stages` row buffers.
 struct RingPlan {
@@ -207,6 +207,8 @@ struct CombinePlan {
 };
 CombinePlan plan_combine(int64_t row_bytes, int parts, int max_smem_bytes, int reduce_stages, int reduce_chunk_bytes);
 constexpr int kCombineThreads = 512;  // transfer warps + reduce warps of one combine CTA
+// Grid of the kernels that sum (or, with one row per token, copy) whole rows: reduce, local_combine.
+int row_sum_grid(int64_t tokens, int hidden, bool sums, int sms);
 int stage_smem_bytes(const WindowLayout& l);
 int plan_smem_bytes(const WindowLayout& l);
 

@@ -627,7 +627,8 @@ CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::T
             c10::cuda::CUDAStreamGuard on_comm(s.work);
             g_marks.mark("begin", cs);
             PeerWindow::launches += 1;
-            cuda_check(launch_local_combine(&p, LaunchShape{2 * lim.sms, 1}, cs), "local combine launch");
+            cuda_check(launch_local_combine(&p, LaunchShape{row_sum_grid(p.tokens, L.hidden, expand, lim.sms), 1}, !expand, cs),
+                       "local combine launch");
             g_marks.mark("local_combine", cs);
         }
         std::vector<at::Tensor> inputs{xs[0]}, results;
@@ -761,9 +762,11 @@ std::vector<at::Tensor> combine_finish(const std::vector<PeerWindow*>& wins, con
     const BarrierParams* bdev = upload(barrier, keep, cs);
     PeerWindow::launches += 1;
     cuda_check(launch_barrier(bdev, LaunchShape{1, n}, cs), "barrier launch");
+    int64_t max_tokens_now = 1;
+    for (int i = 0; i < n; ++i) max_tokens_now = std::max<int64_t>(max_tokens_now, meta[i][5].size(0));
     const ReduceParams* rdev = upload(reduce, keep, cs);
     PeerWindow::launches += 1;
-    cuda_check(launch_reduce(rdev, LaunchShape{2 * lim.sms, n}, cs), "reduce launch");
+    cuda_check(launch_reduce(rdev, LaunchShape{row_sum_grid(max_tokens_now, L.hidden, true, lim.sms), n}, cs), "reduce launch");
     // Tell every peer that this rank has finished reading its return area (nobody waits): the next combine kernel
     // waits for this epoch before it overwrites the area, exactly as it does after a combine kernel.
     std::vector<BarrierParams> done(n);

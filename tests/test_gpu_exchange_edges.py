@@ -33,3 +33,49 @@ def test_padding_rows_of_many_experts(world, experts_per_rank, alignment):
             for r in range(world):
                 assert_dispatch_matches(got[r], case.xs, case.indices, case.weights, case.num_experts, r, expand=True, alignment=alignment,
                                         zero_padding=True)
+
+
+def _values(case, seed=3):
+    gen = torch.Generator().manual_seed(seed)
+    return [torch.randn(idx.shape[0], case.num_topk, case.hidden, generator=gen).to(torch.bfloat16) for idx in case.indices]
+
+
+def _expert_rows(values, meta, capacity):
+    y = torch.full((capacity, values.shape[-1]), float("nan"), dtype=torch.bfloat16)  # padding must not be read
+    slots, tok = meta[:, 2:], meta[:, 1]
+    row, k = (slots >= 0).nonzero(as_tuple=True)
+    y[slots[row, k]] = values[tok[row], k]
+    return y
+
+
+@pytest.mark.parametrize("tokens,topk,hidden", [(1, 8, 256), (2, 1, 768), (5, 9, 7168), (37, 17, 1280), (700, 4, 512)])
+@pytest.mark.parametrize("multiple", [False, True])
+def test_single_rank_combine_shapes(tokens, topk, hidden, multiple):
+    """Row sums of a single-rank group: rows shorter and longer than a work item, one to three batches of eight rows per
+    token, masked choices, tokens without a row, both rounding modes, both layouts."""
+    case = make_case(1, kind="random", seed=tokens, hidden=hidden, tokens=tokens, experts_per_rank=max(4, topk), topk=topk)
+    if tokens > 2:
+        case.indices[0][tokens // 2] = -1
+    cfg = EPConfig(case.num_experts, case.num_topk, case.hidden, case.capacity)
+    values = _values(case)
+    bias = torch.randn(tokens, hidden).to(torch.bfloat16)
+    with EmulatedGroup(1, cfg, allow_multiple_reduction=multiple) as group:
+        for expand in (True, False):
+            got = group.dispatch(_cuda(case.xs), topk_idx=_cuda(case.indices), weights=_cuda(case.weights), do_expand=expand, alignment=4 if expand else 1)[0]
+            meta = got.handle.layout.recv_metadata.cpu().long()
+            y = _expert_rows(values[0], meta, got.handle.layout.expanded_capacity) if expand else values[0][meta[:, 1], 0]
+            back = group.combine([y.cuda()], [got.handle], weights=[got.topk_weights], bias=[bias.cuda()])[0]
+            torch.cuda.synchronize()
+            group.check_status()
+            valid = case.indices[0] >= 0
+            want = torch.zeros(tokens, hidden)
+            if expand:
+                for k in range(topk):  # FP32 in ascending choice
+                    want = torch.where(valid[:, k, None], want + values[0][:, k].float(), want)
+                if multiple:
+                    want = want.to(torch.bfloat16).float()
+            else:
+                want = torch.where(valid.any(1)[:, None], want + values[0][:, 0].float(), want)
+            want = (want + bias.float()).to(torch.bfloat16)
+            assert torch.equal(back.x.cpu().view(torch.int16), want.view(torch.int16)), expand
+            torch.testing.assert_close(back.topk_weights.cpu(), case.weights[0].masked_fill(~valid, 0), rtol=0, atol=0)
