@@ -61,6 +61,26 @@ struct PlanParams {
     int expand;
 };
 
+// The whole plan of a single-rank group's fresh dispatch (counts, offsets, receive rows, slots) in one launch.
+struct LocalPlanParams {
+    CommonParams c;
+    const int64_t* topk;  // [T,K]
+    int tokens;
+    int expand;
+    int alignment;
+    // handle tensors (as in StageParams); `meta` has room for T rows, `slot_map` for the largest possible capacity
+    int64_t* snapshot;
+    int64_t* dst_slots;
+    int64_t* send_counts;
+    int64_t* recv_rank_prefix;
+    int64_t* expert_counts;
+    int64_t* expert_offsets;
+    int* meta;
+    int* slot_map;  // expert-major layout only
+    volatile int64_t* mailbox;
+};
+constexpr int kLocalPlanMaxTokens = 32768, kLocalPlanMaxExperts = 2048;  // larger calls use the stage and plan kernels
+
 struct PullParams {
     CommonParams c;
     const int* meta;  // [N,K+2] plan scratch (fresh) or handle metadata (cached)
@@ -176,6 +196,8 @@ struct LaunchShape {
 // memory) or to a device array of ranks_y blocks.
 cudaError_t launch_stage(const StageParams* params, LaunchShape shape, size_t smem, cudaStream_t stream);
 cudaError_t launch_plan(const PlanParams* params, LaunchShape shape, size_t smem, cudaStream_t stream);
+bool local_plan_fits(const WindowLayout& l, int64_t tokens);
+cudaError_t launch_local_plan(const LocalPlanParams& params, cudaStream_t stream);
 cudaError_t launch_pull(const PullParams* params, LaunchShape shape, int warps, size_t smem, cudaStream_t stream);
 // Fresh dispatch for small calls: stage, plan and pull in ONE cooperative launch; outputs sized at an upper bound.
 cudaError_t launch_fused_fresh_dispatch(const StageParams* stage, const PlanParams* plan, const PullParams* pull, LaunchShape shape, int warps,

@@ -292,6 +292,13 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     const auto f32 = at::TensorOptions().dtype(at::kFloat).device(at::kCUDA, device);
     const auto bf16 = at::TensorOptions().dtype(at::kBFloat16).device(at::kCUDA, device);
 
+    int64_t max_tokens_now = 0;
+    for (int i = 0; i < n; ++i) max_tokens_now = std::max<int64_t>(max_tokens_now, xs[i].size(0));
+    // A single-rank group exchanges nothing: a fresh dispatch plans in one launch that writes the handle's tensors itself
+    // (allocated at their upper bounds and trimmed), a cached one goes straight to the pull.
+    const bool local = L.ranks == 1;
+    const bool plan_locally = local && fresh && local_plan_fits(L, max_tokens_now);
+
     DispatchOut out;
     out.metadata.resize(n);
     out.outputs.resize(n);
@@ -336,7 +343,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             p.fresh = fresh;
             p.parity = parity[i];
             p.alignment = int(alignment);
-            p.skip_copy = L.ranks == 1 ? 1 : 0;
+            p.skip_copy = local ? 1 : 0;
             p.epoch = wins[i]->reserve_epochs(1);
             if (fresh) {
                 p.snapshot = m[5].data_ptr<int64_t>();
@@ -347,7 +354,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
                 p.expert_offsets = m[2].data_ptr<int64_t>();
                 wins[i]->arm_mailbox();
                 p.mailbox = wins[i]->mailbox_device();
-                if (g_trace.enabled && n == 1) {
+                if (g_trace.enabled && n == 1 && !plan_locally) {
                     if (!g_trace.stage_words.defined())
                         g_trace.stage_words = at::empty({5}, at::TensorOptions().dtype(at::kLong).device(at::kCUDA, device));
                     p.trace = reinterpret_cast<unsigned long long*>(g_trace.stage_words.data_ptr<int64_t>());
@@ -355,19 +362,21 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             }
         }
     }
-    int64_t max_tokens_now = 0;
-    for (int i = 0; i < n; ++i) max_tokens_now = std::max<int64_t>(max_tokens_now, xs[i].size(0));
     // Small cached calls: stage, peer barrier and pull go out as ONE cooperative launch.
     bool gated = false;
     for (const auto& t : tile_ready) gated = gated || t.has_value();
-    const bool fuse_small = !fresh && !gated && max_tokens_now <= fused_dispatch_max_tokens();
+    const bool fuse_small = !fresh && !gated && !local && max_tokens_now <= fused_dispatch_max_tokens();
     // Small fresh calls: stage, plan and pull as ONE cooperative launch writing into outputs sized at an upper bound
     // (every rank may send all of its Tmax tokens here), trimmed to N / C once the mailbox has them.  Only when that
     // bound is modest, i.e. for buffers configured for small batches.
-    const int64_t bound_rows_n = int64_t(L.ranks) * L.max_tokens;
-    const int64_t bound_rows_c = bound_rows_n * std::min<int64_t>(L.topk, L.local_experts) + int64_t(L.local_experts) * (alignment - 1);
+    // A single-rank group knows its bound from this call's own tokens, and its pull needs nothing from the host: it is
+    // launched behind the plan without waiting for the counts, under the same limit on the bound.
+    const int64_t bound_rows_n = local ? max_tokens_now : int64_t(L.ranks) * L.max_tokens;
+    const int64_t bound_choices = bound_rows_n * std::min<int64_t>(L.topk, L.local_experts);
+    const int64_t bound_rows_c = bound_choices + std::min<int64_t>(L.local_experts, local ? bound_choices : L.local_experts) * (alignment - 1);
     const int64_t bound_bytes = (expand ? bound_rows_c : bound_rows_n) * L.hidden * 2;
-    const bool fuse_fresh = fresh && !gated && !g_gate.word.defined() && max_tokens_now <= fused_fresh_max_tokens() &&
+    const bool early_pull = plan_locally && !gated && !g_gate.word.defined() && bound_bytes <= kFusedFreshMaxOutputBytes;
+    const bool fuse_fresh = fresh && !gated && !local && !g_gate.word.defined() && max_tokens_now <= fused_fresh_max_tokens() &&
                             bound_bytes <= kFusedFreshMaxOutputBytes && (!expand || bound_rows_c <= L.slot_scratch_ints) &&
                             ring.warps >= 2 && ring.smem_bytes >= size_t(stage_smem_bytes(L)) &&
                             ring.smem_bytes >= size_t(ring.warps) * 32 * L.topk * 4;
@@ -378,19 +387,45 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         c10::cuda::CUDAStreamGuard on_comm(s.work);
         for (int i = 0; i < n; ++i) stage[i].fused = (fuse_small || fuse_fresh) ? 1 : 0;
         stage_dev = upload(stage, keep, cs);
-        if (fresh && g_trace.enabled && n == 1) {
+        if (fresh && g_trace.enabled && n == 1 && !plan_locally) {
             const int64_t init[5] = {INT64_MAX, 0, 0, 0, 0};
             cuda_check(cudaMemcpyAsync(g_trace.stage_words.data_ptr(), init, sizeof(init), cudaMemcpyHostToDevice, cs), "trace reset");
         }
         g_marks.mark("begin", cs);
-        if (!fuse_small && !fuse_fresh) {
+        if (plan_locally) {
+            auto& m = out.metadata[0];
+            const int64_t cells = bound_rows_n * (L.topk + 2), slots = expand ? bound_rows_c : 0;
+            c10::cuda::CUDAStreamGuard pool(consumer);
+            at::Tensor block = at::empty({cells + slots}, i32);
+            m[0] = block.narrow(0, 0, cells).view({bound_rows_n, L.topk + 2});
+            m[7] = block.narrow(0, cells, slots);
+            LocalPlanParams lp{};
+            const StageParams& sp = stage[0];
+            lp.c = sp.c;
+            lp.topk = sp.topk;
+            lp.tokens = sp.tokens;
+            lp.expand = expand;
+            lp.alignment = sp.alignment;
+            lp.snapshot = sp.snapshot;
+            lp.dst_slots = sp.dst_slots;
+            lp.send_counts = sp.send_counts;
+            lp.recv_rank_prefix = sp.recv_rank_prefix;
+            lp.expert_counts = sp.expert_counts;
+            lp.expert_offsets = sp.expert_offsets;
+            lp.meta = m[0].data_ptr<int>();
+            lp.slot_map = expand ? m[7].data_ptr<int>() : nullptr;
+            lp.mailbox = sp.mailbox;
+            PeerWindow::launches += 1;
+            cuda_check(launch_local_plan(lp, cs), "local plan launch");
+            g_marks.mark("plan", cs);
+        } else if (!fuse_small && !fuse_fresh && !(local && !fresh)) {
             PeerWindow::launches += 1;
             // 16 warps per block, 4 row quarters per token: small calls get small grids
             const int stage_grid = int(std::max<int64_t>(1, std::min<int64_t>(2 * num_sms, (max_tokens_now * 4 + 15) / 16)));
             cuda_check(launch_stage(stage_dev, LaunchShape{stage_grid, n}, size_t(stage_smem_bytes(L)), cs), "stage launch");
             g_marks.mark("stage", cs);
         }
-        if (fresh) {
+        if (fresh && !plan_locally) {
             for (int i = 0; i < n; ++i) {
                 plan[i].c = stage[i].c;
                 plan[i].parity = parity[i];
@@ -407,7 +442,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         }
     }
     for (int i = 0; i < n; ++i) {
-        if (fuse_fresh) {
+        if (fuse_fresh || early_pull) {
             out.counts[i] = {bound_rows_n, expand ? bound_rows_c : 0};  // allocation sizes; the real counts follow the launch
         } else if (fresh) {
             std::pair<int64_t, int64_t> nc;
@@ -426,7 +461,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         for (int i = 0; i < n; ++i) {
             const int64_t N = out.counts[i].first, C = out.counts[i].second;
             auto& m = out.metadata[i];
-            if (fresh) {
+            if (fresh && !plan_locally) {
                 const int64_t cells = N * (L.topk + 2), slots = expand ? C : 0;
                 at::Tensor block = at::empty({cells + slots}, i32);
                 m[0] = block.narrow(0, 0, cells).view({N, L.topk + 2});
@@ -439,20 +474,20 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             o[2] = !weighted ? at::empty({0}, f32) : expand ? at::empty({C}, f32) : at::empty({N, L.topk}, f32);
             PullParams& p = pull[i];
             p.c = stage[i].c;
-            p.meta = fresh ? reinterpret_cast<const int*>(static_cast<char*>(wins[i]->base()) + L.meta_scratch_offset) : m[0].data_ptr<int>();
+            p.meta = fresh && !plan_locally ? reinterpret_cast<const int*>(static_cast<char*>(wins[i]->base()) + L.meta_scratch_offset) : m[0].data_ptr<int>();
             p.rows = int(N);
             p.parity = parity[i];
-            p.data_epoch = (fresh && L.ranks > 1) ? stage[i].epoch : 0;  // a single-rank group pulls from the caller's tensor
+            p.data_epoch = (fresh && !local) ? stage[i].epoch : 0;  // a single-rank group pulls from the caller's tensor
             p.expand = expand;
             p.zero_padding = zero_padding;
-            p.write_meta = fresh;
+            p.write_meta = fresh && !plan_locally;
             p.stages = ring.stages;
             p.zero_bytes = ring.zero_bytes;
             p.x_out = reinterpret_cast<__nv_bfloat16*>(o[0].data_ptr());
             p.topk_out = expand ? nullptr : o[1].data_ptr<int64_t>();
             p.w_out = weighted ? o[2].data_ptr<float>() : nullptr;
-            p.meta_out = fresh ? m[0].data_ptr<int>() : nullptr;
-            p.slot_map = (expand && fresh) ? m[7].data_ptr<int>() : nullptr;
+            p.meta_out = p.write_meta ? m[0].data_ptr<int>() : nullptr;
+            p.slot_map = (expand && p.write_meta) ? m[7].data_ptr<int>() : nullptr;
             p.expert_counts = m[1].data_ptr<int64_t>();
             p.expert_offsets = m[2].data_ptr<int64_t>();
             p.recv_rank_prefix = m[6].data_ptr<int64_t>();
@@ -466,8 +501,8 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
                             "tile_ready must be a zeroed CUDA int32 tensor with one entry per 128 expert-major rows");
                 p.tile_ready = t.data_ptr<int>();
                 // Consumers gated by the counters want row blocks to complete front to back.
-                if (!fresh || C <= L.slot_scratch_ints) {
-                    p.slot_src = fresh ? reinterpret_cast<const int*>(static_cast<char*>(wins[i]->base()) + L.slot_scratch_offset)
+                if (!fresh || plan_locally || C <= L.slot_scratch_ints) {
+                    p.slot_src = fresh && !plan_locally ? reinterpret_cast<const int*>(static_cast<char*>(wins[i]->base()) + L.slot_scratch_offset)
                                        : m[7].data_ptr<int>();
                     p.capacity = int(C);
                 }
@@ -505,7 +540,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             g_marks.mark("pull", cs);
         }
     }
-    if (fuse_fresh) {
+    if (fuse_fresh || early_pull) {
         // The kernel is on its way; now wait for N and C and trim the outputs to their exact sizes (leading-dimension
         // views of the bound-sized allocations: contiguous, same storage).
         for (int i = 0; i < n; ++i) {
@@ -517,13 +552,17 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             const int64_t N = nc.first, C = nc.second;
             TORCH_CHECK(N <= bound_rows_n && (!expand || C <= bound_rows_c), "receive counts exceed the single-launch bound");
             out.counts[i] = {N, C};
-            auto& m = out.metadata[i];
             auto& o = out.outputs[i];
-            m[0] = m[0].narrow(0, 0, N);
-            if (expand) m[7] = m[7].narrow(0, 0, C);
             o[0] = o[0].narrow(0, 0, expand ? C : N);
             if (!expand) o[1] = o[1].narrow(0, 0, N);
             if (weighted) o[2] = o[2].narrow(0, 0, expand ? C : N);
+        }
+    }
+    if (fuse_fresh || plan_locally) {
+        for (int i = 0; i < n; ++i) {
+            auto& m = out.metadata[i];
+            m[0] = m[0].narrow(0, 0, out.counts[i].first);
+            if (expand) m[7] = m[7].narrow(0, 0, out.counts[i].second);
         }
     }
     std::vector<at::Tensor> inputs, results;

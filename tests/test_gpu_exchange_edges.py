@@ -79,3 +79,22 @@ def test_single_rank_combine_shapes(tokens, topk, hidden, multiple):
             want = (want + bias.float()).to(torch.bfloat16)
             assert torch.equal(back.x.cpu().view(torch.int16), want.view(torch.int16)), expand
             torch.testing.assert_close(back.topk_weights.cpu(), case.weights[0].masked_fill(~valid, 0), rtol=0, atol=0)
+
+
+@pytest.mark.parametrize("tokens,experts,topk,kind", [
+    (1, 1, 1, "random"), (31, 7, 3, "mixed"), (33, 40, 32, "random"), (64, 5, 2, "masked"), (512, 64, 2, "mixed"), (513, 9, 3, "random"),
+    (1025, 300, 2, "mixed"), (4200, 16, 2, "random"), (8300, 3, 1, "random"),
+])
+def test_single_rank_plan(tokens, experts, topk, kind):
+    """The one-launch plan of a single-rank group: one to eight CTAs, one or several chunks per warp, ragged last chunk."""
+    case = make_case(1, kind=kind, seed=tokens, hidden=256, tokens=tokens, experts_per_rank=experts, topk=topk)
+    case.indices[0][::7] = -1  # tokens without a row
+    cfg = EPConfig(case.num_experts, case.num_topk, case.hidden, case.capacity)
+    with EmulatedGroup(1, cfg) as group:
+        for expand, alignment in ((True, 1), (True, 24), (False, 1)):
+            got = group.dispatch(_cuda(case.xs), topk_idx=_cuda(case.indices), weights=_cuda(case.weights), do_expand=expand, alignment=alignment,
+                                 zero_padding=True)
+            torch.cuda.synchronize()
+            group.check_status()
+            assert_dispatch_matches(got[0], case.xs, case.indices, case.weights, case.num_experts, 0, expand=expand, alignment=alignment,
+                                    zero_padding=True)
