@@ -798,14 +798,21 @@ std::vector<at::Tensor> combine_finish(const std::vector<PeerWindow*>& wins, con
         r.tokens = int(T);
         r.sum_all_choices = 1;
     }
-    const BarrierParams* bdev = upload(barrier, keep, cs);
-    PeerWindow::launches += 1;
-    cuda_check(launch_barrier(bdev, LaunchShape{1, n}, cs), "barrier launch");
+    // A single-rank group has no peer to wait for or to tell: the rows come from an earlier kernel of the same stream and
+    // the next kernel that writes the return area is ordered behind the reduction (the two launches took 20 us with
+    // their gaps, of 100 us that a 64-token layer spent outside its GEMMs).
+    const bool local = L.ranks == 1;
+    if (!local) {
+        const BarrierParams* bdev = upload(barrier, keep, cs);
+        PeerWindow::launches += 1;
+        cuda_check(launch_barrier(bdev, LaunchShape{1, n}, cs), "barrier launch");
+    }
     int64_t max_tokens_now = 1;
     for (int i = 0; i < n; ++i) max_tokens_now = std::max<int64_t>(max_tokens_now, meta[i][5].size(0));
     const ReduceParams* rdev = upload(reduce, keep, cs);
     PeerWindow::launches += 1;
     cuda_check(launch_reduce(rdev, LaunchShape{row_sum_grid(max_tokens_now, L.hidden, true, lim.sms), n}, cs), "reduce launch");
+    if (local) return outs;
     // Tell every peer that this rank has finished reading its return area (nobody waits): the next combine kernel
     // waits for this epoch before it overwrites the area, exactly as it does after a combine kernel.
     std::vector<BarrierParams> done(n);

@@ -80,7 +80,11 @@ class ExpertParallelMoE:
             self._tile_ready.zero_()
         got = buf.dispatch(
             x, topk_idx=None if handle is not None else topk_idx, weights=topk_weights, handle=handle,
-            do_expand=True if handle is None else None, alignment=ALIGNMENT if handle is None else None, zero_padding=True,
+            do_expand=True if handle is None else None, alignment=ALIGNMENT if handle is None else None,
+            # Row blocks are gated by counters that include the padding rows.  Without gating nobody reads what the padding
+            # rows hold: a GEMM row depends on its own input row alone, and the combine takes real rows only (writing
+            # the zeros was 51 MB of 58 MB in a dispatch of 64 tokens to 32 experts, 27 us).
+            zero_padding=overlap,
             async_op=overlap, tile_ready=self._tile_ready if overlap else None,
             ring_smem_limit=self.comm_ring_bytes if overlap else 0,
         )
