@@ -25,15 +25,15 @@ EncodeFn encode_fn() {
     return fn;
 }
 
-// Row-major bf16 [rows, cols]; box = 64 columns (128 bytes, one swizzle row) x 128 rows.
-CUtensorMap make_map(const void* base, int64_t rows, int64_t cols) {
+// Row-major bf16 [outer, rows, cols]; box = 64 columns (128 bytes, one swizzle row) x `box_rows` rows x `box_outer`.
+CUtensorMap make_map(const void* base, int64_t rows, int64_t cols, int box_rows = 128, int64_t outer = 1, int box_outer = 0) {
     TORCH_CHECK(reinterpret_cast<uintptr_t>(base) % 16 == 0 && (cols * 2) % 16 == 0, "TMA operand must be 16-byte aligned with 16-byte row pitch");
     CUtensorMap map;
-    const cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
-    const cuuint64_t strides[1] = {cuuint64_t(cols) * 2};
-    const cuuint32_t box[2] = {64, 128};
-    const cuuint32_t elem[2] = {1, 1};
-    CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+    const cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(outer)};
+    const cuuint64_t strides[2] = {cuuint64_t(cols) * 2, cuuint64_t(rows) * cuuint64_t(cols) * 2};
+    const cuuint32_t box[3] = {64, cuuint32_t(box_rows), cuuint32_t(box_outer)};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, box_outer > 0 ? 3 : 2, const_cast<void*>(base), dims, strides, box, elem,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     TORCH_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed");
@@ -67,6 +67,7 @@ GemmCommon prepare(const at::Tensor& a, const at::Tensor& w, const at::Tensor& e
     GemmCommon g;
     g.args.expert_offsets = expert_offsets.data_ptr<int64_t>();
     g.args.num_experts = int(E);
+    g.args.rows = rows;
     g.args.m_blocks = int(rows / 128);
     g.args.k_blocks = int(K / 64);
     g.args.b_rows_per_expert = int(NW);
@@ -87,6 +88,26 @@ GemmCommon prepare(const at::Tensor& a, const at::Tensor& w, const at::Tensor& e
     return g;
 }
 
+cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& w, const c10::optional<at::Tensor>& counts, int mode,
+                          int64_t max_expert_rows, int64_t max_ctas) {
+    if (counts.has_value()) {
+        TORCH_CHECK(counts->is_cuda() && counts->device() == a.device() && counts->scalar_type() == at::kLong && counts->is_contiguous() &&
+                        counts->dim() == 1 && counts->size(0) == w.size(0),
+                    "expert_counts must be an int64 tensor of num_experts entries on the activations' device");
+        g.args.expert_counts = counts->data_ptr<int64_t>();
+    }
+    const int64_t rows = a.size(0), K = a.size(1), E = w.size(0), NW = w.size(1);
+    gemm::ExpertMaps maps;
+    maps.weights = mode == gemm::kSwiGLU ? make_map(w.data_ptr(), NW / 2, K, 16, 2 * E, 2) : make_map(w.data_ptr(), E * NW, K);
+    for (int b = 0; b < 4; ++b) maps.tokens[b] = make_map(a.data_ptr(), rows, K, 128 >> b);
+    // A smaller token tile deepens the operand pipeline, which weights streamed from memory need (64 tokens over 32 experts of
+    // 7168 x 2048: 287 us with tiles of 64 or 128, 302 with 256); more rows than that would only read the weights again.
+    const int tile = max_expert_rows <= 0 || max_expert_rows > 128 ? 256 : max_expert_rows > 64 ? 128 : 64;
+    const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    const int grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : sms;
+    return gemm::launch_expert(maps, g.args, mode, tile, grid, c10::cuda::getCurrentCUDAStream().stream());
+}
+
 }  // namespace
 
 void bind_gemm(pybind11::module_& m) {
@@ -95,7 +116,7 @@ void bind_gemm(pybind11::module_& m) {
         "grouped_gemm",
         [](const at::Tensor& a, const at::Tensor& w, const at::Tensor& expert_offsets, at::Tensor& out, at::Tensor& status, int64_t mode,
            c10::optional<at::Tensor> tile_ready, c10::optional<at::Tensor> tile_expected, int64_t max_ctas, double timeout_s,
-           c10::optional<at::Tensor> row_scale, int64_t stages, bool pair) {
+           c10::optional<at::Tensor> row_scale, int64_t stages, bool pair, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows) {
             c10::cuda::CUDAGuard guard(a.device());
             TORCH_CHECK(mode == gemm::kPlain || mode == gemm::kSwiGLU, "mode must be 0 (plain) or 1 (SwiGLU)");
             auto g = prepare(a, w, expert_offsets, status, int(mode), timeout_s);
@@ -123,12 +144,17 @@ void bind_gemm(pybind11::module_& m) {
             if (a.size(0) == 0) return;
             const int grid = max_ctas > 0 ? std::min<int>(g.grid, int(max_ctas)) : g.grid;
             PeerWindow::launches += 1;
+            // The kernel with tokens as N unless its row blocks are gated by counters (that one shares the SMs with the
+            // dispatch and has to leave it shared memory) or the caller allows a single CTA (it needs pairs).
+            if (!tile_ready.has_value() && max_ctas != 1) {
+                cudaError_t ee = launch_expert(g, a, w, expert_counts, int(mode), max_expert_rows, max_ctas);
+                TORCH_CHECK(ee == cudaSuccess, "grouped GEMM (expert) launch failed: ", cudaGetErrorString(ee));
+                return;
+            }
             if (pair) {
                 const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
                 const int pair_grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : sms;
-                // gated by tile counters = meant to share the SMs with the pull kernel: shorter pipeline
-                cudaError_t pe = gemm::launch_pair(g.map_a, g.map_b, g.args, int(mode), pair_grid, c10::cuda::getCurrentCUDAStream().stream(),
-                                                   tile_ready.has_value() ? 4 : 6);
+                cudaError_t pe = gemm::launch_pair(g.map_a, g.map_b, g.args, int(mode), pair_grid, c10::cuda::getCurrentCUDAStream().stream());
                 TORCH_CHECK(pe == cudaSuccess, "grouped GEMM (CTA pairs) launch failed: ", cudaGetErrorString(pe));
                 return;
             }
@@ -138,7 +164,8 @@ void bind_gemm(pybind11::module_& m) {
         pybind11::arg("a"), pybind11::arg("w"), pybind11::arg("expert_offsets"), pybind11::arg("out"), pybind11::arg("status"),
         pybind11::arg("mode"), pybind11::arg("tile_ready") = c10::nullopt, pybind11::arg("tile_expected") = c10::nullopt,
         pybind11::arg("max_ctas") = 0, pybind11::arg("timeout_s") = 5.0, pybind11::arg("row_scale") = c10::nullopt,
-        pybind11::arg("stages") = 4, pybind11::arg("pair") = false);
+        pybind11::arg("stages") = 4, pybind11::arg("pair") = false, pybind11::arg("expert_counts") = c10::nullopt,
+        pybind11::arg("max_expert_rows") = 0);
 
     // Down projection fused with the combine push: row r of (A @ W[e]^T) * slot_weight[r] is stored
     // (bf16) into the return partition of the row's source rank; padding rows are skipped.  The return area
@@ -148,8 +175,9 @@ void bind_gemm(pybind11::module_& m) {
         "grouped_gemm_scatter",
         [](PeerWindow& window, const at::Tensor& a, const at::Tensor& w, const at::Tensor& expert_offsets,
            const at::Tensor& slot_map, const at::Tensor& recv_metadata, c10::optional<at::Tensor> slot_weights, at::Tensor& status,
-           int64_t max_ctas, double timeout_s, bool pair) {
+           int64_t max_ctas, double timeout_s, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows) {
             c10::cuda::CUDAGuard guard(a.device());
+            TORCH_CHECK(max_ctas != 1, "the fused combine needs pairs of CTAs");
             auto g = prepare(a, w, expert_offsets, status, gemm::kScatter, timeout_s);
             const WindowLayout& L = window.layout();
             TORCH_CHECK(w.size(1) == L.hidden, "down-projection N must equal the buffer's hidden size");
@@ -175,24 +203,17 @@ void bind_gemm(pybind11::module_& m) {
             g.args.recv_rows = int(recv_metadata.size(0));
             g.args.ldo = L.hidden;
             if (a.size(0) == 0) return;
-            const int grid = max_ctas > 0 ? std::min<int>(g.grid, int(max_ctas)) : g.grid;
             PeerWindow::launches += 1;
-            cudaError_t e;
-            if (pair) {
-                const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-                e = gemm::launch_pair(g.map_a, g.map_b, g.args, gemm::kScatter, max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : sms,
-                                      c10::cuda::getCurrentCUDAStream().stream());
-            } else {
-                e = gemm::launch(g.map_a, g.map_b, g.args, gemm::kScatter, 3, grid, c10::cuda::getCurrentCUDAStream().stream());
-            }
+            const cudaError_t e = launch_expert(g, a, w, expert_counts, gemm::kScatter, max_expert_rows, max_ctas);
             TORCH_CHECK(e == cudaSuccess, "grouped GEMM (scatter) launch failed: ", cudaGetErrorString(e));
         },
         pybind11::arg("window"), pybind11::arg("a"), pybind11::arg("w"), pybind11::arg("expert_offsets"),
         pybind11::arg("slot_map"), pybind11::arg("recv_metadata"), pybind11::arg("slot_weights"), pybind11::arg("status"),
-        pybind11::arg("max_ctas") = 0, pybind11::arg("timeout_s") = 5.0, pybind11::arg("pair") = true);
+        pybind11::arg("max_ctas") = 0, pybind11::arg("timeout_s") = 5.0,
+        pybind11::arg("expert_counts") = c10::nullopt, pybind11::arg("max_expert_rows") = 0);
 
     m.def("gemm_kernel_registers", [](int64_t mode) { return gemm::kernel_registers(int(mode)); });
-    m.def("gemm_shared_bytes", [](int64_t mode, int64_t stages) { return int64_t(gemm::shared_bytes(int(mode), int(stages))); });
+    m.def("gemm_shared_bytes", [](int64_t stages) { return int64_t(gemm::shared_bytes(int(stages))); });
 }
 
 }  // namespace nep

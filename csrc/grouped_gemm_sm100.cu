@@ -4,7 +4,8 @@
 //   out[m, :] = epilogue( A[m, :] @ W[e(m)]^T )     for every 128-row block m of the expert-major
 //                                                   activation matrix; e(m) from expert_offsets.
 //
-// The reference library has no GEMM at all (its kernels only move data); this kernel is what lets
+// It runs where row blocks are gated by counters (beside the dispatch that fills them) or a caller allows one CTA only;
+// everything else is expert_gemm_sm100.cu.  The reference library has no GEMM at all (its kernels only move data); this kernel is what lets
 // dispatch feed the expert up-projection and the down-projection feed combine on the same GPU.
 //
 // Roles per CTA (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner, warps 2..5 =
@@ -16,8 +17,6 @@
 //   kPlain   : out[128 x 256] = bf16(acc)
 //   kSwiGLU  : the B tile holds 128 gate rows and the 128 matching up rows of the fused [2I, H]
 //              weight; out[128 x 128] = bf16(silu(gate) * up)
-//   kScatter : (fused down-projection + combine) acc * gate weight of the slot -> bf16 -> stored
-//              straight into the source rank's return partition over NVLink (peer pointer).
 // Optional tile gating (fused dispatch + up-projection): the producer waits until the row block's
 // ready counter reaches its expected value before loading A.
 //
@@ -42,11 +41,6 @@ constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kThreads = 192;
 constexpr int kTmemCols = 512;
 constexpr int kMaxExperts = 1024;
-// kScatter stages its 128 x 256 bf16 output tile in shared memory (one 512-byte row per thread,
-// padded to 528 bytes against bank conflicts) and sends each row with one bulk store.
-constexpr int kOutRowBytes = BN * 2;
-constexpr int kOutPitch = kOutRowBytes + 16;
-constexpr int kOutStageBytes = 4 * 32 * kOutPitch;
 
 // 2-D tiled TMA load into this CTA's shared memory (unicast).
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -95,7 +89,6 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(const __grid_
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* tiles = smem;  // kStages x (A 16 KB | B 32 KB), 1024-byte aligned
     SharedStorage& sh = *reinterpret_cast<SharedStorage*>(smem + kStages * kStageBytes);
-    uint8_t* out_stage = smem + kStages * kStageBytes + ((sizeof(SharedStorage) + 127) / 128) * 128;  // kScatter only
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t limit_ns = args.timeout_ns;
 
@@ -266,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(const __grid_
 #pragma unroll
                     for (int q = 0; q < 4; ++q) st_v4(out_row + c + q * 8, o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
                 }
-            } else if (kMode == kPlain) {
+            } else {
                 __nv_bfloat16* out_row = args.out + int64_t(row) * args.ldo + nt * BN;
                 const float scale = args.row_scale != nullptr ? args.row_scale[row] : 1.f;
                 uint32_t v[2][32];
@@ -282,60 +275,10 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(const __grid_
 #pragma unroll
                     for (int q = 0; q < 4; ++q) st_v4(out_row + c + q * 8, o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
                 }
-            } else {
-                // kScatter: acc * gate weight -> bf16 row in shared memory -> one 512-byte bulk store into
-                // the source rank's return partition (peer memory over NVLink, or local).  Padding rows
-                // are skipped.
-                __nv_bfloat16* out_row = nullptr;
-                float scale = 1.f;
-                const int a = args.slot_map[row];
-                if (a >= 0) {
-                    const int recv_row = a / args.topk, k = a % args.topk;
-                    const int* meta = args.recv_metadata + int64_t(recv_row) * (args.topk + 2);
-                    const int src = meta[0], tok = meta[1];
-                    scale = args.slot_weights != nullptr ? args.slot_weights[row] : 1.f;
-                    if (recv_row >= args.recv_rows || src < 0 || src >= args.ranks || tok < 0 || tok >= args.max_tokens) {
-                        // impossible provenance: skip the row and report it, as the push kernel does
-                        if (atomicCAS(args.status, 0u, uint32_t(kGemmBadMetadata)) == 0u) args.status[1] = uint32_t(row);
-                    } else
-                    out_row = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(args.peers[src]) + args.ret_offset +
-                                                               (int64_t(k) * args.max_tokens + tok) * int64_t(args.ldo) * 2) +
-                              nt * BN;
-                }
-                uint8_t* my_row = out_stage + (quarter * 32 + lane) * kOutPitch;
-                // the previous tile's bulk store must have finished reading this row buffer
-                // The row is sent as two 256-byte halves, each its own bulk group: before a half of the
-                // staging row is overwritten only the store that last read THAT half has to be done
-                // (wait_group.read 1 = everything but the newest group), so a store is always in flight.
-                uint32_t v[2][32];
-                tmem_ld32(taddr, v[0]);
-#pragma unroll
-                for (int step = 0; step < BN / 32; ++step) {
-                    const int cur = step & 1, c = step * 32;
-                    if (step == 0 || step == BN / 64) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                    tmem_ld_wait();
-                    if (step + 1 < BN / 32) tmem_ld32(taddr + c + 32, v[cur ^ 1]);
-                    uint32_t o[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        o[j] = pack_bf16(__uint_as_float(v[cur][2 * j]) * scale, __uint_as_float(v[cur][2 * j + 1]) * scale);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) st_shared_v4(my_row + c * 2 + q * 16, o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
-                    if (step == BN / 64 - 1 || step == BN / 32 - 1) {
-                        const int half = step == BN / 64 - 1 ? 0 : 1;
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        if (out_row != nullptr) bulk_store_row(out_row + half * (BN / 2), my_row + half * (kOutRowBytes / 2), kOutRowBytes / 2);
-                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    }
-                }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.tmem_empty[acc]);
-        }
-        if (kMode == kScatter) {
-            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-            __threadfence_system();
         }
     }
     tc_fence_before();
@@ -348,14 +291,14 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_kernel(const __grid_
 
 }  // namespace
 
-size_t shared_bytes(int mode, int stages) {
-    return size_t(stages) * kStageBytes + ((sizeof(SharedStorage) + 127) / 128) * 128 + (mode == kScatter ? kOutStageBytes : 0) + 128;
+size_t shared_bytes(int stages) {
+    return size_t(stages) * kStageBytes + ((sizeof(SharedStorage) + 127) / 128) * 128 + 128;
 }
 
 template <int kMode, int kStages>
 cudaError_t launch_mode(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int grid, cudaStream_t stream) {
     auto* fn = grouped_gemm_kernel<kMode, kStages>;
-    const size_t smem = shared_bytes(kMode, kStages);
+    const size_t smem = shared_bytes(kStages);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     fn<<<grid, kThreads, smem, stream>>>(a, b, args);
@@ -369,15 +312,13 @@ cudaError_t launch(const CUtensorMap& a, const CUtensorMap& b, const Args& args,
     if (mode == kPlain && stages == 3) return launch_mode<kPlain, 3>(a, b, args, grid, stream);
     if (mode == kSwiGLU && stages == 4) return launch_mode<kSwiGLU, 4>(a, b, args, grid, stream);
     if (mode == kSwiGLU && stages == 3) return launch_mode<kSwiGLU, 3>(a, b, args, grid, stream);
-    if (mode == kScatter) return launch_mode<kScatter, 3>(a, b, args, grid, stream);
     return cudaErrorInvalidValue;
 }
 
 int kernel_registers(int mode) {
     cudaFuncAttributes attr{};
     const void* fn = mode == kPlain ? (const void*)grouped_gemm_kernel<kPlain, 4>
-                   : mode == kSwiGLU ? (const void*)grouped_gemm_kernel<kSwiGLU, 4>
-                                     : (const void*)grouped_gemm_kernel<kScatter, 3>;
+                                      : (const void*)grouped_gemm_kernel<kSwiGLU, 4>;
     if (cudaFuncGetAttributes(&attr, fn) != cudaSuccess) {
         cudaGetLastError();
         return -1;

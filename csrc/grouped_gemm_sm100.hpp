@@ -14,6 +14,8 @@ enum GemmStatus : uint32_t { kGemmOk = 0, kGemmPipeTimeout = 101, kGemmTileTimeo
 struct Args {
     const int64_t* expert_offsets;  // [E+1] padded exclusive row offsets, multiples of 128
     int num_experts;
+    const int64_t* expert_counts;   // expert kernel: [E] rows that exist per expert, or null (all rows of the range)
+    int64_t rows;            // total rows
     int m_blocks;            // total rows / 128
     int n_tiles;             // output column tiles per row block (256 wide; 128 wide for SwiGLU)
     int k_blocks;            // K / 64
@@ -39,11 +41,21 @@ struct Args {
     int recv_rows;  // kScatter: rows of recv_metadata
 };
 
-size_t shared_bytes(int mode, int stages);
+// Tensor maps of the expert kernel: weights (for SwiGLU as [2E][I][K], gate and up halves), token rows in boxes of
+// 128, 64, 32 and 16 rows.
+struct ExpertMaps {
+    CUtensorMap weights;
+    CUtensorMap tokens[4];
+};
+
+size_t shared_bytes(int stages);
 cudaError_t launch(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int mode, int stages, int grid, cudaStream_t stream);
 int kernel_registers(int mode);
 // CTA-pair variant (tcgen05 cta_group::2, 256 x 256 tiles on two SMs); modes kPlain and kSwiGLU.
-cudaError_t launch_pair(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int mode, int grid, cudaStream_t stream, int stages = 6);
+cudaError_t launch_pair(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int mode, int grid, cudaStream_t stream);
+
+// Weights as M, tokens as N (expert_gemm_sm100.cu); `tile_tokens` = largest token tile wanted (64, 128 or 256).
+cudaError_t launch_expert(const ExpertMaps& maps, const Args& args, int mode, int tile_tokens, int grid, cudaStream_t stream);
 
 }  // namespace gemm
 }  // namespace nep

@@ -4,8 +4,8 @@
 // cluster of two CTAs shares every B tile: each CTA loads its own 128 activation rows and HALF of
 // the 256 weight rows, the leader CTA issues one MMA for the pair, and each CTA keeps the
 // accumulator of its own 128 rows in its own TMEM.  Per CTA and k-block that is 32 KB of operand
-// traffic instead of 48 KB, which is what limits the single-CTA kernel (L2 -> SM bandwidth), and it
-// leaves room for six pipeline stages.
+// traffic instead of 48 KB, which is what limits the single-CTA kernel (L2 -> SM bandwidth).
+// It runs where row blocks are gated by counters; everything else is expert_gemm_sm100.cu.
 //
 // Work unit = (expert, pair of consecutive 128-row blocks of that expert, output column tile).
 // An expert with an odd number of row blocks leaves the second CTA of its last pair without rows:
@@ -40,54 +40,7 @@ constexpr int kThreads = 192;
 constexpr int kTmemCols = 512;
 constexpr int kMaxExperts = 1024;
 constexpr int kMaxStages = 6;
-// kScatter stages each 512-byte output row in shared memory (padded rows) before one bulk store.
-constexpr int kOutRowBytes = BN * 2;
-constexpr int kOutPitch = kOutRowBytes + 16;
-constexpr int kOutStageBytes = 4 * 32 * kOutPitch;
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// shared::cluster address of the same shared-memory location in CTA `rank` of this cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
-    uint32_t out;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_addr), "r"(rank));
-    return out;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// arrive on a barrier given by its shared::cluster address (own or peer CTA)
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// 2-D tiled TMA load into this CTA's shared memory; completion bytes go to the barrier at
-// `bar_cluster_addr`, which may live in the peer CTA of the pair (unicast data path).
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, int x, int y, uint32_t bar_cluster_addr) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-                     smem_u32(smem_dst)),
-                 "l"(map), "r"(bar_cluster_addr), "r"(x), "r"(y)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t addr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
-}
-// completion of all earlier MMAs of the pair -> one arrival on the barrier at `bar_cluster_addr`
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
-}
-__device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
-                 "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-                 : "memory");
-}
 // pair tile: M = 256 (128 rows per CTA), N = 256
 constexpr uint32_t kInstrDescPair = instr_desc_bf16(2 * BM, BN);
 
@@ -125,7 +78,6 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_pair_kernel(const __
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* tiles = smem;
     PairShared& sh = *reinterpret_cast<PairShared*>(smem + kStages * kStageBytes);
-    uint8_t* out_stage = smem + kStages * kStageBytes + ((sizeof(PairShared) + 127) / 128) * 128;  // kScatter only
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t cta = cluster_ctarank();
     const bool leader = cta == 0;
@@ -312,50 +264,6 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_pair_kernel(const __
 #pragma unroll
                         for (int q = 0; q < 4; ++q) st_v4(out_row + c + q * 8, o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
                     }
-                } else if (kMode == kScatter) {
-                    // acc * gate weight -> bf16 row in shared memory -> one 512-byte bulk store into the
-                    // source rank's return partition (peer memory over NVLink, or local); padding rows skipped
-                    __nv_bfloat16* out_row = nullptr;
-                    float scale = 1.f;
-                    const int a = args.slot_map[row];
-                    if (a >= 0) {
-                        const int recv_row = a / args.topk, k = a % args.topk;
-                        const int* meta = args.recv_metadata + int64_t(recv_row) * (args.topk + 2);
-                        const int src = meta[0], tok = meta[1];
-                        scale = args.slot_weights != nullptr ? args.slot_weights[row] : 1.f;
-                        if (recv_row >= args.recv_rows || src < 0 || src >= args.ranks || tok < 0 || tok >= args.max_tokens) {
-                            // impossible provenance: skip the row and report it, as the push kernel does
-                            if (atomicCAS(args.status, 0u, uint32_t(kGemmBadMetadata)) == 0u) args.status[1] = uint32_t(row);
-                        } else
-                        out_row = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(args.peers[src]) + args.ret_offset +
-                                                                   (int64_t(k) * args.max_tokens + tok) * int64_t(args.ldo) * 2) +
-                                  nt * BN;
-                    }
-                    uint8_t* my_row = out_stage + (quarter * 32 + lane) * kOutPitch;
-                    // The row is sent as two 256-byte halves, each its own bulk group: before a half of the
-                    // staging row is overwritten only the store that last read THAT half has to be done
-                    // (wait_group.read 1 = everything but the newest group), so a store is always in flight.
-                    uint32_t v[2][32];
-                    tmem_ld32(taddr, v[0]);
-#pragma unroll
-                    for (int step = 0; step < BN / 32; ++step) {
-                        const int cur = step & 1, c = step * 32;
-                        if (step == 0 || step == BN / 64) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                        tmem_ld_wait();
-                        if (step + 1 < BN / 32) tmem_ld32(taddr + c + 32, v[cur ^ 1]);
-                        uint32_t o[16];
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            o[j] = pack_bf16(__uint_as_float(v[cur][2 * j]) * scale, __uint_as_float(v[cur][2 * j + 1]) * scale);
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) st_shared_v4(my_row + c * 2 + q * 16, o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
-                        if (step == BN / 64 - 1 || step == BN / 32 - 1) {
-                            const int half = step == BN / 64 - 1 ? 0 : 1;
-                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                            if (out_row != nullptr) bulk_store_row(out_row + half * (BN / 2), my_row + half * (kOutRowBytes / 2), kOutRowBytes / 2);
-                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                        }
-                    }
                 } else {
                     __nv_bfloat16* out_row = args.out + int64_t(row) * args.ldo + nt * BN;
                     const float scale = args.row_scale != nullptr ? args.row_scale[row] : 1.f;
@@ -379,10 +287,6 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_pair_kernel(const __
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh.tmem_empty[acc]), 0));
         }
-        if (kMode == kScatter) {
-            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-            __threadfence_system();
-        }
     }
     tc_fence_before();
     __syncthreads();
@@ -396,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_pair_kernel(const __
 template <int kMode, int kStages>
 cudaError_t launch_pair_mode(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int grid, cudaStream_t stream) {
     auto* fn = grouped_gemm_pair_kernel<kMode, kStages>;
-    const size_t smem = size_t(kStages) * kStageBytes + ((sizeof(PairShared) + 127) / 128) * 128 + (kMode == kScatter ? kOutStageBytes : 0) + 256;
+    const size_t smem = size_t(kStages) * kStageBytes + ((sizeof(PairShared) + 127) / 128) * 128 + 256;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t config{};
@@ -416,17 +320,14 @@ cudaError_t launch_pair_mode(const CUtensorMap& a, const CUtensorMap& b, const A
 
 }  // namespace
 
-// `grid` is rounded down to an even number of CTAs (one cluster = two CTAs on two SMs).  Plain and
-// SwiGLU run six operand stages; the scatter epilogue needs shared memory for its row staging and runs four.
-cudaError_t launch_pair(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int mode, int grid, cudaStream_t stream, int stages) {
+// `grid` is rounded down to an even number of CTAs (one cluster = two CTAs on two SMs).  SwiGLU runs four operand stages, which
+// leaves ~95 KB of shared memory per SM for a co-resident transfer kernel; plain runs six.
+cudaError_t launch_pair(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int mode, int grid, cudaStream_t stream) {
     if (args.num_experts > kMaxExperts) return cudaErrorInvalidValue;
     grid &= ~1;
     if (grid < 2) return cudaErrorInvalidValue;
     if (mode == kPlain) return launch_pair_mode<kPlain, 6>(a, b, args, grid, stream);
-    // four stages leave ~95 KB of shared memory per SM for a co-resident transfer kernel
-    if (mode == kSwiGLU && stages == 4) return launch_pair_mode<kSwiGLU, 4>(a, b, args, grid, stream);
-    if (mode == kSwiGLU) return launch_pair_mode<kSwiGLU, 6>(a, b, args, grid, stream);
-    if (mode == kScatter) return launch_pair_mode<kScatter, 4>(a, b, args, grid, stream);
+    if (mode == kSwiGLU) return launch_pair_mode<kSwiGLU, 4>(a, b, args, grid, stream);
     return cudaErrorInvalidValue;
 }
 

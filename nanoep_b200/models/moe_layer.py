@@ -49,9 +49,9 @@ class ExpertParallelMoE:
         self.overlap_dispatch = overlap_dispatch
         self.device = w13.device
         self.comm_ring_bytes = int(comm_ring_bytes)
-        # tcgen05 cta_group::2 kernels (two SMs share each weight tile).  None = decide per call: a pair
-        # needs two row blocks of the same expert, so with few blocks per expert the half-empty last
-        # pairs cost more than the shared weight tiles save.
+        # Which kernel runs the up-projection that is gated by row counters (overlap_dispatch): CTA pairs, where two SMs share
+        # each weight tile, or single CTAs.  None = decide per call: a pair needs two row blocks of the same expert, so with few
+        # blocks per expert the half-empty last pairs cost more than the shared weight tiles save.
         self.cta_pairs = cta_pairs
         self.local_experts = local
         rows_cap = buffer.world_size * cfg.num_max_tokens_per_rank * min(cfg.num_topk, local) + local * (ALIGNMENT - 1)
@@ -89,10 +89,12 @@ class ExpertParallelMoE:
             ring_smem_limit=self.comm_ring_bytes if overlap else 0,
         )
         h_in, offsets = got.x, got.handle.layout.expert_offsets
-        pairs = self.cta_pairs
-        if pairs is None:
-            pairs = got.handle.layout.expanded_capacity >= 6 * ALIGNMENT * self.local_experts
+        # how many rows of an expert's range exist, and the most that any expert can hold
+        counts, most = got.handle.layout.expert_counts, max(1, got.handle.layout.recv_count)
         if overlap:
+            pairs = self.cta_pairs
+            if pairs is None:
+                pairs = got.handle.layout.expanded_capacity >= 6 * ALIGNMENT * self.local_experts
             # The GEMM must not wait for the whole dispatch: it is gated per row block by the counters.
             h_in.record_stream(stream)
             if self.serialize_overlap:
@@ -104,19 +106,19 @@ class ExpertParallelMoE:
             mark("dispatch+up_gemm")
         else:
             mark("dispatch")
-            h = gg.grouped_gemm(h_in, self.w13, offsets, swiglu=True, pair=pairs)
+            h = gg.grouped_gemm(h_in, self.w13, offsets, swiglu=True, expert_counts=counts, max_expert_rows=most)
             mark("up_gemm")
         self.last_handle = got.handle
         if self.fuse_combine:
             window = buf.window
             self._ext.grouped_gemm_scatter(window, h, self.w2, offsets, got.handle.slot_map, got.handle.layout.recv_metadata,
-                                           got.topk_weights, gg.status_tensor(self.device), 0, 5.0, pairs)
+                                           got.topk_weights, gg.status_tensor(self.device), 0, 5.0, counts, most)
             mark("down_gemm_scatter")
             out = self._ext.combine_finish([window], [handle_metadata(got.handle)], [bias])[0]
             mark("barrier+reduce")
             self._collect(marks)
             return out
-        y = gg.grouped_gemm(h, self.w2, offsets, row_scale=got.topk_weights, pair=pairs)  # gate weight in FP32 in the epilogue
+        y = gg.grouped_gemm(h, self.w2, offsets, row_scale=got.topk_weights, expert_counts=counts, max_expert_rows=most)  # gate weight in FP32
         mark("down_gemm")
         out = buf.combine(y, got.handle, bias=bias).x
         mark("combine")

@@ -1,4 +1,5 @@
-"""Grouped GEMM over expert-major rows (tcgen05 / TMEM kernel, csrc/grouped_gemm_sm100.cu).
+"""Grouped GEMM over expert-major rows (tcgen05 / TMEM kernels, csrc/expert_gemm_sm100.cu; gated by row counters:
+csrc/grouped_gemm_sm100.cu and its CTA-pair variant).
 
 ``rows`` come from a dispatch with ``do_expand=True, alignment=128, zero_padding=True``: every
 128-row block belongs to one expert, padding rows are zero.  The reference library stops at
@@ -40,21 +41,23 @@ def check_status(device=None):
 
 
 def grouped_gemm(a, w, expert_offsets, *, swiglu: bool = False, out=None, tile_ready=None, tile_expected=None, max_ctas: int = 0,
-                 timeout_s: float = 5.0, row_scale=None, stages: int = 4, pair: bool = False) -> torch.Tensor:
+                 timeout_s: float = 5.0, row_scale=None, stages: int = 4, pair: bool = False, expert_counts=None, max_expert_rows: int = 0) -> torch.Tensor:
     """``out[r] = a[r] @ w[e(r)].T`` (bf16 in, fp32 accumulate, bf16 out).
 
     a: ``[rows, K]`` bf16, rows % 128 == 0;  w: ``[E, N, K]`` bf16 (``[E, 2*I, K]`` gate rows then up
     rows when ``swiglu``);  expert_offsets: int64 ``[E+1]`` row offsets (multiples of 128).
     With ``swiglu`` the result is ``silu(a @ w_gate.T) * (a @ w_up.T)`` of shape ``[rows, I]``.
     ``row_scale`` (fp32 ``[rows]``, plain mode) multiplies each output row in FP32 before the bf16 round.
-    ``stages=3`` shrinks the operand pipeline so that a transfer kernel can share the SMs.
-    ``pair=True`` runs the CTA-pair kernel (tcgen05 ``cta_group::2``: two SMs share every weight tile).
+    ``expert_counts`` (int64 ``[E]``): only so many rows of each expert's range exist; the other rows are neither read as
+    far as the result goes nor defined in the output.  ``max_expert_rows`` (0 = unknown): no expert holds more rows.
+    With ``tile_ready`` (row blocks gated by counters): ``stages=3`` shrinks the operand pipeline so that a transfer kernel can
+    share the SMs, ``pair=True`` runs the CTA-pair kernel (two SMs share every weight tile).
     """
     n_out = w.shape[1] // 2 if swiglu else w.shape[1]
     if out is None:
         out = torch.empty((a.shape[0], n_out), dtype=torch.bfloat16, device=a.device)
     _ext().grouped_gemm(a, w, expert_offsets, out, status_tensor(a.device), SWIGLU if swiglu else PLAIN, tile_ready, tile_expected,
-                        int(max_ctas), float(timeout_s), row_scale, int(stages), bool(pair))
+                        int(max_ctas), float(timeout_s), row_scale, int(stages), bool(pair), expert_counts, int(max_expert_rows))
     return out
 
 

@@ -32,6 +32,7 @@ SOURCES = (
     "ep_kernels.cu",
     "grouped_gemm_sm100.cu",
     "grouped_gemm_sm100_2cta.cu",
+    "expert_gemm_sm100.cu",
 )
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]

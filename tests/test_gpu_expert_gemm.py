@@ -1,0 +1,106 @@
+"""The grouped GEMM with weights as the M operand: experts of any number of rows, token tiles of every size."""
+
+from datetime import timedelta
+
+import pytest
+import torch
+import torch.distributed as dist
+
+from nanoep_b200 import CudaBuffer, EPConfig
+from nanoep_b200.models.moe_layer import ExpertParallelMoE, dense_reference
+from nanoep_b200.ops import grouped_gemm as gg
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(counts, K, N):
+    blocks = [(c + 127) // 128 for c in counts]
+    offsets = torch.tensor([0] + blocks, dtype=torch.int64).cumsum(0) * 128
+    a = torch.full((int(offsets[-1]), K), float("nan"), dtype=torch.bfloat16)
+    real = torch.zeros(int(offsets[-1]), dtype=torch.bool)
+    for e, c in enumerate(counts):
+        lo = int(offsets[e])
+        a[lo : lo + c] = (torch.randn(c, K) * 0.5).to(torch.bfloat16)
+        real[lo : lo + c] = True
+    w = (torch.randn(len(counts), N, K) * 0.1).to(torch.bfloat16)
+    return a.cuda(), w.cuda(), offsets.cuda(), torch.tensor(counts, dtype=torch.int64, device="cuda"), real.cuda()
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("largest", [0, 64, 128])  # token tile 256, 64 and 128: larger experts are split
+@pytest.mark.parametrize("counts,K,N", [([1], 64, 256), ([31, 32, 0, 33, 64], 512, 512), ([0, 129, 255, 256, 257, 0], 256, 768), ([1000, 5, 2304], 1024, 256)])
+def test_rows_that_exist(counts, K, N, largest, swiglu):
+    """Padding rows hold NaN and must not reach a real row; rows of experts end anywhere inside a tile."""
+    torch.manual_seed(7)
+    a, w, offsets, n, real = _problem(counts, K, N)
+    scale = None if swiglu else torch.rand(a.shape[0], device="cuda") + 0.5
+    out = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, row_scale=scale, expert_counts=n, max_expert_rows=largest)
+    few = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, row_scale=scale, expert_counts=n, max_expert_rows=largest, max_ctas=4)
+    torch.cuda.synchronize()
+    gg.check_status()
+    ref = gg.grouped_gemm_reference(a, w, offsets, swiglu=swiglu)
+    if scale is not None:
+        ref = ref * scale[:, None]
+    # one bf16 round of an fp32-accumulated product
+    torch.testing.assert_close(out[real].float(), ref[real], rtol=1e-2, atol=1e-2)
+    assert torch.equal(out[real], few[real]), "the result does not depend on the number of CTAs"
+
+
+@pytest.mark.parametrize("pair", [False, True])
+def test_matches_the_gated_kernels(pair):
+    """The kernels with tokens as M (row blocks gated by counters) add the same products: at most one bf16 step apart."""
+    torch.manual_seed(8)
+    a, w, offsets, n, _ = _problem([128, 256, 384], 512, 512)
+    full = torch.full((a.shape[0] // 128,), 128, dtype=torch.int32, device="cuda")
+    for swiglu in (False, True):
+        got = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, expert_counts=n)
+        gated = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, tile_ready=full, tile_expected=full, pair=pair)
+        torch.testing.assert_close(got.float(), gated.float(), rtol=8e-3, atol=1e-3)
+
+
+def test_bad_offsets_are_reported():
+    a = torch.zeros(256, 128, dtype=torch.bfloat16, device="cuda")
+    w = torch.zeros(2, 256, 128, dtype=torch.bfloat16, device="cuda")
+    n = torch.tensor([100, 100], dtype=torch.int64, device="cuda")
+    for bad in ([0, 100, 256], [0, 128, 128]):
+        gg.grouped_gemm(a, w, torch.tensor(bad, dtype=torch.int64, device="cuda"), expert_counts=n)
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="expert_offsets"):
+            gg.check_status()
+
+
+@pytest.fixture(scope="module")
+def one_rank():
+    own = not dist.is_initialized()
+    if own:
+        dist.init_process_group("gloo", store=dist.HashStore(), rank=0, world_size=1, timeout=timedelta(seconds=60))
+    yield dist.group.WORLD
+    if own:
+        dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("tokens", [1, 64, 65, 129, 700])
+def test_layer_on_one_rank(one_rank, tokens, fused):
+    """Uneven experts, masked choices and a bias; routing changes between two passes and padding rows hold whatever was there."""
+    H, inner, E, K = 512, 384, 5, 3
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    w13 = (torch.randn(E, 2 * inner, H, device="cuda", generator=gen) * 0.06).to(torch.bfloat16)
+    w2 = (torch.randn(E, H, inner, device="cuda", generator=gen) * 0.06).to(torch.bfloat16)
+    with CudaBuffer(one_rank, EPConfig(E, K, H, 700)) as buf:
+        layer = ExpertParallelMoE(buf, w13, w2, fuse_combine=fused)
+        for _ in range(2):
+            x = (torch.randn(tokens, H, device="cuda", generator=gen) * 0.5).to(torch.bfloat16)
+            bias = torch.randn(tokens, H, device="cuda", generator=gen).to(torch.bfloat16)
+            skew = torch.rand(tokens, E, device="cuda", generator=gen) * torch.arange(1, E + 1, device="cuda")
+            gate, idx = skew.topk(K, dim=-1)
+            idx = torch.where(torch.rand(tokens, K, device="cuda", generator=gen) < 0.2, -1, idx)
+            gate = (gate / gate.sum(-1, keepdim=True)).float()
+            poison = torch.full((8 << 20,), float("nan"), dtype=torch.bfloat16, device="cuda")
+            del poison
+            out = layer(x, idx, gate, bias=bias)
+            torch.cuda.synchronize()
+            buf.check_status()
+            gg.check_status()
+            want = dense_reference(x, idx, gate, w13, w2).float() + bias.float()
+            torch.testing.assert_close(out.float(), want, rtol=3e-2, atol=3e-2)
