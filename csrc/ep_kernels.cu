@@ -1423,6 +1423,7 @@ __device__ void combine_reduce_smem_role(const CombineParams& p, int* flow, char
     const int nc = (xb + cw - 1) / cw;
     uint64_t* full = reinterpret_cast<uint64_t*>(area + int64_t(NS) * P * cw);
     uint64_t* empty = full + NS;
+    int* rows_in_stage = flow + 2;  // per stage: partition rows that the loader put there
     const StatusRef status = status_of(p.c);
     const uint32_t tag = combine_tag(p.epoch);
     const int n_tok = p.tokens > int(blockIdx.x) ? (p.tokens - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
@@ -1430,68 +1431,102 @@ __device__ void combine_reduce_smem_role(const CombineParams& p, int* flow, char
     const uint64_t once = l2_evict_first_policy();
 
     if (rwarp == 0) {
-        // ---- loader
+        // ---- loader.  It looks at the flags of several tokens at once: a token has G lanes, one per choice, so a poll, an
+        // acquiring load and a read of the routing serve 32 / G tokens.  (One token at a time, the chain routing -> flag ->
+        // acquire -> gate weights -> load took 3.6 us per token, which a combine of 1000 compact tokens over four ranks
+        // waited for: 138 -> 105 us.  With one system fence for all tokens instead of the acquiring loads it took 141 us.)
         const uint32_t* flag_base = reinterpret_cast<const uint32_t*>(window(p.c, p.c.rank) + L.ret_flag_offset);
         const float* ret_w = reinterpret_cast<const float*>(window(p.c, p.c.rank) + L.ret_w_offset);
-        unsigned parts = 0;
-        int my_part = 0;
-        for (int u = 0; u < units; ++u) {
-            const int c = u % nc, t = int(blockIdx.x) + (u / nc) * int(gridDim.x);
-            const int s = u % NS, n = u / NS;
-            if (c == 0) {
-                bool valid;
-                int dest;
-                parts = expected_parts(p.topk, t, K, E, Le, p.sum_all_choices != 0, valid, dest);
-                my_part = L.rank_indexed ? dest : lane;
-                if (parts != 0) {
-                    const bool mine = (parts >> lane) & 1u;
-                    const uint32_t* flag = flag_base + int64_t(mine ? my_part : 0) * L.max_tokens + t;
+        const int G = K <= 4 ? 4 : K <= 8 ? 8 : K <= 16 ? 16 : 32, W = 32 / G;
+        const unsigned token_lanes = G == 32 ? kFull : (1u << G) - 1u;
+        const int sub = lane / G, k = lane % G;
+        auto token_of = [&](int i) { return int(blockIdx.x) + i * int(gridDim.x); };
+        auto choice_of = [&](int i) -> int64_t { return i < n_tok && k < K ? p.topk[int64_t(token_of(i)) * K + k] : -1; };
+        int64_t next = choice_of(sub);
+        int u = 0;
+        bool alive = true;
+        for (int base = 0; base < n_tok && alive; base += W) {
+            const int t = token_of(base + sub);
+            const int64_t e = next;
+            next = choice_of(base + W + sub);
+            const bool valid = e >= 0 && e < E;
+            const int dest = valid ? int(e) / Le : -1;
+            // one partition per valid choice, or one per destination rank, named by the rank's first choice
+            const unsigned same = __match_any_sync(kFull, valid ? sub * kMaxRanks + dest : 32 * kMaxRanks + lane);
+            const bool mine = valid && (p.sum_all_choices != 0 || lane == __ffs(same) - 1);
+            const unsigned parts = __ballot_sync(kFull, mine);
+            const int my_part = L.rank_indexed ? dest : k;
+            const uint32_t* flag = flag_base + int64_t(mine ? my_part : 0) * L.max_tokens + (mine ? t : 0);
+            const unsigned my_lanes = token_lanes << (sub * G);
+            bool here = !mine;
+            unsigned ordered = 0;  // lanes of the tokens that are complete and may be loaded
+            for (int j = 0; j < W && base + j < n_tok; ++j) {
+                const unsigned lanes = token_lanes << (j * G);
+                const int tok = token_of(base + j);
+                if ((ordered & lanes) != lanes) {
                     const uint64_t start = global_timer_ns();
                     uint32_t spins = 0;
-                    bool arrived = false;
+                    unsigned seen;  // lanes whose row has arrived
                     for (;;) {
-                        const bool here = !mine || ld_relaxed_sys_u32(flag) == tag;
-                        arrived = __all_sync(kFull, here);
-                        if (arrived) break;
+                        if (!here) here = ld_relaxed_sys_u32(flag) == tag;
+                        seen = __ballot_sync(kFull, here);
+                        if ((seen & lanes) == lanes) break;
                         __nanosleep(100);
                         if ((++spins & 15u) == 0u &&
-                            __any_sync(kFull, *(volatile int*)abort_word != 0 || global_timer_ns() - start > p.c.timeout_ns))
+                            __any_sync(kFull, *(volatile int*)abort_word != 0 || global_timer_ns() - start > p.c.timeout_ns)) {
+                            alive = false;
                             break;
+                        }
                     }
-                    // the polls were relaxed; one acquiring load of each flag orders the rows behind them, and the
-                    // proxy fence orders the bulk loads below behind that
-                    if (arrived && mine) (void)ld_acquire_sys_u32(flag);
-                    fence_proxy_async();
-                    __syncwarp();
-                    if (!arrived) {
+                    if (!alive) {
                         if (lane == 0) {
-                            report(status, kBarrierTimeout, uint32_t(t), kTagReduce);
+                            report(status, kBarrierTimeout, uint32_t(tok), kTagReduce);
                             *(volatile int*)abort_word = 1;  // a peer never delivered: the consumers stop at their next wait
                         }
                         break;
                     }
+                    // the polls were relaxed; one acquiring load of each flag orders the rows behind them, and the
+                    // proxy fence orders the bulk loads below behind that
+                    const bool complete = (seen & my_lanes) == my_lanes, fresh = complete && !((ordered >> lane) & 1u);
+                    if (fresh && mine) (void)ld_acquire_sys_u32(flag);
+                    __syncwarp();
+                    if (fresh && p.w_out != nullptr && k < K && base + sub < n_tok)
+                        p.w_out[int64_t(t) * K + k] = valid ? __ldcg(ret_w + int64_t(t) * K + k) : 0.f;
+                    fence_proxy_async();
+                    __syncwarp();
+                    ordered = __ballot_sync(kFull, complete);
                 }
-                if (p.w_out != nullptr && lane < K) p.w_out[int64_t(t) * K + lane] = valid ? __ldcg(ret_w + int64_t(t) * K + lane) : 0.f;
-            }
-            if (n >= 1) {
-                // the stage is free once every consumer warp has read its previous contents
-                bool ok = mbar_wait_or_abort(empty + s, uint32_t(n - 1) & 1u, p.c.timeout_ns, abort_word);
-                ok = __all_sync(kFull, ok);
-                if (!ok) {
-                    if (lane == 0 && *(volatile int*)abort_word == 0) {
-                        report(status, kCopyTimeout, uint32_t(t), kTagReduce);
-                        *(volatile int*)abort_word = 1;
+                const bool own = sub == j;
+                const unsigned token_parts = parts & lanes;
+                const int np = __popc(token_parts);
+                for (int c = 0; c < nc; ++c, ++u) {
+                    const int s = u % NS, n = u / NS;
+                    if (n >= 1) {
+                        // the stage is free once every consumer warp has read its previous contents
+                        bool ok = mbar_wait_or_abort(empty + s, uint32_t(n - 1) & 1u, p.c.timeout_ns, abort_word);
+                        ok = __all_sync(kFull, ok);
+                        if (!ok) {
+                            if (lane == 0 && *(volatile int*)abort_word == 0) {
+                                report(status, kCopyTimeout, uint32_t(tok), kTagReduce);
+                                *(volatile int*)abort_word = 1;
+                            }
+                            alive = false;
+                            break;
+                        }
                     }
-                    break;
+                    const int bytes = min(cw, xb - c * cw);
+                    if (lane == 0) {
+                        rows_in_stage[s] = np;  // the arrival below hands it to the consumers
+                        mbar_expect_tx(full + s, uint32_t(np * bytes));
+                    }
+                    __syncwarp();
+                    if (own && mine) {
+                        const int at = __popc(token_parts & lanemask_lt());
+                        bulk_load_hint(area + (int64_t(s) * P + at) * cw, ret_row(p.c, p.c.rank, my_part, tok) + int64_t(c) * cw, uint32_t(bytes),
+                                       full + s, once);
+                    }
                 }
-            }
-            const int bytes = min(cw, xb - c * cw);
-            if (lane == 0) mbar_expect_tx(full + s, uint32_t(__popc(parts) * bytes));
-            __syncwarp();
-            if ((parts >> lane) & 1u) {
-                const int j = __popc(parts & lanemask_lt());
-                bulk_load_hint(area + (int64_t(s) * P + j) * cw, ret_row(p.c, p.c.rank, my_part, t) + int64_t(c) * cw, uint32_t(bytes),
-                               full + s, once);
+                if (!alive) break;
             }
         }
         return;
@@ -1499,17 +1534,11 @@ __device__ void combine_reduce_smem_role(const CombineParams& p, int* flow, char
 
     // ---- consumers
     const int cwarp = rwarp - 1;
-    unsigned parts = 0;
     unsigned waited = 0, worked = 0, longest = 0, summed = 0;  // nanoseconds
     unsigned long long longest_at = 0, last_seen = 0;
     for (int u = 0; u < units; ++u) {
         const int c = u % nc, t = int(blockIdx.x) + (u / nc) * int(gridDim.x);
         const int s = u % NS, n = u / NS;
-        if (c == 0) {
-            bool valid;
-            int dest;
-            parts = expected_parts(p.topk, t, K, E, Le, p.sum_all_choices != 0, valid, dest);
-        }
         const uint64_t t_wait = p.trace != nullptr ? global_timer_ns() : 0;
         {
             bool ok = mbar_wait_or_abort(full + s, uint32_t(n) & 1u, p.c.timeout_ns, abort_word);
@@ -1523,7 +1552,7 @@ __device__ void combine_reduce_smem_role(const CombineParams& p, int* flow, char
             }
         }
         const uint64_t t_work = p.trace != nullptr ? global_timer_ns() : 0;
-        const int np = __popc(parts);
+        const int np = *(volatile const int*)(rows_in_stage + s);
         const int bytes = min(cw, xb - c * cw);
         const char* rows = area + int64_t(s) * P * cw;
         for (int v = cwarp * 32 + lane; v * 16 < bytes; v += CW * 32) {
@@ -1989,6 +2018,10 @@ CombinePlan plan_combine(int64_t row_bytes, int parts, int max_smem_bytes, int r
         // about half of shared memory for the pipeline unless the caller names a chunk; whole rows when they fit
         chunk = reduce_chunk_bytes > 0 ? align_up(reduce_chunk_bytes, 128) : (int64_t(max_smem_bytes) / 2 / reduce_stages / parts) / 128 * 128;
         chunk = std::min<int64_t>(chunk, pitch);
+        // whole rows that leave room in that half: more tokens in flight
+        while (reduce_chunk_bytes <= 0 && chunk == pitch && reduce_stages < 4 &&
+               (reduce_stages + 1) * parts * chunk <= int64_t(max_smem_bytes) / 2)
+            ++reduce_stages;
     }
     // transfer warps the rings would get without a pipeline: an automatic chunk shrinks rather than take the second one
     const int64_t alone = std::min<int64_t>((int64_t(max_smem_bytes) - fixed) / (pitch + 8) / 2, 8);
