@@ -28,6 +28,8 @@
 
 #include <cuda_bf16.h>
 
+#include <atomic>
+
 #include "tc_prim.cuh"
 
 namespace nep {
@@ -408,8 +410,17 @@ template <int kMode, int kTileTokens>
 cudaError_t launch_tile(const ExpertMaps& maps, const Args& args, int grid, cudaStream_t stream) {
     auto* fn = expert_gemm_kernel<kMode, kTileTokens>;
     using P = Pipe<kMode, kTileTokens>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(P::kSmemBytes));
+    // The limit is the same for every launch of this kernel: raised once per device (a second thread may do it again).
+    static std::atomic<uint64_t> raised{0};
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
+    const uint64_t bit = device < 64 ? uint64_t(1) << device : 0;
+    if ((raised.load(std::memory_order_acquire) & bit) == 0) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(P::kSmemBytes));
+        if (e != cudaSuccess) return e;
+        raised.fetch_or(bit, std::memory_order_release);
+    }
     cudaLaunchConfig_t config{};
     config.gridDim = dim3(unsigned(grid));
     config.blockDim = dim3(kThreads);

@@ -47,7 +47,6 @@ void check_bf16(const at::Tensor& t, int dims, const char* name) {
 
 struct GemmCommon {
     gemm::Args args{};
-    CUtensorMap map_a, map_b;
     int grid = 0;
 };
 
@@ -81,8 +80,9 @@ GemmCommon prepare(const at::Tensor& a, const at::Tensor& w, const at::Tensor& e
     }
     g.args.status = reinterpret_cast<uint32_t*>(status.data_ptr<int>());
     g.args.timeout_ns = uint64_t(timeout_s * 1e9);
-    if (rows > 0) g.map_a = make_map(a.data_ptr(), rows, K);
-    g.map_b = make_map(w.data_ptr(), E * NW, K);
+    // what a tensor map asks for, also where a call turns out to have nothing to do
+    TORCH_CHECK((rows == 0 || reinterpret_cast<uintptr_t>(a.data_ptr()) % 16 == 0) && reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0,
+                "TMA operand must be 16-byte aligned with 16-byte row pitch");
     const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
     g.grid = std::max(1, std::min(sms, g.args.m_blocks * g.args.n_tiles));
     return g;
@@ -97,12 +97,13 @@ cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& 
         g.args.expert_counts = counts->data_ptr<int64_t>();
     }
     const int64_t rows = a.size(0), K = a.size(1), E = w.size(0), NW = w.size(1);
-    gemm::ExpertMaps maps;
+    gemm::ExpertMaps maps{};
     maps.weights = mode == gemm::kSwiGLU ? make_map(w.data_ptr(), NW / 2, K, 16, 2 * E, 2) : make_map(w.data_ptr(), E * NW, K);
-    for (int b = 0; b < 4; ++b) maps.tokens[b] = make_map(a.data_ptr(), rows, K, 128 >> b);
     // A smaller token tile deepens the operand pipeline, which weights streamed from memory need (64 tokens over 32 experts of
     // 7168 x 2048: 287 us with tiles of 64 or 128, 302 with 256); more rows than that would only read the weights again.
     const int tile = max_expert_rows <= 0 || max_expert_rows > 128 ? 256 : max_expert_rows > 64 ? 128 : 64;
+    for (int b = 0; b < 4; ++b)
+        if ((128 >> b) <= tile / 2) maps.tokens[b] = make_map(a.data_ptr(), rows, K, 128 >> b);
     const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
     const int grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : sms;
     return gemm::launch_expert(maps, g.args, mode, tile, grid, c10::cuda::getCurrentCUDAStream().stream());
@@ -151,14 +152,15 @@ void bind_gemm(pybind11::module_& m) {
                 TORCH_CHECK(ee == cudaSuccess, "grouped GEMM (expert) launch failed: ", cudaGetErrorString(ee));
                 return;
             }
+            const CUtensorMap map_a = make_map(a.data_ptr(), a.size(0), a.size(1)), map_b = make_map(w.data_ptr(), w.size(0) * w.size(1), w.size(2));
             if (pair) {
                 const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
                 const int pair_grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : sms;
-                cudaError_t pe = gemm::launch_pair(g.map_a, g.map_b, g.args, int(mode), pair_grid, c10::cuda::getCurrentCUDAStream().stream());
+                cudaError_t pe = gemm::launch_pair(map_a, map_b, g.args, int(mode), pair_grid, c10::cuda::getCurrentCUDAStream().stream());
                 TORCH_CHECK(pe == cudaSuccess, "grouped GEMM (CTA pairs) launch failed: ", cudaGetErrorString(pe));
                 return;
             }
-            cudaError_t e = gemm::launch(g.map_a, g.map_b, g.args, int(mode), int(stages), grid, c10::cuda::getCurrentCUDAStream().stream());
+            cudaError_t e = gemm::launch(map_a, map_b, g.args, int(mode), int(stages), grid, c10::cuda::getCurrentCUDAStream().stream());
             TORCH_CHECK(e == cudaSuccess, "grouped GEMM launch failed: ", cudaGetErrorString(e));
         },
         pybind11::arg("a"), pybind11::arg("w"), pybind11::arg("expert_offsets"), pybind11::arg("out"), pybind11::arg("status"),

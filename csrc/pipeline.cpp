@@ -11,6 +11,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -164,12 +165,25 @@ void check_handle_meta(const std::vector<at::Tensor>& m, const WindowLayout& L, 
     check_meta_tensor(m[7], at::kInt, {expand ? capacity : 0}, device, "slot_map");
 }
 
+// An uninitialised tensor on `device`, and a contiguous piece of one (offset in elements): what empty() and narrow() +
+// view() give, without their way through the dispatcher (~1 us a call; a fresh dispatch makes a dozen of them per rank
+// before and after it waits for the counts).
+at::Tensor make_empty(at::IntArrayRef sizes, at::ScalarType dtype, int device) {
+    return at::Tensor(at::detail::empty_cuda(sizes, dtype, at::Device(at::kCUDA, at::DeviceIndex(device)), c10::nullopt));
+}
+at::Tensor part_of(const at::Tensor& base, int64_t offset, at::IntArrayRef sizes) {
+    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(base.storage()), base.key_set(), base.dtype());
+    t.unsafeGetTensorImpl()->set_storage_offset(base.storage_offset() + offset);
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    return t;
+}
+
 // Upload a host array of parameter blocks for a multi-rank launch.  The device buffer comes from the
 // comm stream's pool, so its reuse is ordered behind the launch that reads it.
 template <typename P>
 const P* upload(const std::vector<P>& host, std::vector<at::Tensor>& keep, cudaStream_t stream) {
     if (host.size() == 1) return host.data();
-    auto buf = at::empty({int64_t(host.size() * sizeof(P))}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA));
+    at::Tensor buf = make_empty({int64_t(host.size() * sizeof(P))}, at::kByte, at::cuda::current_device());
     cuda_check(cudaMemcpyAsync(buf.data_ptr(), host.data(), host.size() * sizeof(P), cudaMemcpyHostToDevice, stream), "parameter upload");
     keep.push_back(buf);
     return static_cast<const P*>(buf.data_ptr());
@@ -287,11 +301,6 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     // Outputs live in the consumer stream's pool: the caller's stream when the call completes on it,
     // the comm stream when completion is handed over through an event.
     const c10::cuda::CUDAStream consumer = async_op ? s.comm : s.compute;
-    const auto i64 = at::TensorOptions().dtype(at::kLong).device(at::kCUDA, device);
-    const auto i32 = at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device);
-    const auto f32 = at::TensorOptions().dtype(at::kFloat).device(at::kCUDA, device);
-    const auto bf16 = at::TensorOptions().dtype(at::kBFloat16).device(at::kCUDA, device);
-
     int64_t max_tokens_now = 0;
     for (int i = 0; i < n; ++i) max_tokens_now = std::max<int64_t>(max_tokens_now, xs[i].size(0));
     // A single-rank group exchanges nothing: a fresh dispatch plans in one launch that writes the handle's tensors itself
@@ -317,19 +326,19 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
                 // one allocation, six views: allocator calls sit on the host's critical path of a small fresh dispatch
                 m.resize(8);
                 const int64_t Le = L.local_experts, R = L.ranks, K = L.topk;
-                at::Tensor block = at::empty({Le + (Le + 1) + T * R + R + T * K + R}, i64);
+                const at::Tensor block = make_empty({Le + (Le + 1) + T * R + R + T * K + R}, at::kLong, device);
                 int64_t at_ = 0;
-                auto take = [&](int64_t count) {
-                    at::Tensor view = block.narrow(0, at_, count);
-                    at_ += count;
+                auto take = [&](at::IntArrayRef sizes) {
+                    at::Tensor view = part_of(block, at_, sizes);
+                    at_ += view.numel();
                     return view;
                 };
-                m[1] = take(Le);
-                m[2] = take(Le + 1);
-                m[3] = take(T * R).view({T, R});
-                m[4] = take(R);
-                m[5] = take(T * K).view({T, K});
-                m[6] = take(R);
+                m[1] = take({Le});
+                m[2] = take({Le + 1});
+                m[3] = take({T, R});
+                m[4] = take({R});
+                m[5] = take({T, K});
+                m[6] = take({R});
             } else {
                 m = cached_meta[i];
             }
@@ -396,9 +405,9 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             auto& m = out.metadata[0];
             const int64_t cells = bound_rows_n * (L.topk + 2), slots = expand ? bound_rows_c : 0;
             c10::cuda::CUDAStreamGuard pool(consumer);
-            at::Tensor block = at::empty({cells + slots}, i32);
-            m[0] = block.narrow(0, 0, cells).view({bound_rows_n, L.topk + 2});
-            m[7] = block.narrow(0, cells, slots);
+            const at::Tensor block = make_empty({cells + slots}, at::kInt, device);
+            m[0] = part_of(block, 0, {bound_rows_n, L.topk + 2});
+            m[7] = part_of(block, cells, {slots});
             LocalPlanParams lp{};
             const StageParams& sp = stage[0];
             lp.c = sp.c;
@@ -463,15 +472,17 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             auto& m = out.metadata[i];
             if (fresh && !plan_locally) {
                 const int64_t cells = N * (L.topk + 2), slots = expand ? C : 0;
-                at::Tensor block = at::empty({cells + slots}, i32);
-                m[0] = block.narrow(0, 0, cells).view({N, L.topk + 2});
-                m[7] = block.narrow(0, cells, slots);
+                const at::Tensor block = make_empty({cells + slots}, at::kInt, device);
+                m[0] = part_of(block, 0, {N, L.topk + 2});
+                m[7] = part_of(block, cells, {slots});
             }
             auto& o = out.outputs[i];
             o.resize(3);
-            o[0] = at::empty({expand ? C : N, L.hidden}, bf16);
-            o[1] = expand ? at::empty({0}, i64) : at::empty({N, L.topk}, i64);
-            o[2] = !weighted ? at::empty({0}, f32) : expand ? at::empty({C}, f32) : at::empty({N, L.topk}, f32);
+            o[0] = make_empty({expand ? C : N, L.hidden}, at::kBFloat16, device);
+            o[1] = expand ? make_empty({0}, at::kLong, device) : make_empty({N, L.topk}, at::kLong, device);
+            o[2] = !weighted ? make_empty({0}, at::kFloat, device)
+                   : expand ? make_empty({C}, at::kFloat, device)
+                            : make_empty({N, L.topk}, at::kFloat, device);
             PullParams& p = pull[i];
             p.c = stage[i].c;
             p.meta = fresh && !plan_locally ? reinterpret_cast<const int*>(static_cast<char*>(wins[i]->base()) + L.meta_scratch_offset) : m[0].data_ptr<int>();
@@ -553,16 +564,16 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             TORCH_CHECK(N <= bound_rows_n && (!expand || C <= bound_rows_c), "receive counts exceed the single-launch bound");
             out.counts[i] = {N, C};
             auto& o = out.outputs[i];
-            o[0] = o[0].narrow(0, 0, expand ? C : N);
-            if (!expand) o[1] = o[1].narrow(0, 0, N);
-            if (weighted) o[2] = o[2].narrow(0, 0, expand ? C : N);
+            o[0] = part_of(o[0], 0, {expand ? C : N, L.hidden});
+            if (!expand) o[1] = part_of(o[1], 0, {N, L.topk});
+            if (weighted) o[2] = expand ? part_of(o[2], 0, {C}) : part_of(o[2], 0, {N, L.topk});
         }
     }
     if (fuse_fresh || plan_locally) {
         for (int i = 0; i < n; ++i) {
             auto& m = out.metadata[i];
-            m[0] = m[0].narrow(0, 0, out.counts[i].first);
-            if (expand) m[7] = m[7].narrow(0, 0, out.counts[i].second);
+            m[0] = part_of(m[0], 0, {out.counts[i].first, L.topk + 2});
+            if (expand) m[7] = part_of(m[7], 0, {out.counts[i].second});
         }
     }
     std::vector<at::Tensor> inputs, results;
@@ -632,8 +643,6 @@ CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::T
     const Streams s = order_inputs(wins, comm_stream, previous_event, device, async_op);
     const c10::cuda::CUDAStream consumer = async_op ? s.comm : s.compute;
     const cudaStream_t cs = s.work.stream();
-    const auto f32 = at::TensorOptions().dtype(at::kFloat).device(at::kCUDA, device);
-    const auto bf16 = at::TensorOptions().dtype(at::kBFloat16).device(at::kCUDA, device);
 
     CombineOut out;
     out.outputs.resize(n);
@@ -646,8 +655,8 @@ CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::T
             const int64_t T = m[5].size(0);
             auto& o = out.outputs[0];
             o.resize(2);
-            o[0] = at::empty({T, L.hidden}, bf16);
-            o[1] = weighted ? at::empty({T, L.topk}, f32) : at::empty({0}, f32);
+            o[0] = make_empty({T, L.hidden}, at::kBFloat16, device);
+            o[1] = weighted ? make_empty({T, L.topk}, at::kFloat, device) : make_empty({0}, at::kFloat, device);
             p.c = wins[0]->common();
             p.y = reinterpret_cast<const __nv_bfloat16*>(xs[0].data_ptr());
             p.w = weighted ? weights[0]->data_ptr<float>() : nullptr;
@@ -689,8 +698,8 @@ CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::T
             const PeerWindow::CombineEpochs epochs = wins[i]->begin_combine();
             auto& o = out.outputs[i];
             o.resize(2);
-            o[0] = at::empty({T, L.hidden}, bf16);
-            o[1] = weighted ? at::empty({T, L.topk}, f32) : at::empty({0}, f32);
+            o[0] = make_empty({T, L.hidden}, at::kBFloat16, device);
+            o[1] = weighted ? make_empty({T, L.topk}, at::kFloat, device) : make_empty({0}, at::kFloat, device);
             CombineParams& p = params[i];
             p.c = wins[i]->common();
             p.y = reinterpret_cast<const __nv_bfloat16*>(xs[i].data_ptr());
@@ -783,7 +792,7 @@ std::vector<at::Tensor> combine_finish(const std::vector<PeerWindow*>& wins, con
         barrier[i].c = wins[i]->common();
         barrier[i].epoch = wins[i]->reserve_epochs(1);
         TORCH_CHECK(L.ret_parts == L.topk, "this buffer's return area holds one partition per rank only");
-        outs[i] = at::empty({T, L.hidden}, at::TensorOptions().dtype(at::kBFloat16).device(at::kCUDA, device));
+        outs[i] = make_empty({T, L.hidden}, at::kBFloat16, device);
         ReduceParams& r = reduce[i];
         r.c = barrier[i].c;
         r.topk = meta[i][5].data_ptr<int64_t>();
