@@ -2018,10 +2018,6 @@ CombinePlan plan_combine(int64_t row_bytes, int parts, int max_smem_bytes, int r
         // about half of shared memory for the pipeline unless the caller names a chunk; whole rows when they fit
         chunk = reduce_chunk_bytes > 0 ? align_up(reduce_chunk_bytes, 128) : (int64_t(max_smem_bytes) / 2 / reduce_stages / parts) / 128 * 128;
         chunk = std::min<int64_t>(chunk, pitch);
-        // whole rows that leave room in that half: more tokens in flight
-        while (reduce_chunk_bytes <= 0 && chunk == pitch && reduce_stages < 4 &&
-               (reduce_stages + 1) * parts * chunk <= int64_t(max_smem_bytes) / 2)
-            ++reduce_stages;
     }
     // transfer warps the rings would get without a pipeline: an automatic chunk shrinks rather than take the second one
     const int64_t alone = std::min<int64_t>((int64_t(max_smem_bytes) - fixed) / (pitch + 8) / 2, 8);

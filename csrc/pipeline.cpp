@@ -633,7 +633,11 @@ CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::T
     // How the source-side sum runs: a positive setting = register path with that many warps per token; a negative one
     // = shared-memory pipeline, -(stages * 1000 + chunk bytes / 128) with chunk 0 = chosen by the plan; 0 = default.
     const int reduce_setting = g_trace.group != 0 ? g_trace.group : kDefaultReduceSetting;
-    const int pipe_stages = reduce_setting < 0 ? (-reduce_setting) / 1000 : 0;
+    int pipe_stages = reduce_setting < 0 ? (-reduce_setting) / 1000 : 0;
+    // by default whole rows that leave room in the pipeline's half of shared memory: more tokens in flight
+    const int64_t token_bytes = (int64_t(L.hidden) * 2 + 127) / 128 * 128 * L.ret_parts;
+    if (g_trace.group == 0)
+        while (pipe_stages < 4 && (pipe_stages + 1) * token_bytes <= lim.smem_optin / 2) ++pipe_stages;
     const int pipe_chunk = reduce_setting < 0 ? ((-reduce_setting) % 1000) * 128 : 0;
     const CombinePlan plan = plan_combine(int64_t(L.hidden) * 2, L.ret_parts, lim.smem_optin, pipe_stages, pipe_chunk);
     const RingPlan ring = plan.ring;
