@@ -1866,17 +1866,21 @@ __global__ void gate_kernel(volatile int* gate, uint64_t timeout_ns) {
 }
 
 // ---------------------------------------------------------------- wrappers
+template <typename P>
+__device__ __forceinline__ const P& block_of(const Many<P>& all) {
+    return all.device != nullptr ? all.device[blockIdx.y] : all.host[blockIdx.y];
+}
 #define NEP_KERNEL_PAIR(name, Params, ...)                                                                          \
     __global__ void __launch_bounds__(__VA_ARGS__) name##_kernel(const __grid_constant__ Params p) { name##_body(p); } \
-    __global__ void __launch_bounds__(__VA_ARGS__) name##_multi_kernel(const Params* all) { name##_body(all[blockIdx.y]); }
+    __global__ void __launch_bounds__(__VA_ARGS__) name##_multi_kernel(const __grid_constant__ Many<Params> all) { name##_body(block_of(all)); }
 
 __global__ void __launch_bounds__(kStageThreads) stage_kernel(const __grid_constant__ StageParams p) { stage_body(p); }
-__global__ void __launch_bounds__(kStageThreads) stage_multi_kernel(const StageParams* all) { stage_body(all[blockIdx.y]); }
+__global__ void __launch_bounds__(kStageThreads) stage_multi_kernel(const __grid_constant__ Many<StageParams> all) { stage_body(block_of(all)); }
 __global__ void __launch_bounds__(kLocalPlanThreads) local_plan_kernel(const __grid_constant__ LocalPlanParams p) { local_plan_body(p); }
 NEP_KERNEL_PAIR(plan, PlanParams, kPlanThreads)
 NEP_KERNEL_PAIR(pull, PullParams, 256)
 __global__ void __launch_bounds__(kCombineThreads, 1) combine_kernel(const __grid_constant__ CombineParams p) { combine_body(p); }
-__global__ void __launch_bounds__(kCombineThreads, 1) combine_multi_kernel(const CombineParams* all) { combine_body(all[blockIdx.y]); }
+__global__ void __launch_bounds__(kCombineThreads, 1) combine_multi_kernel(const __grid_constant__ Many<CombineParams> all) { combine_body(block_of(all)); }
 NEP_KERNEL_PAIR(reduce, ReduceParams, kRowSumThreads, kRowSumBlocks)
 NEP_KERNEL_PAIR(barrier, BarrierParams, 32)
 NEP_KERNEL_PAIR(local_combine, LocalCombineParams, kRowSumThreads, kRowSumBlocks)
@@ -1906,8 +1910,10 @@ __global__ void __launch_bounds__(256) fused_fresh_dispatch_kernel(const __grid_
                                                                    const __grid_constant__ PullParams pp) {
     fused_fresh_dispatch_body(sp, lp, pp);
 }
-__global__ void __launch_bounds__(256) fused_fresh_dispatch_multi_kernel(const StageParams* sp, const PlanParams* lp, const PullParams* pp) {
-    fused_fresh_dispatch_body(sp[blockIdx.y], lp[blockIdx.y], pp[blockIdx.y]);
+__global__ void __launch_bounds__(256) fused_fresh_dispatch_multi_kernel(const __grid_constant__ Many<StageParams> sp,
+                                                                         const __grid_constant__ Many<PlanParams> lp,
+                                                                         const __grid_constant__ Many<PullParams> pp) {
+    fused_fresh_dispatch_body(block_of(sp), block_of(lp), block_of(pp));
 }
 
 // stage + peer barrier + pull in one cooperative launch (cached dispatch, small calls)
@@ -1916,10 +1922,11 @@ __global__ void __launch_bounds__(256) fused_cached_dispatch_kernel(const __grid
     fence_proxy_async();
     pull_body(pp);
 }
-__global__ void __launch_bounds__(256) fused_cached_dispatch_multi_kernel(const StageParams* sp, const PullParams* pp) {
-    if (!stage_body(sp[blockIdx.y])) return;
+__global__ void __launch_bounds__(256) fused_cached_dispatch_multi_kernel(const __grid_constant__ Many<StageParams> sp,
+                                                                          const __grid_constant__ Many<PullParams> pp) {
+    if (!stage_body(block_of(sp))) return;
     fence_proxy_async();
-    pull_body(pp[blockIdx.y]);
+    pull_body(block_of(pp));
 }
 
 // Raises a kernel's dynamic shared-memory limit when a launch needs more than it was granted so far.  The limit belongs
@@ -1962,8 +1969,18 @@ cudaError_t launch_dependent(void (*fn)(const Params), const Params& params, int
     return cudaLaunchKernelEx(&config, fn, params);
 }
 
+template <typename P>
+Many<P> make_many(const P* params, int ranks) {
+    Many<P> many{};
+    if (ranks > kInlineRanks)
+        many.device = params;
+    else
+        for (int r = 0; r < ranks; ++r) many.host[r] = params[r];
+    return many;
+}
+
 template <typename Params>
-cudaError_t launch_pair(void (*single)(const Params), void (*multi)(const Params*), const Params* params, LaunchShape shape, int threads,
+cudaError_t launch_pair(void (*single)(const Params), void (*multi)(const Many<Params>), const Params* params, LaunchShape shape, int threads,
                         size_t smem, cudaStream_t stream) {
     if (smem > 48 * 1024) {
         const cudaError_t e = allow_shared_memory(shape.ranks_y > 1 ? (const void*)multi : (const void*)single, smem);
@@ -1971,7 +1988,7 @@ cudaError_t launch_pair(void (*single)(const Params), void (*multi)(const Params
     }
     const dim3 grid(shape.grid_x, shape.ranks_y > 1 ? shape.ranks_y : 1);
     if (shape.ranks_y > 1)
-        multi<<<grid, threads, smem, stream>>>(params);
+        multi<<<grid, threads, smem, stream>>>(make_many(params, shape.ranks_y));
     else
         single<<<grid, threads, smem, stream>>>(*params);
     return cudaGetLastError();
@@ -2082,54 +2099,51 @@ cudaError_t launch_barrier(const BarrierParams* params, LaunchShape shape, cudaS
 }
 
 namespace {
-// Cooperative launch of a two-parameter-block kernel: fails instead of deadlocking if the grid cannot be resident at once.
-cudaError_t launch_cooperative(const void* single, const void* multi_fn, const void* first, const void* second, LaunchShape shape, int warps,
-                               size_t smem, cudaStream_t stream) {
-    const bool multi = shape.ranks_y > 1;
-    const void* fn = multi ? multi_fn : single;
+// Cooperative launch: fails instead of deadlocking if the grid cannot be resident at once.
+cudaError_t launch_cooperative(const void* fn, void** args, LaunchShape shape, int threads, size_t smem, cudaStream_t stream) {
     if (smem > 48 * 1024) {
         const cudaError_t e = allow_shared_memory(fn, smem);
         if (e != cudaSuccess) return e;
     }
-    const dim3 grid(shape.grid_x, multi ? shape.ranks_y : 1);
-    // multi: the kernel takes the two device arrays; single: the two blocks by value
-    void* args_multi[2] = {(void*)&first, (void*)&second};
-    void* args_single[2] = {(void*)first, (void*)second};
-    return cudaLaunchCooperativeKernel(fn, grid, dim3(warps * 32), multi ? args_multi : args_single, smem, stream);
+    return cudaLaunchCooperativeKernel(fn, dim3(shape.grid_x, shape.ranks_y > 1 ? shape.ranks_y : 1), dim3(threads), args, smem, stream);
 }
+static_assert(sizeof(Many<StageParams>) + sizeof(Many<PlanParams>) + sizeof(Many<PullParams>) <= 32764, "kernel parameters");
 }  // namespace
 
 cudaError_t launch_fused_cached_dispatch(const StageParams* stage, const PullParams* pull, LaunchShape shape, int warps, size_t smem,
                                          cudaStream_t stream) {
-    return launch_cooperative((const void*)fused_cached_dispatch_kernel, (const void*)fused_cached_dispatch_multi_kernel, stage, pull, shape,
-                              warps, smem, stream);
+    if (shape.ranks_y <= 1) {
+        void* args[2] = {(void*)stage, (void*)pull};
+        return launch_cooperative((const void*)fused_cached_dispatch_kernel, args, shape, warps * 32, smem, stream);
+    }
+    auto sp = make_many(stage, shape.ranks_y);
+    auto pp = make_many(pull, shape.ranks_y);
+    void* args[2] = {&sp, &pp};
+    return launch_cooperative((const void*)fused_cached_dispatch_multi_kernel, args, shape, warps * 32, smem, stream);
 }
 
 cudaError_t launch_fused_fresh_dispatch(const StageParams* stage, const PlanParams* plan, const PullParams* pull, LaunchShape shape, int warps,
                                         size_t smem, cudaStream_t stream) {
-    const bool multi = shape.ranks_y > 1;
-    const void* fn = multi ? (const void*)fused_fresh_dispatch_multi_kernel : (const void*)fused_fresh_dispatch_kernel;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = allow_shared_memory(fn, smem);
-        if (e != cudaSuccess) return e;
+    if (shape.ranks_y <= 1) {
+        void* args[3] = {(void*)stage, (void*)plan, (void*)pull};
+        return launch_cooperative((const void*)fused_fresh_dispatch_kernel, args, shape, warps * 32, smem, stream);
     }
-    const dim3 grid(shape.grid_x, multi ? shape.ranks_y : 1);
-    void* args_multi[3] = {(void*)&stage, (void*)&plan, (void*)&pull};
-    void* args_single[3] = {(void*)stage, (void*)plan, (void*)pull};
-    return cudaLaunchCooperativeKernel(fn, grid, dim3(warps * 32), multi ? args_multi : args_single, smem, stream);
+    auto sp = make_many(stage, shape.ranks_y);
+    auto lp = make_many(plan, shape.ranks_y);
+    auto pp = make_many(pull, shape.ranks_y);
+    void* args[3] = {&sp, &lp, &pp};
+    return launch_cooperative((const void*)fused_fresh_dispatch_multi_kernel, args, shape, warps * 32, smem, stream);
 }
 
 cudaError_t launch_combine(const CombineParams* params, LaunchShape shape, size_t smem, cudaStream_t stream, bool cooperative) {
     if (!cooperative) return launch_pair<CombineParams>(combine_kernel, combine_multi_kernel, params, shape, kCombineThreads, smem, stream);
-    const bool multi = shape.ranks_y > 1;
-    const void* fn = multi ? (const void*)combine_multi_kernel : (const void*)combine_kernel;
-    if (smem > 48 * 1024) {
-        const cudaError_t e = allow_shared_memory(fn, smem);
-        if (e != cudaSuccess) return e;
+    if (shape.ranks_y <= 1) {
+        void* args[1] = {(void*)params};
+        return launch_cooperative((const void*)combine_kernel, args, shape, kCombineThreads, smem, stream);
     }
-    const dim3 grid(shape.grid_x, multi ? shape.ranks_y : 1);
-    void* args[1] = {multi ? (void*)&params : (void*)params};
-    return cudaLaunchCooperativeKernel(fn, grid, dim3(kCombineThreads), args, smem, stream);
+    auto all = make_many(params, shape.ranks_y);
+    void* args[1] = {&all};
+    return launch_cooperative((const void*)combine_multi_kernel, args, shape, kCombineThreads, smem, stream);
 }
 
 cudaError_t launch_gate(int* gate, uint64_t timeout_ns, cudaStream_t stream) {

@@ -1,9 +1,10 @@
 // Parameter blocks and launch entry points of the dispatch/combine kernels (torch-free).
 //
 // Every kernel exists as one device body with two __global__ wrappers: the production wrapper
-// takes the parameter block by value for one rank; the multi-rank wrapper reads the block of
-// logical rank blockIdx.y from a device array, so a whole group can run as ONE launch on one GPU
-// (ranks that wait on one another must never be separate launches on the same device).
+// takes the parameter block by value for one rank; the multi-rank wrapper runs logical rank blockIdx.y,
+// so a whole group can run as ONE launch on one GPU (ranks that wait on one another must never be
+// separate launches on the same device).  Its blocks come by value too for up to kInlineRanks ranks and
+// from a device array beyond.
 //
 // Protocol (differs from the reference's push + epilogue design, csrc/dispatch_main.cuh:356-453):
 //   dispatch = stage (copy tokens into the own window, count, exchange counts, peer barrier)
@@ -28,6 +29,15 @@ struct CommonParams {
     uint64_t timeout_ns;
     uint32_t* status_dev;
     volatile uint32_t* status_host;
+};
+
+// Ranks whose parameter blocks a multi-rank launch takes by value.  An upload in front of the launch costs a pageable copy and
+// an allocation on the host and 4 us on the device, four times in a round trip: eight ranks of 16 tokens 164 -> 152 us.
+constexpr int kInlineRanks = 8;
+template <typename P>
+struct Many {
+    const P* device;  // null: the blocks are in `host`
+    P host[kInlineRanks];
 };
 
 struct StageParams {
@@ -189,11 +199,11 @@ struct BarrierParams {
 
 struct LaunchShape {
     int grid_x;
-    int ranks_y;  // 1 = production wrapper, >1 = multi-rank wrapper (params is then a device array)
+    int ranks_y;  // 1 = production wrapper, >1 = multi-rank wrapper (its blocks: see kInlineRanks)
 };
 
 // Each returns the CUDA error of the launch.  `params` points to one block (ranks_y == 1, host
-// memory) or to a device array of ranks_y blocks.
+// memory) or to ranks_y of them, in host memory up to kInlineRanks and in device memory beyond.
 cudaError_t launch_stage(const StageParams* params, LaunchShape shape, size_t smem, cudaStream_t stream);
 cudaError_t launch_plan(const PlanParams* params, LaunchShape shape, size_t smem, cudaStream_t stream);
 bool local_plan_fits(const WindowLayout& l, int64_t tokens);

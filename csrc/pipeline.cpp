@@ -178,11 +178,11 @@ at::Tensor part_of(const at::Tensor& base, int64_t offset, at::IntArrayRef sizes
     return t;
 }
 
-// Upload a host array of parameter blocks for a multi-rank launch.  The device buffer comes from the
-// comm stream's pool, so its reuse is ordered behind the launch that reads it.
+// Parameter blocks of a launch: passed by value, from the host array, for as many ranks as fit; uploaded for more.  The device
+// buffer comes from the comm stream's pool, so its reuse is ordered behind the launch that reads it.
 template <typename P>
 const P* upload(const std::vector<P>& host, std::vector<at::Tensor>& keep, cudaStream_t stream) {
-    if (host.size() == 1) return host.data();
+    if (host.size() <= size_t(kInlineRanks)) return host.data();
     at::Tensor buf = make_empty({int64_t(host.size() * sizeof(P))}, at::kByte, at::cuda::current_device());
     cuda_check(cudaMemcpyAsync(buf.data_ptr(), host.data(), host.size() * sizeof(P), cudaMemcpyHostToDevice, stream), "parameter upload");
     keep.push_back(buf);

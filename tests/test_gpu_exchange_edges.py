@@ -98,3 +98,25 @@ def test_single_rank_plan(tokens, experts, topk, kind):
             group.check_status()
             assert_dispatch_matches(got[0], case.xs, case.indices, case.weights, case.num_experts, 0, expand=expand, alignment=alignment,
                                     zero_padding=True)
+
+
+@pytest.mark.parametrize("world", [8, 16])  # parameter blocks by value, and from device memory
+def test_many_logical_ranks(world):
+    case = make_case(world, kind="mixed", seed=world, hidden=512, tokens=9, experts_per_rank=3, topk=4)
+    cfg = EPConfig(case.num_experts, case.num_topk, case.hidden, case.capacity)
+    with EmulatedGroup(world, cfg) as group:
+        first = group.dispatch(_cuda(case.xs), topk_idx=_cuda(case.indices), weights=_cuda(case.weights), do_expand=True, alignment=8, zero_padding=True)
+        again = group.dispatch(_cuda(case.xs), handles=[f.handle for f in first], weights=_cuda(case.weights), zero_padding=True)
+        back = [group.combine([g.x for g in got], [g.handle for g in got], weights=[g.topk_weights for g in got]) for got in (first, again)]
+        torch.cuda.synchronize()
+        group.check_status()
+        for got in (first, again):
+            for r in range(world):
+                assert_dispatch_matches(got[r], case.xs, case.indices, case.weights, case.num_experts, r, expand=True, alignment=8, zero_padding=True)
+        for r in range(world):
+            idx, x = case.indices[r], case.xs[r].float()
+            # the sum of up to four equal bf16 values is exact in FP32 and rounded once
+            want = (x * (idx >= 0).sum(-1, keepdim=True)).to(torch.bfloat16)
+            for b in back:
+                assert torch.equal(b[r].x.cpu(), want)
+                assert torch.equal(b[r].topk_weights.cpu(), torch.where(idx >= 0, case.weights[r], 0.0))
