@@ -99,9 +99,13 @@ cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& 
     const int64_t rows = a.size(0), K = a.size(1), E = w.size(0), NW = w.size(1);
     gemm::ExpertMaps maps{};
     maps.weights = mode == gemm::kSwiGLU ? make_map(w.data_ptr(), NW / 2, K, 16, 2 * E, 2) : make_map(w.data_ptr(), E * NW, K);
-    // A smaller token tile deepens the operand pipeline, which weights streamed from memory need (64 tokens over 32 experts of
-    // 7168 x 2048: 287 us with tiles of 64 or 128, 302 with 256); more rows than that would only read the weights again.
-    const int tile = max_expert_rows <= 0 || max_expert_rows > 128 ? 256 : max_expert_rows > 64 ? 128 : 64;
+    // A smaller token tile deepens the operand pipeline, which weights streamed from memory need; more rows than a tile holds
+    // read the weights again, from L2.  Experts of 7168 x 2048, 32 of them, up-projection with tiles of 64, 128 and 256: 64
+    // tokens 283, 287 and 302 us; 256 tokens (at most 78 rows an expert) 324, 293 and 310-329 us; 512 tokens (at most 158) 526,
+    // 374 and 319 us.  So: the smallest tile that no expert can outgrow, and 128 also where every expert has at most one
+    // block of 128 rows on average and none can hold more than four.
+    const bool one_block = max_expert_rows <= 512 && rows <= 128 * E;
+    const int tile = max_expert_rows <= 0 ? 256 : max_expert_rows <= 64 ? 64 : max_expert_rows <= 128 || one_block ? 128 : 256;
     for (int b = 0; b < 4; ++b)
         if ((128 >> b) <= tile / 2) maps.tokens[b] = make_map(a.data_ptr(), rows, K, 128 >> b);
     const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;

@@ -27,7 +27,7 @@ def _problem(counts, K, N):
 
 
 @pytest.mark.parametrize("swiglu", [False, True])
-@pytest.mark.parametrize("largest", [0, 64, 128])  # token tile 256, 64 and 128: larger experts are split
+@pytest.mark.parametrize("largest", [0, 64, 128, 300])  # token tile 256, 64 and 128 (300: where the experts are small); larger experts are split
 @pytest.mark.parametrize("counts,K,N", [([1], 64, 256), ([31, 32, 0, 33, 64], 512, 512), ([0, 129, 255, 256, 257, 0], 256, 768), ([1000, 5, 2304], 1024, 256)])
 def test_rows_that_exist(counts, K, N, largest, swiglu):
     """Padding rows hold NaN and must not reach a real row; rows of experts end anywhere inside a tile."""
