@@ -83,14 +83,16 @@ def gemm_only(args, device):
     w2 = (torch.randn(local, args.hidden, args.inter, device=device) * 0.02).to(torch.bfloat16)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=device)
     h = gg.grouped_gemm(a, w13, offsets, swiglu=True)
+    full = torch.full((rows // 128,), 128, dtype=torch.int32, device=device)
+    gated = dict(tile_ready=full, tile_expected=full)  # the kernels of gated row blocks, every counter full
     out = {}
     for name, fn, flops in (
         ("up_swiglu", lambda: gg.grouped_gemm(a, w13, offsets, swiglu=True), 2.0 * rows * args.hidden * 2 * args.inter),
-        ("up_swiglu_3stage", lambda: gg.grouped_gemm(a, w13, offsets, swiglu=True, stages=3), 2.0 * rows * args.hidden * 2 * args.inter),
-        ("up_swiglu_pair", lambda: gg.grouped_gemm(a, w13, offsets, swiglu=True, pair=True), 2.0 * rows * args.hidden * 2 * args.inter),
-        ("down_pair", lambda: gg.grouped_gemm(h, w2, offsets, pair=True), 2.0 * rows * args.hidden * args.inter),
+        ("up_swiglu_gated_3stage", lambda: gg.grouped_gemm(a, w13, offsets, swiglu=True, stages=3, **gated), 2.0 * rows * args.hidden * 2 * args.inter),
+        ("up_swiglu_gated_pair", lambda: gg.grouped_gemm(a, w13, offsets, swiglu=True, pair=True, **gated), 2.0 * rows * args.hidden * 2 * args.inter),
+        ("down_gated_pair", lambda: gg.grouped_gemm(h, w2, offsets, pair=True, **gated), 2.0 * rows * args.hidden * args.inter),
         ("down", lambda: gg.grouped_gemm(h, w2, offsets), 2.0 * rows * args.hidden * args.inter),
-        ("down_3stage", lambda: gg.grouped_gemm(h, w2, offsets, stages=3), 2.0 * rows * args.hidden * args.inter),
+        ("down_gated_3stage", lambda: gg.grouped_gemm(h, w2, offsets, stages=3, **gated), 2.0 * rows * args.hidden * args.inter),
         ("cublas_up", lambda: torch.bmm(a.view(local, rows_per, args.hidden), w13.transpose(1, 2)), 2.0 * rows * args.hidden * 2 * args.inter),
         ("cublas_down", lambda: torch.bmm(h.view(local, rows_per, args.inter), w2.transpose(1, 2)), 2.0 * rows * args.hidden * args.inter),
     ):

@@ -45,9 +45,11 @@ def run_gemm():
     for _ in range(2):
         h = gg.grouped_gemm(a, w13, offsets, swiglu=True)
         y = gg.grouped_gemm(h, w2, offsets)
-    for _ in range(2):  # CTA-pair kernels (tcgen05 cta_group::2)
-        h = gg.grouped_gemm(a, w13, offsets, swiglu=True, pair=True)
-        y = gg.grouped_gemm(h, w2, offsets, pair=True)
+    full = torch.full((experts * rows_per // 128,), 128, dtype=torch.int32, device="cuda")
+    gated = dict(tile_ready=full, tile_expected=full)
+    for _ in range(2):  # the kernels of gated row blocks: CTA pairs (every counter is full here)
+        h = gg.grouped_gemm(a, w13, offsets, swiglu=True, pair=True, **gated)
+        y = gg.grouped_gemm(h, w2, offsets, pair=True, **gated)
     torch.cuda.synchronize()
     gg.check_status()
     print("gemm rows", a.shape[0], "flops up", 2 * a.shape[0] * H * 2 * I, "down", 2 * a.shape[0] * H * I)
