@@ -697,7 +697,9 @@ __device__ void pull_body(const PullParams& p) {
     const WindowLayout& L = p.c.layout;
     const int R = L.ranks, K = L.topk, H = L.hidden, Le = L.local_experts;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const int gw = blockIdx.x * wpb + warp, GW = gridDim.x * wpb;
+    // neighbouring rows go to different SMs: 32 rows to eight slots each leave through 32 of them instead of 7 (12.5 -> 5.2 us,
+    // 64 rows 18.3 -> 11.3, 4096 rows 131-136 -> 129)
+    const int gw = warp * gridDim.x + blockIdx.x, GW = gridDim.x * wpb;
     const int64_t rb = L.row_bytes();
     const StatusRef status = status_of(p.c);
     const int MW = K + 2;
