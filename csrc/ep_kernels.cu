@@ -76,6 +76,16 @@ __device__ bool wait_go(int* ctrl, uint64_t epoch, uint64_t timeout_ns, StatusRe
     return s_go != 0;
 }
 
+// Receive counts to the host, which returns from the dispatch with them.  Later kernels of this stream see everything else
+// that this kernel writes, so no fence stands here in general.  A gated dispatch is the exception: its consumer runs on
+// another stream and reads expert_offsets and expert_counts as soon as the host has the counts, ordered behind nothing but
+// the mailbox.  Called by the thread that has observed (block or warp barrier) all of the block's writes to those two.
+__device__ __forceinline__ void publish_counts(volatile int64_t* mailbox, int64_t rows, int64_t capacity, bool gated) {
+    if (gated) __threadfence_system();
+    mailbox[1] = capacity;
+    mailbox[0] = rows;
+}
+
 // ------------------------------------------------------------------------------------------
 // stage: copy this rank's tokens (x + gate weights) into its own window, snapshot and count the
 // routing, send the per-destination counts to the peers, peer barrier, derive N / C / offsets.
@@ -238,9 +248,8 @@ __device__ bool stage_body(const StageParams& p) {
             return false;
         }
         const int* in = reinterpret_cast<const int*>(win + L.counts_in_offset + int64_t(p.parity) * L.counts_in_stride);
-        // The host waits for what follows: loads are issued in groups, not one behind the other, and only N and C go into the
-        // mailbox (everything else is for later kernels of this stream), so no fence stands before or after it.
-        // Eight ranks of 16 tokens: counts in the mailbox 20 -> 14 us after the kernel's start.
+        // The host waits for what follows: loads are issued in groups, not one behind the other, and the mailbox is written
+        // before the chunk prefixes.  Eight ranks of 16 tokens: counts in the mailbox 20 -> 14 us after the kernel's start.
         // Phase 1 (all threads): per local expert, sum the sources' counts and round up to the alignment.
         // The padded sizes reuse the dynamic shared array (R + E ints >= L ints).
         int* s_padded = s_counts;
@@ -289,11 +298,11 @@ __device__ bool stage_body(const StageParams& p) {
                 carry += __shfl_sync(kFull, incl, 31);
             }
             if (lane == 0) {
-                p.mailbox[1] = carry;
-                p.mailbox[0] = s_rows;
                 p.expert_offsets[Le] = carry;
                 ctrl[L.ctrl_expert_offsets() + Le] = carry;
             }
+            __syncwarp();  // the other lanes' offsets; the counts are behind the block barrier above
+            if (lane == 0) publish_counts(p.mailbox, s_rows, carry, p.gated != 0);
         }
         // Every source's per-chunk row counts become exclusive prefixes: chunk c of source s starts at receive row
         // recv_prefix[s] + chunk_prefix[s][c].  The total must equal the source's announced row count.
@@ -473,13 +482,13 @@ __device__ void local_plan_body(const LocalPlanParams& p) {
         if (lane == 0) {
             s_capacity = carry;
             if (cta == 0) {
-                p.mailbox[1] = carry;
-                p.mailbox[0] = s_all;
                 p.expert_offsets[E] = carry;
                 p.recv_rank_prefix[0] = s_all;
                 p.send_counts[0] = s_all;
             }
         }
+        __syncwarp();  // the other lanes' offsets; the counts are behind the block barrier above
+        if (lane == 0 && cta == 0) publish_counts(p.mailbox, s_all, carry, p.gated != 0);
     }
     __syncthreads();
     // ---- assign rows and slots

@@ -51,6 +51,7 @@ struct StageParams {
     int alignment;
     int skip_copy;  // single-rank groups: the pull reads x directly, nothing is staged
     int fused;      // stage + pull in one launch: blocks wait for the barrier result instead of exiting
+    int gated;      // a consumer on another stream reads expert_offsets / expert_counts once the host has N and C
     uint64_t epoch;
     // handle tensors written by a fresh dispatch
     int64_t* snapshot;          // [T,K] copy of topk
@@ -78,6 +79,7 @@ struct LocalPlanParams {
     int tokens;
     int expand;
     int alignment;
+    int gated;  // as in StageParams
     // handle tensors (as in StageParams); `meta` has room for T rows, `slot_map` for the largest possible capacity
     int64_t* snapshot;
     int64_t* dst_slots;

@@ -307,6 +307,9 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     // (allocated at their upper bounds and trimmed), a cached one goes straight to the pull.
     const bool local = L.ranks == 1;
     const bool plan_locally = local && fresh && local_plan_fits(L, max_tokens_now);
+    // The caller starts a consumer on another stream as soon as this call returns (see dispatch() in Python).
+    bool gated = false;
+    for (const auto& t : tile_ready) gated = gated || t.has_value();
 
     DispatchOut out;
     out.metadata.resize(n);
@@ -353,6 +356,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             p.parity = parity[i];
             p.alignment = int(alignment);
             p.skip_copy = local ? 1 : 0;
+            p.gated = gated;
             p.epoch = wins[i]->reserve_epochs(1);
             if (fresh) {
                 p.snapshot = m[5].data_ptr<int64_t>();
@@ -372,8 +376,6 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         }
     }
     // Small cached calls: stage, peer barrier and pull go out as ONE cooperative launch.
-    bool gated = false;
-    for (const auto& t : tile_ready) gated = gated || t.has_value();
     const bool fuse_small = !fresh && !gated && !local && max_tokens_now <= fused_dispatch_max_tokens();
     // Small fresh calls: stage, plan and pull as ONE cooperative launch writing into outputs sized at an upper bound
     // (every rank may send all of its Tmax tokens here), trimmed to N / C once the mailbox has them.  Only when that
@@ -415,6 +417,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             lp.tokens = sp.tokens;
             lp.expand = expand;
             lp.alignment = sp.alignment;
+            lp.gated = sp.gated;
             lp.snapshot = sp.snapshot;
             lp.dst_slots = sp.dst_slots;
             lp.send_counts = sp.send_counts;

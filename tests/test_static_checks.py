@@ -106,3 +106,30 @@ def test_nvtx_range_is_a_shared_noop_when_disabled():
         assert tracing.nvtx_range("a") is tracing.nvtx_range("b")
     with tracing.nvtx_range("anything"):
         pass
+
+
+def _body(text, name):
+    """Brace-matched body of the function whose definition starts at ``name(``."""
+    start = text.index("{", text.index(f"{name}("))
+    depth = 0
+    for i in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[start : i + 1]
+    raise AssertionError(name)
+
+
+def test_receive_counts_follow_the_offsets_a_gated_consumer_reads():
+    """A GEMM gated by tile counters runs on another stream and reads expert_offsets once the host has N and C, ordered by
+    nothing but the mailbox: both planning kernels finish those tensors first and a gated dispatch fences in between."""
+    text = re.sub(r"//[^\n]*", "", (ROOT / "csrc" / "ep_kernels.cu").read_text())
+    publish = _body(text, "void publish_counts")
+    assert re.search(r"if \(gated\) __threadfence_system\(\);.*mailbox\[1\] = .*mailbox\[0\] = ", publish, re.S)
+    assert set(re.findall(r"mailbox\[[01]\] = ([^;]+);", text.replace(publish, ""))) == {"-2"}, "only the failure code goes another way"
+    for kernel in ("bool stage_body", "void local_plan_body"):
+        body = _body(text, kernel)
+        assert body.count("publish_counts(") == 1 and re.search(r"__syncwarp\(\);\s*if \(lane == 0[^)]*\) publish_counts\([^;]*p\.gated", body)
+        after = body[body.index("publish_counts(") :]
+        assert not re.search(r"p\.expert_(offsets|counts)\[[^\]]*\] = ", after), kernel
+    host = (ROOT / "csrc" / "pipeline.cpp").read_text()
+    assert re.search(r"gated = gated \|\| t\.has_value\(\);.*p\.gated = gated;.*lp\.gated = sp\.gated;", host, re.S)
