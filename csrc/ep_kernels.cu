@@ -1430,8 +1430,7 @@ __device__ __forceinline__ char* reduce_area(const CombineParams& p, char* smem)
 // keeps no registers busy, so all partitions of a chunk are in flight at once and several chunks ahead: what is left
 // of the kernel after the last row has landed is one load latency and a sum from shared memory, where the register
 // path needs seven dependent batches of loads per token.
-__device__ void combine_reduce_smem_role(const CombineParams& p, int* flow, char* area) {
-    int* abort_word = flow;
+__device__ void combine_reduce_smem_role(const CombineParams& p, int* abort_word, char* area) {
     const WindowLayout& L = p.c.layout;
     const int K = L.topk, Le = L.local_experts, E = int(L.num_experts), H = L.hidden, P = L.ret_parts;
     const int lane = threadIdx.x & 31;
@@ -1440,9 +1439,10 @@ __device__ void combine_reduce_smem_role(const CombineParams& p, int* flow, char
     const int CW = RW - 1;  // consumer warps
     const int NS = p.reduce_stages, cw = p.reduce_chunk_bytes, xb = H * 2;
     const int nc = (xb + cw - 1) / cw;
-    uint64_t* full = reinterpret_cast<uint64_t*>(area + int64_t(NS) * P * cw);
+    const ReduceArea place = ReduceArea::make(NS, P, cw);
+    uint64_t* full = reinterpret_cast<uint64_t*>(area + place.barriers);
     uint64_t* empty = full + NS;
-    int* rows_in_stage = flow + 2;  // per stage: partition rows that the loader put there
+    int* rows_in_stage = reinterpret_cast<int*>(area + place.rows);
     const StatusRef status = status_of(p.c);
     const uint32_t tag = combine_tag(p.epoch);
     const int n_tok = p.tokens > int(blockIdx.x) ? (p.tokens - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x) : 0;
@@ -1622,7 +1622,7 @@ __device__ void combine_body(const CombineParams& p) {
         if (p.reduce_stages >= 2) {
             // full: the loader's arrival plus the bytes of its bulk loads; empty: one arrival per consumer warp
             char* area = reduce_area(p, s_ring);
-            uint64_t* full = reinterpret_cast<uint64_t*>(area + int64_t(p.reduce_stages) * L.ret_parts * p.reduce_chunk_bytes);
+            uint64_t* full = reinterpret_cast<uint64_t*>(area + ReduceArea::make(p.reduce_stages, L.ret_parts, p.reduce_chunk_bytes).barriers);
             const int consumers = int(blockDim.x >> 5) - p.push_warps - 2;
             for (int s = 0; s < p.reduce_stages; ++s) {
                 mbar_init(full + s, 1);
@@ -2045,7 +2045,7 @@ RingPlan plan_ring(int64_t row_bytes, int max_smem_bytes) {
 
 CombinePlan plan_combine(int64_t row_bytes, int parts, int max_smem_bytes, int reduce_stages, int reduce_chunk_bytes) {
     // smem = transfer rings (warps x stages x (row pitch + mbarrier)) + flag board + reduce pipeline
-    // (stages x parts x chunk + two mbarriers per stage) + alignment slack + static smem.
+    // (ReduceArea) + alignment slack + static smem.
     CombinePlan c{};
     const int64_t pitch = align_up(row_bytes, 128);
     const int64_t fixed = int64_t(sizeof(FlagBoard)) + 16 + 128 + 512;
@@ -2059,7 +2059,7 @@ CombinePlan plan_combine(int64_t row_bytes, int parts, int max_smem_bytes, int r
     const int64_t alone = std::min<int64_t>((int64_t(max_smem_bytes) - fixed) / (pitch + 8) / 2, 8);
     for (;;) {
         const bool piped = reduce_stages >= 2 && chunk >= 128;
-        const int64_t pipe = piped ? int64_t(reduce_stages) * parts * chunk + 16 * reduce_stages : 0;
+        const int64_t pipe = piped ? ReduceArea::make(reduce_stages, parts, chunk).bytes : 0;
         const int64_t slots = (int64_t(max_smem_bytes) - fixed - pipe) / (pitch + 8);
         // three stages per transfer warp when there is room for at least four such warps, else two
         const int stages = slots >= 12 ? 3 : 2;

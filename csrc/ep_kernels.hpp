@@ -239,6 +239,15 @@ struct CombinePlan {
     RingPlan ring;
     int reduce_stages, reduce_chunk_bytes;
 };
+// The pipeline's area: `stages` stages of `parts` chunks, then per stage a full and an empty mbarrier, then per stage the number
+// of rows that the loader put there.  Any number of stages that the plan grants has its words here.
+struct ReduceArea {
+    int64_t barriers, rows, bytes;  // offsets of the mbarriers and the row counts, size of the whole
+    NEP_HD static constexpr ReduceArea make(int stages, int parts, int64_t chunk) {
+        const int64_t barriers = int64_t(stages) * parts * chunk, rows = barriers + 16 * int64_t(stages);
+        return ReduceArea{barriers, rows, align_up(rows + 4 * int64_t(stages), 16)};
+    }
+};
 CombinePlan plan_combine(int64_t row_bytes, int parts, int max_smem_bytes, int reduce_stages, int reduce_chunk_bytes);
 constexpr int kCombineThreads = 512;  // transfer warps + reduce warps of one combine CTA
 // Grid of the kernels that sum (or, with one row per token, copy) whole rows: reduce, local_combine.

@@ -120,3 +120,27 @@ def test_many_logical_ranks(world):
             for b in back:
                 assert torch.equal(b[r].x.cpu(), want)
                 assert torch.equal(b[r].topk_weights.cpu(), torch.where(idx >= 0, case.weights[r], 0.0))
+
+
+@pytest.mark.parametrize("setting", [-3000, -40001, -200001])  # stages * 1000 + chunk / 128: three whole-row stages, 40 and 200 of 128 bytes
+def test_reduction_with_many_stages(setting):
+    """Every stage of the reduce ring has its own row count; token counts of neighbouring stages differ here."""
+    from nanoep_b200.utils.build import load_extension
+
+    world = 2
+    case = make_case(world, kind="mixed", seed=5, hidden=256, tokens=300, experts_per_rank=4, topk=4)
+    cfg = EPConfig(case.num_experts, case.num_topk, case.hidden, case.capacity)
+    ext = load_extension()
+    ext.set_combine_trace(False, 0, setting)
+    try:
+        with EmulatedGroup(world, cfg) as group:
+            got = group.dispatch(_cuda(case.xs), topk_idx=_cuda(case.indices), weights=_cuda(case.weights), do_expand=True, alignment=1)
+            back = group.combine([g.x for g in got], [g.handle for g in got], weights=[g.topk_weights for g in got])
+            torch.cuda.synchronize()
+            group.check_status()
+            for r in range(world):
+                idx, x = case.indices[r], case.xs[r].float()
+                want = (x * (idx >= 0).sum(-1, keepdim=True)).to(torch.bfloat16)  # up to four equal bf16 values: exact in FP32
+                assert torch.equal(back[r].x.cpu(), want)
+    finally:
+        ext.set_combine_trace(False, 0, 0)

@@ -378,3 +378,21 @@ def test_combine_shared_memory_plan():
     assert ext.combine_plan(7168, 8, limit, 4, 1700)[4] == 1792
     # a row that leaves no room for a pipeline falls back to the register path instead of failing
     assert ext.combine_plan(49152, 8, limit, 2, 0)[3] in (0, 2)
+
+
+def test_combine_plan_has_words_for_every_stage_it_grants():
+    """The reduce pipeline keeps two mbarriers and a row count per stage; the number of stages is a setting, so they have to be
+    part of what the plan hands out (40 stages of 128 bytes are a legal one)."""
+    from nanoep_b200.utils.build import load_extension
+
+    ext = load_extension()
+    limit = 227 * 1024
+    for hidden, parts, stages in ((256, 8, 40), (256, 1, 200), (7168, 4, 64), (512, 2, 3)):
+        pitch = (hidden * 2 + 127) // 128 * 128
+
+        def beside_the_rings(n):
+            warps, ring_stages, smem, granted, chunk = ext.combine_plan(hidden, parts, limit, n, 128)
+            assert granted == n
+            return smem - warps * ring_stages * (pitch + 8) - granted * parts * chunk
+
+        assert beside_the_rings(stages) - beside_the_rings(0) >= stages * (2 * 8 + 4), (hidden, parts, stages)
