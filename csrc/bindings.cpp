@@ -183,6 +183,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         },
         py::arg("hidden"), py::arg("parts"), py::arg("max_smem_bytes"), py::arg("reduce_stages") = 2, py::arg("reduce_chunk_bytes") = 0,
         "Shared-memory plan of a combine CTA: (transfer warps, ring stages, dynamic bytes, reduce stages, reduce chunk bytes)");
+    m.def(
+        "ring_plan",
+        [](int64_t hidden, int64_t topk, int64_t max_smem_bytes, bool shared) {
+            const nep::RingPlan ring = nep::plan_ring(nep::wire_row_bytes(int(hidden), int(topk)), int(max_smem_bytes), shared);
+            return std::make_tuple(ring.warps, ring.stages, ring.zero_bytes, int64_t(ring.smem_bytes));
+        },
+        py::arg("hidden"), py::arg("topk"), py::arg("max_smem_bytes"), py::arg("shared"),
+        "Shared-memory plan of a pull CTA: (transfer warps, ring stages, bytes of the zero source, dynamic bytes)");
     m.def("set_combine_trace", &nep::set_combine_trace, py::arg("enabled"), py::arg("store_depth") = 0, py::arg("reduce_group") = 0);
     m.def("take_combine_trace", &nep::take_combine_trace);
     m.def("take_stage_trace", &nep::take_stage_trace);

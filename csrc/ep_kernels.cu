@@ -2017,7 +2017,7 @@ int row_sum_grid(int64_t tokens, int hidden, bool sums, int sms) {
 int stage_smem_bytes(const WindowLayout& l) { return int((l.ranks + l.num_experts) * 4); }
 int plan_smem_bytes(const WindowLayout& l) { return (kPlanThreads / 32) * 32 * l.topk * 4; }
 
-RingPlan plan_ring(int64_t row_bytes, int max_smem_bytes) {
+RingPlan plan_ring(int64_t row_bytes, int max_smem_bytes, bool shared) {
     // smem = warps * stages * (row pitch + one mbarrier) + zero buffer + alignment slack + static smem.
     // The software pipeline needs at least two stages; a row that does not fit twice is rejected by
     // the caller (warps == 0).
@@ -2036,9 +2036,12 @@ RingPlan plan_ring(int64_t row_bytes, int max_smem_bytes) {
     if (warps < 1) warps = 0;
     r.warps = warps > 8 ? 8 : warps;
     // What the rings leave goes to the zero source of the padding rows, up to a whole row: stores of 2 KB reach
-    // 4.8 TB/s, of 3.5 KB and more 5.9 TB/s (rows in random order).
+    // 4.8 TB/s, of 3.5 KB and more 5.9 TB/s (rows in random order).  Not beside a gated GEMM: its blocks wait for this
+    // kernel's rows, so both have to fit an SM, and at hidden 4096 a ring of 80 KB leaves the three-stage GEMM (148 KB of the
+    // SM's 228) its place with 2 KB of zeros (75.4 KB) but not with 6 KB (79.7 KB).
     const int64_t used = int64_t(r.warps) * r.stages * (pitch + 8);
-    r.zero_bytes = int(std::max<int64_t>(kZeroBytes, std::min(pitch, (int64_t(max_smem_bytes) - 512 - used) / 128 * 128)));
+    const int64_t left = shared ? 0 : std::min(pitch, (int64_t(max_smem_bytes) - 512 - used) / 128 * 128);
+    r.zero_bytes = int(std::max<int64_t>(kZeroBytes, left));
     r.smem_bytes = size_t(used) + r.zero_bytes + 256;
     return r;
 }

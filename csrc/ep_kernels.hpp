@@ -232,7 +232,8 @@ struct RingPlan {
     int zero_bytes;  // pull only: size of the zero source behind the rings
     size_t smem_bytes;
 };
-RingPlan plan_ring(int64_t row_bytes, int max_smem_bytes);
+// `shared`: a kernel of another stream runs on the same SMs, and what the rings leave of max_smem_bytes is left to it.
+RingPlan plan_ring(int64_t row_bytes, int max_smem_bytes, bool shared);
 // Shared memory of a combine CTA: the transfer warps' rings, the flag board and (reduce_stages >= 2) the reduce
 // pipeline.  reduce_chunk_bytes == 0 lets the plan pick the chunk.
 struct CombinePlan {

@@ -293,7 +293,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     TORCH_CHECK(num_sms >= 1 && num_sms <= lim.sms, "num_sms out of range");
     // A smaller ring leaves shared memory for a compute kernel that shares the SMs with the pull.
     const int ring_budget = ring_smem_limit > 0 ? int(std::min<int64_t>(ring_smem_limit, lim.smem_optin)) : lim.smem_optin;
-    const RingPlan ring = plan_ring(L.row_bytes(), ring_budget);
+    const RingPlan ring = plan_ring(L.row_bytes(), ring_budget, ring_smem_limit > 0);
     TORCH_CHECK(ring.warps >= 1, "hidden size too large for the shared-memory row ring");
     reject_graph_capture(device, fresh ? "fresh dispatch waits for receive counts on the host" : "barrier epochs and buffer parities are kernel arguments");
 

@@ -396,3 +396,24 @@ def test_combine_plan_has_words_for_every_stage_it_grants():
             return smem - warps * ring_stages * (pitch + 8) - granted * parts * chunk
 
         assert beside_the_rings(stages) - beside_the_rings(0) >= stages * (2 * 8 + 4), (hidden, parts, stages)
+
+
+def test_limited_ring_leaves_the_sm_to_the_gated_gemm():
+    """Blocks of a gated GEMM wait for rows of the pull, so one block of each has to fit an SM: a pull with a ring limit takes its
+    rings and the smallest zero source, not what is left of the limit."""
+    import inspect
+
+    from nanoep_b200.models.moe_layer import ExpertParallelMoE
+    from nanoep_b200.utils.build import load_extension
+
+    ext = load_extension()
+    limit = inspect.signature(ExpertParallelMoE).parameters["comm_ring_bytes"].default
+    sm, reserved = 228 * 1024, 1024  # shared memory of an SM; the system's share of every resident block
+    for hidden in (1536, 2048, 3072, 4096, 5120, 5632, 6144, 7168, 8192):
+        warps, stages, zeros, smem = ext.ring_plan(hidden, 8, limit, True)
+        pitch = (hidden * 2 + 32 + 127) // 128 * 128
+        assert warps >= 2 and zeros == 2048 and smem == warps * stages * (pitch + 8) + zeros + 256
+        assert smem + reserved + ext.gemm_shared_bytes(3) + reserved <= sm, hidden
+        # without a limit the zero source is as long as a row where there is room
+        assert ext.ring_plan(hidden, 8, 227 * 1024, False)[2] >= 2048
+    assert ext.ring_plan(7168, 8, 227 * 1024, False)[2] > 2048
