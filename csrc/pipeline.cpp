@@ -29,6 +29,7 @@ namespace {
 constexpr int kFusedDispatchDefaultTokens = 64;
 constexpr int kFusedFreshDefaultTokens = 0;  // single-launch fresh dispatch: off unless asked for (the host waits for N and C either way)
 constexpr int64_t kFusedFreshMaxOutputBytes = int64_t(256) << 20;  // single-launch fresh dispatch: largest bound-sized output
+constexpr int64_t kEarlyPullMaxOutputBytes = int64_t(32) << 20;    // single-rank pull that does not wait for N and C: see dispatch()
 constexpr int kFusedDefaultBlocks = 1024;  // i.e. bounded by the SM budget and co-residency only
 
 void cuda_check(cudaError_t e, const char* what) {
@@ -381,12 +382,15 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     // (every rank may send all of its Tmax tokens here), trimmed to N / C once the mailbox has them.  Only when that
     // bound is modest, i.e. for buffers configured for small batches.
     // A single-rank group knows its bound from this call's own tokens, and its pull needs nothing from the host: it is
-    // launched behind the plan without waiting for the counts, under the same limit on the bound.
+    // launched behind the plan without waiting for the counts where the bound is what a call without masked choices
+    // receives (with an alignment the bound counts padding that hardly any routing has).  A call that receives less gets its
+    // outputs copied to their exact size below, so the limit on the bound lies where that copy takes as long as the wait.
     const int64_t bound_rows_n = local ? max_tokens_now : int64_t(L.ranks) * L.max_tokens;
     const int64_t bound_choices = bound_rows_n * std::min<int64_t>(L.topk, L.local_experts);
     const int64_t bound_rows_c = bound_choices + std::min<int64_t>(L.local_experts, local ? bound_choices : L.local_experts) * (alignment - 1);
     const int64_t bound_bytes = (expand ? bound_rows_c : bound_rows_n) * L.hidden * 2;
-    const bool early_pull = plan_locally && !gated && !g_gate.word.defined() && bound_bytes <= kFusedFreshMaxOutputBytes;
+    const bool early_pull =
+        plan_locally && (!expand || alignment == 1) && !gated && !g_gate.word.defined() && bound_bytes <= kEarlyPullMaxOutputBytes;
     const bool fuse_fresh = fresh && !gated && !local && !g_gate.word.defined() && max_tokens_now <= fused_fresh_max_tokens() &&
                             bound_bytes <= kFusedFreshMaxOutputBytes && (!expand || bound_rows_c <= L.slot_scratch_ints) &&
                             ring.warps >= 2 && ring.smem_bytes >= size_t(stage_smem_bytes(L)) &&
@@ -555,8 +559,14 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         }
     }
     if (fuse_fresh || early_pull) {
-        // The kernel is on its way; now wait for N and C and trim the outputs to their exact sizes (leading-dimension
-        // views of the bound-sized allocations: contiguous, same storage).
+        // The kernel is on its way; now wait for N and C and trim the outputs to their exact sizes: the single-launch path
+        // (off by default) to leading-dimension views of the bound-sized allocations, a single rank's early pull to
+        // tensors that own no more than they show.
+        c10::cuda::CUDAStreamGuard pool(consumer);
+        auto trim = [&](at::Tensor& t, at::IntArrayRef sizes) {
+            const at::Tensor view = part_of(t, 0, sizes);
+            if (view.numel() < t.numel()) t = early_pull ? view.clone() : view;
+        };
         for (int i = 0; i < n; ++i) {
             std::pair<int64_t, int64_t> nc;
             {
@@ -567,9 +577,10 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             TORCH_CHECK(N <= bound_rows_n && (!expand || C <= bound_rows_c), "receive counts exceed the single-launch bound");
             out.counts[i] = {N, C};
             auto& o = out.outputs[i];
-            o[0] = part_of(o[0], 0, {expand ? C : N, L.hidden});
-            if (!expand) o[1] = part_of(o[1], 0, {N, L.topk});
-            if (weighted) o[2] = expand ? part_of(o[2], 0, {C}) : part_of(o[2], 0, {N, L.topk});
+            trim(o[0], {expand ? C : N, L.hidden});
+            if (!expand) trim(o[1], {N, L.topk});
+            if (weighted && expand) trim(o[2], {C});
+            if (weighted && !expand) trim(o[2], {N, L.topk});
         }
     }
     if (fuse_fresh || plan_locally) {

@@ -144,3 +144,30 @@ def test_reduction_with_many_stages(setting):
                 assert torch.equal(back[r].x.cpu(), want)
     finally:
         ext.set_combine_trace(False, 0, 0)
+
+
+@pytest.mark.parametrize("masked", ["none", "choices", "tokens", "all"])
+@pytest.mark.parametrize("expand,alignment", [(False, 1), (True, 1), (True, 16)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_outputs_own_exactly_what_they_show(masked, expand, alignment, weighted):
+    """Whatever a single rank allocates before it knows its receive counts, the outputs keep no more memory than they show."""
+    case = make_case(1, kind="random", seed=3, hidden=256, tokens=40, experts_per_rank=12, topk=4)
+    idx = torch.stack([torch.randperm(case.num_experts)[: case.num_topk] for _ in range(40)])
+    if masked == "choices":
+        idx[::3, 1:] = -1
+    elif masked == "tokens":
+        idx[5:] = -1
+    elif masked == "all":
+        idx[:] = -1
+    case.indices[0] = idx
+    cfg = EPConfig(case.num_experts, case.num_topk, case.hidden, case.capacity)
+    with EmulatedGroup(1, cfg) as group:
+        got = group.dispatch(_cuda(case.xs), topk_idx=_cuda(case.indices), weights=_cuda(case.weights) if weighted else None, do_expand=expand,
+                             alignment=alignment, zero_padding=True)[0]
+        torch.cuda.synchronize()
+        group.check_status()
+        assert_dispatch_matches(got, case.xs, case.indices, case.weights, case.num_experts, 0, expand=expand, alignment=alignment,
+                                zero_padding=True, weighted=weighted)
+        for out in (got.x, got.topk_idx, got.topk_weights):
+            if out is not None:
+                assert out.untyped_storage().nbytes() == out.numel() * out.element_size() and out.storage_offset() == 0
