@@ -29,6 +29,7 @@ namespace {
 constexpr int kFusedDispatchDefaultTokens = 64;
 constexpr int kFusedFreshDefaultTokens = 0;  // single-launch fresh dispatch: off unless asked for (the host waits for N and C either way)
 constexpr int64_t kFusedFreshMaxOutputBytes = int64_t(256) << 20;  // single-launch fresh dispatch: largest bound-sized output
+constexpr int64_t kLocalPlanMaxHandleBytes = int64_t(16) << 20;    // single-rank plan: largest bound-sized handle
 constexpr int64_t kEarlyPullMaxOutputBytes = int64_t(32) << 20;    // single-rank pull that does not wait for N and C: see dispatch()
 constexpr int kFusedDefaultBlocks = 1024;  // i.e. bounded by the SM budget and co-residency only
 
@@ -304,10 +305,18 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     const c10::cuda::CUDAStream consumer = async_op ? s.comm : s.compute;
     int64_t max_tokens_now = 0;
     for (int i = 0; i < n; ++i) max_tokens_now = std::max<int64_t>(max_tokens_now, xs[i].size(0));
-    // A single-rank group exchanges nothing: a fresh dispatch plans in one launch that writes the handle's tensors itself
-    // (allocated at their upper bounds and trimmed), a cached one goes straight to the pull.
+    // A single-rank group exchanges nothing: a fresh dispatch plans in one launch that writes the handle's tensors itself,
+    // a cached one goes straight to the pull.  Those tensors are allocated before the counts are known, so the one launch takes
+    // calls whose upper bound is modest (4096 tokens x top-8 of 256 experts, alignment 128: 0.4 MB); an alignment
+    // far above the experts' counts goes through the stage and plan kernels, which write a handle of exact size.
     const bool local = L.ranks == 1;
-    const bool plan_locally = local && fresh && local_plan_fits(L, max_tokens_now);
+    // Upper bounds of the receive counts: all of this call's tokens on one rank, all that every rank may send in a group.
+    const int64_t bound_rows_n = local ? max_tokens_now : int64_t(L.ranks) * L.max_tokens;
+    const int64_t bound_choices = bound_rows_n * std::min<int64_t>(L.topk, L.local_experts);
+    const int64_t bound_rows_c = bound_choices + std::min<int64_t>(L.local_experts, local ? bound_choices : L.local_experts) * (alignment - 1);
+    const int64_t bound_cells = bound_rows_n * (L.topk + 2), bound_slots = expand ? bound_rows_c : 0;
+    const bool plan_locally =
+        local && fresh && local_plan_fits(L, max_tokens_now) && (bound_cells + bound_slots) * 4 <= kLocalPlanMaxHandleBytes;
     // The caller starts a consumer on another stream as soon as this call returns (see dispatch() in Python).
     bool gated = false;
     for (const auto& t : tile_ready) gated = gated || t.has_value();
@@ -385,9 +394,6 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     // launched behind the plan without waiting for the counts where the bound is what a call without masked choices
     // receives (with an alignment the bound counts padding that hardly any routing has).  A call that receives less gets its
     // outputs copied to their exact size below, so the limit on the bound lies where that copy takes as long as the wait.
-    const int64_t bound_rows_n = local ? max_tokens_now : int64_t(L.ranks) * L.max_tokens;
-    const int64_t bound_choices = bound_rows_n * std::min<int64_t>(L.topk, L.local_experts);
-    const int64_t bound_rows_c = bound_choices + std::min<int64_t>(L.local_experts, local ? bound_choices : L.local_experts) * (alignment - 1);
     const int64_t bound_bytes = (expand ? bound_rows_c : bound_rows_n) * L.hidden * 2;
     const bool early_pull =
         plan_locally && (!expand || alignment == 1) && !gated && !g_gate.word.defined() && bound_bytes <= kEarlyPullMaxOutputBytes;
@@ -409,11 +415,10 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         g_marks.mark("begin", cs);
         if (plan_locally) {
             auto& m = out.metadata[0];
-            const int64_t cells = bound_rows_n * (L.topk + 2), slots = expand ? bound_rows_c : 0;
             c10::cuda::CUDAStreamGuard pool(consumer);
-            const at::Tensor block = make_empty({cells + slots}, at::kInt, device);
+            const at::Tensor block = make_empty({bound_cells + bound_slots}, at::kInt, device);
             m[0] = part_of(block, 0, {bound_rows_n, L.topk + 2});
-            m[7] = part_of(block, cells, {slots});
+            m[7] = part_of(block, bound_cells, {bound_slots});
             LocalPlanParams lp{};
             const StageParams& sp = stage[0];
             lp.c = sp.c;
@@ -584,10 +589,18 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         }
     }
     if (fuse_fresh || plan_locally) {
+        c10::cuda::CUDAStreamGuard pool(consumer);
         for (int i = 0; i < n; ++i) {
             auto& m = out.metadata[i];
             m[0] = part_of(m[0], 0, {out.counts[i].first, L.topk + 2});
             if (expand) m[7] = part_of(m[7], 0, {out.counts[i].second});
+            // A handle may live long (cached dispatches): it does not keep a bound of which it uses less than half,
+            // unless that is no more than what the allocator rounds up anyway.
+            const int64_t used = m[0].numel() + m[7].numel(), held = bound_cells + bound_slots;
+            if (plan_locally && held * 4 > (int64_t(1) << 20) && used * 2 < held) {
+                m[0] = m[0].clone();
+                m[7] = m[7].clone();
+            }
         }
     }
     std::vector<at::Tensor> inputs, results;

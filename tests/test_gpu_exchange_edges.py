@@ -171,3 +171,40 @@ def test_outputs_own_exactly_what_they_show(masked, expand, alignment, weighted)
         for out in (got.x, got.topk_idx, got.topk_weights):
             if out is not None:
                 assert out.untyped_storage().nbytes() == out.numel() * out.element_size() and out.storage_offset() == 0
+
+
+def _one_rank_dispatch(idx, experts, hidden, **layout):
+    gen = torch.Generator().manual_seed(idx.shape[0])
+    x = torch.randn(idx.shape[0], hidden, generator=gen).to(torch.bfloat16)
+    w = torch.rand(idx.shape, generator=gen)
+    with EmulatedGroup(1, EPConfig(experts, idx.shape[1], hidden, idx.shape[0])) as group:
+        got = group.dispatch([x.cuda()], topk_idx=[idx.cuda()], weights=[w.cuda()], zero_padding=True, **layout)[0]
+        torch.cuda.synchronize()
+        group.check_status()
+    assert_dispatch_matches(got, [x], [idx], [w], experts, 0, expand=layout["do_expand"], alignment=layout["alignment"], zero_padding=True)
+    lay = got.handle.layout
+    kept = {t.untyped_storage().data_ptr(): t.untyped_storage().nbytes() for t in (lay.recv_metadata, got.handle.slot_map)}
+    used = sum(t.numel() * t.element_size() for t in (lay.recv_metadata, got.handle.slot_map))
+    assert sum(kept.values()) <= max(2 * used, 1 << 20)
+
+
+@pytest.mark.parametrize("tokens", [32768, 32769])  # the one-launch plan's largest call, and one for the stage and plan kernels
+@pytest.mark.parametrize("expand", [False, True])
+def test_single_rank_plan_limit(tokens, expand):
+    idx = torch.arange(tokens)[:, None] % 4
+    _one_rank_dispatch(idx, 4, 256, do_expand=expand, alignment=8 if expand else 1)
+
+
+@pytest.mark.parametrize("expand", [False, True])
+def test_single_rank_handle_keeps_what_it_uses(expand):
+    """20000 tokens, nearly all masked: the plan's bound is 1.4 MB (expert-major), the handle uses less than 1 KB."""
+    idx = torch.full((20000, 8), -1)
+    idx[::4000] = torch.arange(8)
+    _one_rank_dispatch(idx, 16, 256, do_expand=expand, alignment=1)
+
+
+def test_single_rank_alignment_far_above_the_counts():
+    """16 choices could fill 16 experts of 2^19 rows; they go to one, so the handle needs a sixteenth of the bound."""
+    idx = torch.full((4, 4), -1)
+    idx[:, 2] = 3
+    _one_rank_dispatch(idx, 16, 256, do_expand=True, alignment=1 << 19)
