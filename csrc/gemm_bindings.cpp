@@ -113,6 +113,16 @@ cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& 
     return gemm::launch_expert(maps, g.args, mode, tile, grid, c10::cuda::getCurrentCUDAStream().stream());
 }
 
+// Which kernel a grouped_gemm call runs.  The one with tokens as N is the faster one (expert_gemm_sm100.cu has both sides), but it
+// takes all of an SM's shared memory and works in pairs of CTAs: row blocks gated by counters (which share the SMs with the dispatch that fills them), a
+// caller who asks for CTA pairs or for the three-stage pipeline (smaller, to run beside another kernel), and a call that
+// may use a single CTA get the kernels with tokens as M.
+enum Kernel { kExpertKernel, kPairKernel, kSingleKernel };
+Kernel choose_kernel(bool gated, bool pair, int64_t stages, int64_t max_ctas) {
+    if (pair) return kPairKernel;
+    return gated || stages == 3 || max_ctas == 1 ? kSingleKernel : kExpertKernel;
+}
+
 }  // namespace
 
 void bind_gemm(pybind11::module_& m) {
@@ -149,18 +159,19 @@ void bind_gemm(pybind11::module_& m) {
             if (a.size(0) == 0) return;
             const int grid = max_ctas > 0 ? std::min<int>(g.grid, int(max_ctas)) : g.grid;
             PeerWindow::launches += 1;
-            // The kernel with tokens as N unless its row blocks are gated by counters (that one shares the SMs with the
-            // dispatch and has to leave it shared memory) or the caller allows a single CTA (it needs pairs).
-            if (!tile_ready.has_value() && max_ctas != 1) {
+            const Kernel kernel = choose_kernel(tile_ready.has_value(), pair, stages, max_ctas);
+            if (kernel == kExpertKernel) {
                 cudaError_t ee = launch_expert(g, a, w, expert_counts, int(mode), max_expert_rows, max_ctas);
                 TORCH_CHECK(ee == cudaSuccess, "grouped GEMM (expert) launch failed: ", cudaGetErrorString(ee));
                 return;
             }
             const CUtensorMap map_a = make_map(a.data_ptr(), a.size(0), a.size(1)), map_b = make_map(w.data_ptr(), w.size(0) * w.size(1), w.size(2));
-            if (pair) {
+            if (kernel == kPairKernel) {
                 const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
                 const int pair_grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : sms;
-                cudaError_t pe = gemm::launch_pair(map_a, map_b, g.args, int(mode), pair_grid, c10::cuda::getCurrentCUDAStream().stream());
+                // gated by tile counters = meant to share the SMs with the pull kernel: shorter pipeline
+                cudaError_t pe = gemm::launch_pair(map_a, map_b, g.args, int(mode), pair_grid, c10::cuda::getCurrentCUDAStream().stream(),
+                                                   tile_ready.has_value() ? 4 : 6);
                 TORCH_CHECK(pe == cudaSuccess, "grouped GEMM (CTA pairs) launch failed: ", cudaGetErrorString(pe));
                 return;
             }
@@ -218,6 +229,14 @@ void bind_gemm(pybind11::module_& m) {
         pybind11::arg("max_ctas") = 0, pybind11::arg("timeout_s") = 5.0,
         pybind11::arg("expert_counts") = c10::nullopt, pybind11::arg("max_expert_rows") = 0);
 
+    m.def(
+        "grouped_gemm_choice",
+        [](bool gated, bool pair, int64_t stages, int64_t max_ctas) -> std::string {
+            const Kernel kernel = choose_kernel(gated, pair, stages, max_ctas);
+            return kernel == kExpertKernel ? "expert" : kernel == kPairKernel ? "pair" : "single";
+        },
+        pybind11::arg("gated") = false, pybind11::arg("pair") = false, pybind11::arg("stages") = 4, pybind11::arg("max_ctas") = 0,
+        "Kernel that a grouped_gemm call with these arguments runs");
     m.def("gemm_kernel_registers", [](int64_t mode) { return gemm::kernel_registers(int(mode)); });
     m.def("gemm_shared_bytes", [](int64_t stages) { return int64_t(gemm::shared_bytes(int(stages))); });
 }

@@ -4,8 +4,8 @@
 //   out[m, :] = epilogue( A[m, :] @ W[e(m)]^T )     for every 128-row block m of the expert-major
 //                                                   activation matrix; e(m) from expert_offsets.
 //
-// It runs where row blocks are gated by counters (beside the dispatch that fills them) or a caller allows one CTA only;
-// everything else is expert_gemm_sm100.cu.  The reference library has no GEMM at all (its kernels only move data); this kernel is what lets
+// It runs where row blocks are gated by counters (beside the dispatch that fills them) or a caller allows one CTA only or asks
+// for the three-stage pipeline; everything else is expert_gemm_sm100.cu.  The reference library has no GEMM at all (its kernels only move data); this kernel is what lets
 // dispatch feed the expert up-projection and the down-projection feed combine on the same GPU.
 //
 // Roles per CTA (192 threads): warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner, warps 2..5 =

@@ -5,7 +5,7 @@
 // the 256 weight rows, the leader CTA issues one MMA for the pair, and each CTA keeps the
 // accumulator of its own 128 rows in its own TMEM.  Per CTA and k-block that is 32 KB of operand
 // traffic instead of 48 KB, which is what limits the single-CTA kernel (L2 -> SM bandwidth).
-// It runs where row blocks are gated by counters; everything else is expert_gemm_sm100.cu.
+// It runs where row blocks are gated by counters or the caller asks for it; everything else is expert_gemm_sm100.cu.
 //
 // Work unit = (expert, pair of consecutive 128-row blocks of that expert, output column tile).
 // An expert with an odd number of row blocks leaves the second CTA of its last pair without rows:
@@ -320,14 +320,15 @@ cudaError_t launch_pair_mode(const CUtensorMap& a, const CUtensorMap& b, const A
 
 }  // namespace
 
-// `grid` is rounded down to an even number of CTAs (one cluster = two CTAs on two SMs).  SwiGLU runs four operand stages, which
-// leaves ~95 KB of shared memory per SM for a co-resident transfer kernel; plain runs six.
-cudaError_t launch_pair(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int mode, int grid, cudaStream_t stream) {
+// `grid` is rounded down to an even number of CTAs (one cluster = two CTAs on two SMs).  Six operand stages; SwiGLU also with
+// four, which leave ~95 KB of shared memory per SM for a co-resident transfer kernel.
+cudaError_t launch_pair(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int mode, int grid, cudaStream_t stream, int stages) {
     if (args.num_experts > kMaxExperts) return cudaErrorInvalidValue;
     grid &= ~1;
     if (grid < 2) return cudaErrorInvalidValue;
     if (mode == kPlain) return launch_pair_mode<kPlain, 6>(a, b, args, grid, stream);
-    if (mode == kSwiGLU) return launch_pair_mode<kSwiGLU, 4>(a, b, args, grid, stream);
+    if (mode == kSwiGLU && stages == 4) return launch_pair_mode<kSwiGLU, 4>(a, b, args, grid, stream);
+    if (mode == kSwiGLU) return launch_pair_mode<kSwiGLU, 6>(a, b, args, grid, stream);
     return cudaErrorInvalidValue;
 }
 

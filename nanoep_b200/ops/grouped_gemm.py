@@ -50,8 +50,9 @@ def grouped_gemm(a, w, expert_offsets, *, swiglu: bool = False, out=None, tile_r
     ``row_scale`` (fp32 ``[rows]``, plain mode) multiplies each output row in FP32 before the bf16 round.
     ``expert_counts`` (int64 ``[E]``): only so many rows of each expert's range exist; the other rows are neither read as
     far as the result goes nor defined in the output.  ``max_expert_rows`` (0 = unknown): no expert holds more rows.
-    With ``tile_ready`` (row blocks gated by counters): ``stages=3`` shrinks the operand pipeline so that a transfer kernel can
-    share the SMs, ``pair=True`` runs the CTA-pair kernel (two SMs share every weight tile).
+    ``stages=3`` runs the single-CTA kernel with a pipeline that leaves a third of an SM's shared memory to another kernel,
+    ``pair=True`` the CTA-pair kernel (two SMs share every weight tile); both compute every row of every range, and they are
+    what runs with ``tile_ready`` (row blocks gated by counters).
     """
     n_out = w.shape[1] // 2 if swiglu else w.shape[1]
     if out is None:

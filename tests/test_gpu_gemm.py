@@ -15,8 +15,25 @@ def _offsets(blocks_per_expert):
     return torch.tensor(rows, dtype=torch.int64, device="cuda")
 
 
-def _check(a, w, offsets, swiglu):
-    out = gg.grouped_gemm(a, w, offsets, swiglu=swiglu)
+# Arguments that select each kernel; "gated" stands for row counters that are all full.
+KERNELS = {
+    "expert": {}, "single, three stages": dict(stages=3), "single, four stages": dict(gated=True), "pair, six stages": dict(pair=True),
+    "pair, four stages": dict(pair=True, gated=True),
+}
+
+
+def _select(kernel, a):
+    args = dict(KERNELS[kernel])
+    if args.pop("gated", False):
+        full = torch.full((a.shape[0] // 128,), 128, dtype=torch.int32, device="cuda")
+        args.update(tile_ready=full, tile_expected=full)
+    choice = gg._ext().grouped_gemm_choice(gated="tile_ready" in args, **{k: v for k, v in args.items() if k in ("pair", "stages")})
+    assert choice == kernel.split(",")[0]
+    return args
+
+
+def _check(a, w, offsets, swiglu, kernel="expert"):
+    out = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select(kernel, a))
     torch.cuda.synchronize()
     gg.check_status()
     ref = gg.grouped_gemm_reference(a, w, offsets, swiglu=swiglu)
@@ -25,32 +42,43 @@ def _check(a, w, offsets, swiglu):
     return out
 
 
+@pytest.mark.parametrize("kernel", KERNELS)
 @pytest.mark.parametrize("swiglu", [False, True])
 @pytest.mark.parametrize("blocks,K,N", [([1], 64, 256), ([1, 2, 0, 1], 256, 512), ([3, 1, 2], 1024, 768)])
-def test_small_shapes(blocks, K, N, swiglu):
+def test_small_shapes(blocks, K, N, swiglu, kernel):
     torch.manual_seed(1)
     offsets = _offsets(blocks)
     rows = int(offsets[-1])
     a = (torch.randn(rows, K, device="cuda") * 0.5).to(torch.bfloat16)
     w = (torch.randn(len(blocks), N, K, device="cuda") * 0.1).to(torch.bfloat16)
-    _check(a, w, offsets, swiglu)
+    _check(a, w, offsets, swiglu, kernel)
 
 
-def test_identity_weights_expose_layout_errors():
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_identity_weights_expose_layout_errors(kernel):
     """W = stacked identity blocks: the output must reproduce the input columns exactly."""
     K = N = 256
     offsets = _offsets([2, 1])
     a = torch.randn(384, K, device="cuda").to(torch.bfloat16)
     w = torch.eye(N, K, device="cuda").to(torch.bfloat16).repeat(2, 1, 1).contiguous()
     w[1] *= 2
-    out = gg.grouped_gemm(a, w, offsets)
+    out = gg.grouped_gemm(a, w, offsets, **_select(kernel, a))
     torch.cuda.synchronize()
     gg.check_status()
     assert torch.equal(out[:256], a[:256])
     assert torch.equal(out[256:], (a[256:].float() * 2).to(torch.bfloat16))
+    scale = torch.rand(384, device="cuda") + 0.5
+    scaled = gg.grouped_gemm(a, w, offsets, row_scale=scale, **_select(kernel, a))
+    torch.cuda.synchronize()
+    gg.check_status()
+    factor = torch.ones(384, 1, device="cuda")
+    factor[256:] = 2
+    # one exact product per output, times the scale in FP32, one bf16 round
+    assert torch.equal(scaled, (a.float() * factor * scale[:, None]).to(torch.bfloat16))
 
 
-def test_many_tiles_persistent_schedule():
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_many_tiles_persistent_schedule(kernel):
     """More tiles than CTAs and both accumulators in flight (wraps every pipeline several times)."""
     torch.manual_seed(2)
     blocks = [5, 0, 7, 3, 9, 1, 4, 6]
@@ -60,10 +88,10 @@ def test_many_tiles_persistent_schedule():
     a = (torch.randn(rows, K, device="cuda") * 0.3).to(torch.bfloat16)
     w13 = (torch.randn(len(blocks), 2 * I, K, device="cuda") * 0.05).to(torch.bfloat16)
     w2 = (torch.randn(len(blocks), K, I, device="cuda") * 0.05).to(torch.bfloat16)
-    h = _check(a, w13, offsets, True)
-    _check(h, w2, offsets, False)
+    h = _check(a, w13, offsets, True, kernel)
+    _check(h, w2, offsets, False, kernel)
     # a small grid forces many tiles per CTA
-    out_small = gg.grouped_gemm(a, w13, offsets, swiglu=True, max_ctas=3)
+    out_small = gg.grouped_gemm(a, w13, offsets, swiglu=True, max_ctas=3, **_select(kernel, a))
     torch.cuda.synchronize()
     gg.check_status()
     assert torch.equal(out_small, h)
@@ -100,7 +128,7 @@ def test_cta_pair_kernel_matches_reference_and_single_cta(swiglu):
     K, N = 512, 512
     a = (torch.randn(rows, K, device="cuda") * 0.5).to(torch.bfloat16)
     w = (torch.randn(len(blocks), N, K, device="cuda") * 0.1).to(torch.bfloat16)
-    single = gg.grouped_gemm(a, w, offsets, swiglu=swiglu)
+    single = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select("single, four stages", a))
     n_out = N // 2 if swiglu else N
     out = torch.full((rows, n_out), float("nan"), dtype=torch.bfloat16, device="cuda")
     gg.grouped_gemm(a, w, offsets, swiglu=swiglu, pair=True, out=out)
@@ -109,10 +137,12 @@ def test_cta_pair_kernel_matches_reference_and_single_cta(swiglu):
     ref = gg.grouped_gemm_reference(a, w, offsets, swiglu=swiglu)
     torch.testing.assert_close(out.float(), ref, rtol=2e-2, atol=2e-2)
     assert torch.equal(out, single), "pair and single-CTA kernels accumulate in the same order"
+    gated = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select("pair, four stages", a))
+    three = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select("single, three stages", a))
     small = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, pair=True, max_ctas=4)
     torch.cuda.synchronize()
     gg.check_status()
-    assert torch.equal(small, single)
+    assert torch.equal(small, single) and torch.equal(gated, single) and torch.equal(three, single)
 
 
 def test_offsets_off_the_block_grid_are_reported():

@@ -417,3 +417,12 @@ def test_limited_ring_leaves_the_sm_to_the_gated_gemm():
         # without a limit the zero source is as long as a row where there is room
         assert ext.ring_plan(hidden, 8, 227 * 1024, False)[2] >= 2048
     assert ext.ring_plan(7168, 8, 227 * 1024, False)[2] > 2048
+
+
+def test_grouped_gemm_runs_the_kernel_it_is_asked_for():
+    from nanoep_b200.utils.build import load_extension
+
+    choice = load_extension().grouped_gemm_choice
+    assert choice() == "expert" and choice(max_ctas=2) == "expert"
+    assert choice(stages=3) == "single" and choice(max_ctas=1) == "single" and choice(gated=True) == choice(gated=True, stages=3) == "single"
+    assert choice(pair=True) == choice(pair=True, gated=True) == choice(pair=True, stages=3) == "pair"
