@@ -194,7 +194,6 @@ void bind_gemm(pybind11::module_& m) {
            const at::Tensor& slot_map, const at::Tensor& recv_metadata, c10::optional<at::Tensor> slot_weights, at::Tensor& status,
            int64_t max_ctas, double timeout_s, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows) {
             c10::cuda::CUDAGuard guard(a.device());
-            TORCH_CHECK(max_ctas != 1, "the fused combine needs pairs of CTAs");
             auto g = prepare(a, w, expert_offsets, status, gemm::kScatter, timeout_s);
             const WindowLayout& L = window.layout();
             TORCH_CHECK(w.size(1) == L.hidden, "down-projection N must equal the buffer's hidden size");
@@ -221,7 +220,8 @@ void bind_gemm(pybind11::module_& m) {
             g.args.ldo = L.hidden;
             if (a.size(0) == 0) return;
             PeerWindow::launches += 1;
-            const cudaError_t e = launch_expert(g, a, w, expert_counts, gemm::kScatter, max_expert_rows, max_ctas);
+            // the kernel works in pairs of CTAs: a cap of one means one pair
+            const cudaError_t e = launch_expert(g, a, w, expert_counts, gemm::kScatter, max_expert_rows, max_ctas == 1 ? 2 : max_ctas);
             TORCH_CHECK(e == cudaSuccess, "grouped GEMM (scatter) launch failed: ", cudaGetErrorString(e));
         },
         pybind11::arg("window"), pybind11::arg("a"), pybind11::arg("w"), pybind11::arg("expert_offsets"),

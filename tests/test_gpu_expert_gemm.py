@@ -9,6 +9,7 @@ import torch.distributed as dist
 from nanoep_b200 import CudaBuffer, EPConfig
 from nanoep_b200.models.moe_layer import ExpertParallelMoE, dense_reference
 from nanoep_b200.ops import grouped_gemm as gg
+from nanoep_b200.parallel.cuda_buffer import handle_metadata
 
 pytestmark = pytest.mark.gpu
 
@@ -104,3 +105,31 @@ def test_layer_on_one_rank(one_rank, tokens, fused):
             gg.check_status()
             want = dense_reference(x, idx, gate, w13, w2).float() + bias.float()
             torch.testing.assert_close(out.float(), want, rtol=3e-2, atol=3e-2)
+
+
+@pytest.mark.parametrize("max_ctas", [1, 2, 6])
+def test_scatter_on_a_small_grid(one_rank, max_ctas):
+    """The down-projection with the scatter epilogue takes any cap on its grid and gives the same bits."""
+    T, H, inner, E, K = 150, 256, 128, 3, 2
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x = (torch.randn(T, inner, device="cuda", generator=gen) * 0.5).to(torch.bfloat16)
+    w2 = (torch.randn(E, H, inner, device="cuda", generator=gen) * 0.1).to(torch.bfloat16)
+    idx = torch.rand(T, E, device="cuda", generator=gen).topk(K, dim=-1).indices
+    gate = torch.rand(T, K, device="cuda", generator=gen)
+    with CudaBuffer(one_rank, EPConfig(E, K, H, T)) as buf:
+        got = buf.dispatch(torch.zeros(T, H, dtype=torch.bfloat16, device="cuda"), topk_idx=idx, weights=gate, do_expand=True, alignment=128)
+        lay = got.handle.layout
+        h = torch.zeros(lay.expanded_capacity, inner, dtype=torch.bfloat16, device="cuda")
+        slots = lay.recv_metadata[:, 2:].long()
+        h[slots] = x[lay.recv_metadata[:, 1].long()][:, None].expand(-1, K, -1)
+        outs = []
+        for cap in (0, max_ctas):
+            gg._ext().grouped_gemm_scatter(buf.window, h, w2, lay.expert_offsets, got.handle.slot_map, lay.recv_metadata, got.topk_weights,
+                                           gg.status_tensor(h.device), cap, 5.0, lay.expert_counts, lay.recv_count)
+            outs.append(gg._ext().combine_finish([buf.window], [handle_metadata(got.handle)], [None])[0])
+        torch.cuda.synchronize()
+        buf.check_status()
+        gg.check_status()
+        assert torch.equal(outs[0], outs[1])
+        want = sum((x.float()[:, None] @ w2[idx[:, k]].float().transpose(1, 2))[:, 0] * gate[:, k, None] for k in range(K))
+        torch.testing.assert_close(outs[0].float(), want, rtol=1e-2, atol=2e-2)  # bf16 round per row and of the sum
