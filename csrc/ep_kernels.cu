@@ -79,9 +79,9 @@ __device__ bool wait_go(int* ctrl, uint64_t epoch, uint64_t timeout_ns, StatusRe
 // Receive counts to the host, which returns from the dispatch with them.  Later kernels of this stream see everything else
 // that this kernel writes, so no fence stands here in general.  A gated dispatch is the exception: its consumer runs on
 // another stream and reads expert_offsets and expert_counts as soon as the host has the counts, ordered behind nothing but
-// the mailbox.  Called by the thread that has observed (block or warp barrier) all of the block's writes to those two.
-__device__ __forceinline__ void publish_counts(volatile int64_t* mailbox, int64_t rows, int64_t capacity, bool gated) {
-    if (gated) __threadfence_system();
+// the mailbox (`ordered`).  Called by the thread that has observed (block or warp barrier) all of the block's writes to those two.
+__device__ __forceinline__ void publish_counts(volatile int64_t* mailbox, int64_t rows, int64_t capacity, bool ordered) {
+    if (ordered) __threadfence_system();
     mailbox[1] = capacity;
     mailbox[0] = rows;
 }
@@ -302,7 +302,9 @@ __device__ bool stage_body(const StageParams& p) {
                 ctrl[L.ctrl_expert_offsets() + Le] = carry;
             }
             __syncwarp();  // the other lanes' offsets; the counts are behind the block barrier above
-            if (lane == 0) publish_counts(p.mailbox, s_rows, carry, p.gated != 0);
+            // reports of invalid ids reach the host before the counts do (a group has passed the system fence of its
+            // peer barrier): the call after this one raises them
+            if (lane == 0) publish_counts(p.mailbox, s_rows, carry, p.gated != 0 || R == 1);
         }
         // Every source's per-chunk row counts become exclusive prefixes: chunk c of source s starts at receive row
         // recv_prefix[s] + chunk_prefix[s][c].  The total must equal the source's announced row count.
@@ -386,12 +388,14 @@ __device__ void local_plan_body(const LocalPlanParams& p) {
     int* s_rows = s_real + E;       // [kLocalPlanChunks] rows of this CTA's chunks of 32 tokens, then their prefix
     int* mine = s_rows + kLocalPlanChunks + warp * 32 * K;  // [32 * K] experts of the warp's chunk
     __shared__ int s_total;         // rows of this CTA (read by the other CTAs)
-    __shared__ int s_first, s_all, s_capacity;
+    __shared__ int s_invalid;       // a token of this CTA names an expert that does not exist (read by the other CTAs)
+    __shared__ int s_first, s_all, s_capacity, s_any_invalid;
     allow_dependents();
     wait_for_previous();
     const int chunks = (p.tokens + 31) / 32, per_cta = (chunks + ctas - 1) / ctas;
     const int first_chunk = cta * per_cta, my_chunks = max(0, min(per_cta, chunks - first_chunk));
     for (int i = tid; i < E; i += kLocalPlanThreads) s_count[i] = 0;
+    if (tid == 0) s_invalid = 0;
     __syncthreads();
 
     // experts of a chunk into the warp's buffer; `first` also snapshots, validates and counts them
@@ -414,8 +418,12 @@ __device__ void local_plan_body(const LocalPlanParams& p) {
                 mine[i] = valid ? int(raw[j]) : -1;
                 if (first) {
                     p.snapshot[base + i] = raw[j];
-                    if (valid) atomicAdd(&s_count[int(raw[j])], 1);
-                    else if (raw[j] != -1) report(status, kBadExpertId, uint32_t(tok0 + i / K), kTagStage);
+                    if (valid) {
+                        atomicAdd(&s_count[int(raw[j])], 1);
+                    } else if (raw[j] != -1) {
+                        report(status, kBadExpertId, uint32_t(tok0 + i / K), kTagStage);
+                        s_invalid = 1;
+                    }
                 }
             }
         }
@@ -462,7 +470,11 @@ __device__ void local_plan_body(const LocalPlanParams& p) {
         const int v = lane < ctas ? ld_cluster_smem(&s_total, uint32_t(lane)) : 0;
         const int incl = warp_inclusive_sum(v);
         if (lane == cta) s_first = incl - v;
-        if (lane == 31) s_all = incl;
+        const bool any = __any_sync(kFull, lane < ctas && ld_cluster_smem(&s_invalid, uint32_t(lane)) != 0);
+        if (lane == 31) {
+            s_all = incl;
+            s_any_invalid = any;
+        }
     }
     cluster_arrive();  // this CTA has read the others' counts; they may exit once everybody has
     __syncthreads();
@@ -488,7 +500,8 @@ __device__ void local_plan_body(const LocalPlanParams& p) {
             }
         }
         __syncwarp();  // the other lanes' offsets; the counts are behind the block barrier above
-        if (lane == 0 && cta == 0) publish_counts(p.mailbox, s_all, carry, p.gated != 0);
+        // the report of an invalid id reaches the host before the counts do: the call after this one raises it
+        if (lane == 0 && cta == 0) publish_counts(p.mailbox, s_all, carry, p.gated != 0 || s_any_invalid != 0);
     }
     __syncthreads();
     // ---- assign rows and slots

@@ -208,3 +208,24 @@ def test_single_rank_alignment_far_above_the_counts():
     idx = torch.full((4, 4), -1)
     idx[:, 2] = 3
     _one_rank_dispatch(idx, 16, 256, do_expand=True, alignment=1 << 19)
+
+
+@pytest.mark.parametrize("world", [1, 2])
+@pytest.mark.parametrize("tokens", [1, 700, 5000, 33000])  # one to eight CTAs, and no longer in one launch; the bad id is in the last token
+def test_invalid_expert_id_stops_the_next_call(world, tokens):
+    cfg = EPConfig(8, 2, 256, tokens)
+    with EmulatedGroup(world, cfg) as group:
+        x = [torch.zeros(tokens, 256, dtype=torch.bfloat16, device="cuda") for _ in range(world)]
+        idx = [torch.zeros(tokens, 2, dtype=torch.int64, device="cuda") for _ in range(world)]
+        for i in idx:
+            i[:, 1] = 1
+        idx[-1][-1, 1] = 8
+        torch.cuda.synchronize()
+        for _ in range(5):
+            group.dispatch(x, topk_idx=idx, do_expand=True, alignment=1)
+            with pytest.raises(RuntimeError, match="expert id"):  # no synchronisation in between
+                group.check_status()
+            torch.cuda.synchronize()
+            for w in group.windows:
+                w.clear_status(group.comm_stream.cuda_stream)
+            torch.cuda.synchronize()

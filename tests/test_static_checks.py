@@ -124,7 +124,7 @@ def test_receive_counts_follow_the_offsets_a_gated_consumer_reads():
     nothing but the mailbox: both planning kernels finish those tensors first and a gated dispatch fences in between."""
     text = re.sub(r"//[^\n]*", "", (ROOT / "csrc" / "ep_kernels.cu").read_text())
     publish = _body(text, "void publish_counts")
-    assert re.search(r"if \(gated\) __threadfence_system\(\);.*mailbox\[1\] = .*mailbox\[0\] = ", publish, re.S)
+    assert re.search(r"if \(ordered\) __threadfence_system\(\);.*mailbox\[1\] = .*mailbox\[0\] = ", publish, re.S)
     assert set(re.findall(r"mailbox\[[01]\] = ([^;]+);", text.replace(publish, ""))) == {"-2"}, "only the failure code goes another way"
     for kernel in ("bool stage_body", "void local_plan_body"):
         body = _body(text, kernel)
@@ -133,3 +133,18 @@ def test_receive_counts_follow_the_offsets_a_gated_consumer_reads():
         assert not re.search(r"p\.expert_(offsets|counts)\[[^\]]*\] = ", after), kernel
     host = (ROOT / "csrc" / "pipeline.cpp").read_text()
     assert re.search(r"gated = gated \|\| t\.has_value\(\);.*p\.gated = gated;.*lp\.gated = sp\.gated;", host, re.S)
+
+
+def test_an_invalid_expert_id_is_reported_before_the_counts():
+    """The call that follows a dispatch raises what the dispatch found, so the host sees the status word no later than N and C.
+    In a group the peer barrier's system fence lies between; a single rank fences, in the one-launch plan when a CTA of its
+    cluster reported."""
+    text = re.sub(r"//[^\n]*", "", (ROOT / "csrc" / "ep_kernels.cu").read_text())
+    body = _body(text, "void local_plan_body")
+    assert re.search(r"report\(status, kBadExpertId[^;]*;\s*s_invalid = 1;", body)
+    assert body.index("s_invalid = 1;") < body.index("cluster_wait();") < body.index("ld_cluster_smem(&s_invalid")
+    assert re.search(r"publish_counts\([^;]*s_any_invalid", body)
+    stage = _body(text, "bool stage_body")
+    assert re.search(r"publish_counts\([^;]*R == 1", stage)
+    assert stage.index("kBadExpertId") < stage.index("peer_barrier_warp(") < stage.index("publish_counts(")
+    assert re.search(r"if \(R > 1\) \{\s*__threadfence_system\(\);\s*__syncthreads\(\);\s*if \(warp == 0\) \{\s*const bool ok = peer_barrier_warp", stage)
