@@ -260,8 +260,9 @@ __device__ __forceinline__ uint32_t cluster_size() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
     return n;
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Not the `.aligned` forms: those ask for all threads of a warp at once, and the callers come out of loops that lanes leave early.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // the same shared-memory word in CTA `rank` of this cluster
 __device__ __forceinline__ int ld_cluster_smem(const int* own, uint32_t rank) {
     uint32_t addr;

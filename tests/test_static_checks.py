@@ -148,3 +148,14 @@ def test_an_invalid_expert_id_is_reported_before_the_counts():
     assert re.search(r"publish_counts\([^;]*R == 1", stage)
     assert stage.index("kBadExpertId") < stage.index("peer_barrier_warp(") < stage.index("publish_counts(")
     assert re.search(r"if \(R > 1\) \{\s*__threadfence_system\(\);\s*__syncthreads\(\);\s*if \(warp == 0\) \{\s*const bool ok = peer_barrier_warp", stage)
+
+
+def test_cluster_barriers_ask_for_a_whole_warp_only_behind_a_block_barrier():
+    """The `.aligned` cluster barrier needs every thread of a warp at the same instruction.  Lanes of the one-launch plan leave
+    its loops at different points; the GEMM kernels reach theirs through __syncthreads()."""
+    for path in _native_sources():
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(r"barrier\.cluster\.(arrive|wait)\.\w+\.aligned", text):
+            assert path.name == "tc_prim.cuh" and "void cluster_sync" in text[max(0, m.start() - 250) : m.start()], path.name
+        for m in re.finditer(r"\bcluster_sync\(\);", text):
+            assert re.search(r"__syncthreads\(\);\s*$", text[: m.start()]), path.name
