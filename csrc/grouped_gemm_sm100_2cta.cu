@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_pair_kernel(const __
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    __syncthreads();  // the abort flag is clear before anyone sets it
     for (int i = threadIdx.x; i <= args.num_experts; i += kThreads) {
         const int64_t off = args.expert_offsets[i];
         sh.offsets[i] = int(off);

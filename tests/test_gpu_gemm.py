@@ -145,14 +145,25 @@ def test_cta_pair_kernel_matches_reference_and_single_cta(swiglu):
     assert torch.equal(small, single) and torch.equal(gated, single) and torch.equal(three, single)
 
 
-def test_offsets_off_the_block_grid_are_reported():
+@pytest.mark.parametrize("kernel", KERNELS)
+def test_offsets_off_the_block_grid_are_reported(kernel):
     """One expert per 128-row block: offsets that are not multiples of 128, or that do not end at the row count, are refused."""
     a = torch.zeros(256, 128, dtype=torch.bfloat16, device="cuda")
     w = torch.zeros(2, 256, 128, dtype=torch.bfloat16, device="cuda")
     for bad in ([0, 100, 256], [0, 128, 128]):
-        out = gg.grouped_gemm(a, w, torch.tensor(bad, dtype=torch.int64, device="cuda"))
+        out = gg.grouped_gemm(a, w, torch.tensor(bad, dtype=torch.int64, device="cuda"), **_select(kernel, a))
         torch.cuda.synchronize()
         with pytest.raises(RuntimeError, match="expert_offsets"):
             gg.check_status()
         del out
+    # the only bad one of many: checked by a thread of another warp than the one that set the kernel up, and nothing is computed
+    w = torch.ones(70, 256, 128, dtype=torch.bfloat16, device="cuda")
+    bad = torch.zeros(71, dtype=torch.int64, device="cuda")
+    bad[65:] = 128
+    out = torch.full((256, 256), 7.0, dtype=torch.bfloat16, device="cuda")
+    gg.grouped_gemm(a, w, bad, out=out, **_select(kernel, a))
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="expert_offsets.*detail 70"):
+        gg.check_status()
+    assert (out == 7).all()
     assert torch.ones(2, device="cuda").sum().item() == 2

@@ -159,3 +159,10 @@ def test_cluster_barriers_ask_for_a_whole_warp_only_behind_a_block_barrier():
             assert path.name == "tc_prim.cuh" and "void cluster_sync" in text[max(0, m.start() - 250) : m.start()], path.name
         for m in re.finditer(r"\bcluster_sync\(\);", text):
             assert re.search(r"__syncthreads\(\);\s*$", text[: m.start()]), path.name
+
+
+def test_gemm_kernels_clear_their_abort_flag_before_anyone_sets_it():
+    """Every thread checks offsets and may set the flag; the thread that clears it must have done so before."""
+    for name in ("grouped_gemm_sm100.cu", "grouped_gemm_sm100_2cta.cu", "expert_gemm_sm100.cu"):
+        text = re.sub(r"//[^\n]*", "", (ROOT / "csrc" / name).read_text())
+        assert "__syncthreads();" in text[text.index("sh.abort = 0;") : text.index("sh.abort = 1;")], name
