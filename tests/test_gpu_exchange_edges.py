@@ -135,7 +135,8 @@ def test_reduction_with_many_stages(setting):
     try:
         with EmulatedGroup(world, cfg) as group:
             got = group.dispatch(_cuda(case.xs), topk_idx=_cuda(case.indices), weights=_cuda(case.weights), do_expand=True, alignment=1)
-            back = group.combine([g.x for g in got], [g.handle for g in got], weights=[g.topk_weights for g in got])
+            # two CTAs per rank: 150 tokens of one to four chunks each go round the ring
+            back = group.combine([g.x for g in got], [g.handle for g in got], weights=[g.topk_weights for g in got], num_sms=2)
             torch.cuda.synchronize()
             group.check_status()
             for r in range(world):

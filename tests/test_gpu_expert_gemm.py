@@ -133,3 +133,30 @@ def test_scatter_on_a_small_grid(one_rank, max_ctas):
         assert torch.equal(outs[0], outs[1])
         want = sum((x.float()[:, None] @ w2[idx[:, k]].float().transpose(1, 2))[:, 0] * gate[:, k, None] for k in range(K))
         torch.testing.assert_close(outs[0].float(), want, rtol=1e-2, atol=2e-2)  # bf16 round per row and of the sum
+
+
+@pytest.mark.parametrize("hidden", [512, 4096])  # 4096: the pull's rings fill their limit, and the gated GEMM has to fit beside them
+@pytest.mark.parametrize("pairs", [None, False, True])
+def test_overlapped_layer_on_one_rank(one_rank, hidden, pairs):
+    """The gated up-projection beside the dispatch that fills its row blocks: same result as one after the other, no wait runs out."""
+    T, inner, E, K = 1500, 256, 6, 3
+    gen = torch.Generator(device="cuda").manual_seed(hidden)
+    w13 = (torch.randn(E, 2 * inner, hidden, device="cuda", generator=gen) * 0.03).to(torch.bfloat16)
+    w2 = (torch.randn(E, hidden, inner, device="cuda", generator=gen) * 0.06).to(torch.bfloat16)
+    with CudaBuffer(one_rank, EPConfig(E, K, hidden, T)) as buf:
+        overlapped = ExpertParallelMoE(buf, w13, w2, overlap_dispatch=True, cta_pairs=pairs)
+        plain = ExpertParallelMoE(buf, w13, w2)
+        for _ in range(3):
+            x = (torch.randn(T, hidden, device="cuda", generator=gen) * 0.5).to(torch.bfloat16)
+            gate, idx = torch.rand(T, E, device="cuda", generator=gen).topk(K, dim=-1)
+            idx = torch.where(torch.rand(T, K, device="cuda", generator=gen) < 0.1, -1, idx)
+            for handle in (None, True):
+                routing = dict(handle=overlapped.last_handle) if handle else {}
+                got = overlapped(x, None if handle else idx, gate, **routing)
+                torch.cuda.synchronize()
+                buf.check_status()
+                gg.check_status()
+                want = plain(x, idx, gate)
+                torch.cuda.synchronize()
+                # the same products, added in another order by the two GEMM kernels: bf16 rounds of h, of a row and of the sum
+                torch.testing.assert_close(got.float(), want.float(), rtol=3e-2, atol=3e-2)

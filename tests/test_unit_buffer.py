@@ -409,11 +409,12 @@ def test_limited_ring_leaves_the_sm_to_the_gated_gemm():
     ext = load_extension()
     limit = inspect.signature(ExpertParallelMoE).parameters["comm_ring_bytes"].default
     sm, reserved = 228 * 1024, 1024  # shared memory of an SM; the system's share of every resident block
+    static = 128  # the pull kernel's own variables
     for hidden in (1536, 2048, 3072, 4096, 5120, 5632, 6144, 7168, 8192):
         warps, stages, zeros, smem = ext.ring_plan(hidden, 8, limit, True)
         pitch = (hidden * 2 + 32 + 127) // 128 * 128
         assert warps >= 2 and zeros == 2048 and smem == warps * stages * (pitch + 8) + zeros + 256
-        assert smem + reserved + ext.gemm_shared_bytes(3) + reserved <= sm, hidden
+        assert smem + static + reserved + ext.gemm_shared_bytes(3) + reserved <= sm, hidden
         # without a limit the zero source is as long as a row where there is room
         assert ext.ring_plan(hidden, 8, 227 * 1024, False)[2] >= 2048
     assert ext.ring_plan(7168, 8, 227 * 1024, False)[2] > 2048
