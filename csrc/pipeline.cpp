@@ -3,9 +3,9 @@
 //
 // Same responsibilities as the reference's host pipeline (csrc/pipeline.cu:26-489 plus
 // dispatch_epilogue.cpp / combine_epilogue.cpp): one native call per Python operation; inputs are
-// ordered behind the caller's stream or an explicit event; outputs are allocated with their exact
-// size in the consumer stream's allocator pool; the only host wait is the N/C mailbox of a fresh
-// dispatch.  Every entry point takes a *list* of ranks: one element in production, R elements when a
+// ordered behind the caller's stream or an explicit event; outputs have their exact size (a small call of a
+// single rank fills tensors of its upper bound first and copies what is smaller) and live in the consumer stream's
+// allocator pool; the only host wait is the N/C mailbox of a fresh dispatch.  Every entry point takes a *list* of ranks: one element in production, R elements when a
 // whole logical group shares one GPU (tests) -- then each phase is a single multi-rank launch.
 #include "pipeline.hpp"
 

@@ -5,14 +5,16 @@
 The reference library leaves the expert computation to the caller (its example uses element-wise
 experts, nano_ep/examples/moe.py:19-40).  This layer is the fused path:
 
-* dispatch runs with the expert-major layout, 128-row alignment and zero padding, with a small
-  shared-memory ring per SM, and announces every finished row in per-block counters;
-* the up/gate grouped GEMM (SwiGLU epilogue) starts at once on the SAME SMs (its operand pipeline is
-  one stage shorter so both kernels fit in shared memory) and consumes row blocks as their counters
-  fill, so the NVLink pull hides under tensor-core work;
-* the down-projection GEMM applies the gate weight in FP32 in its epilogue, stages each bf16 output
-  row in shared memory and bulk-stores it straight into the source rank's return partition over
-  NVLink; a peer barrier and the source-side FP32 reduction finish the combine.
+* dispatch with the expert-major layout and 128-row alignment; its padding rows are not written, because a GEMM row
+  depends on its own input row alone and the combine takes real rows only;
+* the up/gate grouped GEMM (SwiGLU epilogue) and the down-projection compute the rows that exist (the dispatch's counts);
+* the down-projection applies the gate weight in FP32 in its epilogue and stores whole bf16 token rows straight into
+  the source rank's return partition, over NVLink or locally; a peer barrier (more than one rank) and the source-side
+  FP32 reduction finish the combine.
+
+With ``overlap_dispatch=True`` the dispatch runs on the communication stream with zero padding and a small shared-memory
+ring per SM and announces every finished row in per-block counters; the up/gate GEMM starts at once on the SAME SMs (its
+operand pipeline is shorter so that both kernels fit in shared memory) and consumes row blocks as their counters fill.
 
 ``fuse_combine=False`` / ``overlap_dispatch=False`` select the unfused compositions of the same
 public operations (used as correctness and performance baselines).

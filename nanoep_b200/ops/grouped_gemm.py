@@ -1,8 +1,9 @@
 """Grouped GEMM over expert-major rows (tcgen05 / TMEM kernels, csrc/expert_gemm_sm100.cu; gated by row counters:
 csrc/grouped_gemm_sm100.cu and its CTA-pair variant).
 
-``rows`` come from a dispatch with ``do_expand=True, alignment=128, zero_padding=True``: every
-128-row block belongs to one expert, padding rows are zero.  The reference library stops at
+``rows`` come from a dispatch with ``do_expand=True, alignment=128``: every 128-row block belongs to one expert.  Padding rows
+may hold anything (``expert_counts`` says how many rows of an expert exist) unless row blocks are gated by counters, which
+count them too (``zero_padding=True``).  The reference library stops at
 dispatch/combine; these ops are the expert compute that sits between them on the same GPU.
 """
 
