@@ -30,7 +30,7 @@ constexpr int kFusedDispatchDefaultTokens = 64;
 constexpr int kFusedFreshDefaultTokens = 0;  // single-launch fresh dispatch: off unless asked for (the host waits for N and C either way)
 constexpr int64_t kFusedFreshMaxOutputBytes = int64_t(256) << 20;  // single-launch fresh dispatch: largest bound-sized output
 constexpr int64_t kLocalPlanMaxHandleBytes = int64_t(16) << 20;    // single-rank plan: largest bound-sized handle
-constexpr int64_t kEarlyPullMaxOutputBytes = int64_t(32) << 20;    // single-rank pull that does not wait for N and C: see dispatch()
+constexpr int64_t kEarlyPullMaxOutputBytes = int64_t(16) << 20;    // single-rank pull that does not wait for N and C: see dispatch()
 constexpr int kFusedDefaultBlocks = 1024;  // i.e. bounded by the SM budget and co-residency only
 
 void cuda_check(cudaError_t e, const char* what) {
@@ -177,6 +177,13 @@ at::Tensor part_of(const at::Tensor& base, int64_t offset, at::IntArrayRef sizes
     at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(base.storage()), base.key_set(), base.dtype());
     t.unsafeGetTensorImpl()->set_storage_offset(base.storage_offset() + offset);
     t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    return t;
+}
+
+// A tensor of its own with what `piece` shows (clone() without the dispatcher).
+at::Tensor own_copy(const at::Tensor& piece, int device, cudaStream_t stream) {
+    at::Tensor t = make_empty(piece.sizes(), piece.scalar_type(), device);
+    if (piece.numel() > 0) cuda_check(cudaMemcpyAsync(t.data_ptr(), piece.data_ptr(), piece.nbytes(), cudaMemcpyDeviceToDevice, stream), "copy to exact size");
     return t;
 }
 
@@ -570,7 +577,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         c10::cuda::CUDAStreamGuard pool(consumer);
         auto trim = [&](at::Tensor& t, at::IntArrayRef sizes) {
             const at::Tensor view = part_of(t, 0, sizes);
-            if (view.numel() < t.numel()) t = early_pull ? view.clone() : view;
+            if (view.numel() < t.numel()) t = early_pull ? own_copy(view, device, cs) : view;
         };
         for (int i = 0; i < n; ++i) {
             std::pair<int64_t, int64_t> nc;
@@ -598,8 +605,8 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             // unless that is no more than what the allocator rounds up anyway.
             const int64_t used = m[0].numel() + m[7].numel(), held = bound_cells + bound_slots;
             if (plan_locally && held * 4 > (int64_t(1) << 20) && used * 2 < held) {
-                m[0] = m[0].clone();
-                m[7] = m[7].clone();
+                m[0] = own_copy(m[0], device, cs);
+                m[7] = own_copy(m[7], device, cs);
             }
         }
     }
