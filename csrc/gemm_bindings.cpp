@@ -114,13 +114,28 @@ cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& 
 }
 
 // Which kernel a grouped_gemm call runs.  The one with tokens as N is the faster one (expert_gemm_sm100.cu has both sides), but it
-// takes all of an SM's shared memory and works in pairs of CTAs: row blocks gated by counters (which share the SMs with the dispatch that fills them), a
-// caller who asks for CTA pairs or for the three-stage pipeline (smaller, to run beside another kernel), and a call that
-// may use a single CTA get the kernels with tokens as M.
+// takes all of an SM's shared memory and works in pairs of CTAs: row blocks gated by counters (which share the SMs with the
+// dispatch that fills them), a caller who asks for CTA pairs or for the three-stage pipeline (smaller, to run beside another
+// kernel), and a call that may use a single CTA get the kernels with tokens as M.
+// So do two kinds of call that the single-CTA kernel serves better, where every row of every range exists (with counts the other
+// kernel leaves rows out).  Nearly no K: the accumulator's way out is the whole kernel, and it is longer for the transposed
+// one (K = 64, N = 256 to 4096, 1 to 128 experts of 1 to 9 blocks: 12-444 us against 12-485, 1.11x on average; at K = 256 1.03x,
+// from 768 on the other way).  And calls whose 128-row tiles fit the GPU once while the pairs' tiles need a second wave
+// (one expert of 1152 rows, N = 4096: 32 against 50 us at K = 2048, 52 against 71 with SwiGLU at K = 4096).
 enum Kernel { kExpertKernel, kPairKernel, kSingleKernel };
-Kernel choose_kernel(bool gated, bool pair, int64_t stages, int64_t max_ctas) {
-    if (pair) return kPairKernel;
-    return gated || stages == 3 || max_ctas == 1 ? kSingleKernel : kExpertKernel;
+struct Choice {
+    bool gated, pair;
+    int64_t stages, max_ctas;
+    bool swiglu, counts;
+    int64_t m_blocks, n_tiles, K, sms;
+};
+Kernel choose_kernel(const Choice& c) {
+    if (c.pair) return kPairKernel;
+    if (c.gated || c.stages == 3 || c.max_ctas == 1) return kSingleKernel;
+    if (c.counts) return kExpertKernel;
+    const int64_t ctas = c.max_ctas > 0 ? std::min(c.max_ctas, c.sms) : c.sms;
+    const bool one_wave_of_singles = c.m_blocks * c.n_tiles <= ctas && (c.m_blocks + 1) / 2 * c.n_tiles > ctas / 2;
+    return (!c.swiglu && c.K <= 128) || one_wave_of_singles ? kSingleKernel : kExpertKernel;
 }
 
 }  // namespace
@@ -159,7 +174,9 @@ void bind_gemm(pybind11::module_& m) {
             if (a.size(0) == 0) return;
             const int grid = max_ctas > 0 ? std::min<int>(g.grid, int(max_ctas)) : g.grid;
             PeerWindow::launches += 1;
-            const Kernel kernel = choose_kernel(tile_ready.has_value(), pair, stages, max_ctas);
+            const Kernel kernel = choose_kernel(Choice{tile_ready.has_value(), pair, stages, max_ctas, mode == gemm::kSwiGLU, expert_counts.has_value(),
+                                                       g.args.m_blocks, g.args.n_tiles, a.size(1),
+                                                       at::cuda::getCurrentDeviceProperties()->multiProcessorCount});
             if (kernel == kExpertKernel) {
                 cudaError_t ee = launch_expert(g, a, w, expert_counts, int(mode), max_expert_rows, max_ctas);
                 TORCH_CHECK(ee == cudaSuccess, "grouped GEMM (expert) launch failed: ", cudaGetErrorString(ee));
@@ -231,11 +248,13 @@ void bind_gemm(pybind11::module_& m) {
 
     m.def(
         "grouped_gemm_choice",
-        [](bool gated, bool pair, int64_t stages, int64_t max_ctas) -> std::string {
-            const Kernel kernel = choose_kernel(gated, pair, stages, max_ctas);
+        [](bool gated, bool pair, int64_t stages, int64_t max_ctas, bool swiglu, bool counts, int64_t rows, int64_t n, int64_t k, int64_t sms) -> std::string {
+            const Kernel kernel = choose_kernel(Choice{gated, pair, stages, max_ctas, swiglu, counts, rows / 128, n / 256, k, sms});
             return kernel == kExpertKernel ? "expert" : kernel == kPairKernel ? "pair" : "single";
         },
         pybind11::arg("gated") = false, pybind11::arg("pair") = false, pybind11::arg("stages") = 4, pybind11::arg("max_ctas") = 0,
+        pybind11::arg("swiglu") = false, pybind11::arg("counts") = false, pybind11::arg("rows") = 1 << 16, pybind11::arg("n") = 4096,
+        pybind11::arg("k") = 4096, pybind11::arg("sms") = 148,
         "Kernel that a grouped_gemm call with these arguments runs");
     m.def("gemm_kernel_registers", [](int64_t mode) { return gemm::kernel_registers(int(mode)); });
     m.def("gemm_shared_bytes", [](int64_t stages) { return int64_t(gemm::shared_bytes(int(stages))); });

@@ -15,25 +15,27 @@ def _offsets(blocks_per_expert):
     return torch.tensor(rows, dtype=torch.int64, device="cuda")
 
 
-# Arguments that select each kernel; "gated" stands for row counters that are all full.
+# Arguments that select each kernel; "gated" stands for row counters that are all full, "counts" for experts whose rows all exist.
 KERNELS = {
-    "expert": {}, "single, three stages": dict(stages=3), "single, four stages": dict(gated=True), "pair, six stages": dict(pair=True),
+    "by size": {}, "expert": dict(counts=True), "single, three stages": dict(stages=3), "single, four stages": dict(gated=True), "pair, six stages": dict(pair=True),
     "pair, four stages": dict(pair=True, gated=True),
 }
 
 
-def _select(kernel, a):
+def _select(kernel, a, offsets):
     args = dict(KERNELS[kernel])
+    choice = gg._ext().grouped_gemm_choice(rows=128, n=256, k=64, **args)
+    assert choice == ("single" if kernel == "by size" else kernel.split(",")[0])
     if args.pop("gated", False):
         full = torch.full((a.shape[0] // 128,), 128, dtype=torch.int32, device="cuda")
         args.update(tile_ready=full, tile_expected=full)
-    choice = gg._ext().grouped_gemm_choice(gated="tile_ready" in args, **{k: v for k, v in args.items() if k in ("pair", "stages")})
-    assert choice == kernel.split(",")[0]
+    if args.pop("counts", False):
+        args.update(expert_counts=(offsets[1:] - offsets[:-1]).contiguous())
     return args
 
 
-def _check(a, w, offsets, swiglu, kernel="expert"):
-    out = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select(kernel, a))
+def _check(a, w, offsets, swiglu, kernel="by size"):
+    out = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select(kernel, a, offsets))
     torch.cuda.synchronize()
     gg.check_status()
     ref = gg.grouped_gemm_reference(a, w, offsets, swiglu=swiglu)
@@ -62,13 +64,13 @@ def test_identity_weights_expose_layout_errors(kernel):
     a = torch.randn(384, K, device="cuda").to(torch.bfloat16)
     w = torch.eye(N, K, device="cuda").to(torch.bfloat16).repeat(2, 1, 1).contiguous()
     w[1] *= 2
-    out = gg.grouped_gemm(a, w, offsets, **_select(kernel, a))
+    out = gg.grouped_gemm(a, w, offsets, **_select(kernel, a, offsets))
     torch.cuda.synchronize()
     gg.check_status()
     assert torch.equal(out[:256], a[:256])
     assert torch.equal(out[256:], (a[256:].float() * 2).to(torch.bfloat16))
     scale = torch.rand(384, device="cuda") + 0.5
-    scaled = gg.grouped_gemm(a, w, offsets, row_scale=scale, **_select(kernel, a))
+    scaled = gg.grouped_gemm(a, w, offsets, row_scale=scale, **_select(kernel, a, offsets))
     torch.cuda.synchronize()
     gg.check_status()
     factor = torch.ones(384, 1, device="cuda")
@@ -91,7 +93,7 @@ def test_many_tiles_persistent_schedule(kernel):
     h = _check(a, w13, offsets, True, kernel)
     _check(h, w2, offsets, False, kernel)
     # a small grid forces many tiles per CTA
-    out_small = gg.grouped_gemm(a, w13, offsets, swiglu=True, max_ctas=3, **_select(kernel, a))
+    out_small = gg.grouped_gemm(a, w13, offsets, swiglu=True, max_ctas=3, **_select(kernel, a, offsets))
     torch.cuda.synchronize()
     gg.check_status()
     assert torch.equal(out_small, h)
@@ -118,6 +120,20 @@ def test_tile_gating_waits_for_ready_counters():
     assert torch.ones(2, device="cuda").sum().item() == 2
 
 
+@pytest.mark.parametrize("K,N,blocks", [(64, 512, [1, 2]), (128, 256, [3]), (192, 256, [3]), (256, 4096, [9]), (256, 4096, [10]), (256, 4096, [8])])
+def test_sizes_on_both_sides_of_the_choice(K, N, blocks):
+    """Short K and one wave of single-CTA tiles go to the single-CTA kernel; its neighbours to the expert kernel."""
+    torch.manual_seed(11)
+    offsets = _offsets(blocks)
+    rows = int(offsets[-1])
+    a = (torch.randn(rows, K, device="cuda") * 0.5).to(torch.bfloat16)
+    w = (torch.randn(len(blocks), N, K, device="cuda") * 0.1).to(torch.bfloat16)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    choice = gg._ext().grouped_gemm_choice(rows=rows, n=N, k=K, sms=sms)
+    assert choice == ("single" if K <= 128 or blocks == [9] else "expert")
+    _check(a, w, offsets, False)
+
+
 @pytest.mark.parametrize("swiglu", [False, True])
 def test_cta_pair_kernel_matches_reference_and_single_cta(swiglu):
     """tcgen05 cta_group::2 variant: experts with odd and even block counts, an empty expert, many tiles."""
@@ -128,7 +144,7 @@ def test_cta_pair_kernel_matches_reference_and_single_cta(swiglu):
     K, N = 512, 512
     a = (torch.randn(rows, K, device="cuda") * 0.5).to(torch.bfloat16)
     w = (torch.randn(len(blocks), N, K, device="cuda") * 0.1).to(torch.bfloat16)
-    single = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select("single, four stages", a))
+    single = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select("single, four stages", a, offsets))
     n_out = N // 2 if swiglu else N
     out = torch.full((rows, n_out), float("nan"), dtype=torch.bfloat16, device="cuda")
     gg.grouped_gemm(a, w, offsets, swiglu=swiglu, pair=True, out=out)
@@ -137,8 +153,8 @@ def test_cta_pair_kernel_matches_reference_and_single_cta(swiglu):
     ref = gg.grouped_gemm_reference(a, w, offsets, swiglu=swiglu)
     torch.testing.assert_close(out.float(), ref, rtol=2e-2, atol=2e-2)
     assert torch.equal(out, single), "pair and single-CTA kernels accumulate in the same order"
-    gated = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select("pair, four stages", a))
-    three = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select("single, three stages", a))
+    gated = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select("pair, four stages", a, offsets))
+    three = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, **_select("single, three stages", a, offsets))
     small = gg.grouped_gemm(a, w, offsets, swiglu=swiglu, pair=True, max_ctas=4)
     torch.cuda.synchronize()
     gg.check_status()
@@ -151,7 +167,8 @@ def test_offsets_off_the_block_grid_are_reported(kernel):
     a = torch.zeros(256, 128, dtype=torch.bfloat16, device="cuda")
     w = torch.zeros(2, 256, 128, dtype=torch.bfloat16, device="cuda")
     for bad in ([0, 100, 256], [0, 128, 128]):
-        out = gg.grouped_gemm(a, w, torch.tensor(bad, dtype=torch.int64, device="cuda"), **_select(kernel, a))
+        offsets = torch.tensor(bad, dtype=torch.int64, device="cuda")
+        out = gg.grouped_gemm(a, w, offsets, **_select(kernel, a, offsets))
         torch.cuda.synchronize()
         with pytest.raises(RuntimeError, match="expert_offsets"):
             gg.check_status()
@@ -161,7 +178,7 @@ def test_offsets_off_the_block_grid_are_reported(kernel):
     bad = torch.zeros(71, dtype=torch.int64, device="cuda")
     bad[65:] = 128
     out = torch.full((256, 256), 7.0, dtype=torch.bfloat16, device="cuda")
-    gg.grouped_gemm(a, w, bad, out=out, **_select(kernel, a))
+    gg.grouped_gemm(a, w, bad, out=out, **_select(kernel, a, bad))
     torch.cuda.synchronize()
     with pytest.raises(RuntimeError, match="expert_offsets.*detail 70"):
         gg.check_status()

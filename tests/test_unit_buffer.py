@@ -427,3 +427,18 @@ def test_grouped_gemm_runs_the_kernel_it_is_asked_for():
     assert choice() == "expert" and choice(max_ctas=2) == "expert"
     assert choice(stages=3) == "single" and choice(max_ctas=1) == "single" and choice(gated=True) == choice(gated=True, stages=3) == "single"
     assert choice(pair=True) == choice(pair=True, gated=True) == choice(pair=True, stages=3) == "pair"
+
+
+def test_grouped_gemm_choice_by_size():
+    """Calls that are faster with tokens as M: nearly no K, and one wave of 128-row tiles where pairs of them need two."""
+    from nanoep_b200.utils.build import load_extension
+
+    choice = load_extension().grouped_gemm_choice
+    assert choice(k=128) == "single" and choice(k=192) == "expert" and choice(k=128, swiglu=True) == "expert"
+    assert choice(k=64, counts=True) == "expert"
+    for rows, want in ((7 * 128, "expert"), (8 * 128, "expert"), (9 * 128, "single"), (10 * 128, "expert")):
+        assert choice(rows=rows, n=4096, sms=148) == want, rows
+        assert choice(rows=rows, n=4096, swiglu=True, sms=148) == want, rows
+        assert choice(rows=rows, n=4096, sms=148, counts=True) == "expert"
+    # a cap on the grid moves the line: three tiles, three CTAs, but one pair
+    assert choice(rows=384, n=256, max_ctas=3) == "single" and choice(rows=384, n=256, max_ctas=4) == "expert"
