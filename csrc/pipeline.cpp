@@ -401,6 +401,8 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     // launched behind the plan without waiting for the counts where the bound is what a call without masked choices
     // receives (with an alignment the bound counts padding that hardly any routing has).  A call that receives less gets its
     // outputs copied to their exact size below, so the limit on the bound lies where that copy takes as long as the wait.
+    // Dispatch of 1 to 128 tokens of 7168, top-8, per call: 25 us against 30 with the wait; with a tenth of the choices
+    // masked 33 against 30.
     const int64_t bound_bytes = (expand ? bound_rows_c : bound_rows_n) * L.hidden * 2;
     const bool early_pull =
         plan_locally && (!expand || alignment == 1) && !gated && !g_gate.word.defined() && bound_bytes <= kEarlyPullMaxOutputBytes;
