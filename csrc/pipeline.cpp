@@ -450,8 +450,9 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             g_marks.mark("plan", cs);
         } else if (!fuse_small && !fuse_fresh && !(local && !fresh)) {
             PeerWindow::launches += 1;
-            // 16 warps per block, 4 row quarters per token: small calls get small grids
-            const int stage_grid = int(std::max<int64_t>(1, std::min<int64_t>(2 * num_sms, (max_tokens_now * 4 + 15) / 16)));
+            // 16 warps per block, 4 row quarters per token: small calls get small grids; one block of a fresh dispatch exchanges
+            // the counts instead of copying
+            const int stage_grid = int(std::max<int64_t>(1, std::min<int64_t>(2 * num_sms, (max_tokens_now * 4 + 15) / 16 + (fresh ? 1 : 0))));
             cuda_check(launch_stage(stage_dev, LaunchShape{stage_grid, n}, size_t(stage_smem_bytes(L)), cs), "stage launch");
             g_marks.mark("stage", cs);
         }
