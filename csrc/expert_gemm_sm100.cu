@@ -22,6 +22,16 @@
 // tiles per token tile (a quarter less ingress, one accumulator each) ran at 1.3 GHz and the same power: up 1707, down 823 us.
 // In between, 4662 rows over 32 experts of 4096 x 1536: up 209 -> 163 us, down 121 -> 86 us.
 //
+// Who computes what.  The grid holds a cluster for every unit (one weight tile x one token tile) that the offsets allow; the
+// clusters that run take over the places of those that have not started (cluster launch control), in order, one or two
+// units ahead.  With a fixed share of the units per cluster, clusters that share a weight tile drift apart by more than
+// L2 keeps it (small differences add up over units of 100 us) and fetch it again: the up-projection of 32 experts of 1024
+// rows read 4.0-5.3 GB from memory instead of the 2.35 GB that there are, now 2.5-2.7 GB, and at the power limit every byte costs
+// clock.  us, fixed share -> taken over: 32 x 1024 rows up 1325 -> 1260, 0.8 s in a row 1533 -> 1480, down 660 -> 648, 785 -> 770; 32 x (1024
+// +- 32) up 1410 -> 1345, 0.8 s in a row 1650 -> 1566, down 692 -> 686; 4662 uneven rows (4096 x 1536) up 165 -> 158, down 91 -> 85.  The readers of a unit
+// acknowledge it without a fence: a releasing arrival waits for the thread's bulk loads in flight and drained the
+// operand pipeline at every unit (tensor pipe 98 -> 93 % active up, 96 -> 80 % down).  A launch with a cap on its CTAs keeps fixed shares.
+//
 // All waits are bounded; on expiry a CTA records a code in `status`, stops issuing work, and both CTAs still meet at the
 // final cluster barrier and free their TMEM.
 #include "grouped_gemm_sm100.hpp"
@@ -48,6 +58,8 @@ constexpr int kMaxExperts = 1024;
 constexpr int kMaxStages = 10;
 constexpr int kChunk = 32;                   // token rows staged at a time by a group
 constexpr int kMaxTokens = 256;              // largest N
+constexpr int kUnitReaders = 5;              // readers of a handed-out unit: two producers, the MMA issuer, two epilogues
+constexpr int kUnitSlots = 2;                // units handed out ahead of their readers
 
 template <int kMode>
 struct Out {
@@ -58,10 +70,14 @@ struct Out {
 };
 
 struct Shared {
+    alignas(16) uint32_t cancelled[4];  // answer to a request for the next cluster's place (CTA 1)
     uint64_t full[kMaxStages], empty[kMaxStages], tmem_full[2], tmem_empty[2];
+    uint64_t cancel_done, unit_full[kUnitSlots], unit_empty[kUnitSlots];
     uint32_t tmem_base;
     int abort;
     int go[2];
+    int next_unit[kUnitSlots];  // handed out by the scheduler, -1: none
+    int epi_unit[2];   // the epilogue's unit, by parity of the item
     int offsets[kMaxExperts + 1];       // first row
     int rows[kMaxExperts];              // rows to compute
     int first_tile[kMaxExperts + 1];    // exclusive prefix of token tiles
@@ -114,6 +130,45 @@ __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorM
                  "l"(map), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
                  : "memory");
 }
+// Takes over the place of a cluster of this grid that has not started: 16 bytes of answer, counted in on `bar`.
+__device__ __forceinline__ void request_cluster(void* answer, uint64_t* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(answer)),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
+// First CTA of the cluster taken over, or -1 when none was left.
+__device__ __forceinline__ int cancelled_cta(const void* answer) {
+    uint32_t taken, x;
+    asm volatile(
+        "{\n .reg .b128 r;\n .reg .pred p;\n mov.b32 %1, 0;\n ld.shared.b128 r, [%2];\n"
+        " clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n selp.u32 %0, 1, 0, p;\n"
+        " @p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, _, _, _}, r;\n}"
+        : "=&r"(taken), "=&r"(x)
+        : "r"(smem_u32(answer))
+        : "memory");
+    return taken ? int(x) : -1;
+}
+__device__ __forceinline__ void st_cluster(uint32_t cluster_addr, int v) {
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+}
+// Arrival behind the read that gave `value` (an operand of the statement, so the read is done), without the fence of a releasing one.
+__device__ __forceinline__ void arrive_after(uint32_t cluster_addr, int value) {
+    asm volatile("{\n .reg .b32 v;\n mov.b32 v, %1;\n mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n}" ::"r"(cluster_addr), "r"(value) : "memory");
+}
+// Bounded wait that also orders what the other CTA of the pair wrote before its arrival.
+__device__ __forceinline__ bool mbar_wait_pair(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
+    const uint64_t start = timer_ns();
+    uint32_t spins = 0;
+    for (;;) {
+        uint32_t done;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(smem_u32(bar)), "r"(parity)
+                     : "memory");
+        if (done) return true;
+        if ((++spins & 1023u) == 0u && timer_ns() - start > limit_ns) return false;
+    }
+}
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); }
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory"); }
 
@@ -138,6 +193,11 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
         for (int a = 0; a < 2; ++a) {
             mbar_init(&sh.tmem_full[a], 1);
             mbar_init(&sh.tmem_empty[a], 2 * kEpiThreads / 32);  // leader: the epilogue warps of both CTAs
+        }
+        mbar_init(&sh.cancel_done, 1);
+        for (int u = 0; u < kUnitSlots; ++u) {
+            mbar_init(&sh.unit_full[u], 1);
+            mbar_init(&sh.unit_empty[u], kUnitReaders);
         }
         sh.abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -201,12 +261,27 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
         if (atomicCAS(args.status, 0u, code) == 0u) args.status[1] = blockIdx.x;
     };
 
+    // The unit behind `unit` for one reader (one thread), -1 at the end; `item` counts the reader's units.
+    auto next_unit = [&](int unit, int item) -> int {
+        if (*abort_flag) return -1;
+        if (!args.dynamic) return unit + num_clusters < units ? unit + num_clusters : -1;
+        const int slot = item % kUnitSlots;
+        if (!mbar_wait_pair(&sh.unit_full[slot], uint32_t(item / kUnitSlots) & 1u, limit_ns)) {
+            fail(kGemmPipeTimeout);
+            return -1;
+        }
+        const int next = *(volatile int*)&sh.next_unit[slot];
+        arrive_after(map_to_cta(smem_u32(&sh.unit_empty[slot]), 1), next);
+        return next;
+    };
+    const int first_unit = cluster_id < units ? cluster_id : -1;
+
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)
         if (elect_one()) {
-            int stage = 0;
+            int stage = 0, item = 0;
             uint32_t phase = 0;
-            for (int i = cluster_id; i < units && !*abort_flag; i += num_clusters) {
+            for (int i = first_unit; i >= 0 && !*abort_flag; i = next_unit(i, item++)) {
                 const Tile t = locate(sh, args.num_experts, args.n_tiles, i, kTileTokens);
                 const int half = t.tokens / 2, t_row = t.row0 + int(cta) * half;  // this CTA's token rows
                 for (int kb = 0; kb < k_blocks; ++kb) {
@@ -248,7 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
         if (leader && elect_one()) {
             int stage = 0, item = 0;
             uint32_t phase = 0;
-            for (int i = cluster_id; i < units && !*abort_flag; i += num_clusters, ++item) {
+            for (int i = first_unit; i >= 0 && !*abort_flag; i = next_unit(i, item++)) {
                 const Tile t = locate(sh, args.num_experts, args.n_tiles, i, kTileTokens);
                 const uint32_t idesc = instr_desc_bf16(BW, t.tokens);
                 const int acc = item & 1;
@@ -286,6 +361,35 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
                 commit(&sh.tmem_full[acc]);
             }
         }
+        // ------------------------------------------------------------------ scheduler (the other CTA)
+        // Hands out the units of the clusters that it takes over; those behind the last unit (the offsets may allow more than
+        // the counts give) are taken over as well, so that none of them has to start.  An answer "none left" is the last request.
+        if (!leader && args.dynamic && elect_one()) {
+            int taken = first_unit >= 0 ? 0 : units;
+            for (int n = 0; taken >= 0; ++n) {
+                const int slot = n % kUnitSlots;
+                const bool wanted = taken < units;
+                if (n >= kUnitSlots && wanted && !mbar_wait_pair(&sh.unit_empty[slot], uint32_t(n / kUnitSlots - 1) & 1u, limit_ns)) {
+                    fail(kGemmPipeTimeout);
+                    break;
+                }
+                mbar_expect_tx(&sh.cancel_done, 16);
+                request_cluster(sh.cancelled, &sh.cancel_done);
+                if (!mbar_wait(&sh.cancel_done, uint32_t(n) & 1u, limit_ns)) {
+                    fail(kGemmPipeTimeout);
+                    break;
+                }
+                const int cta_taken = cancelled_cta(sh.cancelled);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next answer comes behind this read
+                taken = cta_taken < 0 ? -1 : cta_taken >> 1;
+                if (!wanted) continue;
+                const int unit = taken < units ? taken : -1;
+                *(volatile int*)&sh.next_unit[slot] = unit;
+                st_cluster(map_to_cta(smem_u32(&sh.next_unit[slot]), 0), unit);
+                mbar_arrive_cluster(map_to_cta(smem_u32(&sh.unit_full[slot]), 1));
+                mbar_arrive_cluster(map_to_cta(smem_u32(&sh.unit_full[slot]), 0));
+            }
+        }
     } else {
         // ------------------------------------------------------------------ epilogue (both CTAs)
         const int quarter = warp & 3;             // TMEM lanes [32 * quarter, +32) belong to this warp
@@ -295,11 +399,20 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
         // stmatrix: matrix m = lane / 8 holds token group m / 2 and feature half m % 2; this lane addresses its row lane % 8
         const int st_tok = (lane >> 4) * 8 + (lane & 7), st_feat = ((lane >> 3) & 1) * 8;
         uint8_t* buf = stage_out + group * O::kBufBytes;
-        int item = 0;
-        for (int i = cluster_id; i < units; i += num_clusters, ++item) {
+        int unit = first_unit;  // warp 2, lane 0
+        for (int item = 0;; ++item) {
+            if (warp == 2) {
+                if (lane == 0) {
+                    if (item > 0) unit = next_unit(unit, item - 1);
+                    *(volatile int*)&sh.epi_unit[item & 1] = unit;
+                }
+                __syncwarp();
+            }
+            epilogue_sync();  // and the previous unit's destinations have been used
+            const int i = *(volatile int*)&sh.epi_unit[item & 1];
+            if (i < 0) break;
             const Tile t = locate(sh, args.num_experts, args.n_tiles, i, kTileTokens);
             if (kMode != kSwiGLU) {
-                epilogue_sync();  // the previous unit's destinations have been used
                 for (int r = tid; r < t.tokens; r += kEpiThreads) {
                     const int row = t.row0 + r;
                     float scale = 1.f;

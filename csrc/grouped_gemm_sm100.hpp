@@ -39,6 +39,7 @@ struct Args {
     int topk;
     int ranks;      // kScatter: valid source ranks are [0, ranks)
     int recv_rows;  // kScatter: rows of recv_metadata
+    int dynamic;    // expert kernel: the grid has a cluster for every unit of work, and running clusters take over the waiting ones' places
 };
 
 // Tensor maps of the expert kernel: weights (for SwiGLU as [2E][I][K], gate and up halves), token rows in boxes of

@@ -47,6 +47,41 @@ def test_rows_that_exist(counts, K, N, largest, swiglu):
     assert torch.equal(out[real], few[real]), "the result does not depend on the number of CTAs"
 
 
+@pytest.mark.parametrize("largest", [0, 64, 128])  # token tiles of 256, 64 and 128
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize(
+    "counts,ranges,K,N",
+    [
+        ([3, 0, 40], [1024, 512, 2048], 128, 512),  # the offsets allow far more units than the counts give
+        ([0, 0], [128, 256], 64, 256),              # no unit at all
+        ([1], [128], 64, 512),                      # fewer units than clusters
+        ([2304, 1000, 129, 0, 777, 256, 1, 511], None, 64, 2048),  # short units, several per cluster
+        ([640, 385, 130], None, 2048, 1280),
+    ],
+)
+def test_units_taken_over_by_running_clusters(counts, ranges, K, N, swiglu, largest):
+    """Without a cap on the CTAs the units are handed out as clusters get free; with one every cluster has a fixed share.
+    Each unit is computed the same way wherever it runs."""
+    torch.manual_seed(11)
+    a, w, offsets, n, real = _problem(counts if ranges is None else ranges, K, N)
+    a = torch.nan_to_num(a, nan=0.25)
+    if ranges is not None:
+        real.zero_()
+        for e, c in enumerate(counts):
+            real[int(offsets[e]) : int(offsets[e]) + c] = True
+        n = torch.tensor(counts, dtype=torch.int64, device="cuda")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    shape = (a.shape[0], N // 2 if swiglu else N)
+    runs = [gg.grouped_gemm(a, w, offsets, swiglu=swiglu, expert_counts=n, max_expert_rows=largest, max_ctas=cap,
+                            out=torch.full(shape, 3.0, dtype=torch.bfloat16, device="cuda")) for cap in (0, sms, 2, 0)]
+    torch.cuda.synchronize()
+    gg.check_status()
+    ref = gg.grouped_gemm_reference(a, w, offsets, swiglu=swiglu)
+    torch.testing.assert_close(runs[0][real].float(), ref[real], rtol=1e-2, atol=1e-2)  # one bf16 round of an fp32-accumulated product
+    for other in runs[1:]:
+        assert torch.equal(runs[0][real], other[real])
+
+
 @pytest.mark.parametrize("pair", [False, True])
 def test_matches_the_gated_kernels(pair):
     """The kernels with tokens as M (row blocks gated by counters) add the same products: at most one bf16 step apart."""
