@@ -185,6 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
     const bool leader = cta == 0;
     const uint64_t limit_ns = args.timeout_ns;
 
+    allow_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(&sh.full[s], 1);   // leader: one expect_tx arrival covering both CTAs' bytes
@@ -284,33 +285,51 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
             for (int i = first_unit; i >= 0 && !*abort_flag; i = next_unit(i, item++)) {
                 const Tile t = locate(sh, args.num_experts, args.n_tiles, i, kTileTokens);
                 const int half = t.tokens / 2, t_row = t.row0 + int(cta) * half;  // this CTA's token rows
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&sh.empty[stage], phase ^ 1u, limit_ns)) {
-                        fail(kGemmPipeTimeout);
-                        break;
-                    }
-                    uint8_t* w_dst = smem + stage * P::kStageBytes;
-                    uint8_t* t_dst = w_dst + kWBytes;
-                    const uint32_t bar = map_to_cta(smem_u32(&sh.full[stage]), 0);
-                    if (leader) mbar_expect_tx(&sh.full[stage], uint32_t(2 * (kWBytes + half * BK * 2)));
+                const uint32_t bytes = uint32_t(2 * (kWBytes + half * BK * 2));    // of a stage, in both CTAs
+                auto load_weights = [&](int kb, int s) {
+                    uint8_t* dst = smem + s * P::kStageBytes;
+                    const uint32_t bar = map_to_cta(smem_u32(&sh.full[s]), 0);
+                    if (leader) mbar_expect_tx(&sh.full[s], bytes);
                     if (kMode == kSwiGLU) {
                         // 16 gate rows followed by their 16 up rows, four times: 64 output features of this CTA
                         const int f0 = t.wt * 128 + int(cta) * 64;
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) tma_load_3d_pair(w_dst + q * 4096, &maps.weights, kb * BK, f0 + 16 * q, 2 * t.expert, bar);
+                        for (int q = 0; q < 4; ++q) tma_load_3d_pair(dst + q * 4096, &maps.weights, kb * BK, f0 + 16 * q, 2 * t.expert, bar);
                     } else {
-                        tma_load_2d_pair(w_dst, &maps.weights, kb * BK, t.expert * args.b_rows_per_expert + t.wt * BW + int(cta) * (BW / 2), bar);
+                        tma_load_2d_pair(dst, &maps.weights, kb * BK, t.expert * args.b_rows_per_expert + t.wt * BW + int(cta) * (BW / 2), bar);
                     }
-                    // token rows: boxes of 128, 64, 32 and 16 rows make up any multiple of 16
+                };
+                auto load_tokens = [&](int kb, int s) {
+                    uint8_t* dst = smem + s * P::kStageBytes + kWBytes;
+                    const uint32_t bar = map_to_cta(smem_u32(&sh.full[s]), 0);
+                    // boxes of 128, 64, 32 and 16 rows make up any multiple of 16
                     int at = 0;
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {
                         const int box = 128 >> b;
                         if (half & box) {
-                            tma_load_2d_pair(t_dst + at * BK * 2, &maps.tokens[b], kb * BK, t_row + at, bar);
+                            tma_load_2d_pair(dst + at * BK * 2, &maps.tokens[b], kb * BK, t_row + at, bar);
                             at += box;
                         }
                     }
+                };
+                int early = 0;  // k-blocks whose weights are on their way already
+                if (item == 0) {
+                    // The ring is empty: fill it with weights while the kernel in front, which writes the token rows, ends.  (A layer of
+                    // 64 tokens, 32 experts of 7168 x 2048, with a cached handle 446 -> 437.7 us; of 777 tokens, 4096 x 1536, 289 -> 284.)
+                    early = min(kStages, k_blocks);
+                    for (int kb = 0; kb < early; ++kb) load_weights(kb, kb);
+                    wait_for_previous();
+                }
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (kb >= early) {
+                        if (!mbar_wait(&sh.empty[stage], phase ^ 1u, limit_ns)) {
+                            fail(kGemmPipeTimeout);
+                            break;
+                        }
+                        load_weights(kb, stage);
+                    }
+                    load_tokens(kb, stage);
                     if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1u;
@@ -399,6 +418,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
         // stmatrix: matrix m = lane / 8 holds token group m / 2 and feature half m % 2; this lane addresses its row lane % 8
         const int st_tok = (lane >> 4) * 8 + (lane & 7), st_feat = ((lane >> 3) & 1) * 8;
         uint8_t* buf = stage_out + group * O::kBufBytes;
+        // Rows, scales and destinations are the work of kernels in front; no CTA ends before those have.
+        wait_for_previous();
         int unit = first_unit;  // warp 2, lane 0
         for (int item = 0;; ++item) {
             if (warp == 2) {
@@ -520,7 +541,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
 }
 
 template <int kMode, int kTileTokens>
-cudaError_t launch_tile(const ExpertMaps& maps, const Args& args, int grid, cudaStream_t stream) {
+cudaError_t launch_tile(const ExpertMaps& maps, const Args& args, int grid, bool early, cudaStream_t stream) {
     auto* fn = expert_gemm_kernel<kMode, kTileTokens>;
     using P = Pipe<kMode, kTileTokens>;
     // The limit is the same for every launch of this kernel: raised once per device (a second thread may do it again).
@@ -539,32 +560,34 @@ cudaError_t launch_tile(const ExpertMaps& maps, const Args& args, int grid, cuda
     config.blockDim = dim3(kThreads);
     config.dynamicSmemBytes = P::kSmemBytes;
     config.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attr;
-    config.numAttrs = 1;
+    config.numAttrs = early ? 2 : 1;
     return cudaLaunchKernelEx(&config, fn, maps, args);
 }
 
 template <int kMode>
-cudaError_t launch_mode(const ExpertMaps& maps, const Args& args, int tile_tokens, int grid, cudaStream_t stream) {
-    if (tile_tokens <= 64) return launch_tile<kMode, 64>(maps, args, grid, stream);
-    if (tile_tokens <= 128) return launch_tile<kMode, 128>(maps, args, grid, stream);
-    return launch_tile<kMode, 256>(maps, args, grid, stream);
+cudaError_t launch_mode(const ExpertMaps& maps, const Args& args, int tile_tokens, int grid, bool early, cudaStream_t stream) {
+    if (tile_tokens <= 64) return launch_tile<kMode, 64>(maps, args, grid, early, stream);
+    if (tile_tokens <= 128) return launch_tile<kMode, 128>(maps, args, grid, early, stream);
+    return launch_tile<kMode, 256>(maps, args, grid, early, stream);
 }
 
 }  // namespace
 
-cudaError_t launch_expert(const ExpertMaps& maps, const Args& args, int mode, int tile_tokens, int grid, cudaStream_t stream) {
+cudaError_t launch_expert(const ExpertMaps& maps, const Args& args, int mode, int tile_tokens, int grid, bool early, cudaStream_t stream) {
     if (args.num_experts > kMaxExperts) return cudaErrorInvalidValue;
     grid &= ~1;
     if (grid < 2) return cudaErrorInvalidValue;
-    if (mode == kPlain) return launch_mode<kPlain>(maps, args, tile_tokens, grid, stream);
-    if (mode == kSwiGLU) return launch_mode<kSwiGLU>(maps, args, tile_tokens, grid, stream);
-    if (mode == kScatter) return launch_mode<kScatter>(maps, args, tile_tokens, grid, stream);
+    if (mode == kPlain) return launch_mode<kPlain>(maps, args, tile_tokens, grid, early, stream);
+    if (mode == kSwiGLU) return launch_mode<kSwiGLU>(maps, args, tile_tokens, grid, early, stream);
+    if (mode == kScatter) return launch_mode<kScatter>(maps, args, tile_tokens, grid, early, stream);
     return cudaErrorInvalidValue;
 }
 

@@ -89,7 +89,7 @@ GemmCommon prepare(const at::Tensor& a, const at::Tensor& w, const at::Tensor& e
 }
 
 cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& w, const c10::optional<at::Tensor>& counts, int mode,
-                          int64_t max_expert_rows, int64_t max_ctas) {
+                          int64_t max_expert_rows, int64_t max_ctas, bool early) {
     if (counts.has_value()) {
         TORCH_CHECK(counts->is_cuda() && counts->device() == a.device() && counts->scalar_type() == at::kLong && counts->is_contiguous() &&
                         counts->dim() == 1 && counts->size(0) == w.size(0),
@@ -114,7 +114,7 @@ cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& 
     const int64_t blocks = rows / 128, tiles = tile <= 128 ? blocks * 128 / tile : (blocks + std::min(E, blocks)) / 2;
     g.args.dynamic = max_ctas <= 0;
     const int grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : int(2 * tiles * g.args.n_tiles);
-    return gemm::launch_expert(maps, g.args, mode, tile, grid, c10::cuda::getCurrentCUDAStream().stream());
+    return gemm::launch_expert(maps, g.args, mode, tile, grid, early, c10::cuda::getCurrentCUDAStream().stream());
 }
 
 // Which kernel a grouped_gemm call runs.  The one with tokens as N is the faster one (expert_gemm_sm100.cu has both sides), but it
@@ -150,7 +150,7 @@ void bind_gemm(pybind11::module_& m) {
         "grouped_gemm",
         [](const at::Tensor& a, const at::Tensor& w, const at::Tensor& expert_offsets, at::Tensor& out, at::Tensor& status, int64_t mode,
            c10::optional<at::Tensor> tile_ready, c10::optional<at::Tensor> tile_expected, int64_t max_ctas, double timeout_s,
-           c10::optional<at::Tensor> row_scale, int64_t stages, bool pair, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows) {
+           c10::optional<at::Tensor> row_scale, int64_t stages, bool pair, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows, bool early) {
             c10::cuda::CUDAGuard guard(a.device());
             TORCH_CHECK(mode == gemm::kPlain || mode == gemm::kSwiGLU, "mode must be 0 (plain) or 1 (SwiGLU)");
             auto g = prepare(a, w, expert_offsets, status, int(mode), timeout_s);
@@ -182,7 +182,7 @@ void bind_gemm(pybind11::module_& m) {
                                                        g.args.m_blocks, g.args.n_tiles, a.size(1),
                                                        at::cuda::getCurrentDeviceProperties()->multiProcessorCount});
             if (kernel == kExpertKernel) {
-                cudaError_t ee = launch_expert(g, a, w, expert_counts, int(mode), max_expert_rows, max_ctas);
+                cudaError_t ee = launch_expert(g, a, w, expert_counts, int(mode), max_expert_rows, max_ctas, early);
                 TORCH_CHECK(ee == cudaSuccess, "grouped GEMM (expert) launch failed: ", cudaGetErrorString(ee));
                 return;
             }
@@ -203,7 +203,7 @@ void bind_gemm(pybind11::module_& m) {
         pybind11::arg("mode"), pybind11::arg("tile_ready") = c10::nullopt, pybind11::arg("tile_expected") = c10::nullopt,
         pybind11::arg("max_ctas") = 0, pybind11::arg("timeout_s") = 5.0, pybind11::arg("row_scale") = c10::nullopt,
         pybind11::arg("stages") = 4, pybind11::arg("pair") = false, pybind11::arg("expert_counts") = c10::nullopt,
-        pybind11::arg("max_expert_rows") = 0);
+        pybind11::arg("max_expert_rows") = 0, pybind11::arg("early") = false);
 
     // Down projection fused with the combine push: row r of (A @ W[e]^T) * slot_weight[r] is stored
     // (bf16) into the return partition of the row's source rank; padding rows are skipped.  The return area
@@ -213,7 +213,7 @@ void bind_gemm(pybind11::module_& m) {
         "grouped_gemm_scatter",
         [](PeerWindow& window, const at::Tensor& a, const at::Tensor& w, const at::Tensor& expert_offsets,
            const at::Tensor& slot_map, const at::Tensor& recv_metadata, c10::optional<at::Tensor> slot_weights, at::Tensor& status,
-           int64_t max_ctas, double timeout_s, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows) {
+           int64_t max_ctas, double timeout_s, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows, bool early) {
             c10::cuda::CUDAGuard guard(a.device());
             auto g = prepare(a, w, expert_offsets, status, gemm::kScatter, timeout_s);
             const WindowLayout& L = window.layout();
@@ -242,13 +242,13 @@ void bind_gemm(pybind11::module_& m) {
             if (a.size(0) == 0) return;
             PeerWindow::launches += 1;
             // the kernel works in pairs of CTAs: a cap of one means one pair
-            const cudaError_t e = launch_expert(g, a, w, expert_counts, gemm::kScatter, max_expert_rows, max_ctas == 1 ? 2 : max_ctas);
+            const cudaError_t e = launch_expert(g, a, w, expert_counts, gemm::kScatter, max_expert_rows, max_ctas == 1 ? 2 : max_ctas, early);
             TORCH_CHECK(e == cudaSuccess, "grouped GEMM (scatter) launch failed: ", cudaGetErrorString(e));
         },
         pybind11::arg("window"), pybind11::arg("a"), pybind11::arg("w"), pybind11::arg("expert_offsets"),
         pybind11::arg("slot_map"), pybind11::arg("recv_metadata"), pybind11::arg("slot_weights"), pybind11::arg("status"),
         pybind11::arg("max_ctas") = 0, pybind11::arg("timeout_s") = 5.0,
-        pybind11::arg("expert_counts") = c10::nullopt, pybind11::arg("max_expert_rows") = 0);
+        pybind11::arg("expert_counts") = c10::nullopt, pybind11::arg("max_expert_rows") = 0, pybind11::arg("early") = false);
 
     m.def(
         "grouped_gemm_choice",

@@ -55,8 +55,10 @@ int kernel_registers(int mode);
 // CTA-pair variant (tcgen05 cta_group::2, 256 x 256 tiles on two SMs); modes kPlain and kSwiGLU.
 cudaError_t launch_pair(const CUtensorMap& a, const CUtensorMap& b, const Args& args, int mode, int grid, cudaStream_t stream, int stages);
 
-// Weights as M, tokens as N (expert_gemm_sm100.cu); `tile_tokens` = largest token tile wanted (64, 128 or 256).
-cudaError_t launch_expert(const ExpertMaps& maps, const Args& args, int mode, int tile_tokens, int grid, cudaStream_t stream);
+// Weights as M, tokens as N (expert_gemm_sm100.cu); `tile_tokens` = largest token tile wanted (64, 128 or 256).  `early`: the kernel may
+// start while the one in front of it on the stream ends (it waits for that one before it reads rows, scales or destinations);
+// whatever writes the weights, offsets and counts has ended by the time that the kernel in front lets its dependents start.
+cudaError_t launch_expert(const ExpertMaps& maps, const Args& args, int mode, int tile_tokens, int grid, bool early, cudaStream_t stream);
 
 }  // namespace gemm
 }  // namespace nep

@@ -91,6 +91,11 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     return v;
 }
 
+// Programmatic dependent launch: the kernel behind this one may be set up from here on; everything in front of this kernel has
+// ended and its writes are visible (both do nothing for a kernel launched or followed without it).
+__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- CTA pairs (clusters of two, tcgen05 cta_group::2)
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;

@@ -108,23 +108,31 @@ class ExpertParallelMoE:
             mark("dispatch+up_gemm")
         else:
             mark("dispatch")
-            h = gg.grouped_gemm(h_in, self.w13, offsets, swiglu=True, expert_counts=counts, max_expert_rows=most)
+            h = self._grouped(h_in, self.w13, offsets, self.inner, gg.SWIGLU, None, counts, most)
             mark("up_gemm")
         self.last_handle = got.handle
         if self.fuse_combine:
             window = buf.window
             self._ext.grouped_gemm_scatter(window, h, self.w2, offsets, got.handle.slot_map, got.handle.layout.recv_metadata,
-                                           got.topk_weights, gg.status_tensor(self.device), 0, 5.0, counts, most)
+                                           got.topk_weights, gg.status_tensor(self.device), 0, 5.0, counts, most, not overlap)
             mark("down_gemm_scatter")
             out = self._ext.combine_finish([window], [handle_metadata(got.handle)], [bias])[0]
             mark("barrier+reduce")
             self._collect(marks)
             return out
-        y = gg.grouped_gemm(h, self.w2, offsets, row_scale=got.topk_weights, expert_counts=counts, max_expert_rows=most)  # gate weight in FP32
+        y = self._grouped(h, self.w2, offsets, self.buffer.config.hidden, gg.PLAIN, got.topk_weights, counts, most, not overlap)  # gate weight in FP32
         mark("down_gemm")
         out = buf.combine(y, got.handle, bias=bias).x
         mark("combine")
         self._collect(marks)
+        return out
+
+    def _grouped(self, a, w, offsets, columns, mode, scale, counts, most, early=True):
+        """A grouped GEMM that may start while the kernel in front of it (the dispatch's pull, the up-projection) ends: nothing
+        from the pull on writes weights, offsets or counts, and the pull lets its dependents start only once all that lies
+        before it has ended."""
+        out = torch.empty((a.shape[0], columns), dtype=torch.bfloat16, device=a.device)
+        self._ext.grouped_gemm(a, w, offsets, out, gg.status_tensor(a.device), mode, None, None, 0, 5.0, scale, 4, False, counts, most, early)
         return out
 
     def _collect(self, marks):
