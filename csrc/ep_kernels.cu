@@ -1775,8 +1775,8 @@ __device__ void reduce_body(const ReduceParams& p) {
 }
 
 // Tokens without any valid choice have no receive row: result = bias (or zero), weights = 0.
-__device__ void finish_rowless_tokens(const LocalCombineParams& p, int first, int step) {
-    if (p.rows == p.tokens) return;
+__device__ void finish_rowless_tokens(const LocalCombineParams& p, int rows, int first, int step) {
+    if (rows == p.tokens) return;
     const WindowLayout& L = p.c.layout;
     const int lane = threadIdx.x & 31, K = L.topk, H = L.hidden;
     for (int t = first; t < p.tokens; t += step) {
@@ -1787,6 +1787,10 @@ __device__ void finish_rowless_tokens(const LocalCombineParams& p, int first, in
         for (int c = lane; c < H / 8; c += 32) out[c] = bias != nullptr ? ld_nc_v4(bias + c) : make_int4(0, 0, 0, 0);
         if (p.w_out != nullptr && lane < K) p.w_out[int64_t(t) * K + lane] = 0.f;
     }
+}
+
+__device__ __forceinline__ int local_rows(const LocalCombineParams& p) {
+    return p.rows_device != nullptr ? int(min(int64_t(p.rows), *p.rows_device)) : p.rows;
 }
 
 // Token and choices of receive row r on all lanes: lane k holds choice k.  False: nothing to add up (or bad metadata).
@@ -1811,7 +1815,8 @@ __device__ void local_combine_body(const LocalCombineParams& p) {
     const int gw = blockIdx.x * wpb + warp, GW = gridDim.x * wpb;
     const int vecs = H / 8, per_row = (vecs + kItemVecs - 1) / kItemVecs;
     const uint64_t once = l2_evict_first_policy();
-    const int64_t items = int64_t(p.rows) * per_row;
+    const int rows = local_rows(p);
+    const int64_t items = int64_t(rows) * per_row;
     for (int64_t item = gw; item < items; item += GW) {
         const int r = int(item / per_row), c = int(item - int64_t(r) * per_row);
         int tok, v;
@@ -1832,7 +1837,7 @@ __device__ void local_combine_body(const LocalCombineParams& p) {
         finish_columns(a0, a1, col, one, two, p.bias != nullptr ? p.bias + int64_t(tok) * H : nullptr, p.out + int64_t(tok) * H, once);
         if (c == 0 && p.w_out != nullptr && lane < K) p.w_out[int64_t(tok) * K + lane] = ((vm >> lane) & 1u) ? p.w[v] : 0.f;
     }
-    finish_rowless_tokens(p, gw, GW);
+    finish_rowless_tokens(p, rows, gw, GW);
 }
 
 // The compact layout: a row is its token's sum already.  A streaming copy (plus bias); few registers, so that many warps
@@ -1845,7 +1850,8 @@ __device__ void local_combine_compact_body(const LocalCombineParams& p) {
     constexpr int kCols = kCopyItemVecs / 32;
     const int vecs = H / 8, per_row = (vecs + kCopyItemVecs - 1) / kCopyItemVecs;
     const uint64_t once = l2_evict_first_policy();
-    const int64_t items = int64_t(p.rows) * per_row;
+    const int rows = local_rows(p);
+    const int64_t items = int64_t(rows) * per_row;
     for (int64_t item = gw; item < items; item += GW) {
         const int r = int(item / per_row), c = int(item - int64_t(r) * per_row);
         const int col = c * kCopyItemVecs + lane;
@@ -1870,7 +1876,7 @@ __device__ void local_combine_compact_body(const LocalCombineParams& p) {
         }
         if (c == 0 && p.w_out != nullptr && lane < K) p.w_out[int64_t(tok) * K + lane] = ((vm >> lane) & 1u) ? p.w[int64_t(r) * K + lane] : 0.f;
     }
-    finish_rowless_tokens(p, gw, GW);
+    finish_rowless_tokens(p, rows, gw, GW);
 }
 
 __device__ void barrier_body(const BarrierParams& p) {

@@ -189,6 +189,7 @@ struct LocalCombineParams {
     __nv_bfloat16* out;          // [T,H]
     float* w_out;                // [T,K] or null
     int rows, capacity, tokens;
+    const int64_t* rows_device;  // how many of `rows` there are, where the host did not know yet, or null
     int expand;
     int round_partial;  // expanded + multiple reduction: bf16 round of the local sum before bias
 };

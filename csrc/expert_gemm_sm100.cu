@@ -208,9 +208,9 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
     for (int i = threadIdx.x; i <= args.num_experts; i += kThreads) {
         const int64_t off = args.expert_offsets[i];
         sh.offsets[i] = int(off);
-        // one expert per 128-row block: offsets must be multiples of 128, start at 0, not fall, and end at the row count
+        // one expert per 128-row block: offsets must be multiples of 128, start at 0, not fall, and end at the row count (or in front of it)
         const bool falls = i > 0 && off < args.expert_offsets[i - 1];
-        if ((off & 127) != 0 || falls || (i == 0 && off != 0) || (i == args.num_experts && off != args.rows)) {
+        if ((off & 127) != 0 || falls || (i == 0 && off != 0) || (i == args.num_experts && (args.rows_bound ? off > args.rows : off != args.rows))) {
             sh.abort = 1;
             if (atomicCAS(args.status, 0u, uint32_t(kGemmBadOffsets)) == 0u) args.status[1] = uint32_t(i);
         }

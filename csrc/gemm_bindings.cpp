@@ -7,6 +7,7 @@
 
 #include "grouped_gemm_sm100.hpp"
 #include "peer_window.hpp"
+#include "pipeline.hpp"
 
 namespace nep {
 namespace {
@@ -89,7 +90,7 @@ GemmCommon prepare(const at::Tensor& a, const at::Tensor& w, const at::Tensor& e
 }
 
 cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& w, const c10::optional<at::Tensor>& counts, int mode,
-                          int64_t max_expert_rows, int64_t max_ctas, bool early) {
+                          int64_t max_expert_rows, int64_t max_ctas, bool early, int64_t assigned) {
     if (counts.has_value()) {
         TORCH_CHECK(counts->is_cuda() && counts->device() == a.device() && counts->scalar_type() == at::kLong && counts->is_contiguous() &&
                         counts->dim() == 1 && counts->size(0) == w.size(0),
@@ -104,7 +105,8 @@ cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& 
     // tokens 283, 287 and 302 us; 256 tokens (at most 78 rows an expert) 324, 293 and 310-329 us; 512 tokens (at most 158) 526,
     // 374 and 319 us.  So: the smallest tile that no expert can outgrow, and 128 also where every expert has at most one
     // block of 128 rows on average and none can hold more than four.
-    const bool one_block = max_expert_rows <= 512 && rows <= 128 * E;
+    // Where `rows` is a bound, the number of choices stands for it: experts of 80 rows on average rarely have a second block.
+    const bool one_block = max_expert_rows <= 512 && (assigned >= 0 ? assigned <= 80 * E : rows <= 128 * E);
     const int tile = max_expert_rows <= 0 ? 256 : max_expert_rows <= 64 ? 64 : max_expert_rows <= 128 || one_block ? 128 : 256;
     for (int b = 0; b < 4; ++b)
         if ((128 >> b) <= tile / 2) maps.tokens[b] = make_map(a.data_ptr(), rows, K, 128 >> b);
@@ -113,6 +115,7 @@ cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& 
     // whole blocks of 128, and tiles of 256 split an odd number of them into one more).
     const int64_t blocks = rows / 128, tiles = tile <= 128 ? blocks * 128 / tile : (blocks + std::min(E, blocks)) / 2;
     g.args.dynamic = max_ctas <= 0;
+    g.args.rows_bound = assigned >= 0;
     const int grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : int(2 * tiles * g.args.n_tiles);
     return gemm::launch_expert(maps, g.args, mode, tile, grid, early, c10::cuda::getCurrentCUDAStream().stream());
 }
@@ -142,114 +145,151 @@ Kernel choose_kernel(const Choice& c) {
     return (!c.swiglu && c.K <= 128) || one_wave_of_singles ? kSingleKernel : kExpertKernel;
 }
 
+// out = A @ W[e]^T per 128-row block (mode 0) or silu(gate) * up with W = [E, 2I, K] (mode 1).  `early` as in launch_expert.
+// `assigned` >= 0: the rows of `a` are an upper bound (the offsets say where they end), and so many of them at most are real.
+void grouped_gemm(const at::Tensor& a, const at::Tensor& w, const at::Tensor& expert_offsets, at::Tensor& out, at::Tensor& status, int64_t mode,
+                  c10::optional<at::Tensor> tile_ready, c10::optional<at::Tensor> tile_expected, int64_t max_ctas, double timeout_s,
+                  c10::optional<at::Tensor> row_scale, int64_t stages, bool pair, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows, bool early, int64_t assigned) {
+    c10::cuda::CUDAGuard guard(a.device());
+    TORCH_CHECK(mode == gemm::kPlain || mode == gemm::kSwiGLU, "mode must be 0 (plain) or 1 (SwiGLU)");
+    auto g = prepare(a, w, expert_offsets, status, int(mode), timeout_s);
+    check_bf16(out, 2, "out");
+    const int64_t n_out = mode == gemm::kSwiGLU ? w.size(1) / 2 : w.size(1);
+    TORCH_CHECK(out.size(0) == a.size(0) && out.size(1) == n_out, "out has the wrong shape");
+    g.args.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
+    g.args.ldo = int(n_out);
+    if (tile_ready.has_value()) {
+        TORCH_CHECK(tile_expected.has_value() && tile_ready->scalar_type() == at::kInt && tile_expected->scalar_type() == at::kInt &&
+                        tile_ready->numel() >= g.args.m_blocks && tile_expected->numel() >= g.args.m_blocks &&
+                        tile_ready->is_cuda() && tile_expected->is_cuda() && tile_ready->device() == a.device() &&
+                        tile_expected->device() == a.device() && tile_ready->is_contiguous() && tile_expected->is_contiguous(),
+                    "tile_ready/tile_expected must be contiguous int32 tensors on the activations' device with one entry per 128-row block");
+        g.args.tile_ready = tile_ready->data_ptr<int>();
+        g.args.tile_expected = tile_expected->data_ptr<int>();
+    }
+    if (row_scale.has_value()) {
+        TORCH_CHECK(mode == gemm::kPlain && row_scale->is_cuda() && row_scale->scalar_type() == at::kFloat &&
+                        row_scale->is_contiguous() && row_scale->numel() == a.size(0),
+                    "row_scale must be float32 [rows] (plain mode only)");
+        g.args.row_scale = row_scale->data_ptr<float>();
+    }
+    TORCH_CHECK(stages == 3 || stages == 4, "stages must be 3 or 4 (single-CTA) or 4 for the gated CTA-pair kernel");
+    if (a.size(0) == 0) return;
+    const int grid = max_ctas > 0 ? std::min<int>(g.grid, int(max_ctas)) : g.grid;
+    PeerWindow::launches += 1;
+    const Kernel kernel = choose_kernel(Choice{tile_ready.has_value(), pair, stages, max_ctas, mode == gemm::kSwiGLU, expert_counts.has_value(),
+                                               g.args.m_blocks, g.args.n_tiles, a.size(1),
+                                               at::cuda::getCurrentDeviceProperties()->multiProcessorCount});
+    if (kernel == kExpertKernel) {
+        cudaError_t ee = launch_expert(g, a, w, expert_counts, int(mode), max_expert_rows, max_ctas, early, assigned);
+        TORCH_CHECK(ee == cudaSuccess, "grouped GEMM (expert) launch failed: ", cudaGetErrorString(ee));
+        return;
+    }
+    const CUtensorMap map_a = make_map(a.data_ptr(), a.size(0), a.size(1)), map_b = make_map(w.data_ptr(), w.size(0) * w.size(1), w.size(2));
+    if (kernel == kPairKernel) {
+        const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+        const int pair_grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : sms;
+        // gated by tile counters = meant to share the SMs with the pull kernel: shorter pipeline
+        cudaError_t pe = gemm::launch_pair(map_a, map_b, g.args, int(mode), pair_grid, c10::cuda::getCurrentCUDAStream().stream(),
+                                           tile_ready.has_value() ? 4 : 6);
+        TORCH_CHECK(pe == cudaSuccess, "grouped GEMM (CTA pairs) launch failed: ", cudaGetErrorString(pe));
+        return;
+    }
+    cudaError_t e = gemm::launch(map_a, map_b, g.args, int(mode), int(stages), grid, c10::cuda::getCurrentCUDAStream().stream());
+    TORCH_CHECK(e == cudaSuccess, "grouped GEMM launch failed: ", cudaGetErrorString(e));
+}
+
+// Down projection fused with the combine push: row r of (A @ W[e]^T) * slot_weight[r] is stored
+// (bf16) into the return partition of the row's source rank; padding rows are skipped.  The return area
+// exists once: a dispatch (whose peer barrier every rank passes only after its previous reduction) must lie
+// between two such calls, as it does in a layer's forward pass.
+void grouped_gemm_scatter(PeerWindow& window, const at::Tensor& a, const at::Tensor& w, const at::Tensor& expert_offsets,
+                          const at::Tensor& slot_map, const at::Tensor& recv_metadata, c10::optional<at::Tensor> slot_weights, at::Tensor& status,
+                          int64_t max_ctas, double timeout_s, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows, bool early, int64_t assigned) {
+    c10::cuda::CUDAGuard guard(a.device());
+    auto g = prepare(a, w, expert_offsets, status, gemm::kScatter, timeout_s);
+    const WindowLayout& L = window.layout();
+    TORCH_CHECK(w.size(1) == L.hidden, "down-projection N must equal the buffer's hidden size");
+    TORCH_CHECK(slot_map.is_cuda() && slot_map.scalar_type() == at::kInt && slot_map.numel() == a.size(0) && slot_map.is_contiguous(),
+                "slot_map must be contiguous int32 [rows]");
+    TORCH_CHECK(recv_metadata.is_cuda() && recv_metadata.scalar_type() == at::kInt && recv_metadata.dim() == 2 &&
+                    recv_metadata.size(1) == L.topk + 2 && recv_metadata.is_contiguous(),
+                "recv_metadata must be int32 [N, topk + 2]");
+    g.args.slot_map = slot_map.data_ptr<int>();
+    g.args.recv_metadata = recv_metadata.data_ptr<int>();
+    if (slot_weights.has_value()) {
+        TORCH_CHECK(slot_weights->is_cuda() && slot_weights->scalar_type() == at::kFloat && slot_weights->numel() == a.size(0),
+                    "slot_weights must be float32 [rows]");
+        g.args.slot_weights = slot_weights->data_ptr<float>();
+    }
+    const CommonParams c = window.common();
+    for (int p = 0; p < kMaxRanks; ++p) g.args.peers[p] = c.peers[p];
+    TORCH_CHECK(L.ret_parts == L.topk, "the fused combine epilogue needs one return partition per choice (allow_multiple_reduction=False)");
+    g.args.ret_offset = L.ret_offset;
+    g.args.max_tokens = L.max_tokens;
+    g.args.topk = L.topk;
+    g.args.ranks = L.ranks;
+    g.args.recv_rows = int(recv_metadata.size(0));
+    g.args.ldo = L.hidden;
+    if (a.size(0) == 0) return;
+    PeerWindow::launches += 1;
+    // the kernel works in pairs of CTAs: a cap of one means one pair
+    const cudaError_t e = launch_expert(g, a, w, expert_counts, gemm::kScatter, max_expert_rows, max_ctas == 1 ? 2 : max_ctas, early, assigned);
+    TORCH_CHECK(e == cudaSuccess, "grouped GEMM (scatter) launch failed: ", cudaGetErrorString(e));
+}
+
+// A whole expert layer: dispatch (fresh with `topk`, cached with `cached` = the handle's tensors and capacity), up-projection with SwiGLU,
+// down-projection, combine, all on the caller's stream.  In one call because the host would otherwise sit between the kernels: where
+// the dispatch allows it everything is queued before the receive counts have reached the host.
+// us before -> after, a layer of 64 tokens (32 experts of 7168 x 2048) 466 -> 447, of 777 tokens (4096 x 1536) 314 -> 306.
+pybind11::tuple moe_forward(PeerWindow& window, const at::Tensor& x, const c10::optional<at::Tensor>& topk, const c10::optional<at::Tensor>& weights,
+                            const std::vector<at::Tensor>& cached, int64_t cached_capacity, bool expand, int64_t alignment, const at::Tensor& w13,
+                            const at::Tensor& w2, at::Tensor& status, const c10::optional<at::Tensor>& bias, bool fuse_combine,
+                            bool allow_multiple_reduction, int64_t num_sms, int64_t comm_stream, double mailbox_timeout_s) {
+    at::Tensor result;
+    const auto behind = [&](DispatchOut& got, bool bound) {
+        const auto& m = got.metadata[0];
+        const at::Tensor &rows = got.outputs[0][0], &counts = m[1], &offsets = m[2];
+        const auto gate = weights.has_value() ? c10::make_optional(got.outputs[0][2]) : c10::nullopt;
+        const at::TensorOptions bf16 = rows.options();
+        const int64_t tokens = x.size(0), most = std::max<int64_t>(1, bound ? tokens : got.counts[0].first);
+        const int64_t assigned = bound ? tokens * window.layout().topk : -1;
+        at::Tensor h = at::empty({rows.size(0), w13.size(1) / 2}, bf16);
+        grouped_gemm(rows, w13, offsets, h, status, gemm::kSwiGLU, {}, {}, 0, 5.0, {}, 4, false, counts, most, true, assigned);
+        if (fuse_combine) {
+            grouped_gemm_scatter(window, h, w2, offsets, m[7], m[0], gate, status, 0, 5.0, counts, most, true, assigned);
+            result = combine_finish({&window}, got.metadata, {bias})[0];
+        } else {
+            at::Tensor y = at::empty({rows.size(0), w2.size(1)}, bf16);
+            grouped_gemm(h, w2, offsets, y, status, gemm::kPlain, {}, {}, 0, 5.0, gate, 4, false, counts, most, true, assigned);  // gate weight in FP32
+            result = combine({&window}, {y}, got.metadata, {rows.size(0)}, {c10::nullopt}, {bias}, expand, allow_multiple_reduction, num_sms, comm_stream,
+                             -1, false, bound).outputs[0][0];
+        }
+    };
+    auto out = dispatch({&window}, {x}, {topk}, {weights}, {cached}, {cached_capacity}, alignment, expand, false, num_sms, comm_stream, -1, false,
+                        mailbox_timeout_s, {c10::nullopt}, 0, behind);
+    return pybind11::make_tuple(result, out.metadata[0], out.counts[0]);
+}
+
 }  // namespace
 
 void bind_gemm(pybind11::module_& m) {
-    // out = A @ W[e]^T per 128-row block (mode 0) or silu(gate) * up with W = [E, 2I, K] (mode 1).
     m.def(
-        "grouped_gemm",
-        [](const at::Tensor& a, const at::Tensor& w, const at::Tensor& expert_offsets, at::Tensor& out, at::Tensor& status, int64_t mode,
-           c10::optional<at::Tensor> tile_ready, c10::optional<at::Tensor> tile_expected, int64_t max_ctas, double timeout_s,
-           c10::optional<at::Tensor> row_scale, int64_t stages, bool pair, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows, bool early) {
-            c10::cuda::CUDAGuard guard(a.device());
-            TORCH_CHECK(mode == gemm::kPlain || mode == gemm::kSwiGLU, "mode must be 0 (plain) or 1 (SwiGLU)");
-            auto g = prepare(a, w, expert_offsets, status, int(mode), timeout_s);
-            check_bf16(out, 2, "out");
-            const int64_t n_out = mode == gemm::kSwiGLU ? w.size(1) / 2 : w.size(1);
-            TORCH_CHECK(out.size(0) == a.size(0) && out.size(1) == n_out, "out has the wrong shape");
-            g.args.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
-            g.args.ldo = int(n_out);
-            if (tile_ready.has_value()) {
-                TORCH_CHECK(tile_expected.has_value() && tile_ready->scalar_type() == at::kInt && tile_expected->scalar_type() == at::kInt &&
-                                tile_ready->numel() >= g.args.m_blocks && tile_expected->numel() >= g.args.m_blocks &&
-                                tile_ready->is_cuda() && tile_expected->is_cuda() && tile_ready->device() == a.device() &&
-                                tile_expected->device() == a.device() && tile_ready->is_contiguous() && tile_expected->is_contiguous(),
-                            "tile_ready/tile_expected must be contiguous int32 tensors on the activations' device with one entry per 128-row block");
-                g.args.tile_ready = tile_ready->data_ptr<int>();
-                g.args.tile_expected = tile_expected->data_ptr<int>();
-            }
-            if (row_scale.has_value()) {
-                TORCH_CHECK(mode == gemm::kPlain && row_scale->is_cuda() && row_scale->scalar_type() == at::kFloat &&
-                                row_scale->is_contiguous() && row_scale->numel() == a.size(0),
-                            "row_scale must be float32 [rows] (plain mode only)");
-                g.args.row_scale = row_scale->data_ptr<float>();
-            }
-            TORCH_CHECK(stages == 3 || stages == 4, "stages must be 3 or 4 (single-CTA) or 4 for the gated CTA-pair kernel");
-            if (a.size(0) == 0) return;
-            const int grid = max_ctas > 0 ? std::min<int>(g.grid, int(max_ctas)) : g.grid;
-            PeerWindow::launches += 1;
-            const Kernel kernel = choose_kernel(Choice{tile_ready.has_value(), pair, stages, max_ctas, mode == gemm::kSwiGLU, expert_counts.has_value(),
-                                                       g.args.m_blocks, g.args.n_tiles, a.size(1),
-                                                       at::cuda::getCurrentDeviceProperties()->multiProcessorCount});
-            if (kernel == kExpertKernel) {
-                cudaError_t ee = launch_expert(g, a, w, expert_counts, int(mode), max_expert_rows, max_ctas, early);
-                TORCH_CHECK(ee == cudaSuccess, "grouped GEMM (expert) launch failed: ", cudaGetErrorString(ee));
-                return;
-            }
-            const CUtensorMap map_a = make_map(a.data_ptr(), a.size(0), a.size(1)), map_b = make_map(w.data_ptr(), w.size(0) * w.size(1), w.size(2));
-            if (kernel == kPairKernel) {
-                const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-                const int pair_grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : sms;
-                // gated by tile counters = meant to share the SMs with the pull kernel: shorter pipeline
-                cudaError_t pe = gemm::launch_pair(map_a, map_b, g.args, int(mode), pair_grid, c10::cuda::getCurrentCUDAStream().stream(),
-                                                   tile_ready.has_value() ? 4 : 6);
-                TORCH_CHECK(pe == cudaSuccess, "grouped GEMM (CTA pairs) launch failed: ", cudaGetErrorString(pe));
-                return;
-            }
-            cudaError_t e = gemm::launch(map_a, map_b, g.args, int(mode), int(stages), grid, c10::cuda::getCurrentCUDAStream().stream());
-            TORCH_CHECK(e == cudaSuccess, "grouped GEMM launch failed: ", cudaGetErrorString(e));
-        },
+        "grouped_gemm", &grouped_gemm,
         pybind11::arg("a"), pybind11::arg("w"), pybind11::arg("expert_offsets"), pybind11::arg("out"), pybind11::arg("status"),
         pybind11::arg("mode"), pybind11::arg("tile_ready") = c10::nullopt, pybind11::arg("tile_expected") = c10::nullopt,
         pybind11::arg("max_ctas") = 0, pybind11::arg("timeout_s") = 5.0, pybind11::arg("row_scale") = c10::nullopt,
         pybind11::arg("stages") = 4, pybind11::arg("pair") = false, pybind11::arg("expert_counts") = c10::nullopt,
-        pybind11::arg("max_expert_rows") = 0, pybind11::arg("early") = false);
+        pybind11::arg("max_expert_rows") = 0, pybind11::arg("early") = false, pybind11::arg("assigned") = -1);
 
-    // Down projection fused with the combine push: row r of (A @ W[e]^T) * slot_weight[r] is stored
-    // (bf16) into the return partition of the row's source rank; padding rows are skipped.  The return area
-    // exists once: a dispatch (whose peer barrier every rank passes only after its previous reduction) must lie
-    // between two such calls, as it does in a layer's forward pass.
     m.def(
-        "grouped_gemm_scatter",
-        [](PeerWindow& window, const at::Tensor& a, const at::Tensor& w, const at::Tensor& expert_offsets,
-           const at::Tensor& slot_map, const at::Tensor& recv_metadata, c10::optional<at::Tensor> slot_weights, at::Tensor& status,
-           int64_t max_ctas, double timeout_s, c10::optional<at::Tensor> expert_counts, int64_t max_expert_rows, bool early) {
-            c10::cuda::CUDAGuard guard(a.device());
-            auto g = prepare(a, w, expert_offsets, status, gemm::kScatter, timeout_s);
-            const WindowLayout& L = window.layout();
-            TORCH_CHECK(w.size(1) == L.hidden, "down-projection N must equal the buffer's hidden size");
-            TORCH_CHECK(slot_map.is_cuda() && slot_map.scalar_type() == at::kInt && slot_map.numel() == a.size(0) && slot_map.is_contiguous(),
-                        "slot_map must be contiguous int32 [rows]");
-            TORCH_CHECK(recv_metadata.is_cuda() && recv_metadata.scalar_type() == at::kInt && recv_metadata.dim() == 2 &&
-                            recv_metadata.size(1) == L.topk + 2 && recv_metadata.is_contiguous(),
-                        "recv_metadata must be int32 [N, topk + 2]");
-            g.args.slot_map = slot_map.data_ptr<int>();
-            g.args.recv_metadata = recv_metadata.data_ptr<int>();
-            if (slot_weights.has_value()) {
-                TORCH_CHECK(slot_weights->is_cuda() && slot_weights->scalar_type() == at::kFloat && slot_weights->numel() == a.size(0),
-                            "slot_weights must be float32 [rows]");
-                g.args.slot_weights = slot_weights->data_ptr<float>();
-            }
-            const CommonParams c = window.common();
-            for (int p = 0; p < kMaxRanks; ++p) g.args.peers[p] = c.peers[p];
-            TORCH_CHECK(L.ret_parts == L.topk, "the fused combine epilogue needs one return partition per choice (allow_multiple_reduction=False)");
-            g.args.ret_offset = L.ret_offset;
-            g.args.max_tokens = L.max_tokens;
-            g.args.topk = L.topk;
-            g.args.ranks = L.ranks;
-            g.args.recv_rows = int(recv_metadata.size(0));
-            g.args.ldo = L.hidden;
-            if (a.size(0) == 0) return;
-            PeerWindow::launches += 1;
-            // the kernel works in pairs of CTAs: a cap of one means one pair
-            const cudaError_t e = launch_expert(g, a, w, expert_counts, gemm::kScatter, max_expert_rows, max_ctas == 1 ? 2 : max_ctas, early);
-            TORCH_CHECK(e == cudaSuccess, "grouped GEMM (scatter) launch failed: ", cudaGetErrorString(e));
-        },
+        "grouped_gemm_scatter", &grouped_gemm_scatter,
         pybind11::arg("window"), pybind11::arg("a"), pybind11::arg("w"), pybind11::arg("expert_offsets"),
         pybind11::arg("slot_map"), pybind11::arg("recv_metadata"), pybind11::arg("slot_weights"), pybind11::arg("status"),
         pybind11::arg("max_ctas") = 0, pybind11::arg("timeout_s") = 5.0,
-        pybind11::arg("expert_counts") = c10::nullopt, pybind11::arg("max_expert_rows") = 0, pybind11::arg("early") = false);
+        pybind11::arg("expert_counts") = c10::nullopt, pybind11::arg("max_expert_rows") = 0, pybind11::arg("early") = false, pybind11::arg("assigned") = -1);
 
+    m.def("moe_forward", &moe_forward);
     m.def(
         "grouped_gemm_choice",
         [](bool gated, bool pair, int64_t stages, int64_t max_ctas, bool swiglu, bool counts, int64_t rows, int64_t n, int64_t k, int64_t sms) -> std::string {

@@ -16,6 +16,7 @@ struct Args {
     int num_experts;
     const int64_t* expert_counts;   // expert kernel: [E] rows that exist per expert, or null (all rows of the range)
     int64_t rows;            // total rows
+    int rows_bound;          // expert kernel: the offsets may end in front of `rows`
     int m_blocks;            // total rows / 128
     int n_tiles;             // output column tiles per row block (256 wide; 128 wide for SwiGLU)
     int k_blocks;            // K / 64

@@ -31,6 +31,7 @@ constexpr int kFusedFreshDefaultTokens = 0;  // single-launch fresh dispatch: of
 constexpr int64_t kFusedFreshMaxOutputBytes = int64_t(256) << 20;  // single-launch fresh dispatch: largest bound-sized output
 constexpr int64_t kLocalPlanMaxHandleBytes = int64_t(16) << 20;    // single-rank plan: largest bound-sized handle
 constexpr int64_t kEarlyPullMaxOutputBytes = int64_t(16) << 20;    // single-rank pull that does not wait for N and C: see dispatch()
+constexpr int64_t kDeferredMaxOutputBytes = int64_t(128) << 20;    // single rank: outputs of their bound for work queued in front of N and C
 constexpr int kFusedDefaultBlocks = 1024;  // i.e. bounded by the SM budget and co-residency only
 
 void cuda_check(cudaError_t e, const char* what) {
@@ -279,7 +280,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
                      const std::vector<std::vector<at::Tensor>>& cached_meta, const std::vector<int64_t>& cached_capacity,
                      int64_t alignment, bool expand, bool zero_padding, int64_t num_sms, int64_t comm_stream, int64_t previous_event,
                      bool async_op, double mailbox_timeout_s, const std::vector<c10::optional<at::Tensor>>& tile_ready,
-                     int64_t ring_smem_limit) {
+                     int64_t ring_smem_limit, const std::function<void(DispatchOut&, bool)>& behind) {
     validate_group(wins);
     const int n = int(wins.size());
     TORCH_CHECK(int(xs.size()) == n && int(topks.size()) == n && int(weights.size()) == n && int(cached_meta.size()) == n &&
@@ -404,8 +405,13 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     // Dispatch of 1 to 128 tokens of 7168, top-8, per call: 25 us against 30 with the wait; with a tenth of the choices
     // masked 33 against 30.
     const int64_t bound_bytes = (expand ? bound_rows_c : bound_rows_n) * L.hidden * 2;
+    // Work that follows on the same stream and takes its sizes from the device need not wait for the host to have the counts: the
+    // pull and what `behind` queues go out at once, on tensors of their upper bound.  Limited to calls that take less time than
+    // the wait matters for (and in the memory that the bound may cost over the exact size).
+    const bool deferred = behind && plan_locally && !async_op && expand && !gated && !g_gate.word.defined() && bound_bytes <= kDeferredMaxOutputBytes;
+    const int64_t deferred_rows_c = bound_rows_c / alignment * alignment;  // C is a multiple of the alignment
     const bool early_pull =
-        plan_locally && (!expand || alignment == 1) && !gated && !g_gate.word.defined() && bound_bytes <= kEarlyPullMaxOutputBytes;
+        plan_locally && !deferred && (!expand || alignment == 1) && !gated && !g_gate.word.defined() && bound_bytes <= kEarlyPullMaxOutputBytes;
     const bool fuse_fresh = fresh && !gated && !local && !g_gate.word.defined() && max_tokens_now <= fused_fresh_max_tokens() &&
                             bound_bytes <= kFusedFreshMaxOutputBytes && (!expand || bound_rows_c <= L.slot_scratch_ints) &&
                             ring.warps >= 2 && ring.smem_bytes >= size_t(stage_smem_bytes(L)) &&
@@ -473,7 +479,9 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         }
     }
     for (int i = 0; i < n; ++i) {
-        if (fuse_fresh || early_pull) {
+        if (deferred) {
+            out.counts[i] = {bound_rows_n, deferred_rows_c};
+        } else if (fuse_fresh || early_pull) {
             out.counts[i] = {bound_rows_n, expand ? bound_rows_c : 0};  // allocation sizes; the real counts follow the launch
         } else if (fresh) {
             std::pair<int64_t, int64_t> nc;
@@ -573,6 +581,23 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             g_marks.mark("pull", cs);
         }
     }
+    if (deferred) {
+        auto& m = out.metadata[0];
+        m[7] = part_of(m[7], 0, {deferred_rows_c});
+        auto receive_counts = [&] {
+            pybind11::gil_scoped_release release;
+            return wins[0]->wait_mailbox(cs, mailbox_timeout_s);
+        };
+        try {
+            behind(out, true);
+        } catch (...) {
+            receive_counts();  // the plan writes the mailbox, which the next dispatch arms again
+            throw;
+        }
+        const auto nc = receive_counts();
+        TORCH_CHECK(nc.first <= bound_rows_n && nc.second <= deferred_rows_c, "receive counts exceed their bound");
+        out.counts[0] = {nc.first, nc.second};
+    }
     if (fuse_fresh || early_pull) {
         // The kernel is on its way; now wait for N and C and trim the outputs to their exact sizes: the single-launch path
         // (off by default) to leading-dimension views of the bound-sized allocations, a single rank's early pull to
@@ -613,6 +638,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             }
         }
     }
+    if (behind && !deferred) behind(out, false);
     std::vector<at::Tensor> inputs, results;
     for (int i = 0; i < n; ++i) {
         inputs.push_back(xs[i]);
@@ -628,7 +654,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
 CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::Tensor>& xs, const std::vector<std::vector<at::Tensor>>& meta,
                    const std::vector<int64_t>& capacity, const std::vector<c10::optional<at::Tensor>>& weights,
                    const std::vector<c10::optional<at::Tensor>>& bias, bool expand, bool allow_multiple_reduction, int64_t num_sms,
-                   int64_t comm_stream, int64_t previous_event, bool async_op) {
+                   int64_t comm_stream, int64_t previous_event, bool async_op, bool rows_bound) {
     validate_group(wins);
     const int n = int(wins.size());
     TORCH_CHECK(int(xs.size()) == n && int(meta.size()) == n && int(capacity.size()) == n && int(weights.size()) == n && int(bias.size()) == n,
@@ -707,6 +733,7 @@ CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::T
             p.out = reinterpret_cast<__nv_bfloat16*>(o[0].data_ptr());
             p.w_out = weighted ? o[1].data_ptr<float>() : nullptr;
             p.rows = int(m[0].size(0));
+            p.rows_device = rows_bound ? m[6].data_ptr<int64_t>() : nullptr;
             p.capacity = int(capacity[0]);
             p.tokens = int(T);
             p.expand = expand;

@@ -5,6 +5,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <c10/util/Optional.h>
 
+#include <functional>
 #include <memory>
 #include <string>
 #include <utility>
@@ -40,17 +41,20 @@ struct CombineOut {
     std::shared_ptr<CompletionEvent> event;
 };
 
+// `behind` queues what follows the dispatch on the same stream.  It is called once: a synchronous, fresh, expert-major dispatch of a
+// single rank with outputs of at most kDeferredMaxOutputBytes calls it before the host has the counts, with outputs and handle tensors of
+// their upper bound (second argument true; a device word has N, the offsets end at C), and waits for the counts afterwards.
 DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at::Tensor>& xs,
                      const std::vector<c10::optional<at::Tensor>>& topks, const std::vector<c10::optional<at::Tensor>>& weights,
                      const std::vector<std::vector<at::Tensor>>& cached_meta, const std::vector<int64_t>& cached_capacity,
                      int64_t alignment, bool expand, bool zero_padding, int64_t num_sms, int64_t comm_stream, int64_t previous_event,
                      bool async_op, double mailbox_timeout_s, const std::vector<c10::optional<at::Tensor>>& tile_ready = {},
-                     int64_t ring_smem_limit = 0);
+                     int64_t ring_smem_limit = 0, const std::function<void(DispatchOut&, bool)>& behind = {});
 
 CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::Tensor>& xs, const std::vector<std::vector<at::Tensor>>& meta,
                    const std::vector<int64_t>& capacity, const std::vector<c10::optional<at::Tensor>>& weights,
                    const std::vector<c10::optional<at::Tensor>>& bias, bool expand, bool allow_multiple_reduction, int64_t num_sms,
-                   int64_t comm_stream, int64_t previous_event, bool async_op);
+                   int64_t comm_stream, int64_t previous_event, bool async_op, bool rows_bound = false);
 
 std::vector<at::Tensor> combine_finish(const std::vector<PeerWindow*>& wins, const std::vector<std::vector<at::Tensor>>& meta,
                                        const std::vector<c10::optional<at::Tensor>>& bias);

@@ -66,6 +66,14 @@ class ExpertParallelMoE:
         self.last_profile: dict[str, float] = {}
 
     def forward(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor, *, handle=None, bias=None) -> torch.Tensor:
+        if not self.overlap_dispatch and not self.profile:
+            out, self.last_handle = self.buffer._run_layer(x, topk_idx, topk_weights, handle, bias, self.w13, self.w2, gg.status_tensor(self.device),
+                                                          ALIGNMENT, self.fuse_combine)
+            return out
+        return self._forward_in_steps(x, topk_idx, topk_weights, handle, bias)
+
+    def _forward_in_steps(self, x, topk_idx, topk_weights, handle, bias) -> torch.Tensor:
+        """The same layer from the public operations, one by one: gated by row counters, or with the steps timed."""
         buf = self.buffer
         stream = torch.cuda.current_stream(self.device)
         overlap = self.overlap_dispatch

@@ -223,6 +223,18 @@ class CudaBuffer:
         return self._auto_num_sms
 
     # ------------------------------------------------------------------ dispatch
+    def _check_dispatch(self, x, topk_idx, handle, do_expand, alignment):
+        check_torch_deterministic()
+        if self._closed:
+            raise RuntimeError("CudaBuffer is closed")
+        expand, expert_alignment = resolve_layout_args(self, handle, topk_idx, do_expand, alignment)
+        routing = handle.topk_idx if handle is not None else topk_idx
+        if x.dim() != 2 or x.shape[1] != self._config.hidden:
+            raise ValueError("x hidden dimension does not match the buffer configuration")
+        if routing.shape != (x.shape[0], self._config.num_topk):
+            raise ValueError("routing snapshot/topk_idx shape must match the buffer configuration")
+        return expand, expert_alignment, routing
+
     def dispatch(
         self,
         x: torch.Tensor,
@@ -247,16 +259,7 @@ class CudaBuffer:
         ``ring_smem_limit`` caps the pull kernel's shared-memory ring (bytes per CTA) so that such a
         consumer can share the SMs with it; 0 uses all of the CTA's shared memory.
         """
-        check_torch_deterministic()
-        if self._closed:
-            raise RuntimeError("CudaBuffer is closed")
-        expand, expert_alignment = resolve_layout_args(self, handle, topk_idx, do_expand, alignment)
-        routing = handle.topk_idx if handle is not None else topk_idx
-        if x.dim() != 2 or x.shape[1] != self._config.hidden:
-            raise ValueError("x hidden dimension does not match the buffer configuration")
-        if routing.shape != (x.shape[0], self._config.num_topk):
-            raise ValueError("routing snapshot/topk_idx shape must match the buffer configuration")
-
+        expand, expert_alignment, routing = self._check_dispatch(x, topk_idx, handle, do_expand, alignment)
         main_sms = self._resolve_num_sms(num_sms, handle)
         if handle is not None and handle.native_state is not None:
             with _OnDevice(self._device), nvtx_range("nanoep.dispatch.cached"):
@@ -350,6 +353,25 @@ class CudaBuffer:
         event = CudaEvent(completed, keepalive=(self, x, handle, weights, bias)) if async_op else None
         out = outputs[0]
         return NativeCombineResult(x=out[0], topk_weights=out[1] if weights is not None else None, event=event)
+
+    # ------------------------------------------------------------------ expert layer
+    def _run_layer(self, x, topk_idx, weights, handle, bias, w13, w2, gemm_status, alignment, fuse_combine):
+        """Dispatch, SwiGLU experts and combine in one native call (models/moe_layer.py): ``(result, handle)``."""
+        fresh = handle is None
+        expand, expert_alignment, _ = self._check_dispatch(x, None if not fresh else topk_idx, handle, True if fresh else None, alignment if fresh else None)
+        if bias is not None and not fuse_combine:  # the fused path checks it in front of its reduction
+            check_combine_bias(bias, (x.shape[0], self._config.hidden), x.dtype, torch.device("cuda", self._device))
+        main_sms = self._resolve_num_sms(None, handle)
+        cached_metadata, cached_capacity = ([], 0) if fresh else (handle_metadata(handle), handle.layout.expanded_capacity)
+        with _OnDevice(self._device), nvtx_range("nanoep.layer"):
+            out, metadata, counts = self._backend.moe_forward(
+                self._window, x, topk_idx if fresh else None, weights, cached_metadata, cached_capacity, expand, expert_alignment, w13, w2,
+                gemm_status, bias, fuse_combine, self._allow_multiple_reduction, main_sms, self._comm_stream.cuda_stream, self._mailbox_timeout_s,
+            )
+        if fresh:
+            handle = build_handle(self, metadata, counts, expand, expert_alignment, x.dtype, main_sms)
+            handle.native_state = self._backend.HandleState(list(metadata), int(counts[1]), bool(expand))
+        return out, handle
 
     # ------------------------------------------------------------------ misc
     def barrier(self):
@@ -457,8 +479,10 @@ def validate_combine_inputs(config: EPConfig, handle: NativeHandle, x, weights, 
         weights.device != device or weights.dtype != torch.float32 or weights.shape != weight_shape or not weights.is_contiguous()
     ):
         raise ValueError("combine weights must be contiguous float32 on the buffer's device with the handle's receive layout")
-    tokens = handle.topk_idx.shape[0]
-    if bias is not None and (
-        bias.device != device or bias.dtype != x.dtype or bias.shape != (tokens, config.hidden) or not bias.is_contiguous()
-    ):
+    if bias is not None:
+        check_combine_bias(bias, (handle.topk_idx.shape[0], config.hidden), x.dtype, device)
+
+
+def check_combine_bias(bias, shape, dtype, device) -> None:
+    if bias.device != device or bias.dtype != dtype or bias.shape != shape or not bias.is_contiguous():
         raise ValueError("combine bias must be contiguous source [T,H], with the x dtype on this buffer's device")

@@ -142,6 +142,39 @@ def test_layer_on_one_rank(one_rank, tokens, fused):
             torch.testing.assert_close(out.float(), want, rtol=3e-2, atol=3e-2)
 
 
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("hidden,tokens,masked", [(512, 0, 0.0), (512, 1, 0.0), (512, 200, 0.2), (512, 200, 0.97), (512, 40, 1.0), (16384, 4000, 0.0)])
+def test_layer_queued_in_front_of_its_counts(one_rank, hidden, tokens, masked, fused):
+    """One native call, on tensors of their bound where the call is small, against the layer step by step: the same bits and
+    the same handle, also without a single choice, with tokens that have none, and beyond the limit on the bound."""
+    inner, E, K = 256, 4, 2
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    w13 = (torch.randn(E, 2 * inner, hidden, device="cuda", generator=gen) * 0.03).to(torch.bfloat16)
+    w2 = (torch.randn(E, hidden, inner, device="cuda", generator=gen) * 0.06).to(torch.bfloat16)
+    with CudaBuffer(one_rank, EPConfig(E, K, hidden, max(tokens, 8))) as buf:
+        layer = ExpertParallelMoE(buf, w13, w2, fuse_combine=fused)
+        x = (torch.randn(tokens, hidden, device="cuda", generator=gen) * 0.5).to(torch.bfloat16)
+        bias = torch.randn(tokens, hidden, device="cuda", generator=gen).to(torch.bfloat16)
+        gate, idx = torch.rand(tokens, E, device="cuda", generator=gen).topk(K, dim=-1)
+        idx = torch.where(torch.rand(tokens, K, device="cuda", generator=gen) < masked, -1, idx)
+        for weights in (gate, None):
+            steps = layer._forward_in_steps(x, idx, weights, None, bias)
+            old = layer.last_handle
+            poison = torch.full((64 << 20,), float("nan"), dtype=torch.bfloat16, device="cuda")
+            del poison
+            whole = layer(x, idx, weights, bias=bias)
+            new = layer.last_handle
+            again = layer(x, None, weights, handle=new, bias=bias)
+            torch.cuda.synchronize()
+            buf.check_status()
+            gg.check_status()
+            assert torch.equal(whole, steps) and torch.equal(again, steps)
+            assert (new.layout.recv_count, new.layout.expanded_capacity) == (old.layout.recv_count, old.layout.expanded_capacity)
+            for a, b in zip(handle_metadata(new), handle_metadata(old)):
+                assert a.shape == b.shape and a.dtype == b.dtype
+            assert torch.equal(new.layout.expert_counts, old.layout.expert_counts) and torch.equal(new.topk_idx, old.topk_idx)
+
+
 @pytest.mark.parametrize("max_ctas", [1, 2, 6])
 def test_scatter_on_a_small_grid(one_rank, max_ctas):
     """The down-projection with the scatter epilogue takes any cap on its grid and gives the same bits."""
