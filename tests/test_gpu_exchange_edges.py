@@ -189,6 +189,15 @@ def _one_rank_dispatch(idx, experts, hidden, **layout):
     assert sum(kept.values()) <= max(2 * used, 1 << 20)
 
 
+@pytest.mark.parametrize("tokens,experts,topk", [(40, 511, 2), (40, 512, 2), (600, 513, 3), (1500, 1025, 4), (300, 2048, 9)])
+def test_single_rank_plan_of_many_experts(tokens, experts, topk):
+    """The plan scans 512 experts at a time; counts, offsets and alignment gaps go on across that line."""
+    idx = torch.rand(tokens, experts, generator=torch.Generator().manual_seed(experts)).topk(topk, dim=-1).indices
+    idx[::5, 0] = -1
+    for layout in (dict(do_expand=True, alignment=1), dict(do_expand=True, alignment=12), dict(do_expand=False, alignment=1)):
+        _one_rank_dispatch(idx, experts, 256, **layout)
+
+
 @pytest.mark.parametrize("tokens", [32768, 32769])  # the one-launch plan's largest call, and one for the stage and plan kernels
 @pytest.mark.parametrize("expand", [False, True])
 def test_single_rank_plan_limit(tokens, expand):
