@@ -228,8 +228,7 @@ __device__ bool stage_body(const StageParams& p) {
         }
         if (tid == 0) ctrl[WindowLayout::kTicketStage] = 0;
         if (R > 1) {
-            __threadfence_system();
-            __syncthreads();
+            __syncthreads();  // the signalling warp's fence stands for the block's (a second one here, by every thread, took 4 us)
             if (warp == 0) {
                 const bool ok = peer_barrier_warp(p.c.peers, p.c.rank, R, L.signal_offset, p.epoch, p.c.timeout_ns, status, kTagStage);
                 if (lane == 0) s_ok = ok;
@@ -1019,16 +1018,15 @@ struct FlagBoard {
     int finished[kMaxPushWarps];   // the transfer warp has no more work
 };
 
-struct FlagWriter {  // a transfer warp's end of the board (all lanes hold the same values)
+struct FlagWriter {  // a transfer warp's end of the board (all lanes hold the same values, except `mark`)
     FlagBoard* board;
     int warp;
-    int produced;
     int depth;  // bulk stores that may be pending before the warp waits
     uint64_t timeout_ns;
-    // Call right after committing the bulk group of the row that `flag` announces.
-    __device__ __forceinline__ void push(uint32_t* flag) {
-        const int lane = threadIdx.x & 31;
-        if (lane == 0) {
+    int produced = 0, handed = 0;  // flags on the ring, flags that the publisher may write
+    int groups = 0, mark = 0;      // bulk groups committed; lane g % 32: flags on the ring at the commit of group g
+    __device__ __forceinline__ void append(uint32_t* flag) {
+        if ((threadIdx.x & 31) == 0) {
             volatile int* published = board->published + warp;
             if (produced - *published >= kFlagRing) {  // ring full: the publisher is behind (bounded wait)
                 const uint64_t start = global_timer_ns();
@@ -1037,18 +1035,34 @@ struct FlagWriter {  // a transfer warp's end of the board (all lanes hold the s
             board->ring[warp][produced % kFlagRing] = flag;
         }
         ++produced;
+    }
+    __device__ __forceinline__ void hand_over(int count) {
+        __syncwarp();  // other lanes' stores are ordered before the hand-over
+        handed = count;
+        if ((threadIdx.x & 31) == 0) st_release_cta_smem(board->completed + warp, count);
+    }
+    // Call right after committing the bulk group of the row that `flag` announces.
+    __device__ __forceinline__ void push(uint32_t* flag) {
+        append(flag);
+        if ((threadIdx.x & 31) == (groups & 31)) mark = produced;
+        ++groups;
         bulk_wait_read<1>();              // the ring stage of the previous row may be refilled
         bulk_wait_depth(depth);           // everything older than the newest `depth` rows has landed
-        __syncwarp();                     // other lanes' gate-weight stores are ordered before the hand-over below
-        if (lane == 0 && produced > depth) st_release_cta_smem(board->completed + warp, produced - depth);
+        if (groups > depth) hand_over(__shfl_sync(kFull, mark, (groups - 1 - depth) & 31));
+        __syncwarp();
+    }
+    // A flag that announces no bulk store: handed over with the next one that does, or on its own where many have come together.
+    __device__ __forceinline__ void note(uint32_t* flag) {
+        append(flag);
+        if (produced - handed >= kFlagRing / 2) {
+            bulk_wait<0>();
+            hand_over(produced);
+        }
     }
     __device__ __forceinline__ void finish() {
         bulk_wait<0>();
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) {
-            st_release_cta_smem(board->completed + warp, produced);
-            st_release_cta_smem(board->finished + warp, 1);
-        }
+        hand_over(produced);
+        if ((threadIdx.x & 31) == 0) st_release_cta_smem(board->finished + warp, 1);
     }
 };
 
@@ -1086,6 +1100,11 @@ __device__ void combine_publish_role(const CombineParams& p, FlagBoard* board) {
     }
 }
 
+// Eight ranks of 512 tokens on one GPU: combine 238 -> 228 us (one row in eight is a rank's own: its copy was 2 x 59 MB through L2 and 59 MB
+// to memory); four ranks of 1000 skewed tokens 94 -> 92.  Whether the rows of a rank's own tokens stay in the expert output for the reduction to read: in the modes that return rows as
+// they are, and with the reduction that takes rows from anywhere (bulk loads into its ring).
+__device__ __forceinline__ bool own_rows_in_place(const CombineParams& p) { return p.reduce_stages >= 2 && p.mode != kPushExpandedReduce; }
+
 // Transfer warps.  Receive rows are visited round-robin over the source ranks (SourceWalk), so at every moment
 // the warps of a GPU address all destinations evenly; a row of the expert-major layout yields one transfer per
 // local slot.
@@ -1117,7 +1136,7 @@ __device__ void combine_push_role(const CombineParams& p, char* smem, FlagBoard*
     };
     request();
     const int depth = (p.store_depth == 4 || p.store_depth == 6 || p.store_depth == 8 || p.store_depth == 12) ? p.store_depth : 2;
-    FlagWriter flags{board, warp, 0, depth, p.c.timeout_ns};
+    FlagWriter flags{board, warp, depth, p.c.timeout_ns};
 
     if (p.mode == kPushExpandedReduce) {
         // FP32 sum of the row's local slots, one bf16 round, one store per (token, this rank).
@@ -1190,7 +1209,8 @@ __device__ void combine_push_role(const CombineParams& p, char* smem, FlagBoard*
 
     // One bulk load + one bulk store per transfer.  A cursor enumerates the transfers of this warp's rows:
     // compact layout = one per receive row; expert-major layout = one per local slot of the row.
-    const bool by_slot = p.mode == kPushExpanded;
+    // Rows of this rank's own tokens are not transferred where the reduction can read them in place (see combine_body).
+    const bool by_slot = p.mode == kPushExpanded, direct = own_rows_in_place(p);
     struct Cursor {
         unsigned left;  // choices of the current row that still need a transfer
         unsigned vm;    // all valid choices of the current row
@@ -1206,8 +1226,6 @@ __device__ void combine_push_role(const CombineParams& p, char* smem, FlagBoard*
                 const int item = take();
                 if (item >= walk.items) return false;
                 if (!walk.locate(item, r)) continue;
-                if (lane == (q_head & 31)) queued = r;
-                ++q_head;
             } else {
                 if (q_tail == q_head) return false;
                 r = __shfl_sync(kFull, queued, q_tail & 31);
@@ -1225,6 +1243,18 @@ __device__ void combine_push_role(const CombineParams& p, char* smem, FlagBoard*
                 c.vm = 0;
             }
             c.left = by_slot ? c.vm : (c.vm & (0u - c.vm));  // compact: the first valid choice names the partition
+            if (!leading) continue;
+            if (direct && c.src == p.c.rank) {
+                // The row stays where it is: its place in the return area takes its index, and the reduction reads the row itself.
+                const int part = L.rank_indexed ? p.c.rank : lane;
+                if ((c.left >> lane) & 1u) *reinterpret_cast<int*>(ret_row(p.c, c.src, part, c.tok)) = by_slot ? c.v : c.r;
+                if (p.w != nullptr && ((c.vm >> lane) & 1u))
+                    st_relaxed_sys_f32(ret_w_row(p.c, c.src, c.tok) + lane, by_slot ? p.w[c.v] : p.w[int64_t(c.r) * K + lane]);
+                for (; c.left != 0; c.left &= c.left - 1) flags.note(ret_flag(p.c, c.src, __shfl_sync(kFull, part, __ffs(c.left) - 1), c.tok));
+                continue;
+            }
+            if (lane == (q_head & 31)) queued = r;
+            ++q_head;
         }
         c.k = __ffs(c.left) - 1;
         c.left &= c.left - 1;
@@ -1473,7 +1503,7 @@ __device__ __forceinline__ char* reduce_area(const CombineParams& p, char* smem)
 // path needs seven dependent batches of loads per token.
 __device__ void combine_reduce_smem_role(const CombineParams& p, int* abort_word, char* area) {
     const WindowLayout& L = p.c.layout;
-    const int K = L.topk, Le = L.local_experts, E = int(L.num_experts), H = L.hidden, P = L.ret_parts;
+    const int K = L.topk, Le = L.local_experts, E = int(L.num_experts), H = L.hidden, P = p.reduce_parts;
     const int lane = threadIdx.x & 31;
     const int RW = (blockDim.x >> 5) - p.push_warps - 1;
     const int rwarp = (threadIdx.x >> 5) - p.push_warps - 1;
@@ -1500,6 +1530,7 @@ __device__ void combine_reduce_smem_role(const CombineParams& p, int* abort_word
         const int G = K <= 4 ? 4 : K <= 8 ? 8 : K <= 16 ? 16 : 32, W = 32 / G;
         const unsigned token_lanes = G == 32 ? kFull : (1u << G) - 1u;
         const int sub = lane / G, k = lane % G;
+        const bool direct = own_rows_in_place(p);
         auto token_of = [&](int i) { return int(blockIdx.x) + i * int(gridDim.x); };
         auto choice_of = [&](int i) -> int64_t { return i < n_tok && k < K ? p.topk[int64_t(token_of(i)) * K + k] : -1; };
         int64_t next = choice_of(sub);
@@ -1518,6 +1549,8 @@ __device__ void combine_reduce_smem_role(const CombineParams& p, int* abort_word
             const int my_part = L.rank_indexed ? dest : k;
             const uint32_t* flag = flag_base + int64_t(mine ? my_part : 0) * L.max_tokens + (mine ? t : 0);
             const unsigned my_lanes = token_lanes << (sub * G);
+            const bool in_place = mine && dest == p.c.rank && direct;
+            const char* from = ret_row(p.c, p.c.rank, mine ? my_part : 0, mine ? t : 0);  // the lane's row
             bool here = !mine;
             unsigned ordered = 0;  // lanes of the tokens that are complete and may be loaded
             for (int j = 0; j < W && base + j < n_tok; ++j) {
@@ -1549,6 +1582,7 @@ __device__ void combine_reduce_smem_role(const CombineParams& p, int* abort_word
                     // proxy fence orders the bulk loads below behind that
                     const bool complete = (seen & my_lanes) == my_lanes, fresh = complete && !((ordered >> lane) & 1u);
                     if (fresh && mine) (void)ld_acquire_sys_u32(flag);
+                    if (fresh && in_place) from = reinterpret_cast<const char*>(p.y + int64_t(*reinterpret_cast<const volatile int*>(from)) * H);
                     __syncwarp();
                     if (fresh && p.w_out != nullptr && k < K && base + sub < n_tok)
                         p.w_out[int64_t(t) * K + k] = valid ? __ldcg(ret_w + int64_t(t) * K + k) : 0.f;
@@ -1582,7 +1616,7 @@ __device__ void combine_reduce_smem_role(const CombineParams& p, int* abort_word
                     __syncwarp();
                     if (own && mine) {
                         const int at = __popc(token_parts & lanemask_lt());
-                        bulk_load_hint(area + (int64_t(s) * P + at) * cw, ret_row(p.c, p.c.rank, my_part, tok) + int64_t(c) * cw, uint32_t(bytes),
+                        bulk_load_hint(area + (int64_t(s) * P + at) * cw, from + int64_t(c) * cw, uint32_t(bytes),
                                        full + s, once);
                     }
                 }
@@ -1663,7 +1697,7 @@ __device__ void combine_body(const CombineParams& p) {
         if (p.reduce_stages >= 2) {
             // full: the loader's arrival plus the bytes of its bulk loads; empty: one arrival per consumer warp
             char* area = reduce_area(p, s_ring);
-            uint64_t* full = reinterpret_cast<uint64_t*>(area + ReduceArea::make(p.reduce_stages, L.ret_parts, p.reduce_chunk_bytes).barriers);
+            uint64_t* full = reinterpret_cast<uint64_t*>(area + ReduceArea::make(p.reduce_stages, p.reduce_parts, p.reduce_chunk_bytes).barriers);
             const int consumers = int(blockDim.x >> 5) - p.push_warps - 2;
             for (int s = 0; s < p.reduce_stages; ++s) {
                 mbar_init(full + s, 1);

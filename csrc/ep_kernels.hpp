@@ -156,6 +156,7 @@ struct CombineParams {
     // of a token are bulk-loaded into a ring of reduce_stages stages, reduce_chunk_bytes of every partition per stage.
     int reduce_stages;
     int reduce_chunk_bytes;
+    int reduce_parts;     // rows that a token can have: places in a stage
     int store_depth;      // bulk stores a transfer warp may have pending before it waits (2, 4, 6, 8 or 12; anything else means 2)
     // Optional diagnostics (null = off): [0] earliest start, [1] latest end of the transfer warps, [2] of the
     // publisher warps, [3] of the reduce warps, as %globaltimer nanoseconds; [4] nanoseconds the reduce groups spent

@@ -698,11 +698,14 @@ CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::T
     const int reduce_setting = g_trace.group != 0 ? g_trace.group : kDefaultReduceSetting;
     int pipe_stages = reduce_setting < 0 ? (-reduce_setting) / 1000 : 0;
     // by default whole rows that leave room in the pipeline's half of shared memory: more tokens in flight
-    const int64_t token_bytes = (int64_t(L.hidden) * 2 + 127) / 128 * 128 * L.ret_parts;
+    // One row per choice, or one per rank that a token went to: a stage has no places for more (compact rows of 4096 from four ranks,
+    // top-6: three stages instead of two, 95 -> 92 us).
+    const int parts = expand && !allow_multiple_reduction ? L.ret_parts : std::min({L.ret_parts, L.ranks, L.topk});
+    const int64_t token_bytes = (int64_t(L.hidden) * 2 + 127) / 128 * 128 * parts;
     if (g_trace.group == 0)
         while (pipe_stages < 4 && (pipe_stages + 1) * token_bytes <= lim.smem_optin / 2) ++pipe_stages;
     const int pipe_chunk = reduce_setting < 0 ? ((-reduce_setting) % 1000) * 128 : 0;
-    const CombinePlan plan = plan_combine(int64_t(L.hidden) * 2, L.ret_parts, lim.smem_optin, pipe_stages, pipe_chunk);
+    const CombinePlan plan = plan_combine(int64_t(L.hidden) * 2, parts, lim.smem_optin, pipe_stages, pipe_chunk);
     const RingPlan ring = plan.ring;
     TORCH_CHECK(ring.warps >= 1, "hidden size too large for the shared-memory row ring");
     reject_graph_capture(device, "barrier epochs and buffer parities are kernel arguments");
@@ -793,6 +796,7 @@ CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::T
             p.reduce_group = reduce_setting > 0 ? reduce_setting : 2;
             p.reduce_stages = plan.reduce_stages;
             p.reduce_chunk_bytes = plan.reduce_chunk_bytes;
+            p.reduce_parts = parts;
             if (g_trace.enabled && n == 1) {
                 if (!g_trace.words.defined()) g_trace.words = at::empty({9}, at::TensorOptions().dtype(at::kLong).device(at::kCUDA, device));
                 p.trace = reinterpret_cast<unsigned long long*>(g_trace.words.data_ptr<int64_t>());

@@ -147,6 +147,59 @@ def test_reduction_with_many_stages(setting):
         ext.set_combine_trace(False, 0, 0)
 
 
+@pytest.mark.parametrize("own_share", [0.0, 0.6, 1.0])  # of the choices that name an expert of the token's own rank
+@pytest.mark.parametrize("setting", [0, 2])  # reduction through its ring (own rows are read in place) and in registers (they are returned like others)
+@pytest.mark.parametrize("num_sms", [1, 3, None])  # one CTA: every row of a rank in one sequence, far more than a transfer warp's board of flags
+def test_rows_of_own_tokens(own_share, setting, num_sms):
+    from nanoep_b200.utils.build import load_extension
+
+    world, tokens, hidden, local, topk = 2, 230, 256, 6, 4
+    gen = torch.Generator().manual_seed(int(own_share * 10))
+    cfg = EPConfig(world * local, topk, hidden, tokens)
+    xs = [torch.randn(tokens, hidden, generator=gen).to(torch.bfloat16) for _ in range(world)]
+    ws = [torch.rand(tokens, topk, generator=gen) for _ in range(world)]
+    idxs = []
+    for r in range(world):
+        own = torch.rand(tokens, topk, generator=gen) < own_share
+        within = torch.rand(tokens, local, generator=gen).topk(topk, dim=-1).indices
+        idx = torch.where(own, within + r * local, within + (1 - r) * local)
+        idxs.append(idx.masked_fill(torch.rand(tokens, topk, generator=gen) < 0.15, -1))
+    values = [torch.randn(tokens, topk, hidden, generator=gen).to(torch.bfloat16) for _ in range(world)]  # what a choice's expert returns
+    ext = load_extension()
+    ext.set_combine_trace(False, 0, setting)
+    try:
+        with EmulatedGroup(world, cfg) as group:
+            for expand in (True, False, True):
+                got = group.dispatch(_cuda(xs), topk_idx=_cuda(idxs), weights=_cuda(ws), do_expand=expand, alignment=8 if expand else 1)
+                ys = []
+                for r in range(world):
+                    meta = got[r].handle.layout.recv_metadata.cpu().long()
+                    src, tok, v = meta[:, 0], meta[:, 1], meta[:, 2:]
+                    row, k = (v >= 0).nonzero(as_tuple=True)
+                    if expand:
+                        y = torch.full((got[r].handle.layout.expanded_capacity, hidden), float("nan"), dtype=torch.bfloat16)
+                        y[v[row, k]] = torch.stack(values)[src[row], tok[row], k]
+                    else:
+                        y = torch.stack(values)[src, tok, (v >= 0).int().argmax(-1)]  # the rank's first choice names the row
+                    ys.append(y.cuda())
+                back = group.combine(ys, [g.handle for g in got], weights=[g.topk_weights for g in got], num_sms=num_sms)
+                torch.cuda.synchronize()
+                group.check_status()
+                for r in range(world):
+                    want = torch.zeros(tokens, hidden)
+                    for k in range(topk):  # FP32 in ascending choice
+                        e = idxs[r][:, k]
+                        counts = e >= 0
+                        if not expand:  # one row per rank, with its first choice
+                            earlier = (idxs[r][:, :k] >= 0) & (idxs[r][:, :k] // local == (e // local)[:, None])
+                            counts = counts & ~earlier.any(-1)
+                        want = torch.where(counts[:, None], want + values[r][:, k].float(), want)
+                    assert torch.equal(back[r].x.cpu().view(torch.int16), want.to(torch.bfloat16).view(torch.int16)), (expand, r)
+                    assert torch.equal(back[r].topk_weights.cpu(), ws[r].masked_fill(idxs[r] < 0, 0))
+    finally:
+        ext.set_combine_trace(False, 0, 0)
+
+
 @pytest.mark.parametrize("masked", ["none", "choices", "tokens", "all"])
 @pytest.mark.parametrize("expand,alignment", [(False, 1), (True, 1), (True, 16)])
 @pytest.mark.parametrize("weighted", [False, True])
