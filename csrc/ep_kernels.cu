@@ -1963,8 +1963,8 @@ __device__ __forceinline__ const P& block_of(const Many<P>& all) {
     __global__ void __launch_bounds__(__VA_ARGS__) name##_kernel(const __grid_constant__ Params p) { name##_body(p); } \
     __global__ void __launch_bounds__(__VA_ARGS__) name##_multi_kernel(const __grid_constant__ Many<Params> all) { name##_body(block_of(all)); }
 
-__global__ void __launch_bounds__(kStageThreads) stage_kernel(const __grid_constant__ StageParams p) { stage_body(p); }
-__global__ void __launch_bounds__(kStageThreads) stage_multi_kernel(const __grid_constant__ Many<StageParams> all) { stage_body(block_of(all)); }
+__global__ void __launch_bounds__(kStageThreads, 2) stage_kernel(const __grid_constant__ StageParams p) { stage_body(p); }
+__global__ void __launch_bounds__(kStageThreads, 2) stage_multi_kernel(const __grid_constant__ Many<StageParams> all) { stage_body(block_of(all)); }
 __global__ void __launch_bounds__(kLocalPlanThreads) local_plan_kernel(const __grid_constant__ LocalPlanParams p) { local_plan_body(p); }
 NEP_KERNEL_PAIR(plan, PlanParams, kPlanThreads)
 NEP_KERNEL_PAIR(pull, PullParams, 256)
