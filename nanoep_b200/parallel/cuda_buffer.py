@@ -223,18 +223,6 @@ class CudaBuffer:
         return self._auto_num_sms
 
     # ------------------------------------------------------------------ dispatch
-    def _check_dispatch(self, x, topk_idx, handle, do_expand, alignment):
-        check_torch_deterministic()
-        if self._closed:
-            raise RuntimeError("CudaBuffer is closed")
-        expand, expert_alignment = resolve_layout_args(self, handle, topk_idx, do_expand, alignment)
-        routing = handle.topk_idx if handle is not None else topk_idx
-        if x.dim() != 2 or x.shape[1] != self._config.hidden:
-            raise ValueError("x hidden dimension does not match the buffer configuration")
-        if routing.shape != (x.shape[0], self._config.num_topk):
-            raise ValueError("routing snapshot/topk_idx shape must match the buffer configuration")
-        return expand, expert_alignment, routing
-
     def dispatch(
         self,
         x: torch.Tensor,
@@ -259,7 +247,16 @@ class CudaBuffer:
         ``ring_smem_limit`` caps the pull kernel's shared-memory ring (bytes per CTA) so that such a
         consumer can share the SMs with it; 0 uses all of the CTA's shared memory.
         """
-        expand, expert_alignment, routing = self._check_dispatch(x, topk_idx, handle, do_expand, alignment)
+        check_torch_deterministic()
+        if self._closed:
+            raise RuntimeError("CudaBuffer is closed")
+        expand, expert_alignment = resolve_layout_args(self, handle, topk_idx, do_expand, alignment)
+        routing = handle.topk_idx if handle is not None else topk_idx
+        if x.dim() != 2 or x.shape[1] != self._config.hidden:
+            raise ValueError("x hidden dimension does not match the buffer configuration")
+        if routing.shape != (x.shape[0], self._config.num_topk):
+            raise ValueError("routing snapshot/topk_idx shape must match the buffer configuration")
+
         main_sms = self._resolve_num_sms(num_sms, handle)
         if handle is not None and handle.native_state is not None:
             with _OnDevice(self._device), nvtx_range("nanoep.dispatch.cached"):
@@ -358,14 +355,22 @@ class CudaBuffer:
     def _run_layer(self, x, topk_idx, weights, handle, bias, w13, w2, gemm_status, alignment, fuse_combine):
         """Dispatch, SwiGLU experts and combine in one native call (models/moe_layer.py): ``(result, handle)``."""
         fresh = handle is None
-        expand, expert_alignment, _ = self._check_dispatch(x, None if not fresh else topk_idx, handle, True if fresh else None, alignment if fresh else None)
+        check_torch_deterministic()
+        if self._closed:
+            raise RuntimeError("CudaBuffer is closed")
+        topk_idx = topk_idx if fresh else None
+        expand, expert_alignment = resolve_layout_args(self, handle, topk_idx, True if fresh else None, alignment if fresh else None)
+        if x.dim() != 2 or x.shape[1] != self._config.hidden:
+            raise ValueError("x hidden dimension does not match the buffer configuration")
+        if (topk_idx if fresh else handle.topk_idx).shape != (x.shape[0], self._config.num_topk):
+            raise ValueError("routing snapshot/topk_idx shape must match the buffer configuration")
         if bias is not None and not fuse_combine:  # the fused path checks it in front of its reduction
             check_combine_bias(bias, (x.shape[0], self._config.hidden), x.dtype, torch.device("cuda", self._device))
         main_sms = self._resolve_num_sms(None, handle)
         cached_metadata, cached_capacity = ([], 0) if fresh else (handle_metadata(handle), handle.layout.expanded_capacity)
         with _OnDevice(self._device), nvtx_range("nanoep.layer"):
             out, metadata, counts = self._backend.moe_forward(
-                self._window, x, topk_idx if fresh else None, weights, cached_metadata, cached_capacity, expand, expert_alignment, w13, w2,
+                self._window, x, topk_idx, weights, cached_metadata, cached_capacity, expand, expert_alignment, w13, w2,
                 gemm_status, bias, fuse_combine, self._allow_multiple_reduction, main_sms, self._comm_stream.cuda_stream, self._mailbox_timeout_s,
             )
         if fresh:
