@@ -228,7 +228,8 @@ __device__ bool stage_body(const StageParams& p) {
         }
         if (tid == 0) ctrl[WindowLayout::kTicketStage] = 0;
         if (R > 1) {
-            __syncthreads();  // the signalling warp's fence stands for the block's (a second one here, by every thread, took 4 us)
+            __threadfence_system();
+            __syncthreads();
             if (warp == 0) {
                 const bool ok = peer_barrier_warp(p.c.peers, p.c.rank, R, L.signal_offset, p.epoch, p.c.timeout_ns, status, kTagStage);
                 if (lane == 0) s_ok = ok;
@@ -380,7 +381,7 @@ __device__ bool stage_body(const StageParams& p) {
 // the handle's tensors, and N and C reach the host before the rows are assigned.
 // Against stage + plan, top-8 of 256 experts: 1 token 22 -> 6.6 us, 256 tokens 14.6 -> 8.1 us, 4096 tokens 25 -> 14 us;
 // the pull of a call whose output bound is modest no longer waits for the host: 1 token and its combine 59 -> 52 us.
-// A chain of latencies throughout, so: the counts reach the host in front of the stores that nothing waits for, all threads scan
+// A chain of latencies throughout, so: all threads scan
 // the experts instead of one warp in waves, the other CTAs' counts and the slots of eight choices are asked for at once, and a warp
 // keeps the choices of its only chunk.  1 token 6.2 -> 5.1 us, 256 tokens 7.6 -> 6.1, 4096 tokens 13.8 -> 12.4; calls of
 // 1, 32 and 256 tokens with their combine 37.3 -> 36.7, 38.3 -> 37.7 and 41.0 -> 39.9 us, of 4096 tokens 226.5 -> 225.1.
@@ -516,14 +517,14 @@ __device__ void local_plan_body(const LocalPlanParams& p) {
         p.expert_offsets[E] = capacity;
         p.recv_rank_prefix[0] = s_all;
         p.send_counts[0] = s_all;
-        // nothing that the host or a later kernel of this stream does with the counts needs the stores above
-        if (p.gated == 0 && s_any_invalid == 0) publish_counts(p.mailbox, s_all, capacity, false);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        __syncwarp();  // everybody's offsets and counts are behind the block barrier above
+        // the report of an invalid id reaches the host before the counts do: the call after this one raises it
+        if (lane == 0 && cta == 0) publish_counts(p.mailbox, s_all, capacity, p.gated != 0 || s_any_invalid != 0);
     }
     cluster_arrive();  // this CTA has read the others' counts; they may exit once everybody has
-    __syncthreads();
-    // a consumer on another stream relies on offsets and counts, all written before the block barrier; the report of an
-    // invalid id reaches the host before the counts do: the call after this one raises it
-    if (cta == 0 && tid == 0 && (p.gated != 0 || s_any_invalid != 0)) publish_counts(p.mailbox, s_all, capacity, true);
     // ---- assign rows and slots
     for (int ch = warp; ch < my_chunks; ch += kWarps) {
         const int tok0 = (first_chunk + ch) * 32;
