@@ -755,7 +755,7 @@ __device__ void pull_body(const PullParams& p) {
     Ring ring = make_ring(s_ring, wpb, p.stages, rb);
     const int S = p.stages;
     wait_for_previous();
-    allow_dependents();  // behind the wait: what a dependent reads before its own has been written by then (offsets, counts)
+    if (p.dependents) allow_dependents();  // behind the wait: what a dependent reads before its own has been written by then (offsets, counts)
     if (p.data_epoch != 0) {
         // A fresh dispatch stages its rows underneath the count exchange: every source signals when its rows are in place.
         __shared__ int s_staged;

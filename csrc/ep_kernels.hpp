@@ -101,6 +101,7 @@ struct PullParams {
     int expand;
     int zero_padding;
     int write_meta;
+    int dependents;  // the kernel behind this one may be set up while it runs (the expert layer's up-projection)
     int stages;
     int zero_bytes;  // zero source in shared memory behind the rings (see RingPlan)
     __nv_bfloat16* x_out;

@@ -522,6 +522,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             p.expand = expand;
             p.zero_padding = zero_padding;
             p.write_meta = fresh && !plan_locally;
+            p.dependents = behind ? 1 : 0;
             p.stages = ring.stages;
             p.zero_bytes = ring.zero_bytes;
             p.x_out = reinterpret_cast<__nv_bfloat16*>(o[0].data_ptr());
