@@ -2,6 +2,7 @@
 // diagnostics.  Same boundary as the reference's csrc/bindings.cpp:11-86.
 #include <torch/extension.h>
 
+#include "flag_queue.hpp"
 #include "gemm_api.hpp"
 #include "pipeline.hpp"
 
@@ -16,6 +17,25 @@ struct HandleState {
     std::vector<at::Tensor> metadata;  // same order as DispatchOut::metadata
     int64_t capacity;
     bool expand;
+};
+
+// Host side of a FlagQueue: what a transfer warp would have done, step by step.
+struct FlagModel {
+    int marks[32] = {}, groups = 0, landed = 0, completed = 0;
+    std::vector<int> group_of;  // per flag: the bulk group that it announces, -1: none
+    bool early = false;         // a flag was handed over in front of its row
+    void append(int group, int at) {
+        if (at != int(group_of.size())) throw std::logic_error("flags out of order");
+        group_of.push_back(group);
+        groups = std::max(groups, group + 1);
+    }
+    void set_mark(int i, int count) { marks[i] = count; }
+    int mark(int i) const { return marks[i]; }
+    void wait_landed(int depth) { landed = std::max(landed, groups - depth); }
+    void publish_up_to(int count) {
+        completed = count;
+        for (int i = 0; i < count; ++i) early = early || group_of.at(size_t(i)) >= landed;
+    }
 };
 
 py::dict layout_dict(const nep::WindowLayout& w) {
@@ -191,6 +211,23 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         },
         py::arg("hidden"), py::arg("topk"), py::arg("max_smem_bytes"), py::arg("shared"),
         "Shared-memory plan of a pull CTA: (transfer warps, ring stages, bytes of the zero source, dynamic bytes)");
+    m.def(
+        "flag_queue_trace",
+        [](const std::string& steps, int depth) {
+            nep::FlagQueue<FlagModel, int> queue{FlagModel{}, depth};
+            std::vector<std::tuple<int, int, bool>> out;
+            for (const char step : steps) {
+                if (step == 'n') queue.note(-1); else queue.push(queue.groups);
+                out.emplace_back(queue.produced, queue.io.completed, queue.io.early);
+            }
+            queue.finish();
+            out.emplace_back(queue.produced, queue.io.completed, queue.io.early);
+            return out;
+        },
+        py::arg("steps"), py::arg("depth"),
+        "Flags of a combine's transfer warp ('p': of a row that it stores, 'n': of a row that stays): after every step and at the end "
+        "(on the ring, handed to the publisher, whether one was handed over before its row had landed)");
+    m.def("flag_ring", [] { return std::make_pair(nep::kFlagRing, nep::kMaxStoreDepth); });
     m.def("set_combine_trace", &nep::set_combine_trace, py::arg("enabled"), py::arg("store_depth") = 0, py::arg("reduce_group") = 0);
     m.def("take_combine_trace", &nep::take_combine_trace);
     m.def("take_stage_trace", &nep::take_stage_trace);

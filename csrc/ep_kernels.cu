@@ -6,6 +6,7 @@
 #include <mutex>
 #include <utility>
 
+#include "flag_queue.hpp"
 #include "prim.cuh"
 
 namespace nep {
@@ -999,16 +1000,15 @@ __device__ __forceinline__ int4 pack8(const float* acc) {
 // Arrival flags are published by a dedicated warp, not by the transfer warps: a flag needs a system-scope
 // release after its row has landed, and that fence waits for remote stores in flight.  A transfer warp only
 // appends the flag's address to its ring on this board and reports how many of its bulk stores have COMPLETED
-// (cp.async.bulk.wait_group, not .read; up to kStoresInFlight may be pending).  The publisher warp sweeps the
+// (cp.async.bulk.wait_group, not .read; up to a FlagQueue's depth may be pending).  The publisher warp sweeps the
 // boards, fences once per sweep and writes the flags of everything that completed since its last sweep.
-constexpr int kFlagRing = 32;  // entries per transfer warp
 constexpr int kMaxPushWarps = 8;
 __device__ __forceinline__ void bulk_wait_depth(int depth) {
     switch (depth) {
         case 4: bulk_wait<4>(); break;
         case 6: bulk_wait<6>(); break;
         case 8: bulk_wait<8>(); break;
-        case 12: bulk_wait<12>(); break;
+        case kMaxStoreDepth: bulk_wait<kMaxStoreDepth>(); break;
         default: bulk_wait<2>(); break;
     }
 }
@@ -1019,50 +1019,43 @@ struct FlagBoard {
     int finished[kMaxPushWarps];   // the transfer warp has no more work
 };
 
-struct FlagWriter {  // a transfer warp's end of the board (all lanes hold the same values, except `mark`)
+// A transfer warp's end of the board, under a FlagQueue (all lanes hold the same values, except `kept`).
+struct FlagWriter {
     FlagBoard* board;
     int warp;
-    int depth;  // bulk stores that may be pending before the warp waits
     uint64_t timeout_ns;
-    int produced = 0, handed = 0;  // flags on the ring, flags that the publisher may write
-    int groups = 0, mark = 0;      // bulk groups committed; lane g % 32: flags on the ring at the commit of group g
-    __device__ __forceinline__ void append(uint32_t* flag) {
+    StatusRef status;
+    int kept = 0;  // lane i: mark i
+    __device__ __forceinline__ void append(uint32_t* flag, int at) {
         if ((threadIdx.x & 31) == 0) {
             volatile int* published = board->published + warp;
-            if (produced - *published >= kFlagRing) {  // ring full: the publisher is behind (bounded wait)
+            if (at - *published >= kFlagRing) {  // ring full: the publisher is behind (bounded wait)
                 const uint64_t start = global_timer_ns();
-                while (produced - *published >= kFlagRing && global_timer_ns() - start < timeout_ns) __nanosleep(64);
+                while (at - *published >= kFlagRing && global_timer_ns() - start < timeout_ns) __nanosleep(64);
             }
-            board->ring[warp][produced % kFlagRing] = flag;
+            if (at - *published < kFlagRing)
+                board->ring[warp][at % kFlagRing] = flag;
+            else  // the entry still holds a flag that has to go out
+                report(status, kCopyTimeout, uint32_t(warp), kTagPush);
         }
-        ++produced;
     }
-    __device__ __forceinline__ void hand_over(int count) {
-        __syncwarp();  // other lanes' stores are ordered before the hand-over
-        handed = count;
+    __device__ __forceinline__ void set_mark(int i, int count) {
+        if ((threadIdx.x & 31) == i) kept = count;
+    }
+    __device__ __forceinline__ int mark(int i) const { return __shfl_sync(kFull, kept, i); }
+    __device__ __forceinline__ void wait_landed(int depth) {
+        if (depth == 0) {
+            bulk_wait<0>();
+        } else {
+            bulk_wait_read<1>();  // the ring stage of the previous row may be refilled
+            bulk_wait_depth(depth);
+        }
+        __syncwarp();  // by any lane; and other lanes' stores are ordered before a hand-over
+    }
+    __device__ __forceinline__ void publish_up_to(int count) {
         if ((threadIdx.x & 31) == 0) st_release_cta_smem(board->completed + warp, count);
     }
-    // Call right after committing the bulk group of the row that `flag` announces.
-    __device__ __forceinline__ void push(uint32_t* flag) {
-        append(flag);
-        if ((threadIdx.x & 31) == (groups & 31)) mark = produced;
-        ++groups;
-        bulk_wait_read<1>();              // the ring stage of the previous row may be refilled
-        bulk_wait_depth(depth);           // everything older than the newest `depth` rows has landed
-        if (groups > depth) hand_over(__shfl_sync(kFull, mark, (groups - 1 - depth) & 31));
-        __syncwarp();
-    }
-    // A flag that announces no bulk store: handed over with the next one that does, or on its own where many have come together.
-    __device__ __forceinline__ void note(uint32_t* flag) {
-        append(flag);
-        if (produced - handed >= kFlagRing / 2) {
-            bulk_wait<0>();
-            hand_over(produced);
-        }
-    }
-    __device__ __forceinline__ void finish() {
-        bulk_wait<0>();
-        hand_over(produced);
+    __device__ __forceinline__ void no_more() {
         if ((threadIdx.x & 31) == 0) st_release_cta_smem(board->finished + warp, 1);
     }
 };
@@ -1136,8 +1129,8 @@ __device__ void combine_push_role(const CombineParams& p, char* smem, FlagBoard*
         return v;
     };
     request();
-    const int depth = (p.store_depth == 4 || p.store_depth == 6 || p.store_depth == 8 || p.store_depth == 12) ? p.store_depth : 2;
-    FlagWriter flags{board, warp, depth, p.c.timeout_ns};
+    const int depth = (p.store_depth == 4 || p.store_depth == 6 || p.store_depth == 8 || p.store_depth == kMaxStoreDepth) ? p.store_depth : 2;
+    FlagQueue<FlagWriter, uint32_t*> flags{FlagWriter{board, warp, p.c.timeout_ns, status}, depth};
 
     if (p.mode == kPushExpandedReduce) {
         // FP32 sum of the row's local slots, one bf16 round, one store per (token, this rank).
@@ -1205,6 +1198,7 @@ __device__ void combine_push_role(const CombineParams& p, char* smem, FlagBoard*
             flags.push(ret_flag(p.c, src, part, tok));
         }
         flags.finish();
+        flags.io.no_more();
         return;
     }
 
@@ -1293,6 +1287,7 @@ __device__ void combine_push_role(const CombineParams& p, char* smem, FlagBoard*
         if (more && (more = next(ahead, true))) issue(ahead, issued++);
     }
     flags.finish();
+    flags.io.no_more();
 }
 
 // Which return partitions hold a row for source token `t`, as a mask over the lanes (choices) that name them;

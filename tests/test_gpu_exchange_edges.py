@@ -147,24 +147,30 @@ def test_reduction_with_many_stages(setting):
         ext.set_combine_trace(False, 0, 0)
 
 
-@pytest.mark.parametrize("own_share", [0.0, 0.6, 1.0])  # of the choices that name an expert of the token's own rank
-@pytest.mark.parametrize("setting", [0, 2])  # reduction through its ring (own rows are read in place) and in registers (they are returned like others)
-@pytest.mark.parametrize("num_sms", [1, 3, None])  # one CTA: every row of a rank in one sequence, far more than a transfer warp's board of flags
-def test_rows_of_own_tokens(own_share, setting, num_sms):
+def _own_rows_round_trip(tokens, own_shares, setting, num_sms, seed, run=1):
+    """Two ranks with `tokens` tokens each (one number per rank) of which a share of the choices names an expert of the token's own
+    rank (drawn for `run` tokens at a time); every choice comes back with values of its own."""
     from nanoep_b200.utils.build import load_extension
 
-    world, tokens, hidden, local, topk = 2, 230, 256, 6, 4
-    gen = torch.Generator().manual_seed(int(own_share * 10))
-    cfg = EPConfig(world * local, topk, hidden, tokens)
-    xs = [torch.randn(tokens, hidden, generator=gen).to(torch.bfloat16) for _ in range(world)]
-    ws = [torch.rand(tokens, topk, generator=gen) for _ in range(world)]
+    world, hidden, local, topk = 2, 256, 6, 4
+    gen = torch.Generator().manual_seed(seed)
+    cfg = EPConfig(world * local, topk, hidden, max(tokens))
+    xs = [torch.randn(n, hidden, generator=gen).to(torch.bfloat16) for n in tokens]
+    ws = [torch.rand(n, topk, generator=gen) for n in tokens]
     idxs = []
-    for r in range(world):
-        own = torch.rand(tokens, topk, generator=gen) < own_share
-        within = torch.rand(tokens, local, generator=gen).topk(topk, dim=-1).indices
+    for r, n in enumerate(tokens):
+        if run == 1:
+            own = torch.rand(n, topk, generator=gen) < own_shares[r]
+        else:
+            own = (torch.rand((n + run - 1) // run, 1, generator=gen) < own_shares[r]).repeat_interleave(run, 0)[:n].expand(n, topk)
+        within = torch.rand(n, local, generator=gen).topk(topk, dim=-1).indices
         idx = torch.where(own, within + r * local, within + (1 - r) * local)
-        idxs.append(idx.masked_fill(torch.rand(tokens, topk, generator=gen) < 0.15, -1))
-    values = [torch.randn(tokens, topk, hidden, generator=gen).to(torch.bfloat16) for _ in range(world)]  # what a choice's expert returns
+        idxs.append(idx.masked_fill(torch.rand(n, topk, generator=gen) < 0.15, -1))
+    # what a choice's expert returns; ranks may have different numbers of tokens
+    values = [torch.randn(n, topk, hidden, generator=gen).to(torch.bfloat16) for n in tokens]
+    padded = torch.zeros(world, max(tokens), topk, hidden, dtype=torch.bfloat16)
+    for r, v in enumerate(values):
+        padded[r, : v.shape[0]] = v
     ext = load_extension()
     ext.set_combine_trace(False, 0, setting)
     try:
@@ -178,15 +184,15 @@ def test_rows_of_own_tokens(own_share, setting, num_sms):
                     row, k = (v >= 0).nonzero(as_tuple=True)
                     if expand:
                         y = torch.full((got[r].handle.layout.expanded_capacity, hidden), float("nan"), dtype=torch.bfloat16)
-                        y[v[row, k]] = torch.stack(values)[src[row], tok[row], k]
+                        y[v[row, k]] = padded[src[row], tok[row], k]
                     else:
-                        y = torch.stack(values)[src, tok, (v >= 0).int().argmax(-1)]  # the rank's first choice names the row
+                        y = padded[src, tok, (v >= 0).int().argmax(-1)]  # the rank's first choice names the row
                     ys.append(y.cuda())
                 back = group.combine(ys, [g.handle for g in got], weights=[g.topk_weights for g in got], num_sms=num_sms)
                 torch.cuda.synchronize()
                 group.check_status()
-                for r in range(world):
-                    want = torch.zeros(tokens, hidden)
+                for r, n in enumerate(tokens):
+                    want = torch.zeros(n, hidden)
                     for k in range(topk):  # FP32 in ascending choice
                         e = idxs[r][:, k]
                         counts = e >= 0
@@ -198,6 +204,20 @@ def test_rows_of_own_tokens(own_share, setting, num_sms):
                     assert torch.equal(back[r].topk_weights.cpu(), ws[r].masked_fill(idxs[r] < 0, 0))
     finally:
         ext.set_combine_trace(False, 0, 0)
+
+
+@pytest.mark.parametrize("own_share", [0.0, 0.6, 1.0])  # of the choices that name an expert of the token's own rank
+@pytest.mark.parametrize("setting", [0, 2])  # reduction through its ring (own rows are read in place) and in registers (they are returned like others)
+@pytest.mark.parametrize("num_sms", [1, 3, None])  # one CTA: every row of a rank in one sequence, far more than a transfer warp's board of flags
+def test_rows_of_own_tokens(own_share, setting, num_sms):
+    _own_rows_round_trip([230, 230], [own_share] * 2, setting, num_sms, int(own_share * 10))
+
+
+@pytest.mark.parametrize("tokens,own_shares,run", [([700, 5], [0.98, 0.5], 1), ([613, 40], [0.9, 0.0], 37), ([64, 1000], [1.0, 0.95], 50), ([0, 333], [0.0, 1.0], 1)])
+@pytest.mark.parametrize("num_sms", [1, 2])
+def test_runs_of_own_tokens_between_few_others(tokens, own_shares, run, num_sms):
+    """Flags of rows that stay where they are come in runs longer than a transfer warp's board, with few stored rows between."""
+    _own_rows_round_trip(tokens, own_shares, 0, num_sms, sum(tokens) + run, run)
 
 
 @pytest.mark.parametrize("masked", ["none", "choices", "tokens", "all"])

@@ -442,3 +442,37 @@ def test_grouped_gemm_choice_by_size():
         assert choice(rows=rows, n=4096, sms=148, counts=True) == "expert"
     # a cap on the grid moves the line: three tiles, three CTAs, but one pair
     assert choice(rows=384, n=256, max_ctas=3) == "single" and choice(rows=384, n=256, max_ctas=4) == "expert"
+
+
+def _flag_steps(rng, length, share_of_notes, run):
+    """Rows that are stored ('p') and rows that stay ('n') in runs, as routing that favours the own rank gives them."""
+    steps = ""
+    while len(steps) < length:
+        steps += ("n" if rng.random() < share_of_notes else "p") * rng.randint(1, run)
+    return steps[:length]
+
+
+@pytest.mark.parametrize("depth", [2, 4, 6, 8, 12])
+@pytest.mark.parametrize("share_of_notes", [0.0, 0.3, 0.7, 0.95, 1.0])
+def test_flags_of_a_combine_are_handed_over_once_and_in_time(depth, share_of_notes):
+    """What a transfer warp hands to the publisher never falls (the publisher may have written it already, and would wait for
+    more while the warp waits for room), leaves room on the ring, comes behind the rows, and is everything in the end."""
+    import random
+
+    from nanoep_b200.utils.build import load_extension
+
+    ext = load_extension()
+    ring, deepest = ext.flag_ring()
+    assert deepest == 12
+    rng = random.Random(depth * 100 + int(share_of_notes * 10))
+    steps = [_flag_steps(rng, rng.randint(0, 200), share_of_notes, run) for run in (1, 3, 20, 60) for _ in range(50)]
+    steps += ["n" * 40 + "p" * 20, "p" * 40, ("n" * 15 + "p") * 9, ("n" * 16 + "p" * depth) * 5, "p" + "n" * 100 + "p"]
+    for case in steps:
+        before = 0
+        for produced, handed, early in ext.flag_queue_trace(case, depth):
+            assert not early, case
+            assert before <= handed <= produced, (case, produced, before, handed)
+            # the next flag finds room as soon as the publisher has written what it was handed
+            assert produced - handed < ring, (case, produced, handed)
+            before = handed
+        assert handed == produced == len(case)
