@@ -255,7 +255,7 @@ pybind11::tuple moe_forward(PeerWindow& window, const at::Tensor& x, const c10::
         const int64_t tokens = x.size(0), most = std::max<int64_t>(1, bound ? tokens : got.counts[0].first);
         const int64_t assigned = bound ? tokens * window.layout().topk : -1;
         at::Tensor h = at::empty({rows.size(0), w13.size(1) / 2}, bf16);
-        grouped_gemm(rows, w13, offsets, h, status, gemm::kSwiGLU, {}, {}, 0, 5.0, {}, 4, false, counts, most, true, assigned);
+        grouped_gemm(rows, w13, offsets, h, status, gemm::kSwiGLU, {}, {}, 0, 5.0, {}, 4, false, counts, most, got.early, assigned);
         if (fuse_combine) {
             grouped_gemm_scatter(window, h, w2, offsets, m[7], m[0], gate, status, 0, 5.0, counts, most, true, assigned);
             result = combine_finish({&window}, got.metadata, {bias})[0];

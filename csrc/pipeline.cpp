@@ -416,6 +416,8 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
                             bound_bytes <= kFusedFreshMaxOutputBytes && (!expand || bound_rows_c <= L.slot_scratch_ints) &&
                             ring.warps >= 2 && ring.smem_bytes >= size_t(stage_smem_bytes(L)) &&
                             ring.smem_bytes >= size_t(ring.warps) * 32 * L.topk * 4;
+    // The single-launch fresh kernel writes offsets and counts itself: what follows it is ordered behind all of it.
+    out.early = behind && !fuse_fresh;
     const StageParams* stage_dev = nullptr;
     const PlanParams* plan_dev = nullptr;
     std::vector<PlanParams> plan(fresh ? n : 0);  // outlives the launches: a single-rank call passes it by host pointer
@@ -522,7 +524,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             p.expand = expand;
             p.zero_padding = zero_padding;
             p.write_meta = fresh && !plan_locally;
-            p.dependents = behind ? 1 : 0;
+            p.dependents = out.early;
             p.stages = ring.stages;
             p.zero_bytes = ring.zero_bytes;
             p.x_out = reinterpret_cast<__nv_bfloat16*>(o[0].data_ptr());

@@ -33,6 +33,9 @@ struct DispatchOut {
     //            recv_rank_prefix, slot_map]
     std::vector<std::vector<at::Tensor>> metadata;
     std::vector<std::pair<int64_t, int64_t>> counts;  // (N, C)
+    // The dispatch's last kernel lets the one behind it start while it runs, and what that one may read without waiting (the handle's
+    // offsets and counts) is the work of kernels that have ended by then.
+    bool early = false;
     std::shared_ptr<CompletionEvent> event;            // null unless async_op
 };
 

@@ -116,7 +116,7 @@ class ExpertParallelMoE:
             mark("dispatch+up_gemm")
         else:
             mark("dispatch")
-            h = self._grouped(h_in, self.w13, offsets, self.inner, gg.SWIGLU, None, counts, most)
+            h = self._grouped(h_in, self.w13, offsets, self.inner, gg.SWIGLU, None, counts, most, False)
             mark("up_gemm")
         self.last_handle = got.handle
         if self.fuse_combine:
@@ -135,10 +135,10 @@ class ExpertParallelMoE:
         self._collect(marks)
         return out
 
-    def _grouped(self, a, w, offsets, columns, mode, scale, counts, most, early=True):
-        """A grouped GEMM that may start while the kernel in front of it (the dispatch's pull, the up-projection) ends: nothing
-        from the pull on writes weights, offsets or counts, and the pull lets its dependents start only once all that lies
-        before it has ended."""
+    def _grouped(self, a, w, offsets, columns, mode, scale, counts, most, early):
+        """A grouped GEMM that may start while the kernel in front of it ends (``early``): the down-projection behind the
+        up-projection, since neither writes weights, offsets or counts and those are complete before the up-projection starts.
+        The up-projection itself follows a dispatch that was not told about it, and waits for its end."""
         out = torch.empty((a.shape[0], columns), dtype=torch.bfloat16, device=a.device)
         self._ext.grouped_gemm(a, w, offsets, out, gg.status_tensor(a.device), mode, None, None, 0, 5.0, scale, 4, False, counts, most, early)
         return out

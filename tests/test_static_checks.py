@@ -166,3 +166,17 @@ def test_gemm_kernels_clear_their_abort_flag_before_anyone_sets_it():
     for name in ("grouped_gemm_sm100.cu", "grouped_gemm_sm100_2cta.cu", "expert_gemm_sm100.cu"):
         text = re.sub(r"//[^\n]*", "", (ROOT / "csrc" / name).read_text())
         assert "__syncthreads();" in text[text.index("sh.abort = 0;") : text.index("sh.abort = 1;")], name
+
+
+def test_what_starts_early_reads_only_what_ended_kernels_wrote():
+    """The expert GEMM reads offsets and counts in front of its wait for the previous kernel.  Behind a dispatch that is safe where
+    the last kernel has not written them itself: the single-launch fresh dispatch has."""
+    host, layer = (re.sub(r"//[^\n]*", "", (ROOT / "csrc" / name).read_text()) for name in ("pipeline.cpp", "gemm_bindings.cpp"))
+    assert re.findall(r"out\.early = ([^;]+);", host) == ["behind && !fuse_fresh"]
+    assert re.findall(r"\.dependents = ([^;]+);", host) == ["out.early"]
+    assert host.index("const bool fuse_fresh =") < host.index("out.early =") < host.index("p.dependents =")
+    body = _body(layer, "pybind11::tuple moe_forward")
+    up = re.search(r"grouped_gemm\(rows, w13,[^;]*;", body).group(0)
+    assert "got.early" in up and "true" not in up
+    steps = (ROOT / "nanoep_b200" / "models" / "moe_layer.py").read_text()
+    assert re.search(r"self\._grouped\(h_in, self\.w13,[^)]*, False\)", steps)
