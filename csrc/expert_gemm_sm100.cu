@@ -342,6 +342,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
         if (leader && elect_one()) {
             int stage = 0, item = 0;
             uint32_t phase = 0;
+            wait_for_previous();  // the time limits below are this kernel's, not those of a pull that waits for its peers in front of it
             for (int i = first_unit; i >= 0 && !*abort_flag; i = next_unit(i, item++)) {
                 const Tile t = locate(sh, args.num_experts, args.n_tiles, i, kTileTokens);
                 const uint32_t idesc = instr_desc_bf16(BW, t.tokens);
@@ -388,6 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
             for (int n = 0; taken >= 0; ++n) {
                 const int slot = n % kUnitSlots;
                 const bool wanted = taken < units;
+                if (n == kUnitSlots) wait_for_previous();  // as the readers do
                 if (n >= kUnitSlots && wanted && !mbar_wait_pair(&sh.unit_empty[slot], uint32_t(n / kUnitSlots - 1) & 1u, limit_ns)) {
                     fail(kGemmPipeTimeout);
                     break;

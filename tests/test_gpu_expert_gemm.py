@@ -82,6 +82,32 @@ def test_units_taken_over_by_running_clusters(counts, ranges, K, N, swiglu, larg
         assert torch.equal(runs[0][real], other[real])
 
 
+def test_limits_start_when_the_kernel_in_front_has_ended():
+    """A GEMM that starts early sits on its SMs while the kernel in front of it runs (a pull may wait for its peers): that time
+    does not count towards its own limits, and what that kernel writes is what it reads."""
+    torch.manual_seed(12)
+    a, w, offsets, n, _ = _problem([4096] * 2, 4096, 4096)
+    a *= 0.1
+    w2 = (torch.randn(2, 512, 4096) * 0.02).to(torch.bfloat16).cuda()
+    h, late, early = (torch.empty(a.shape[0], cols, dtype=torch.bfloat16, device="cuda") for cols in (4096, 512, 512))
+    ext, status = gg._ext(), gg.status_tensor(a.device)
+
+    def run(out, front_ctas, is_early, limit_s):
+        gg.grouped_gemm(a, w, offsets, expert_counts=n, max_ctas=front_ctas, out=h)
+        ext.grouped_gemm(h, w2, offsets, out, status, gg.PLAIN, None, None, 0, limit_s, None, 4, False, n, 0, is_early)
+
+    run(late, 0, False, 5.0)
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    h.zero_()
+    start.record()
+    run(early, 2, True, 2e-3)  # one pair of CTAs in front, the others are free
+    end.record()
+    torch.cuda.synchronize()
+    gg.check_status()
+    assert start.elapsed_time(end) > 6, "the kernel in front ran far longer than the limit"
+    assert torch.equal(early, late)
+
+
 @pytest.mark.parametrize("pair", [False, True])
 def test_matches_the_gated_kernels(pair):
     """The kernels with tokens as M (row blocks gated by counters) add the same products: at most one bf16 step apart."""
