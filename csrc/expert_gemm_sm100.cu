@@ -151,9 +151,13 @@ __device__ __forceinline__ int cancelled_cta(const void* answer) {
 __device__ __forceinline__ void st_cluster(uint32_t cluster_addr, int v) {
     asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
-// Arrival behind the read that gave `value` (an operand of the statement, so the read is done), without the fence of a releasing one.
-__device__ __forceinline__ void arrive_after(uint32_t cluster_addr, int value) {
-    asm volatile("{\n .reg .b32 v;\n mov.b32 v, %1;\n mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n}" ::"r"(cluster_addr), "r"(value) : "memory");
+// Arrival behind the read that gave `unit`, without the fence of a releasing one.  The barrier's address is computed from the value
+// (units lie between -1 and 2^31 - 2, so the added term is 0, which the compiler does not know), so the arrival cannot be on its
+// way before the value is there.  Whoever rewrites the slot waits for the arrival first: a read that returned the rewritten
+// value would be its own cause, through a chain of dependencies.
+__device__ __forceinline__ void arrive_behind(uint32_t cluster_addr, int unit) {
+    const uint32_t zero = (uint32_t(unit) + 1u) >> 31;
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr + 8u * zero) : "memory");
 }
 // Bounded wait that also orders what the other CTA of the pair wrote before its arrival.
 __device__ __forceinline__ bool mbar_wait_pair(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
@@ -272,7 +276,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
             return -1;
         }
         const int next = *(volatile int*)&sh.next_unit[slot];
-        arrive_after(map_to_cta(smem_u32(&sh.unit_empty[slot]), 1), next);
+        arrive_behind(map_to_cta(smem_u32(&sh.unit_empty[slot]), 1), next);
         return next;
     };
     const int first_unit = cluster_id < units ? cluster_id : -1;

@@ -180,3 +180,14 @@ def test_what_starts_early_reads_only_what_ended_kernels_wrote():
     assert "got.early" in up and "true" not in up
     steps = (ROOT / "nanoep_b200" / "models" / "moe_layer.py").read_text()
     assert re.search(r"self\._grouped\(h_in, self\.w13,[^)]*, False\)", steps)
+
+
+def test_a_unit_is_acknowledged_behind_its_read():
+    """A relaxed arrival orders no read in front of it, and an operand that the statement does not use orders nothing: the address
+    that the arrival goes to is computed from the value read."""
+    text = re.sub(r"//[^\n]*", "", (ROOT / "csrc" / "expert_gemm_sm100.cu").read_text())
+    assert text.count("mbarrier.arrive.relaxed") == 1
+    body = _body(text, "void arrive_behind")
+    assert re.search(r"(\w+) = \(uint32_t\(unit\) \+ 1u\) >> 31;.*_, \[%0\];\" *::\"r\"\(cluster_addr \+ 8u \* \1\)", body, re.S)
+    # the value that is acknowledged is the one read from the slot
+    assert re.search(r"next = \*\(volatile int\*\)&sh\.next_unit\[slot\];\s*arrive_behind\([^;]*, next\);", text)
