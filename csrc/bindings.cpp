@@ -5,6 +5,7 @@
 #include "flag_queue.hpp"
 #include "gemm_api.hpp"
 #include "pipeline.hpp"
+#include "unit_queue.hpp"
 
 namespace py = pybind11;
 using nep::PeerWindow;
@@ -35,6 +36,28 @@ struct FlagModel {
     void publish_up_to(int count) {
         completed = count;
         for (int i = 0; i < count; ++i) early = early || group_of.at(size_t(i)) >= landed;
+    }
+};
+
+// Host side of hand_out_units: answers in a given order, then "none left".
+struct UnitModel {
+    std::vector<int> answers;
+    size_t asked = 0;
+    int handed = 0;
+    std::vector<std::pair<std::string, int>> log;
+    bool wait_read(int n) {
+        log.emplace_back("wait", n);
+        return true;
+    }
+    bool request(int& unit) {
+        unit = asked < answers.size() ? answers[asked] : -1;
+        ++asked;
+        log.emplace_back("answer", unit);
+        return true;
+    }
+    void hand_out(int n, int unit) {
+        if (n != handed++) throw std::logic_error("hand-outs out of order");
+        log.emplace_back("unit", unit);
     }
 };
 
@@ -228,6 +251,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "Flags of a combine's transfer warp ('p': of a row that it stores, 'n': of a row that stays): after every step and at the end "
         "(on the ring, handed to the publisher, whether one was handed over before its row had landed)");
     m.def("flag_ring", [] { return std::make_pair(nep::kFlagRing, nep::kMaxStoreDepth); });
+    m.def("hand_out_units",
+          [](std::vector<int> answers, int units) {
+              UnitModel model{std::move(answers)};
+              if (!nep::gemm::hand_out_units(model, units)) throw std::logic_error("gave up");
+              return model.log;
+          },
+          py::arg("answers"), py::arg("units"),
+          "What an expert GEMM's scheduler does with a series of answers: waits for slots, answers and units handed out, in order");
     m.def("set_combine_trace", &nep::set_combine_trace, py::arg("enabled"), py::arg("store_depth") = 0, py::arg("reduce_group") = 0);
     m.def("take_combine_trace", &nep::take_combine_trace);
     m.def("take_stage_trace", &nep::take_stage_trace);

@@ -30,11 +30,13 @@
 // clock.  us, fixed share -> taken over: 32 x 1024 rows up 1325 -> 1260, 0.8 s in a row 1533 -> 1480, down 660 -> 648, 785 -> 770; 32 x (1024
 // +- 32) up 1410 -> 1345, 0.8 s in a row 1650 -> 1566, down 692 -> 686; 4662 uneven rows (4096 x 1536) up 165 -> 158, down 91 -> 85.  The readers of a unit
 // acknowledge it without a fence: a releasing arrival waits for the thread's bulk loads in flight and drained the
-// operand pipeline at every unit (tensor pipe 98 -> 93 % active up, 96 -> 80 % down).  A launch with a cap on its CTAs keeps fixed shares.
+// operand pipeline at every unit (tensor pipe 98 -> 93 % active up, 96 -> 80 % down).  Which unit comes when is hand_out_units
+// (unit_queue.hpp): every unit taken over is computed, whatever the order of the answers.  A launch with a cap on its CTAs keeps fixed shares.
 //
 // All waits are bounded; on expiry a CTA records a code in `status`, stops issuing work, and both CTAs still meet at the
 // final cluster barrier and free their TMEM.
 #include "grouped_gemm_sm100.hpp"
+#include "unit_queue.hpp"
 
 #include <cuda_bf16.h>
 
@@ -59,7 +61,6 @@ constexpr int kMaxStages = 10;
 constexpr int kChunk = 32;                   // token rows staged at a time by a group
 constexpr int kMaxTokens = 256;              // largest N
 constexpr int kUnitReaders = 5;              // readers of a handed-out unit: two producers, the MMA issuer, two epilogues
-constexpr int kUnitSlots = 2;                // units handed out ahead of their readers
 
 template <int kMode>
 struct Out {
@@ -266,12 +267,14 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
         if (atomicCAS(args.status, 0u, code) == 0u) args.status[1] = blockIdx.x;
     };
 
-    // The unit behind `unit` for one reader (one thread), -1 at the end; `item` counts the reader's units.
+    // The unit that a reader (one thread) computes behind `unit`, its `item`-th; -1 at the end.  A cluster without a unit of its own
+    // asks for its first one as well.
+    const bool own_unit = cluster_id < units;
     auto next_unit = [&](int unit, int item) -> int {
         if (*abort_flag) return -1;
         if (!args.dynamic) return unit + num_clusters < units ? unit + num_clusters : -1;
-        const int slot = item % kUnitSlots;
-        if (!mbar_wait_pair(&sh.unit_full[slot], uint32_t(item / kUnitSlots) & 1u, limit_ns)) {
+        const int handed = own_unit ? item : item + 1, slot = handed % kUnitSlots;
+        if (!mbar_wait_pair(&sh.unit_full[slot], uint32_t(handed / kUnitSlots) & 1u, limit_ns)) {
             fail(kGemmPipeTimeout);
             return -1;
         }
@@ -279,14 +282,14 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
         arrive_behind(map_to_cta(smem_u32(&sh.unit_empty[slot]), 1), next);
         return next;
     };
-    const int first_unit = cluster_id < units ? cluster_id : -1;
+    auto first_unit = [&]() { return own_unit ? cluster_id : args.dynamic ? next_unit(-1, -1) : -1; };
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)
         if (elect_one()) {
             int stage = 0, item = 0;
             uint32_t phase = 0;
-            for (int i = first_unit; i >= 0 && !*abort_flag; i = next_unit(i, item++)) {
+            for (int i = first_unit(); i >= 0 && !*abort_flag; i = next_unit(i, item++)) {
                 const Tile t = locate(sh, args.num_experts, args.n_tiles, i, kTileTokens);
                 const int half = t.tokens / 2, t_row = t.row0 + int(cta) * half;  // this CTA's token rows
                 const uint32_t bytes = uint32_t(2 * (kWBytes + half * BK * 2));    // of a stage, in both CTAs
@@ -347,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
             int stage = 0, item = 0;
             uint32_t phase = 0;
             wait_for_previous();  // the time limits below are this kernel's, not those of a pull that waits for its peers in front of it
-            for (int i = first_unit; i >= 0 && !*abort_flag; i = next_unit(i, item++)) {
+            for (int i = first_unit(); i >= 0 && !*abort_flag; i = next_unit(i, item++)) {
                 const Tile t = locate(sh, args.num_experts, args.n_tiles, i, kTileTokens);
                 const uint32_t idesc = instr_desc_bf16(BW, t.tokens);
                 const int acc = item & 1;
@@ -386,34 +389,33 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
             }
         }
         // ------------------------------------------------------------------ scheduler (the other CTA)
-        // Hands out the units of the clusters that it takes over; those behind the last unit (the offsets may allow more than
-        // the counts give) are taken over as well, so that none of them has to start.  An answer "none left" is the last request.
         if (!leader && args.dynamic && elect_one()) {
-            int taken = first_unit >= 0 ? 0 : units;
-            for (int n = 0; taken >= 0; ++n) {
-                const int slot = n % kUnitSlots;
-                const bool wanted = taken < units;
-                if (n == kUnitSlots) wait_for_previous();  // as the readers do
-                if (n >= kUnitSlots && wanted && !mbar_wait_pair(&sh.unit_empty[slot], uint32_t(n / kUnitSlots - 1) & 1u, limit_ns)) {
-                    fail(kGemmPipeTimeout);
-                    break;
+            struct {
+                Shared& sh;
+                uint64_t limit_ns;
+                int answers;
+                __device__ bool wait_read(int n) {
+                    if (n == kUnitSlots) wait_for_previous();  // as the readers do
+                    return mbar_wait_pair(&sh.unit_empty[n % kUnitSlots], uint32_t(n / kUnitSlots - 1) & 1u, limit_ns);
                 }
-                mbar_expect_tx(&sh.cancel_done, 16);
-                request_cluster(sh.cancelled, &sh.cancel_done);
-                if (!mbar_wait(&sh.cancel_done, uint32_t(n) & 1u, limit_ns)) {
-                    fail(kGemmPipeTimeout);
-                    break;
+                __device__ bool request(int& unit) {
+                    mbar_expect_tx(&sh.cancel_done, 16);
+                    request_cluster(sh.cancelled, &sh.cancel_done);
+                    if (!mbar_wait(&sh.cancel_done, uint32_t(answers++) & 1u, limit_ns)) return false;
+                    const int cta_taken = cancelled_cta(sh.cancelled);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next answer comes behind this read
+                    unit = cta_taken < 0 ? -1 : cta_taken >> 1;
+                    return true;
                 }
-                const int cta_taken = cancelled_cta(sh.cancelled);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next answer comes behind this read
-                taken = cta_taken < 0 ? -1 : cta_taken >> 1;
-                if (!wanted) continue;
-                const int unit = taken < units ? taken : -1;
-                *(volatile int*)&sh.next_unit[slot] = unit;
-                st_cluster(map_to_cta(smem_u32(&sh.next_unit[slot]), 0), unit);
-                mbar_arrive_cluster(map_to_cta(smem_u32(&sh.unit_full[slot]), 1));
-                mbar_arrive_cluster(map_to_cta(smem_u32(&sh.unit_full[slot]), 0));
-            }
+                __device__ void hand_out(int n, int unit) {
+                    const int at = n % kUnitSlots;
+                    *(volatile int*)&sh.next_unit[at] = unit;
+                    st_cluster(map_to_cta(smem_u32(&sh.next_unit[at]), 0), unit);
+                    mbar_arrive_cluster(map_to_cta(smem_u32(&sh.unit_full[at]), 1));
+                    mbar_arrive_cluster(map_to_cta(smem_u32(&sh.unit_full[at]), 0));
+                }
+            } io{sh, limit_ns, 0};
+            if (!hand_out_units(io, units)) fail(kGemmPipeTimeout);
         }
     } else {
         // ------------------------------------------------------------------ epilogue (both CTAs)
@@ -426,11 +428,11 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
         uint8_t* buf = stage_out + group * O::kBufBytes;
         // Rows, scales and destinations are the work of kernels in front; no CTA ends before those have.
         wait_for_previous();
-        int unit = first_unit;  // warp 2, lane 0
+        int unit = -1;  // warp 2, lane 0
         for (int item = 0;; ++item) {
             if (warp == 2) {
                 if (lane == 0) {
-                    if (item > 0) unit = next_unit(unit, item - 1);
+                    unit = item > 0 ? next_unit(unit, item - 1) : first_unit();
                     *(volatile int*)&sh.epi_unit[item & 1] = unit;
                 }
                 __syncwarp();

@@ -476,3 +476,33 @@ def test_flags_of_a_combine_are_handed_over_once_and_in_time(depth, share_of_not
             assert produced - handed < ring, (case, produced, handed)
             before = handed
         assert handed == produced == len(case)
+
+
+@pytest.mark.parametrize("units,total", [(0, 0), (0, 7), (1, 1), (5, 5), (40, 40), (40, 90), (3, 200)])
+@pytest.mark.parametrize("order", ["ascending", "descending", "shuffled"])
+def test_every_unit_taken_over_is_handed_out(units, total, order):
+    """Each answer below `units` reaches the readers, whatever comes in front of it, and "none" ends the series; a slot is
+    written only once its previous contents have been read, and nothing is asked for that would have to wait for one."""
+    import random
+
+    from nanoep_b200.utils.build import load_extension
+
+    answers = list(range(total))
+    if order == "descending":
+        answers.reverse()
+    elif order == "shuffled":
+        random.Random(units + total).shuffle(answers)
+    log = load_extension().hand_out_units(answers, units)
+    assert [v for what, v in log if what == "unit"] == [a for a in answers if a < units] + [-1]
+    assert [v for what, v in log if what == "answer"] == answers + [-1]
+    handed, last_free, last = 0, 1, 0  # the first two slots are free
+    for what, v in log:
+        if what == "wait":
+            assert v == last_free + 1 == handed
+            last_free = v
+        elif what == "answer":
+            assert last >= units or last_free >= handed, "asked while every slot is taken"
+            last = v
+        else:
+            assert last_free >= handed
+            handed += 1
