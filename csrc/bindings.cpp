@@ -49,10 +49,10 @@ struct UnitModel {
         log.emplace_back("wait", n);
         return true;
     }
-    bool request(int& unit) {
-        unit = asked < answers.size() ? answers[asked] : -1;
+    bool request(int& place) {
+        place = asked < answers.size() ? answers[asked] : -1;
         ++asked;
-        log.emplace_back("answer", unit);
+        log.emplace_back("answer", place);
         return true;
     }
     void hand_out(int n, int unit) {
@@ -251,13 +251,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "Flags of a combine's transfer warp ('p': of a row that it stores, 'n': of a row that stays): after every step and at the end "
         "(on the ring, handed to the publisher, whether one was handed over before its row had landed)");
     m.def("flag_ring", [] { return std::make_pair(nep::kFlagRing, nep::kMaxStoreDepth); });
+    m.def("unit_places", &nep::gemm::unit_places, py::arg("allowed"), py::arg("experts"), py::arg("largest"), py::arg("tile_tokens"),
+          py::arg("weight_tiles"));
     m.def("hand_out_units",
-          [](std::vector<int> answers, int units) {
+          [](std::vector<int> answers, int units, int places, int own) {
               UnitModel model{std::move(answers)};
-              if (!nep::gemm::hand_out_units(model, units)) throw std::logic_error("gave up");
+              if (!nep::gemm::hand_out_units(model, units, places, own)) throw std::logic_error("gave up");
               return model.log;
           },
-          py::arg("answers"), py::arg("units"),
+          py::arg("answers"), py::arg("units"), py::arg("places"), py::arg("own"),
           "What an expert GEMM's scheduler does with a series of answers: waits for slots, answers and units handed out, in order");
     m.def("set_combine_trace", &nep::set_combine_trace, py::arg("enabled"), py::arg("store_depth") = 0, py::arg("reduce_group") = 0);
     m.def("take_combine_trace", &nep::take_combine_trace);

@@ -22,8 +22,8 @@
 // tiles per token tile (a quarter less ingress, one accumulator each) ran at 1.3 GHz and the same power: up 1707, down 823 us.
 // In between, 4662 rows over 32 experts of 4096 x 1536: up 209 -> 163 us, down 121 -> 86 us.
 //
-// Who computes what.  The grid holds a cluster for every unit (one weight tile x one token tile) that the offsets allow; the
-// clusters that run take over the places of those that have not started (cluster launch control), in order, one or two
+// Who computes what.  The grid holds a cluster for every unit (one weight tile x one token tile) that the offsets allow (see
+// unit_places for where it holds fewer); the clusters that run take over the places of those that have not started (cluster launch control), in order, one or two
 // units ahead.  With a fixed share of the units per cluster, clusters that share a weight tile drift apart by more than
 // L2 keeps it (small differences add up over units of 100 us) and fetch it again: the up-projection of 32 experts of 1024
 // rows read 4.0-5.3 GB from memory instead of the 2.35 GB that there are, now 2.5-2.7 GB, and at the power limit every byte costs
@@ -398,13 +398,13 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
                     if (n == kUnitSlots) wait_for_previous();  // as the readers do
                     return mbar_wait_pair(&sh.unit_empty[n % kUnitSlots], uint32_t(n / kUnitSlots - 1) & 1u, limit_ns);
                 }
-                __device__ bool request(int& unit) {
+                __device__ bool request(int& place) {
                     mbar_expect_tx(&sh.cancel_done, 16);
                     request_cluster(sh.cancelled, &sh.cancel_done);
                     if (!mbar_wait(&sh.cancel_done, uint32_t(answers++) & 1u, limit_ns)) return false;
                     const int cta_taken = cancelled_cta(sh.cancelled);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next answer comes behind this read
-                    unit = cta_taken < 0 ? -1 : cta_taken >> 1;
+                    place = cta_taken < 0 ? -1 : cta_taken >> 1;
                     return true;
                 }
                 __device__ void hand_out(int n, int unit) {
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_gemm_kernel(const __grid_c
                     mbar_arrive_cluster(map_to_cta(smem_u32(&sh.unit_full[at]), 0));
                 }
             } io{sh, limit_ns, 0};
-            if (!hand_out_units(io, units)) fail(kGemmPipeTimeout);
+            if (!hand_out_units(io, units, num_clusters, cluster_id)) fail(kGemmPipeTimeout);
         }
     } else {
         // ------------------------------------------------------------------ epilogue (both CTAs)

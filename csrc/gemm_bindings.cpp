@@ -8,6 +8,7 @@
 #include "grouped_gemm_sm100.hpp"
 #include "peer_window.hpp"
 #include "pipeline.hpp"
+#include "unit_queue.hpp"
 
 namespace nep {
 namespace {
@@ -111,12 +112,12 @@ cudaError_t launch_expert(GemmCommon& g, const at::Tensor& a, const at::Tensor& 
     for (int b = 0; b < 4; ++b)
         if ((128 >> b) <= tile / 2) maps.tokens[b] = make_map(a.data_ptr(), rows, K, 128 >> b);
     const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-    // Without a cap on the CTAs there is a cluster for every unit that the offsets allow (an expert of n rows has a range of
-    // whole blocks of 128, and tiles of 256 split an odd number of them into one more).
+    // Units that the offsets allow: an expert of n rows has a range of whole blocks of 128, and tiles of 256 split an odd number of
+    // them into one more.  Without a cap on the CTAs clusters take over one another's places.
     const int64_t blocks = rows / 128, tiles = tile <= 128 ? blocks * 128 / tile : (blocks + std::min(E, blocks)) / 2;
     g.args.dynamic = max_ctas <= 0;
     g.args.rows_bound = assigned >= 0;
-    const int grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : int(2 * tiles * g.args.n_tiles);
+    const int grid = max_ctas > 0 ? std::min<int>(sms, int(max_ctas)) : int(2 * gemm::unit_places(tiles * g.args.n_tiles, E, max_expert_rows, tile, g.args.n_tiles));
     return gemm::launch_expert(maps, g.args, mode, tile, grid, early, c10::cuda::getCurrentCUDAStream().stream());
 }
 

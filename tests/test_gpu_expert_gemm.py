@@ -57,6 +57,7 @@ def test_rows_that_exist(counts, K, N, largest, swiglu):
         ([1], [128], 64, 512),                      # fewer units than clusters
         ([2304, 1000, 129, 0, 777, 256, 1, 511], None, 64, 2048),  # short units, several per cluster
         ([640, 385, 130], None, 2048, 1280),
+        ([700, 0, 3, 0, 130, 4000], [4096] * 6, 64, 5120),  # largest = 64 is far from true here: 1024 places for 1560 units
     ],
 )
 def test_units_taken_over_by_running_clusters(counts, ranges, K, N, swiglu, largest):

@@ -478,24 +478,29 @@ def test_flags_of_a_combine_are_handed_over_once_and_in_time(depth, share_of_not
         assert handed == produced == len(case)
 
 
-@pytest.mark.parametrize("units,total", [(0, 0), (0, 7), (1, 1), (5, 5), (40, 40), (40, 90), (3, 200)])
+@pytest.mark.parametrize("units,places", [(0, 1), (0, 7), (1, 1), (5, 5), (40, 40), (40, 90), (3, 200), (100, 40), (81, 40), (17, 1)])
 @pytest.mark.parametrize("order", ["ascending", "descending", "shuffled"])
-def test_every_unit_taken_over_is_handed_out(units, total, order):
-    """Each answer below `units` reaches the readers, whatever comes in front of it, and "none" ends the series; a slot is
-    written only once its previous contents have been read, and nothing is asked for that would have to wait for one."""
+@pytest.mark.parametrize("own", [0, -1])  # the first and the last place
+def test_every_unit_taken_over_is_handed_out(units, places, order, own):
+    """Each unit of the cluster's own place but the first and of every place taken over reaches the readers, whatever comes in front
+    of it, and "none" ends the series; a slot is written only once its previous contents have been read, and nothing is asked
+    for that would have to wait for one."""
     import random
 
     from nanoep_b200.utils.build import load_extension
 
-    answers = list(range(total))
+    own %= places
+    answers = [p for p in range(places) if p != own]
     if order == "descending":
         answers.reverse()
     elif order == "shuffled":
-        random.Random(units + total).shuffle(answers)
-    log = load_extension().hand_out_units(answers, units)
-    assert [v for what, v in log if what == "unit"] == [a for a in answers if a < units] + [-1]
+        random.Random(units + places).shuffle(answers)
+    log = load_extension().hand_out_units(answers, units, places, own)
+    want = [u for p in [own] + answers for u in range(p, units, places)]
+    assert [v for what, v in log if what == "unit"] == (want[1:] if own < units else want) + [-1]
+    assert sorted(want) == list(range(units))
     assert [v for what, v in log if what == "answer"] == answers + [-1]
-    handed, last_free, last = 0, 1, 0  # the first two slots are free
+    handed, last_free, last = 0, 1, own  # the first two slots are free
     for what, v in log:
         if what == "wait":
             assert v == last_free + 1 == handed
@@ -506,3 +511,17 @@ def test_every_unit_taken_over_is_handed_out(units, total, order):
         else:
             assert last_free >= handed
             handed += 1
+
+
+def test_places_of_an_expert_gemm():
+    """No more clusters than units that the offsets allow, and not many more than the experts' rows can need: one without a unit
+    costs five nanoseconds."""
+    from nanoep_b200.utils.build import load_extension
+
+    places = load_extension().unit_places
+    assert places(512, 32, 64, 64, 16) == 512 and places(0, 4, 0, 256, 8) == 0
+    assert places(32768, 32, 64, 64, 16) == 1024 == places(32768, 32, 8, 64, 16)  # ranges of 4096 rows, at most 64 of them real
+    assert places(32768, 32, 512, 64, 16) == 32 * 8 * 16
+    assert places(2560, 32, 4096, 256, 16) == 2560  # 4096 tokens, tight ranges
+    assert places(1 << 20, 32, 32768, 256, 28) == 32 * 128 * 28
+    assert places(8192, 32, 0, 256, 16) == 8192 and places(1 << 20, 32, 0, 256, 16) == 16384  # nothing is known of the rows
