@@ -598,6 +598,9 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
             throw;
         }
         const auto nc = receive_counts();
+        // What the plan found has reached the host in front of the counts.  The check of a later call would raise it, but those that `behind`
+        // made came too early.
+        wins[0]->check_status();
         TORCH_CHECK(nc.first <= bound_rows_n && nc.second <= deferred_rows_c, "receive counts exceed their bound");
         out.counts[0] = {nc.first, nc.second};
     }

@@ -202,6 +202,30 @@ def test_layer_queued_in_front_of_its_counts(one_rank, hidden, tokens, masked, f
             assert torch.equal(new.layout.expert_counts, old.layout.expert_counts) and torch.equal(new.topk_idx, old.topk_idx)
 
 
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("tokens", [1, 300, 20000])  # queued in front of the counts, and beyond the limit on the bound
+def test_layer_refuses_an_invalid_expert_id(one_rank, tokens, fused):
+    """The pass that got the bad id raises, however early its kernels were queued; the next pass is not affected."""
+    E, K, hidden, inner = 8, 2, 4096, 128
+    w13 = torch.zeros(E, 2 * inner, hidden, dtype=torch.bfloat16, device="cuda")
+    w2 = torch.zeros(E, hidden, inner, dtype=torch.bfloat16, device="cuda")
+    with CudaBuffer(one_rank, EPConfig(E, K, hidden, tokens)) as buf:
+        layer = ExpertParallelMoE(buf, w13, w2, fuse_combine=fused)
+        x = torch.zeros(tokens, hidden, dtype=torch.bfloat16, device="cuda")
+        good = torch.tensor([0, 1], device="cuda").expand(tokens, K).contiguous()
+        bad = good.clone()
+        bad[-1, 1] = E
+        gate = torch.ones(tokens, K, device="cuda")
+        for _ in range(3):
+            with pytest.raises(RuntimeError, match="expert id"):
+                layer(x, bad, gate)
+            buf.clear_status()
+            assert not layer(x, good, gate).any()
+            torch.cuda.synchronize()
+            buf.check_status()
+            gg.check_status()
+
+
 @pytest.mark.parametrize("max_ctas", [1, 2, 6])
 def test_scatter_on_a_small_grid(one_rank, max_ctas):
     """The down-projection with the scatter epilogue takes any cap on its grid and gives the same bits."""
