@@ -266,6 +266,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("take_stage_trace", &nep::take_stage_trace);
     m.def("take_phase_timings", &nep::take_phase_timings);
     m.def("launch_count", [] { return PeerWindow::launches; });
+    m.def("queued_ahead_count", [] { return PeerWindow::queued_ahead; });
     m.def("format_status", &nep::format_status);
     m.def("peer_access_error", &nep::peer_access_error, py::arg("own_rank"), py::arg("peer_rank"), py::arg("own_device"),
           py::arg("peer_device"), py::arg("can_access"), py::arg("access_supported"));

@@ -268,7 +268,7 @@ pybind11::tuple moe_forward(PeerWindow& window, const at::Tensor& x, const c10::
         }
     };
     auto out = dispatch({&window}, {x}, {topk}, {weights}, {cached}, {cached_capacity}, alignment, expand, false, num_sms, comm_stream, -1, false,
-                        mailbox_timeout_s, {c10::nullopt}, 0, behind);
+                        mailbox_timeout_s, {c10::nullopt}, 0, behind, w13.size(1) / 2 * 2 + (fuse_combine ? 0 : w2.size(1) * 2));
     return pybind11::make_tuple(result, out.metadata[0], out.counts[0]);
 }
 

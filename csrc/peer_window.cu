@@ -11,6 +11,7 @@
 namespace nep {
 
 int64_t PeerWindow::launches = 0;
+int64_t PeerWindow::queued_ahead = 0;
 
 namespace {
 void check(cudaError_t e, const char* what) {

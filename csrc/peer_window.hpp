@@ -86,6 +86,7 @@ public:
 
     // Launch counter for diagnostics and benchmarks.
     static int64_t launches;
+    static int64_t queued_ahead;  // dispatches whose followers were queued before the host had the counts
 
 private:
     int rank_, world_, device_;

@@ -31,7 +31,8 @@ constexpr int kFusedFreshDefaultTokens = 0;  // single-launch fresh dispatch: of
 constexpr int64_t kFusedFreshMaxOutputBytes = int64_t(256) << 20;  // single-launch fresh dispatch: largest bound-sized output
 constexpr int64_t kLocalPlanMaxHandleBytes = int64_t(16) << 20;    // single-rank plan: largest bound-sized handle
 constexpr int64_t kEarlyPullMaxOutputBytes = int64_t(16) << 20;    // single-rank pull that does not wait for N and C: see dispatch()
-constexpr int64_t kDeferredMaxOutputBytes = int64_t(128) << 20;    // single rank: outputs of their bound for work queued in front of N and C
+constexpr int64_t kAheadMaxRowBytes = int64_t(128) << 20;          // single rank, work queued in front of N and C: rows of their bound,
+constexpr int64_t kAheadMaxBytes = int64_t(384) << 20;             // and with what that work allocates for them
 constexpr int kFusedDefaultBlocks = 1024;  // i.e. bounded by the SM budget and co-residency only
 
 void cuda_check(cudaError_t e, const char* what) {
@@ -280,7 +281,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
                      const std::vector<std::vector<at::Tensor>>& cached_meta, const std::vector<int64_t>& cached_capacity,
                      int64_t alignment, bool expand, bool zero_padding, int64_t num_sms, int64_t comm_stream, int64_t previous_event,
                      bool async_op, double mailbox_timeout_s, const std::vector<c10::optional<at::Tensor>>& tile_ready,
-                     int64_t ring_smem_limit, const std::function<void(DispatchOut&, bool)>& behind) {
+                     int64_t ring_smem_limit, const std::function<void(DispatchOut&, bool)>& behind, int64_t behind_row_bytes) {
     validate_group(wins);
     const int n = int(wins.size());
     TORCH_CHECK(int(xs.size()) == n && int(topks.size()) == n && int(weights.size()) == n && int(cached_meta.size()) == n &&
@@ -406,9 +407,12 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
     // masked 33 against 30.
     const int64_t bound_bytes = (expand ? bound_rows_c : bound_rows_n) * L.hidden * 2;
     // Work that follows on the same stream and takes its sizes from the device need not wait for the host to have the counts: the
-    // pull and what `behind` queues go out at once, on tensors of their upper bound.  Limited to calls that take less time than
-    // the wait matters for (and in the memory that the bound may cost over the exact size).
-    const bool deferred = behind && plan_locally && !async_op && expand && !gated && !g_gate.word.defined() && bound_bytes <= kDeferredMaxOutputBytes;
+    // pull and what `behind` queues go out at once, on tensors of their upper bound.  Limited in the memory that these rows and what
+    // `behind` allocates for them may take: the gain falls with the size (padding rows that only the bound has are a bigger grid and
+    // more to allocate).  us with the wait -> without, 32 experts of 4096 x 1536, top-6, separate combine: 64 tokens (35 MB of rows)
+    // 226 -> 212, 256 (44 MB) 234 -> 225, 777 (68 MB) 269 -> 266, 1500 (102 MB) 416 -> 418, 2000 (126 MB) 471 -> 466.
+    const bool deferred = behind && plan_locally && !async_op && expand && !gated && !g_gate.word.defined() && bound_bytes <= kAheadMaxRowBytes &&
+                          bound_bytes + bound_rows_c * behind_row_bytes <= kAheadMaxBytes;
     const int64_t deferred_rows_c = bound_rows_c / alignment * alignment;  // C is a multiple of the alignment
     const bool early_pull =
         plan_locally && !deferred && (!expand || alignment == 1) && !gated && !g_gate.word.defined() && bound_bytes <= kEarlyPullMaxOutputBytes;
@@ -585,6 +589,7 @@ DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at:
         }
     }
     if (deferred) {
+        PeerWindow::queued_ahead += 1;
         auto& m = out.metadata[0];
         m[7] = part_of(m[7], 0, {deferred_rows_c});
         auto receive_counts = [&] {

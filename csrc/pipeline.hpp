@@ -45,14 +45,15 @@ struct CombineOut {
 };
 
 // `behind` queues what follows the dispatch on the same stream.  It is called once: a synchronous, fresh, expert-major dispatch of a
-// single rank with outputs of at most kDeferredMaxOutputBytes calls it before the host has the counts, with outputs and handle tensors of
-// their upper bound (second argument true; a device word has N, the offsets end at C), and waits for the counts afterwards.
+// single rank whose rows, with `behind_row_bytes` more for each of them, stay below a limit (kAheadMaxRowBytes, kAheadMaxBytes) calls it before the
+// host has the counts, with outputs and handle tensors of their upper bound (second argument true; a device word has N, the offsets
+// end at C), and waits for the counts afterwards.
 DispatchOut dispatch(const std::vector<PeerWindow*>& wins, const std::vector<at::Tensor>& xs,
                      const std::vector<c10::optional<at::Tensor>>& topks, const std::vector<c10::optional<at::Tensor>>& weights,
                      const std::vector<std::vector<at::Tensor>>& cached_meta, const std::vector<int64_t>& cached_capacity,
                      int64_t alignment, bool expand, bool zero_padding, int64_t num_sms, int64_t comm_stream, int64_t previous_event,
                      bool async_op, double mailbox_timeout_s, const std::vector<c10::optional<at::Tensor>>& tile_ready = {},
-                     int64_t ring_smem_limit = 0, const std::function<void(DispatchOut&, bool)>& behind = {});
+                     int64_t ring_smem_limit = 0, const std::function<void(DispatchOut&, bool)>& behind = {}, int64_t behind_row_bytes = 0);
 
 CombineOut combine(const std::vector<PeerWindow*>& wins, const std::vector<at::Tensor>& xs, const std::vector<std::vector<at::Tensor>>& meta,
                    const std::vector<int64_t>& capacity, const std::vector<c10::optional<at::Tensor>>& weights,

@@ -226,6 +226,33 @@ def test_layer_refuses_an_invalid_expert_id(one_rank, tokens, fused):
             gg.check_status()
 
 
+@pytest.mark.parametrize(
+    "hidden,inner,tokens,fused,ahead",
+    [
+        (512, 256, 0, True, True), (512, 256, 1, False, True), (512, 256, 200, True, True), (512, 256, 200, False, True),
+        (16384, 256, 4000, True, False), (16384, 256, 4000, False, False),  # 266 MB of rows
+        (4096, 128, 7900, True, True), (4096, 128, 7900, False, True), (4096, 128, 8000, True, False),  # 127 and 129 MB
+        (256, 4096, 20000, True, True), (256, 4096, 24000, True, False), (256, 8192, 24000, False, False),  # 20-24 MB, but 336, 403 and 805 MB with activations
+    ],
+)
+def test_when_a_layer_is_queued_in_front_of_its_counts(one_rank, hidden, inner, tokens, fused, ahead):
+    """Its tensors have the size of their bound then: only so many bytes of rows, and of what the GEMMs make of them."""
+    E, K = 4, 2
+    ext = gg._ext()
+    w13 = torch.zeros(E, 2 * inner, hidden, dtype=torch.bfloat16, device="cuda")
+    w2 = torch.zeros(E, hidden, inner, dtype=torch.bfloat16, device="cuda")
+    with CudaBuffer(one_rank, EPConfig(E, K, hidden, max(tokens, 8))) as buf:
+        layer = ExpertParallelMoE(buf, w13, w2, fuse_combine=fused)
+        x = torch.zeros(tokens, hidden, dtype=torch.bfloat16, device="cuda")
+        gate, idx = torch.rand(tokens, E, device="cuda").topk(K, dim=-1)
+        before = ext.queued_ahead_count()
+        layer(x, idx, gate)
+        assert ext.queued_ahead_count() - before == ahead
+        layer(x, None, gate, handle=layer.last_handle)  # the counts are known
+        assert ext.queued_ahead_count() - before == ahead
+        torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("max_ctas", [1, 2, 6])
 def test_scatter_on_a_small_grid(one_rank, max_ctas):
     """The down-projection with the scatter epilogue takes any cap on its grid and gives the same bits."""
