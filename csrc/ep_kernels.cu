@@ -344,8 +344,8 @@ __device__ bool stage_body(const StageParams& p) {
     if (p.fresh) {
         // The count exchange comes first: every rank and the host wait for it.  The rows are staged underneath it by all
         // the other blocks; the tail block copies only where it is alone.  (With a share of its own behind the tail it was the
-        // last to finish.  Without it, and with one system fence per signal, eight ranks of 16 tokens take 17.6 us instead of 34,
-        // of 512 tokens 39.7 instead of 56; four skewed ranks of 1000 tokens 35.5 instead of 50.)
+        // last to finish.  Without it, with one system fence per signal and two blocks per SM, the kernel alone with cold caches: eight ranks
+        // of 16 tokens 46 -> 26 us, of 512 tokens 62 -> 32; four skewed ranks of 1000 tokens 54 -> 26.)
         bool ok = true;
         if (runs_tail) ok = tail();
         if (share < shares) {
@@ -382,10 +382,10 @@ __device__ bool stage_body(const StageParams& p) {
 // the handle's tensors, and N and C reach the host before the rows are assigned.
 // Against stage + plan, top-8 of 256 experts: 1 token 22 -> 6.6 us, 256 tokens 14.6 -> 8.1 us, 4096 tokens 25 -> 14 us;
 // the pull of a call whose output bound is modest no longer waits for the host: 1 token and its combine 59 -> 52 us.
-// A chain of latencies throughout, so: all threads scan
-// the experts instead of one warp in waves, the other CTAs' counts and the slots of eight choices are asked for at once, and a warp
-// keeps the choices of its only chunk.  1 token 6.2 -> 5.1 us, 256 tokens 7.6 -> 6.1, 4096 tokens 13.8 -> 12.4; calls of
-// 1, 32 and 256 tokens with their combine 37.3 -> 36.7, 38.3 -> 37.7 and 41.0 -> 39.9 us, of 4096 tokens 226.5 -> 225.1.
+// A chain of latencies throughout, so: all threads scan the experts instead of one warp in waves, the other CTAs' counts and the
+// slots of eight choices are asked for at once, and a warp keeps the choices of its only chunk.  The kernel alone with cold
+// caches: 1 token 8.0 -> 6.7 us, 256 tokens 10.5 -> 9.2, 4096 tokens 15.2 -> 13.3.  (In a call, which the host bounds, half a
+// microsecond of 36 to 40, no more than runs of one side differ.)
 // ------------------------------------------------------------------------------------------
 __device__ void local_plan_body(const LocalPlanParams& p) {
     extern __shared__ int s_plan[];
@@ -1094,9 +1094,10 @@ __device__ void combine_publish_role(const CombineParams& p, FlagBoard* board) {
     }
 }
 
-// Eight ranks of 512 tokens on one GPU: combine 238 -> 228 us (one row in eight is a rank's own: its copy was 2 x 59 MB through L2 and 59 MB
-// to memory); four ranks of 1000 skewed tokens 94 -> 92.  Whether the rows of a rank's own tokens stay in the expert output for the reduction to read: in the modes that return rows as
-// they are, and with the reduction that takes rows from anywhere (bulk loads into its ring).
+// Whether the rows of a rank's own tokens stay in the expert output for the reduction to read: in the modes that return rows as they
+// are, and with the reduction that takes rows from anywhere (the loader of combine_reduce_smem_role bulk-loads them into its ring).
+// Eight ranks of 512 tokens on one GPU: combine 238 -> 228 us (one row in eight is a rank's own: its copy was 2 x 59 MB through L2 and
+// 59 MB to memory); four ranks of 1000 skewed tokens 94 -> 92.
 __device__ __forceinline__ bool own_rows_in_place(const CombineParams& p) { return p.reduce_stages >= 2 && p.mode != kPushExpandedReduce; }
 
 // Transfer warps.  Receive rows are visited round-robin over the source ranks (SourceWalk), so at every moment
@@ -1204,7 +1205,7 @@ __device__ void combine_push_role(const CombineParams& p, char* smem, FlagBoard*
 
     // One bulk load + one bulk store per transfer.  A cursor enumerates the transfers of this warp's rows:
     // compact layout = one per receive row; expert-major layout = one per local slot of the row.
-    // Rows of this rank's own tokens are not transferred where the reduction can read them in place (see combine_body).
+    // Rows of this rank's own tokens are not transferred where the reduction can read them in place (own_rows_in_place).
     const bool by_slot = p.mode == kPushExpanded, direct = own_rows_in_place(p);
     struct Cursor {
         unsigned left;  // choices of the current row that still need a transfer
@@ -1959,6 +1960,8 @@ __device__ __forceinline__ const P& block_of(const Many<P>& all) {
     __global__ void __launch_bounds__(__VA_ARGS__) name##_kernel(const __grid_constant__ Params p) { name##_body(p); } \
     __global__ void __launch_bounds__(__VA_ARGS__) name##_multi_kernel(const __grid_constant__ Many<Params> all) { name##_body(block_of(all)); }
 
+// Two blocks per SM, which the grid counts on: the kernel for several ranks took 76 registers and half of its grid waited for a second
+// wave (39.9 -> 35.2 us at eight ranks of 512 tokens, 34.3 -> 25.5 at four of 1000); its 64 registers cost it a few spilled words.
 __global__ void __launch_bounds__(kStageThreads, 2) stage_kernel(const __grid_constant__ StageParams p) { stage_body(p); }
 __global__ void __launch_bounds__(kStageThreads, 2) stage_multi_kernel(const __grid_constant__ Many<StageParams> all) { stage_body(block_of(all)); }
 __global__ void __launch_bounds__(kLocalPlanThreads) local_plan_kernel(const __grid_constant__ LocalPlanParams p) { local_plan_body(p); }
